@@ -184,6 +184,43 @@ __global__ void pass_begin_kernel(const int* plan, PlanLayout lay, uint32_t* exp
   }
 }
 
+// One thread per slice row: the row's expert by bisection of the experts' starts in the stream, its source among the P
+// segments of that expert. (The up-projection gradient's GEMM follows on the same stream; this is a few us beside the
+// chain's GEMMs, where summing inside the dX epilogue kept one column tile's warps busy with strided reads.)
+__global__ void __launch_bounds__(256) return_dw_kernel(const ReturnDwParams p) {
+  if (p.status != nullptr && p.status->code != 0) return;  // an earlier kernel of this pass already gave up
+  const int lane = threadIdx.x & 31;
+  const int row = blockIdx.x * blockDim.x + threadIdx.x, at = p.slice * p.lay.S + row;  // slice row, stream row
+  const int* expert_start = p.plan + p.lay.off_expert_start;
+  int src = -1;
+  if (row < p.lay.S && at < p.plan[1]) {  // plan[1]: rows of this rank's stream
+    int lo = 0, hi = p.lay.L - 1;
+    while (lo < hi) {  // last expert that starts at or before the row (empty experts share the next one's start)
+      const int mid = (lo + hi + 1) >> 1;
+      if (expert_start[mid] <= at) lo = mid; else hi = mid - 1;
+    }
+    float sum = 0.0f;
+    for (int q = 0; q < p.parts; ++q) sum += p.dwp[static_cast<size_t>(row) * p.parts + q];
+    for (int s = 0; s < p.lay.P; ++s) {
+      const int i = s * p.lay.L + lo, off = at - p.plan[p.lay.off_in_start + i];
+      if (off >= 0 && off < p.plan[p.lay.off_in_size + i]) {
+        src = s;
+        p.peer_dw[s][p.plan[p.lay.off_src_send_start + i] + off] = sum;
+      }
+    }
+  }
+  uint32_t sent = 0;  // lane s: rows this warp has stored to source s
+  for (int s = 0; s < p.lay.P; ++s) {
+    const uint32_t cnt = __popc(__ballot_sync(0xffffffffu, src == s));
+    if (lane == s) sent = cnt;
+  }
+  __syncwarp();
+  if (sent > 0) {
+    __threadfence_system();
+    red_add_release_sys(p.peer_count[lane], sent);
+  }
+}
+
 __global__ void __launch_bounds__(256) combine_reduce_kernel(const CombineParams p) {
   __shared__ int s_abort;
   if (threadIdx.x == 0) {
@@ -302,6 +339,10 @@ void launch_slice_done(uint32_t* const* peer_credit, int num_ranks, int me, uint
 void launch_pass_begin(const int* plan, PlanLayout lay, uint32_t* expected_total, uint32_t* pass_base,
                        uint32_t* ready_total, uint32_t* ready_base, cudaStream_t stream) {
   pass_begin_kernel<<<1, 256, 0, stream>>>(plan, lay, expected_total, pass_base, ready_total, ready_base);
+}
+
+void launch_return_dw(const ReturnDwParams& p, cudaStream_t stream) {
+  return_dw_kernel<<<(p.lay.S + 255) / 256, 256, 0, stream>>>(p);
 }
 
 void launch_combine_reduce(const CombineParams& p, cudaStream_t stream) {

@@ -46,6 +46,21 @@ void launch_slice_done(uint32_t* const* peer_credit, int num_ranks, int me, uint
 void launch_pass_begin(const int* plan, PlanLayout lay, uint32_t* expected_total, uint32_t* pass_base,
                        uint32_t* ready_total, uint32_t* ready_base, cudaStream_t stream);
 
+// Backward: adds up each slice row's shares of the router weight's gradient (written per column tile by the SwiGLU'
+// GEMM) and stores the sum to the row's source rank, then counts the rows there like any other returned piece.
+struct ReturnDwParams {
+  const int* plan;
+  PlanLayout lay;
+  int slice;
+  const float* dwp;               // [S, parts]
+  int parts;
+  float* const* peer_dw;          // [P] each source rank's [T*K] d_weight rows
+  uint32_t* const* peer_count;    // [P] each source rank's returned-piece counter
+  StatusBlock* status;
+};
+
+void launch_return_dw(const ReturnDwParams& p, cudaStream_t stream);
+
 struct CombineParams {
   const __nv_bfloat16* rows;  // [T*K, D] returned rows in send order
   const int* inv_order;       // [T*K] send-order position of flat assignment t*K+k

@@ -218,6 +218,10 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
     uint32_t u[32];
     __nv_bfloat16* act_row = p.out0 + static_cast<size_t>(grow) * p.ld0 + tl.n * (kBlockN / 2);
     __nv_bfloat16* h_row = p.out1 ? p.out1 + static_cast<size_t>(grow) * p.ld1 + tl.n * kBlockN : nullptr;
+    // Backward: the router weight is folded into `act` (one rounding of w * act), so that dW_down is the plain product of
+    // `act` and the rows of g as they arrived and no w * g matrix exists.
+    // (Read past L1: the line may also hold weights of rows that had not arrived when another tile read it.)
+    const float w = (p.row_w != nullptr && valid) ? __ldcg(p.row_w + grow) : 1.0f;
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {
       const int f_local = c * 32;
@@ -232,7 +236,7 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
         for (int i = 0; i < 16; ++i) {
           const float g0 = __uint_as_float(r[2 * i]), g1 = __uint_as_float(r[2 * i + 1]);
           const float u0 = __uint_as_float(u[2 * i]), u1 = __uint_as_float(u[2 * i + 1]);
-          o[i] = pack_bf16(silu_f(g0) * u0, silu_f(g1) * u1);
+          o[i] = pack_bf16(silu_f(g0) * u0 * w, silu_f(g1) * u1 * w);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -341,13 +345,6 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
         if (mine) bulk_commit();
       }
     }
-    if constexpr (MODE == kModeDx) {
-      if (tl.n == 0 && src >= 0) {
-        float dw = 0.0f;
-        for (int i = 0; i < p.dwp_tiles; ++i) dw += p.dwp[static_cast<size_t>(grow) * p.dwp_tiles + i];
-        p.peer_dw[src][pos] = dw;
-      }
-    }
     // Lane s keeps the count of row pieces this warp has stored to source rank s; nothing is released here, so the
     // stores of consecutive tiles stay in flight together (`flush_returned` releases once, after the last tile).
     for (int s = 0; s < p.lay.P; ++s) {
@@ -397,6 +394,10 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
     }
     if (valid) p.dwp[static_cast<size_t>(grow) * p.dwp_tiles + tl.n] = partial;
   } else if constexpr (MODE == kModeDswiglu) {
+    // The accumulator is g W_down^T of the UNWEIGHTED gradient rows: d_act = w * acc, and the router weight's gradient is
+    // <g, act W_down> = <acc, act>, so neither y nor w * g is ever formed (see `compute_backward`).
+    const float w = (p.row_w != nullptr && valid) ? p.row_w[grow] : 1.0f;
+    float partial = 0.0f;  // this tile's columns of <acc, act>
     if (p.stripe <= 64 && p.k_blocks < kStagedDswigluMaxKBlocks) {
       // The tile's 512 striped columns of h / dh are four 128-column blocks; with stripes of 32 or 64 columns block b
       // holds the gate and up values of exactly the accumulator columns [64 b, 64 b + 64). The warp brings a block of h
@@ -433,7 +434,8 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               // d_act is rounded to bf16 first, as the unfused reference stores it.
-              const uint32_t db = pack_bf16(__uint_as_float(acc[2 * e]), __uint_as_float(acc[2 * e + 1]));
+              const float a2[2] = {__uint_as_float(acc[2 * e]), __uint_as_float(acc[2 * e + 1])};
+              const uint32_t db = pack_bf16(w * a2[0], w * a2[1]);
               float dg[2], du[2];
 #pragma unroll
               for (int z = 0; z < 2; ++z) {
@@ -442,6 +444,7 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
                 const float up = z ? bf16_hi(uw[e]) : bf16_lo(uw[e]);
                 const float sig = sigmoid_f(gt);
                 const float sl = gt * sig;
+                partial += a2[z] * (sl * up);
                 dg[z] = d * up * (sig + sl * (1.0f - sig));
                 du[z] = d * sl;
               }
@@ -455,6 +458,7 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
         stage_flush(stage_gen, lane, reinterpret_cast<uint8_t*>(p.out0 + block_off + b * 128),
                     static_cast<size_t>(p.ld0) * 2, nvalid);
       }
+      if (valid && p.dwp != nullptr) p.dwp[static_cast<size_t>(grow) * p.dwp_tiles + tl.n] = partial;
       return;
     }
     // Deep contractions (the epilogue hides behind the next tile either way and this form is a little cheaper), and
@@ -507,7 +511,8 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             // d_act is rounded to bf16 first, as the unfused reference stores it.
-            const uint32_t db = pack_bf16(__uint_as_float(r[8 * i + 2 * e]), __uint_as_float(r[8 * i + 2 * e + 1]));
+            const float a2[2] = {__uint_as_float(r[8 * i + 2 * e]), __uint_as_float(r[8 * i + 2 * e + 1])};
+            const uint32_t db = pack_bf16(w * a2[0], w * a2[1]);
             float dg[2], du[2];
 #pragma unroll
             for (int z = 0; z < 2; ++z) {
@@ -516,6 +521,7 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
               const float up = z ? bf16_hi(uw[e]) : bf16_lo(uw[e]);
               const float sig = sigmoid_f(gt);
               const float sl = gt * sig;
+              partial += a2[z] * (sl * up);
               dg[z] = d * up * (sig + sl * (1.0f - sig));
               du[z] = d * sl;
             }
@@ -527,6 +533,7 @@ __device__ __forceinline__ void run_epilogue(const GemmParams& p, const Tile& tl
         }
       }
     }
+    if (valid && p.dwp != nullptr) p.dwp[static_cast<size_t>(grow) * p.dwp_tiles + tl.n] = partial;
   } else {  // kModeTgmm
     const size_t m_total = static_cast<size_t>(p.m_tiles) * kBlockM;
     const bool first = (tl.flags & kGroupFirst) != 0, final = (tl.flags & kGroupFinal) != 0;

@@ -23,9 +23,9 @@ constexpr int kRasterBand = 8;     // row tiles swept together across N so their
 enum GemmMode : int {
   kModeSwiglu = 0,   // act = silu(x Wg) * (x Wu) from striped w_up; optional h          (replaces gmm_swiglu)
   kModeDownFwd = 1,  // y = act Wd; epilogue x router weight, rows stored to their source rank (gmm + combine)
-  kModeDownDw = 2,   // backward remat of y: d_weight partials <g, y> and dy = w * g, y never stored
-  kModeDswiglu = 3,  // d_act = dy Wd^T; epilogue SwiGLU' with h -> dh                     (gmm_dswiglu)
-  kModeDx = 4,       // dx = dh Wu^T; rows (+ d_weight scalar) stored to their source rank  (gmm^T + combine)
+  kModeDownDw = 2,   // d_weight partials <g, y> and dy = w * g, y never stored (kernel entry point only)
+  kModeDswiglu = 3,  // d_act = w * (g Wd^T); epilogue SwiGLU' with h -> dh, d_weight partials (gmm_dswiglu)
+  kModeDx = 4,       // dx = dh Wu^T; rows stored to their source rank                      (gmm^T + combine)
   kModeTgmm = 5,     // dW[g] = lhs[rows_g]^T rhs[rows_g], fp32 carry across slices         (tgmm + accumulate)
 };
 
@@ -72,13 +72,12 @@ struct GemmParams {
   __nv_bfloat16* out0;        // swiglu: act [S,F]; down_dw: dy [S,D]; dswiglu: dh [S,2F]
   __nv_bfloat16* out1;        // swiglu: h [S,2F] or null
   const __nv_bfloat16* in0;   // down_dw: g [S,D]; dswiglu: h [S,2F]
-  const float* row_w;         // down_fwd / down_dw: router weight per slice row [S]
-  float* dwp;                 // down_dw: out [S, n_tiles]; dx: in [S, dwp_tiles]
+  const float* row_w;         // router weight per slice row [S]; swiglu / dswiglu: null = 1
+  float* dwp;                 // down_dw / dswiglu: per-column-tile shares of the router weight's gradient [S, dwp_tiles]
   int dwp_tiles;
   int ld0, ld1;
   // --- combine targets (down_fwd, dx) --------------------------------------------------------
   __nv_bfloat16* const* peer_rows;   // [P] base of each source rank's [T*K, ld] return buffer
-  float* const* peer_dw;             // [P] base of each source rank's [T*K] d_weight rows (dx only)
   uint32_t* const* peer_count;       // [P] each source rank's returned-row counter
   // --- tgmm ---------------------------------------------------------------------------------
   const float* carry_in;   // [M, N] fp32 partial of the expert that straddles the previous slice boundary

@@ -89,9 +89,11 @@ class FusedRank {
   torch::Tensor act() const { return act_[0]; }
   torch::Tensor h() const { return h_[0]; }
   torch::Tensor dh() const { return dh_[0]; }
-  torch::Tensor dy() const { return dy_[0]; }
+  torch::Tensor dy() const { return torch::empty({0}, act_[0].options()); }  // w * g is never materialised
 
  private:
+  // Common start of a pass: counter targets on the device, what the pass will receive back (`pieces_per_row` of T*K rows).
+  void begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row);
   void end_pass(int64_t n_slices);
   void join_streams(bool backward);
   GemmParams base_params(const int* plan, int j) const;
@@ -115,7 +117,7 @@ class FusedRank {
   std::vector<uint8_t*> peers_;
 
   // local scratch (torch-owned)
-  torch::Tensor act_[2], h_[2], dy_[2], dh_[2], dwp_[2];
+  torch::Tensor act_[2], h_[2], dh_[2], dwp_[2];
   torch::Tensor carry_up_, carry_down_, pass_base_, expected_total_, status_, tables_,
       sort_scratch_, my_counts_;
   torch::Tensor ready_, ready_base_, ready_total_;  // fp8 wire: per-expert "rows expanded" counter, its base, its target
@@ -125,14 +127,14 @@ class FusedRank {
   template <typename T>
   T* const* table(int t) const { return reinterpret_cast<T* const*>(tables_.data_ptr<int64_t>() + t * P_); }
 
-  CUtensorMap map_x_k_[2], map_x_mn_[2], map_act_k_[2], map_act_mn_[2], map_dy_k_[2], map_dy_mn_[2], map_dh_k_[2],
+  CUtensorMap map_x_k_[2], map_x_mn_[2], map_act_k_[2], map_act_mn_[2], map_g_k_[2], map_g_mn_[2], map_dh_k_[2],
       map_dh_mn_[2];
   std::map<std::tuple<const void*, uint32_t, int64_t, int64_t>, CUtensorMap> weight_maps_;
 
   cudaStream_t comm_stream_ = nullptr, aux_stream_ = nullptr, chain_[2] = {};
   cudaStream_t expand_stream_ = nullptr;  // fp8 wire: the expansion kernels run here, beside the GEMM chains
   cudaEvent_t ev_expand_[4] = {};  // expansion of slice j (mod 4) has finished
-  cudaEvent_t ev_down_[2] = {}, ev_dd_[2] = {}, ev_ds_[2] = {}, ev_dx_[2] = {}, ev_tgd_[2] = {}, ev_tgu_[2] = {};
+  cudaEvent_t ev_down_[2] = {}, ev_up_[2] = {}, ev_ds_[2] = {}, ev_dx_[2] = {}, ev_tgd_[2] = {}, ev_tgu_[2] = {};
   cudaEvent_t ev_pass_ = nullptr, ev_put_[4] = {}, ev_done_[4] = {}, ev_header_ = nullptr;
   int64_t last_slices_ = -1;  // slice count of the previous forward pass (the next pass's guess)
   int32_t* host_header_ = nullptr;  // pinned: 16 plan header ints + 8 status ints

@@ -44,9 +44,8 @@ KernelRunner::KernelRunner(int L, int S, int stripe, int num_sms, bool cta_pairs
   counts_ = torch::zeros({L}, i32);
   status_ = torch::zeros({8}, i32);
   ones_ = torch::ones({S}, f32);
-  scratch_f32_ = torch::zeros({S}, f32);
   counter_ = torch::zeros({4}, i32);
-  table_ = torch::zeros({4}, torch::TensorOptions().device(torch::kCUDA).dtype(torch::kInt64));
+  table_ = torch::zeros({2}, torch::TensorOptions().device(torch::kCUDA).dtype(torch::kInt64));
 }
 
 void KernelRunner::set_groups(torch::Tensor group_rows) {
@@ -112,8 +111,7 @@ void KernelRunner::gmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out, 
   need_bf16(lhs, S_, K, "lhs");
   need_bf16(out, S_, N, "out");
   // One "rank": rows go back to where they came from, which is their own position in `out`.
-  const int64_t ptrs[4] = {reinterpret_cast<int64_t>(out.data_ptr()), reinterpret_cast<int64_t>(counter_.data_ptr()),
-                           reinterpret_cast<int64_t>(scratch_f32_.data_ptr()), 0};
+  const int64_t ptrs[2] = {reinterpret_cast<int64_t>(out.data_ptr()), reinterpret_cast<int64_t>(counter_.data_ptr())};
   cudaMemcpyAsync(table_.data_ptr(), ptrs, sizeof(ptrs), cudaMemcpyHostToDevice, stream());
   GemmParams p = base();
   p.n_tiles = static_cast<int>(N / kBlockN);
@@ -129,9 +127,6 @@ void KernelRunner::gmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out, 
     launch(kModeDownFwd, p, a, b, nullptr);
   } else {
     p.b_group_rows = static_cast<int>(N);
-    p.peer_dw = reinterpret_cast<float* const*>(table_.data_ptr<int64_t>() + 2);
-    p.dwp = nullptr;
-    p.dwp_tiles = 0;  // no d_weight partials: the scalar that rides along is a plain zero
     const CUtensorMap b = make_bf16_map_2d(rhs.data_ptr(), static_cast<uint64_t>(L_) * N, K, pairs_ ? 128 : 256);
     launch(kModeDx, p, a, b, nullptr);
   }

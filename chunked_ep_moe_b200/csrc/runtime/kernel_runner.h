@@ -47,7 +47,7 @@ class KernelRunner {
   int L_, S_, stripe_, num_sms_;
   bool pairs_;
   PlanLayout lay_;
-  torch::Tensor plan_, counts_, status_, ones_, scratch_f32_, counter_, table_;
+  torch::Tensor plan_, counts_, status_, ones_, counter_, table_;
 };
 
 }  // namespace cem

@@ -10,8 +10,8 @@ reached the host. Compared with the reference's loop
   * no `[T*K, D]` send buffer: the put kernel gathers rows straight from `x[token]`;
   * the router weight is applied in the down-projection epilogue, which stores every finished
     row into the source rank's return buffer; a local K-way fixed-order sum finishes the token;
-  * the backward folds `y` into `d_weight = <g, y>` inside the recomputed down GEMM's epilogue
-    and forms `dy = w * g` there, so `y` never reaches HBM;
+  * the backward recomputes the up-projection only: `d_weight = <g, act Wd>` is `<g Wd^T, act>`, a by-product of the
+    GEMM that yields `d_act = w * (g Wd^T)`, and `dW_down` contracts `w * act` with `g`; neither `y` nor `w * g` exists;
   * weight gradients are written once per expert in bf16; only the (at most one) expert that
     straddles a slice boundary carries an fp32 partial to the next slice.
 
@@ -180,8 +180,8 @@ def expected_launches(num_slices: int, fp8: bool = False) -> int:
     """Kernels one forward+backward of the fused layer launches on a rank that loops `num_slices` slices.
 
     Forward: sort (3) + plan build + pass begin + per slice (put, swiglu, down+combine, slice done) + combine reduce.
-    Backward: pass begin + per slice (put, swiglu+h, down->d_weight/dy, dswiglu, dW_down, dx+combine, dW_up, slice
-    done) + combine reduce. The fp8 wire adds one dequantisation kernel per slice and pass.
+    Backward: pass begin + per slice (put, swiglu+h, dswiglu, dW_down, d_weight return, dx+combine, dW_up, slice done)
+    + combine reduce. The fp8 wire adds one dequantisation kernel per slice and pass.
     """
     per_slice = 12 + (2 if fp8 else 0)
     return 8 + per_slice * num_slices
@@ -198,7 +198,7 @@ def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidd
     tk = tokens_per_rank * top_k if tk_cap is None else tk_cap
     S, D, F = slice_size, hidden, ffn
     arena = int(ext.arena_bytes(world, L, S, D, tk, fp8))
-    scratch = 2 * (S * F * 2 + S * 2 * F * 2 + S * D * 2 + S * 2 * F * 2 + S * (D // 256) * 4)  # act, h, dy, dh, dwp x2
+    scratch = 2 * (S * F * 2 + S * 2 * F * 2 + S * 2 * F * 2 + S * (F // 256) * 4)  # act, h, dh, d_weight shares, x2
     carry = 2 * (D * 2 * F + F * D) * 4
     weights = L * (D * 2 * F + F * D) * 2
     max_slices = max(1, math.ceil(world * tk / S)) + 1
@@ -206,7 +206,7 @@ def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidd
     saved = tokens_per_rank * D * 2 + tk * 4 * 3 + plan  # x, router weights, order, inverse order, plan tables
     out = {
         "arena (slice buffers x2 for x and g, return rows, counters, traffic matrix)": arena,
-        "scratch (act, h, dy, dh, d_weight partials; two slices in flight)": scratch,
+        "scratch (act, h, dh, d_weight shares; two slices in flight)": scratch,
         "weight-gradient carry tiles (fp32, two per matrix)": carry,
         "expert weights (bf16)": weights,
         "expert weight gradients (bf16)": weights,
