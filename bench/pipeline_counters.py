@@ -1,6 +1,7 @@
 """In-kernel pipeline counters of the grouped GEMM modes over a few forward+backward steps (one GPU, no profiler).
 
-For every mode: SM cycles per k-block (512 is the tensor pipe's floor for a 128x256x64 bf16 block), the SM clock the
+For every mode: SM cycles per k-block (512 is the tensor pipe's floor for a full 256-row tile, narrower tiles need
+proportionally less), the SM clock the
 kernels really ran at (cycles / global-timer nanoseconds) and the share of the MMA warp's loop spent waiting for a
 filled stage (loads late), for an accumulator (epilogue late), and of the producer's time waiting for a free stage
 (MMAs late).
@@ -66,8 +67,7 @@ def main():
     stop.record()
     torch.cuda.synchronize()
     fused.pipeline_counters(False)
-    print(f"{args.steps} steps with counters on: {start.elapsed_time(stop) / args.steps:.2f} ms per step; "
-          f"CEM_CTA_PAIRS={os.environ.get('CEM_CTA_PAIRS', '0')}")
+    print(f"{args.steps} steps with counters on: {start.elapsed_time(stop) / args.steps:.2f} ms per step")
     c = sum(t.double() for t in counters).cpu()  # [6, CTAs, 8]
     s = {n: i for i, n in enumerate(fused.PIPELINE_COUNTER_SLOTS)}
     print("mode       k-blocks  cycles/k-block  SM GHz  mma wait loads %  mma wait epilogue %  producer wait mma %  "

@@ -23,7 +23,7 @@ _SOURCES = [
     "runtime/tensor_map.cpp",
     "runtime/fused_rank.cpp",
     "runtime/kernel_runner.cpp",
-    "gemm/grouped_gemm.cu",
+    "gemm/row_gemm.cu",
     "gemm/grouped_gemm_pair.cu",
     "comm/comm_kernels.cu",
     "plan/plan_kernel.cu",

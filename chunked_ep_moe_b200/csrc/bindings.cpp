@@ -14,11 +14,13 @@ namespace {
 py::dict plan_layout_dict(int P, int L, int S, int max_slices) {
   const cem::PlanLayout y = cem::make_plan_layout(P, L, S, max_slices);
   py::dict d;
-  d["max_mtiles"] = y.max_mtiles;
+  // "mtiles" and "ptiles" are one and the same table of GEMM row tiles (at most `tile_m` rows each).
+  for (const std::string kind : {"mtiles", "ptiles"}) {
+    d[("max_" + kind).c_str()] = y.max_tiles;
+    d[("num_" + kind).c_str()] = y.off_num_tiles;
+    d[kind.c_str()] = y.off_tiles;
+  }
   d["max_gtiles"] = y.max_gtiles;
-  d["max_ptiles"] = y.max_ptiles;
-  d["num_ptiles"] = y.off_num_ptiles;
-  d["ptiles"] = y.off_ptiles;
   d["send_start"] = y.off_send_start;
   d["seg_start"] = y.off_seg_start;
   d["seg_size"] = y.off_seg_size;
@@ -27,14 +29,12 @@ py::dict plan_layout_dict(int P, int L, int S, int max_slices) {
   d["src_send_start"] = y.off_src_send_start;
   d["expert_start"] = y.off_expert_start;
   d["expert_rows"] = y.off_expert_rows;
-  d["num_mtiles"] = y.off_num_mtiles;
   d["num_gtiles"] = y.off_num_gtiles;
   d["num_chunks"] = y.off_num_chunks;
-  d["mtiles"] = y.off_mtiles;
   d["gtiles"] = y.off_gtiles;
   d["put"] = y.off_put;
   d["total"] = y.total;
-  d["tile_m"] = cem::kTileM;
+  d["tile_m"] = cem::kTileTokens;
   d["put_chunk_rows"] = cem::kPutChunkRows;
   return d;
 }
@@ -110,8 +110,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("arena_fill", &cem::arena_fill, "cudaMemset of a byte range (tests poison data buffers with NaN patterns)");
   m.def("arena_layout", &arena_layout_dict, "byte offsets inside one rank's symmetric arena");
   m.def("arena_read_i32", &cem::arena_read_i32, "device synchronise + copy int32 values of an arena to the host");
-  m.attr("gemm_smem_bytes") = cem::kGemmSmemBytes;
-  m.def("pair_grid_used", []() { return cem::g_pair_grid_used; }, "grid of the last CTA-pair GEMM launch");
+  m.attr("gemm_smem_bytes") = cem::row_gemm_smem_bytes();
+  m.def("pair_grid_used", []() { return cem::g_pair_grid_used; }, "grid of the last GEMM launch");
   m.def("wait_probe", &wait_probe, "bounded-wait self test kernel");
   m.def("format_status", &cem::format_status, "text of a recorded status block");
   m.def("add_rms_norm_fwd", &cem::add_rms_norm_fwd, "s = x + delta, y = RMSNorm(s) * w -> (s, y, rstd)");
@@ -125,8 +125,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("router_fwd", &cem::router_fwd, "fp32 logits, bias -> (ids, weights, counts, per-block score sums)");
   m.def("router_bwd", &cem::router_bwd, "-> fp32 gradient of the logits");
   py::class_<cem::KernelRunner>(m, "KernelRunner")
-      .def(py::init<int, int, int, int, bool>(), py::arg("L"), py::arg("S"), py::arg("stripe"), py::arg("num_sms"),
-           py::arg("cta_pairs") = false)
+      .def(py::init<int, int, int, int>(), py::arg("L"), py::arg("S"), py::arg("stripe"), py::arg("num_sms"))
       .def("set_groups", &cem::KernelRunner::set_groups)
       .def("gmm_swiglu", &cem::KernelRunner::gmm_swiglu, py::arg("x"), py::arg("w_up"), py::arg("act"),
            py::arg("h") = py::none())
@@ -137,11 +136,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("check_status", &cem::KernelRunner::check_status);
   py::class_<cem::FusedRank>(m, "FusedRank")
       .def(py::init<int, int, int, int, int, int, int, int, int, int, int, bool, int64_t, std::vector<int64_t>, bool,
-                    int64_t, int, bool, bool>(),
+                    int64_t, int>(),
            py::arg("P"), py::arg("L"), py::arg("me"), py::arg("S"), py::arg("D"), py::arg("F"), py::arg("K"),
            py::arg("stripe"), py::arg("tk_cap"), py::arg("max_slices"), py::arg("num_sms"), py::arg("fp8"),
            py::arg("arena"), py::arg("peer_arenas"), py::arg("use_comm_stream"), py::arg("spin_limit"),
-           py::arg("put_blocks"), py::arg("cta_pairs") = true, py::arg("tgmm_pairs") = true)
+           py::arg("put_blocks"))
       .def("begin_forward", &cem::FusedRank::begin_forward)
       .def("begin_forward_async", &cem::FusedRank::begin_forward_async)
       .def("resolve_slices", &cem::FusedRank::resolve_slices)

@@ -25,7 +25,7 @@ namespace cem {
 
 namespace {
 
-constexpr int kPutThreads = 512;
+constexpr int kPutThreads = 256;  // with 64 registers each it fits beside a GEMM CTA (see row_gemm.cu)
 
 __device__ __forceinline__ int find_segment(const int4* put, int n, int chunk) {
   // Last segment whose chunk prefix is <= chunk (empty segments share a prefix with their successor).
@@ -200,7 +200,11 @@ __global__ void __launch_bounds__(256) return_dw_kernel(const ReturnDwParams p) 
       if (expert_start[mid] <= at) lo = mid; else hi = mid - 1;
     }
     float sum = 0.0f;
-    for (int q = 0; q < p.parts; ++q) sum += p.dwp[static_cast<size_t>(row) * p.parts + q];
+    const float4* parts = reinterpret_cast<const float4*>(p.dwp + static_cast<size_t>(row) * p.parts);
+    for (int q = 0; q < p.parts / 4; ++q) {  // F / 32 of them: a multiple of eight
+      const float4 v = parts[q];
+      sum += (v.x + v.y) + (v.z + v.w);
+    }
     for (int s = 0; s < p.lay.P; ++s) {
       const int i = s * p.lay.L + lo, off = at - p.plan[p.lay.off_in_start + i];
       if (off >= 0 && off < p.plan[p.lay.off_in_size + i]) {
@@ -241,9 +245,7 @@ __global__ void __launch_bounds__(256) combine_reduce_kernel(const CombineParams
       for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
       for (int k = 0; k < p.top_k; ++k) {  // fixed k order: bitwise reproducible
         const int pos = p.inv_order[t * p.top_k + k];
-        const size_t at = p.blocked ? (static_cast<size_t>(u >> 5) * p.ret_rows + pos) * 256 + (((u & 31) ^ (pos & 7)) << 3)
-                                    : static_cast<size_t>(pos) * p.hidden + u * 8;
-        const int4 raw = *reinterpret_cast<const int4*>(p.rows + at);
+        const int4 raw = *reinterpret_cast<const int4*>(p.rows + static_cast<size_t>(pos) * p.hidden + u * 8);
         const uint32_t wds[4] = {static_cast<uint32_t>(raw.x), static_cast<uint32_t>(raw.y),
                                  static_cast<uint32_t>(raw.z), static_cast<uint32_t>(raw.w)};
 #pragma unroll

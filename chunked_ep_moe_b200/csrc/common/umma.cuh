@@ -37,16 +37,17 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// Suspends the thread for up to 20 us (no polling while a long mainloop runs).
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t"
       "}\n"
       : "=r"(ok)
-      : "r"(bar), "r"(parity)
+      : "r"(bar), "r"(parity), "r"(20000u)
       : "memory");
   return ok != 0;
 }
@@ -68,32 +69,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
     if ((i & 63u) == 0) {
       if (abort != nullptr && *abort != 0) return false;
       if (global_timer_ns() - t0 > static_cast<uint64_t>(limit_us) * 1000ull) return false;
-    }
-  }
-}
-
-// Non-suspending variant (test_wait polling) for barriers completed by the other CTA of a pair; also gives up as
-// soon as `*abort` is set.
-__device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, uint32_t limit_us,
-                                               const volatile int* abort = nullptr) {
-  uint64_t t0 = 0;
-  for (uint32_t i = 0;; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((i & 255u) == 255u) {
-      if (abort != nullptr && *abort != 0) return false;
-      const uint64_t now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > static_cast<uint64_t>(limit_us) * 1000ull) return false;
     }
   }
 }
@@ -367,7 +342,47 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
       : "memory");
 }
 
+// TMEM -> registers as 8 x 8 matrix fragments: 16 lanes (from `taddr`'s lane) x 32 consecutive fp32 columns. Register
+// 4 j + 2 rr + e of a thread holds lane 8 rr + laneid / 4, column 8 j + 2 (laneid % 4) + e.
+__device__ __forceinline__ void tmem_ld_16x256_x4(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------------------
+// shared-memory accesses by 32-bit address; 8 x 8 b16 matrices stored / loaded transposed (lane 8 i + k gives the address of
+// row k of matrix i; register i holds matrix i's fragment: element (laneid / 4, 2 (laneid % 4) + e) of the TRANSPOSE)
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+__device__ __forceinline__ int4 ld_shared_v4(uint32_t addr) {
+  int4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr)
+               : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t (&m)[4]) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(m[0]),
+               "r"(m[1]), "r"(m[2]), "r"(m[3])
+               : "memory");
+}
+
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&m)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(m[0]), "=r"(m[1]), "=r"(m[2]), "=r"(m[3])
+               : "r"(addr)
+               : "memory");
+}
 
 // ---------------------------------------------------------------------------------------------
 // system-scope flag accesses (flags live in this or a peer GPU's memory)

@@ -1,0 +1,709 @@
+// Row-wise grouped GEMMs (SwiGLU up-projection, down-projection + combine, SwiGLU', dX + combine) on CTA pairs with the
+// WEIGHTS' columns on the MMA's M side and the TOKENS on its N side.
+//
+// A pair of CTAs drives one 256 x N x 16 tcgen05.mma (cta_group::2): M = 256 weight columns (128 per CTA), N = a tile of
+// up to 256 rows of ONE expert, in steps of 32. With tokens on the M side a tile is 128 or 256 rows whatever the expert
+// has left; here an expert's rows are cut into equal tiles of a multiple of 32 (`plan_tile_span`), so the padding is 16
+// rows per expert on average. Each CTA stages its 128 weight columns and half of the tile's rows: 32 KB per k-block at
+// N = 256 (the SM's L2 port carries one request per 128-byte line, see grouped_gemm_pair.cu), less for narrow tiles.
+//
+//   warp 0       TMA producer of the CTA's operands (every load credits the leader's full barrier)
+//   warp 1       leader only: MMA issue; commits to both CTAs' barriers
+//   warps 2-9    epilogue of the CTA's 128 columns x N rows. A warp may read 32 of the 128 TMEM lanes, so four warps form
+//                a group; the two groups take the tile's 32-row chunks in turn (SwiGLU needs a few thousand cycles of one
+//                warp per SM sub-partition for a tile: with 16 k-blocks per tile one group could not keep up).
+//
+// Measured against the token-major kernels this one replaced (128 x 256 tiles on single CTAs below 768 rows per expert, 256 x
+// 256 on pairs above), same box: 490-510 cycles per k-block at D=7168, F=2048 in every mode (the tensor pipe's floor for the
+// mean width; 515-540 for the pairs, 610-700 for single CTAs), layer forward + backward with 256 rows per expert 7.86 -> 7.33
+// ms, Zipf routing in slices of 2048 rows 10.7 -> 9.1 ms, decode of 64 tokens (16 rows per expert) 776 -> 563 us, 2048 rows
+// per expert 21.4 -> 20.4 ms (there the 1000 W power cap sets the clock, so fewer padded rows are what counts).
+//
+// The accumulator is transposed (TMEM lane = weight column, TMEM column = row). `tcgen05.ld.16x256b` hands it out as
+// 8 x 8 matrix fragments, and `stmatrix.trans` / `ldmatrix.trans` turn those around in the group's staging buffer, whose
+// rows are token rows; global accesses then move whole 128- to 512-byte row pieces. 16-byte pieces of a staging row are
+// XOR-ed with the row number (mod 8): fragment and row accesses are both free of bank conflicts.
+#include "grouped_gemm.cuh"
+
+#include "../common/umma.cuh"
+#include "gemm_common.cuh"
+
+namespace cem {
+
+namespace {
+
+constexpr int kRowStages = 6;
+constexpr int kRowStageBytesA = kBlockM * kBlockK * 2;  // this CTA's 128 weight columns
+constexpr int kRowStageBytesB = (kTileTokens / 2) * kBlockK * 2;  // up to 128 rows
+constexpr int kRowStageBytes = kRowStageBytesA + kRowStageBytesB;
+constexpr int kRowBand = 4;                             // token tiles swept together over the weight columns
+constexpr int kRowThreads = 64 + 8 * 32;
+constexpr int kGroupStaging = 16384;                    // per epilogue group
+constexpr int kRowSmemBytes = kSmemAlignSlack + kRowStages * kRowStageBytes + 2 * kGroupStaging + kSmemTailBytes;
+static_assert(kRowSmemBytes + 1024 + 1024 + 16 <= 233472, "no room for a second, small CTA on the SM");
+
+struct RowTile {
+  int g;      // local expert
+  int row0;   // first slice row
+  int nrows;  // rows of the tile
+  int ncols;  // nrows rounded up to a multiple of 32: the MMA's N
+  int n;      // 256-column tile of the weights
+};
+
+__device__ __forceinline__ RowTile decode_row_tile(const GemmParams& p, int t, int num_entries) {
+  RowTile tl;
+  const int band_tiles = kRowBand * p.n_tiles;
+  const int band = t / band_tiles, rem = t - band * band_tiles;
+  int width = num_entries - band * kRowBand;
+  width = width > kRowBand ? kRowBand : width;
+  tl.n = rem / width;
+  const int ti = band * kRowBand + (rem - tl.n * width);
+  const int4 e = reinterpret_cast<const int4*>(p.plan + p.lay.off_tiles + 4 * p.lay.max_tiles * p.slice)[ti];
+  tl.g = e.x; tl.row0 = e.y; tl.nrows = e.z; tl.ncols = e.w;
+  return tl;
+}
+
+template <int MODE>
+struct RowTraits {
+  static constexpr bool kAMn = (MODE == kModeSwiglu || MODE == kModeDownFwd);  // weights read with K along rows
+  static constexpr bool kCombine = (MODE == kModeDownFwd || MODE == kModeDx);
+};
+
+template <int MODE>
+__device__ __forceinline__ void issue_row_kblock(const GemmParams& p, const RowTile& tl, int kb, int rank,
+                                                 const CUtensorMap* map_a, const CUtensorMap* map_b, uint32_t sa,
+                                                 uint32_t bar) {
+  if constexpr (RowTraits<MODE>::kAMn) {
+    const int y = tl.g * p.b_group_rows + kb * kBlockK;
+    if (MODE == kModeSwiglu && p.stripe == 128) {
+      // Stripes of 128: this CTA's 64 gate columns and the 64 up columns that belong to them are 128 columns apart.
+      tma_load_3d_pair(sa, map_a, bar, y, tl.n * 4 + rank);
+      tma_load_3d_pair(sa + kRowStageBytesA / 2, map_a, bar, y, tl.n * 4 + 2 + rank);
+    } else {
+      tma_load_3d_pair(sa, map_a, bar, y, tl.n * 4 + 2 * rank);  // two 64-column chunks
+    }
+  } else {
+    tma_load_2d_pair(sa, map_a, bar, kb * kBlockK, tl.g * p.b_group_rows + tl.n * kBlockN + rank * kBlockM);
+  }
+  tma_load_2d_pair(sa + kRowStageBytesA, map_b, bar, kb * kBlockK, tl.row0 + rank * (tl.ncols >> 1));
+}
+
+// ---------------------------------------------------------------------------------------------
+// Epilogues. `tacc`: TMEM address of this warp's 32 lanes, accumulator buffer included. A group of four warps (128
+// threads, `gt` = thread in the group) works on 32-row chunks h, h + 2, ... of the tile.
+// Register index of a chunk fragment: half * 16 + j * 4 + rr * 2 + e holds weight column 16 half + 8 rr + lane / 4 (of the
+// warp's 32) and row 8 j + 2 (lane & 3) + e (of the chunk's 32).
+// ---------------------------------------------------------------------------------------------
+// (Barrier numbers as immediates: with a register operand the compiler reserves all sixteen of the CTA's barriers.)
+__device__ __forceinline__ void group_sync(int h) {
+  if (h == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+  else asm volatile("bar.sync 2, 128;" ::: "memory");
+}
+
+// True if `ok` holds in every thread of the group.
+__device__ __forceinline__ bool group_vote(int h, bool ok) {
+  uint32_t r;
+#define CEM_VOTE(BAR)                                                                                             \
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, " BAR ", 128, p;\n\t"         \
+               "selp.u32 %0, 1, 0, q;\n\t}\n"                                                                     \
+               : "=r"(r) : "r"(ok ? 1u : 0u) : "memory")
+  if (h == 0) CEM_VOTE("1");
+  else CEM_VOTE("2");
+#undef CEM_VOTE
+  return r != 0;
+}
+
+__device__ __forceinline__ void load_fragment(uint32_t taddr, uint32_t (&r)[32]) {
+  tmem_ld_16x256_x4(taddr, r);
+  tmem_ld_16x256_x4(taddr + (16u << 16), r + 16);
+  tmem_ld_wait();
+}
+
+// Address of 16-byte piece `piece` of staging row `row`, rows of ROWB bytes.
+template <int ROWB>
+__device__ __forceinline__ uint32_t staged(uint32_t buf, int row, int piece) {
+  return buf + row * ROWB + ((piece ^ (row & 7)) << 4);
+}
+
+// Copies staging rows (ROWB bytes = consecutive columns at `out + row * ld`) below `nvalid` to global memory.
+template <int ROWB>
+__device__ __forceinline__ void flush_rows(uint32_t buf, int gt, uint8_t* out, size_t ld_bytes, int nvalid) {
+  constexpr int kPieces = ROWB / 16, kRows = 128 / kPieces;  // rows per sweep of the group
+  const int piece = gt % kPieces;
+#pragma unroll
+  for (int i = 0; i < 32 / kRows; ++i) {
+    const int row = gt / kPieces + i * kRows;
+    const int4 v = ld_shared_v4(staged<ROWB>(buf, row, piece));
+    if (row < nvalid) *reinterpret_cast<int4*>(out + row * ld_bytes + piece * 16) = v;
+  }
+}
+
+struct GroupCtx {
+  int h, q, lane, gt, rank;
+  uint32_t staging;  // this group's staging buffer
+};
+
+template <typename Release>
+__device__ __forceinline__ void swiglu_epilogue(const GemmParams& p, const RowTile& tl, uint32_t tacc,
+                                                const GroupCtx& c, Release&& release) {
+  const int chunks = (tl.nrows + 31) >> 5;
+  // Lanes 0-63 of the accumulator are gate columns and 64-127 the up columns that belong to them (stripes of 32: both
+  // kinds alternate every 32 lanes), so a gate warp and its partner exchange half of a chunk through shared memory
+  // (fp32, thread to thread) and each computes 32 activation columns of 16 rows.
+  const bool narrow = p.stripe == 32;
+  const bool is_gate = narrow ? !(c.q & 1) : c.q < 2;
+  const int partner = narrow ? (c.q ^ 1) : (c.q ^ 2);
+  const int act_piece = (narrow ? (c.q >> 1) : (c.q & 1)) * 4;  // first 16-byte piece of the 32 activation columns
+  const bool with_h = p.out1 != nullptr;
+  const uint32_t hbuf = c.staging, exch = c.staging + 8192;
+  const uint32_t abuf = with_h ? exch : hbuf;  // activations go where the exchange was; without h its place is free
+  const int act_col = tl.n * 128 + c.rank * 64;
+  const int h_col0 = tl.n * kBlockN + c.rank * (p.stripe == 128 ? 64 : 128);
+  const int h_col1 = h_col0 + (p.stripe == 128 ? 128 : 64);
+  for (int ch = c.h; ch < chunks; ch += 2) {
+    const int row0 = tl.row0 + ch * 32, nvalid = tl.nrows - ch * 32;
+    uint32_t r[32];
+    load_fragment(tacc + ch * 32, r);
+    if (ch + 2 >= chunks) release();
+    if (with_h) group_sync(c.h);  // the previous chunk's rows have left the buffers
+    const uint32_t mine = exch + c.q * 2048 + c.lane * 16;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // register quads (half, j) of the rows the partner works on
+      const int half = i >> 1, jj = i & 1;
+      uint32_t v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = is_gate ? r[half * 16 + (2 + jj) * 4 + k] : r[half * 16 + jj * 4 + k];
+      st_shared_v4(mine + i * 512, v[0], v[1], v[2], v[3]);
+    }
+    if (with_h) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t o[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
+          o[s] = pack_bf16(__uint_as_float(r[b]), __uint_as_float(r[b + 1]));
+        }
+        stmatrix_x4_trans(staged<256>(hbuf, 8 * j + (c.lane & 7), c.q * 4 + (c.lane >> 3)), o);
+      }
+    }
+    group_sync(c.h);
+    uint32_t in[16];
+    const uint32_t theirs = exch + partner * 2048 + c.lane * 16;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int4 v = ld_shared_v4(theirs + i * 512);
+      in[4 * i] = v.x; in[4 * i + 1] = v.y; in[4 * i + 2] = v.z; in[4 * i + 3] = v.w;
+    }
+    if (with_h) group_sync(c.h);  // everybody has read the exchange: its place takes the activations
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {
+      const int trow = (is_gate ? 0 : 16) + 8 * jj;
+      float w0 = 1.0f, w1 = 1.0f;
+      if (p.row_w != nullptr) {
+        // (Read past L1: the line may also hold weights of rows that had not arrived when another tile read it. Rows
+        // past the tile's end read their neighbours' weights or, at the end of the slice, nothing; they are not stored.)
+        const int t0 = trow + 2 * (c.lane & 3);
+        if (t0 < nvalid) w0 = __ldcg(p.row_w + row0 + t0);
+        if (t0 + 1 < nvalid) w1 = __ldcg(p.row_w + row0 + t0 + 1);
+      }
+      uint32_t o[4];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int half = s >> 1, rr = s & 1;
+        float a[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t own = is_gate ? r[half * 16 + jj * 4 + rr * 2 + e] : r[half * 16 + (2 + jj) * 4 + rr * 2 + e];
+          const uint32_t other = in[(half * 2 + jj) * 4 + rr * 2 + e];
+          const float gate = __uint_as_float(is_gate ? own : other), up = __uint_as_float(is_gate ? other : own);
+          a[e] = silu_f(gate) * up;
+        }
+        o[s] = pack_bf16(a[0] * w0, a[1] * w1);
+      }
+      stmatrix_x4_trans(staged<128>(abuf, trow + (c.lane & 7), act_piece + (c.lane >> 3)), o);
+    }
+    group_sync(c.h);
+    flush_rows<128>(abuf, c.gt, reinterpret_cast<uint8_t*>(p.out0 + static_cast<size_t>(row0) * p.ld0 + act_col),
+                    static_cast<size_t>(p.ld0) * 2, nvalid);
+    if (with_h) {
+      // 256-byte staging rows: two 128-byte halves whose places in a row of h depend on the stripe
+      const int piece = c.gt & 15;
+      __nv_bfloat16* out = p.out1 + static_cast<size_t>(row0) * p.ld1 + (piece < 8 ? h_col0 : h_col1) + (piece & 7) * 8;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = (c.gt >> 4) + i * 8;
+        const int4 v = ld_shared_v4(staged<256>(hbuf, row, piece));
+        if (row < nvalid) *reinterpret_cast<int4*>(out + static_cast<size_t>(row) * p.ld1) = v;
+      }
+    }
+  }
+  if (c.h >= chunks) release();
+}
+
+// Down-projection / dX: every row's 128 columns go to the rank the row came from, at its send-order position.
+// `dst` (shared memory, one entry per row of this group's chunks): source << 27 | position, or ~0 for rows past the tile;
+// `wts`: the rows' router weights (down-projection).
+template <int MODE, typename Release>
+__device__ __forceinline__ void combine_epilogue(const GemmParams& p, const RowTile& tl, uint32_t tacc,
+                                                 const GroupCtx& c, const uint32_t* dst, const float* wts,
+                                                 Release&& release) {
+  const int chunks = (tl.nrows + 31) >> 5;
+  const int col = tl.n * kBlockN + c.rank * kBlockM;
+  for (int ch = c.h; ch < chunks; ch += 2) {
+    const int list0 = (ch >> 1) * 32;
+    uint32_t r[32];
+    load_fragment(tacc + ch * 32, r);
+    if (ch + 2 >= chunks) release();
+    uint32_t o[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float2 w = make_float2(1.0f, 1.0f);
+      if constexpr (MODE == kModeDownFwd) w = *reinterpret_cast<const float2*>(wts + list0 + 8 * j + 2 * (c.lane & 3));
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
+        o[j][s] = pack_bf16(__uint_as_float(r[b]) * w.x, __uint_as_float(r[b + 1]) * w.y);
+      }
+    }
+    const uint32_t buf = c.staging;
+    group_sync(c.h);  // the previous chunk's rows have left the buffer
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      stmatrix_x4_trans(staged<256>(buf, 8 * j + (c.lane & 7), c.q * 4 + (c.lane >> 3)), o[j]);
+    group_sync(c.h);
+    const int piece = c.gt & 15;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = (c.gt >> 4) + i * 8;
+      const int4 v = ld_shared_v4(staged<256>(buf, row, piece));
+      const uint32_t d = dst[list0 + row];
+      if (d != ~0u)
+        *reinterpret_cast<int4*>(p.peer_rows[d >> 27] + static_cast<size_t>(d & ((1u << 27) - 1)) * p.ld0 + col +
+                                 piece * 8) = v;
+    }
+  }
+  if (c.h >= chunks) release();
+}
+
+// SwiGLU': 128 columns of d_act and the 256 striped columns of h / dh that belong to them (512 bytes of a row). The
+// group brings a chunk of h into its staging buffer (the next chunk's loads are in flight meanwhile), every warp turns
+// its own gate and up columns into gradients in place, the group writes the chunk out as dh.
+template <typename Release>
+__device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowTile& tl, uint32_t tacc,
+                                                 const GroupCtx& c, const int4 (&first)[8], Release&& release) {
+  const int chunks = (tl.nrows + 31) >> 5;
+  const int col = 2 * (tl.n * kBlockN + c.rank * kBlockM);  // first striped column
+  const int f = c.q * 32 + (c.lane >> 3) * 8;               // column (of 128) whose 16-byte piece this lane addresses
+  const int gpiece = (2 * p.stripe * (f / p.stripe) + f % p.stripe) >> 3, upiece = gpiece + (p.stripe >> 3);
+  const size_t ld_bytes = static_cast<size_t>(p.ld0) * 2;
+  const int piece = c.gt & 31, prow = c.gt >> 5;  // 32 threads per 512-byte row, four rows per sweep
+  int4 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = first[i];
+  for (int ch = c.h; ch < chunks; ch += 2) {
+    const int row0 = tl.row0 + ch * 32, nvalid = tl.nrows - ch * 32;
+    group_sync(c.h);  // the previous chunk has left the buffer
+#pragma unroll
+    for (int i = 0; i < 8; ++i) st_shared_v4(staged<512>(c.staging, prow + 4 * i, piece), v[i].x, v[i].y, v[i].z, v[i].w);
+    if (ch + 2 < chunks) {
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(p.in0 + static_cast<size_t>(row0 + 64) * p.ld0 + col) + piece * 16;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (prow + 4 * i < nvalid - 64) v[i] = *reinterpret_cast<const int4*>(src + (prow + 4 * i) * ld_bytes);
+    }
+    group_sync(c.h);
+    uint32_t r[32];
+    load_fragment(tacc + ch * 32, r);
+    if (ch + 2 >= chunks) release();
+    float part[8];  // <acc, act> over this thread's columns, rows 8 j + 2 (lane & 3) + e
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int t0 = 8 * j + 2 * (c.lane & 3);
+      float w[2] = {1.0f, 1.0f};
+      if (p.row_w != nullptr) {
+        if (t0 < nvalid) w[0] = p.row_w[row0 + t0];
+        if (t0 + 1 < nvalid) w[1] = p.row_w[row0 + t0 + 1];
+      }
+      const uint32_t ga = staged<512>(c.staging, 8 * j + (c.lane & 7), gpiece);
+      const uint32_t ua = staged<512>(c.staging, 8 * j + (c.lane & 7), upiece);
+      uint32_t g[4], u[4];
+      ldmatrix_x4_trans(ga, g);
+      ldmatrix_x4_trans(ua, u);
+      part[2 * j] = part[2 * j + 1] = 0.0f;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
+        const float a[2] = {__uint_as_float(r[b]), __uint_as_float(r[b + 1])};
+        // d_act is rounded to bf16 first, as the unfused reference stores it.
+        const uint32_t db = pack_bf16(w[0] * a[0], w[1] * a[1]);
+        float dg[2], du[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float d = e ? bf16_hi(db) : bf16_lo(db);
+          const float gt = e ? bf16_hi(g[s]) : bf16_lo(g[s]);
+          const float up = e ? bf16_hi(u[s]) : bf16_lo(u[s]);
+          const float sig = sigmoid_f(gt);
+          const float sl = gt * sig;
+          part[2 * j + e] += a[e] * (sl * up);
+          dg[e] = d * up * (sig + sl * (1.0f - sig));
+          du[e] = d * sl;
+        }
+        g[s] = pack_bf16(dg[0], dg[1]);
+        u[s] = pack_bf16(du[0], du[1]);
+      }
+      __syncwarp();  // all lanes' ldmatrix reads of these rows are done (they cross lanes) before the rows are overwritten
+      stmatrix_x4_trans(ga, g);
+      stmatrix_x4_trans(ua, u);
+    }
+    if (p.dwp != nullptr) {
+      // Sum over the 8 lanes that hold the same rows, then one partial per (row, 32 columns).
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) part[k] += __shfl_xor_sync(0xffffffffu, part[k], o);
+      }
+      if (c.lane < 4) {
+        float* out = p.dwp + static_cast<size_t>(row0) * p.dwp_tiles + (tl.n * 2 + c.rank) * 4 + c.q;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int t = 8 * (k >> 1) + 2 * c.lane + (k & 1);
+          if (t < nvalid) out[static_cast<size_t>(t) * p.dwp_tiles] = part[k];
+        }
+      }
+    }
+    group_sync(c.h);
+    flush_rows<512>(c.staging, c.gt, reinterpret_cast<uint8_t*>(p.out0 + static_cast<size_t>(row0) * p.ld0 + col),
+                    ld_bytes, nvalid);
+  }
+  if (c.h >= chunks) release();
+}
+
+// 152 registers per thread: 320 threads x 152 leave room in the register file for a 256-thread, 64-register copy CTA (the
+// dispatch put, the fp8 expansion), which has to become resident BESIDE this kernel for the overlap to happen.
+template <int MODE>
+__global__ void __cluster_dims__(2, 1, 1) __maxnreg__(152)
+row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap map_a,
+                const __grid_constant__ TokenMaps maps_b) {
+  using Traits = RowTraits<MODE>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  const uint32_t staging_base = smem_base + kRowStages * kRowStageBytes;
+  uint8_t* staging_gen = smem_gen + kRowStages * kRowStageBytes;
+  const uint32_t bar_base = staging_base + 2 * kGroupStaging;
+  // barriers: full[6], empty[6], acc_full[2], acc_empty[2], drain; then tmem slot, abort flag, early flag
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (kRowStages + s); };
+  auto acc_full_bar = [&](int s) { return bar_base + 8u * (2 * kRowStages + s); };
+  auto acc_empty_bar = [&](int s) { return bar_base + 8u * (2 * kRowStages + 2 + s); };
+  const uint32_t drain_bar = bar_base + 8u * (2 * kRowStages + 4);
+  constexpr int kSlotOff = 8 * (2 * kRowStages + 5);
+  static_assert(kSlotOff + 12 <= kSmemTailBytes, "barrier area too small");
+  const uint32_t tmem_slot = bar_base + kSlotOff;
+  uint8_t* tail_gen = staging_gen + 2 * kGroupStaging;
+  volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(tail_gen + kSlotOff);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tail_gen + kSlotOff + 4);
+  volatile int* early_flag = reinterpret_cast<volatile int*>(tail_gen + kSlotOff + 8);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_cta_rank());
+  const bool leader = rank == 0;
+  const bool counting = p.prof != nullptr;
+  auto prof_add = [&](int slot, long long v) {
+    atomicAdd(p.prof + static_cast<size_t>(blockIdx.x) * kProfSlots + slot, static_cast<unsigned long long>(v));
+  };
+
+  // A CTA that gives up tells its partner too (the flag sits at the same offset in both CTAs), so the partner's waits
+  // end at their next poll instead of running into their own limits.
+  const uint32_t partner_abort = map_to_cta(bar_base + kSlotOff + 4, static_cast<uint32_t>(rank ^ 1));
+  auto raise_abort = [&]() {
+    *abort_flag = 1;
+    st_shared_cluster_u32(partner_abort, 1u);
+  };
+
+  // The aligned layout must fit into what the launch provided. Both CTAs of a pair see the same offsets, so they
+  // leave together.
+  if (smem_base - smem_u32(smem_raw) > static_cast<uint32_t>(kSmemAlignSlack)) {
+    if (threadIdx.x == 0) report_status(p.status, kStatusBadIndex, kKernelGemm, MODE, -1, 1, kSmemAlignSlack,
+                                        smem_base - smem_u32(smem_raw));
+    return;
+  }
+  // An earlier kernel of this pass already gave up: both CTAs of the pair leave together (the leader decides).
+  if (threadIdx.x == 0 && leader) {
+    const uint32_t v = (p.status != nullptr && p.status->code != 0) ? 1u : 0u;
+    *early_flag = static_cast<int>(v);
+    st_shared_cluster_u32(map_to_cta(bar_base + kSlotOff + 8, 1), v);
+  }
+  cluster_sync_all();
+  if (*early_flag) return;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kRowStages; ++s) {
+      mbar_init(full_bar(s), 2);  // leader: one arrival from each CTA's producer (the peer's own barrier is not used)
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(acc_full_bar(s), 1);
+      mbar_init(acc_empty_bar(s), 16);  // eight epilogue warps in each CTA of the pair
+    }
+    mbar_init(drain_bar, 1);
+    *abort_flag = 0;
+    mbar_init_fence();
+    tma_prefetch_desc(&map_a);
+    for (int i = 0; i < 8; ++i) tma_prefetch_desc(&maps_b.by_width[i]);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(tmem_slot, 512);
+    tmem_relinquish_pair();
+  }
+  tcgen05_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers exist before anyone signals across the pair
+  tcgen05_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot_gen;
+
+  const int num_entries = p.plan[p.lay.off_num_tiles + p.slice];
+  const int num_tiles = num_entries * p.n_tiles;
+  const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+
+  if (warp == 0) {
+    // ================================ TMA producer (both CTAs) ==============================
+    // The whole warp walks the k-blocks in step (every lane waits on the stage's barrier, one elected lane issues the
+    // copies), so stage index, phase and addresses stay warp-uniform values.
+    uint32_t it = 0, ps = 0, pph = 0;
+    int waited_expert = -1;
+    long long empty_wait = 0;
+    bool dead = false;
+    // The next tile is decoded one iteration ahead, so its plan-table load is in flight while this tile runs.
+    RowTile nxt = {};
+    if (first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, num_entries);
+    for (int t = first_tile; t < num_tiles && !dead && !*abort_flag; t += tile_step) {
+      const RowTile tl = nxt;
+      if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, num_entries);
+      if constexpr (MODE == kModeSwiglu) {
+        if ((p.arrive != nullptr || p.ready != nullptr) && tl.g != waited_expert) {
+          if (!wait_expert_rows(p, tl.g, lane, abort_flag)) {
+            if (lane == 0) raise_abort();
+            break;
+          }
+          waited_expert = tl.g;
+        }
+      }
+      const CUtensorMap* map_b = &maps_b.by_width[(tl.ncols >> 5) - 1];
+      const uint32_t bytes = kRowStageBytesA + static_cast<uint32_t>(tl.ncols >> 1) * (kBlockK * 2);
+      for (int kb = 0; kb < p.k_blocks; ++kb) {
+        const long long w0 = counting ? clock64() : 0;
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(empty_bar(ps), pph ^ 1u, p.mbar_limit, abort_flag));
+        if (!ok) {
+          if (lane == 0) {
+            report_status(p.status, kStatusMbarTimeout, kKernelGemm, MODE, t, 1100 + ps, 0, 0);
+            raise_abort();
+          }
+          dead = true;
+          break;
+        }
+        if (counting) empty_wait += clock64() - w0;
+        if (elect_one()) {
+          const uint32_t fb = map_to_cta(full_bar(ps), 0);
+          mbar_expect_tx_cluster(fb, bytes);
+          issue_row_kblock<MODE>(p, tl, kb, rank, &map_a, map_b, smem_base + ps * kRowStageBytes, fb);
+        }
+        ++it;
+        if (++ps == kRowStages) { ps = 0; pph ^= 1u; }
+      }
+    }
+    __syncwarp();
+    if (counting && lane == 0) prof_add(kProfEmptyWait, empty_wait);
+    // Unwinding: no exit while a copy may still land in this CTA's shared memory (the leader's barriers see every stage
+    // of both CTAs; the peer leaves after the leader, at the cluster barrier below).
+    if (lane == 0 && *abort_flag && leader) {
+      for (int s = 0; s < kRowStages; ++s) {
+        if (it > static_cast<uint32_t>(s)) {
+          const uint32_t last = it - 1 - ((it - 1 - s) % kRowStages);
+          mbar_wait(full_bar(s), (last / kRowStages) & 1u, p.mbar_limit);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ================================ MMA issuer (leader) ===================================
+    constexpr uint32_t idesc0 = make_instr_desc_bf16(2 * kBlockM, 0, Traits::kAMn, false);
+    constexpr uint32_t kDescStepA = Traits::kAMn ? 2048u : 32u;
+    constexpr uint32_t kDescStepB = 32u;
+    uint32_t it = 0, tcount = 0, cs = 0, cph = 0;
+    long long full_wait = 0, acc_wait = 0;
+    const long long loop_c0 = counting ? clock64() : 0;
+    const uint64_t loop_n0 = counting ? global_timer_ns() : 0;
+    bool dead = false;
+    auto fail = [&](int t, int detail) {
+      if (lane == 0) {
+        report_status(p.status, kStatusMbarTimeout, kKernelGemm, MODE, t, detail, 0, 0);
+        raise_abort();
+      }
+      dead = true;
+    };
+    RowTile nxt = {};
+    if (leader && first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, num_entries);
+    for (int t = first_tile; leader && t < num_tiles && !dead && !*abort_flag; t += tile_step, ++tcount) {
+      const RowTile tl = nxt;
+      if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, num_entries);
+      const int as = tcount & 1;
+      const uint32_t aph = (tcount >> 1) & 1u;
+      const uint32_t tmem_d = tmem_base + as * kTileTokens;
+      const uint32_t idesc = idesc0 | (static_cast<uint32_t>(tl.ncols >> 3) << 17);
+      const long long w0 = counting ? clock64() : 0;
+      bool ok = __all_sync(0xffffffffu, mbar_wait(acc_empty_bar(as), aph ^ 1u, p.mbar_limit, abort_flag));
+      if (counting) acc_wait += clock64() - w0;
+      if (!ok) { fail(t, 1200 + as); break; }
+      tcgen05_fence_after_sync();
+      for (int kb = 0; kb < p.k_blocks; ++kb) {
+        const long long w1 = counting ? clock64() : 0;
+        ok = __all_sync(0xffffffffu, mbar_wait(full_bar(cs), cph, p.mbar_limit, abort_flag));
+        if (counting) full_wait += clock64() - w1;
+        if (!ok) { fail(t, 1300 + cs); break; }
+        tcgen05_fence_after_sync();
+        const uint32_t sa = smem_base + cs * kRowStageBytes;
+        const uint64_t da = Traits::kAMn ? make_smem_desc(sa, 8192, 1024) : make_smem_desc(sa, 16, 1024);
+        const uint64_t db = make_smem_desc(sa + kRowStageBytesA, 16, 1024);
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < kBlockK / kUmmaK; ++k)
+            umma_bf16_pair(tmem_d, da + ((k * kDescStepA) >> 4), db + ((k * kDescStepB) >> 4), idesc,
+                           (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit_pair_both(empty_bar(cs));
+        }
+        ++it;
+        if (++cs == kRowStages) { cs = 0; cph ^= 1u; }
+      }
+      if (dead) break;
+      if (elect_one()) umma_commit_pair_both(acc_full_bar(as));
+    }
+    __syncwarp();
+    if (counting && leader && lane == 0) {
+      prof_add(kProfLoopCycles, clock64() - loop_c0);
+      prof_add(kProfLoopNs, static_cast<long long>(global_timer_ns() - loop_n0));
+      prof_add(kProfFullWait, full_wait);
+      prof_add(kProfAccWait, acc_wait);
+      prof_add(kProfKBlocks, it);
+      prof_add(kProfTiles, tcount);
+    }
+    if (leader && *abort_flag) {
+      __syncwarp();
+      if (elect_one()) umma_commit_pair(drain_bar);
+      mbar_wait(drain_bar, 0, p.mbar_limit);
+    }
+  } else {
+    // ================================ epilogue (both CTAs) ==================================
+    GroupCtx c;
+    c.h = (warp - 2) >> 2;
+    c.q = warp & 3;  // TMEM lane quarter this warp may read
+    c.lane = lane;
+    c.gt = c.q * 32 + lane;
+    c.rank = rank;
+    c.staging = staging_base + c.h * kGroupStaging;
+    const uint32_t leader_acc_empty0 = map_to_cta(acc_empty_bar(0), 0);
+    // Combine modes: the row tables sit behind the 8 KB that a chunk is staged in.
+    uint32_t* s_dst = reinterpret_cast<uint32_t*>(staging_gen + c.h * kGroupStaging + 8192);
+    float* s_wts = reinterpret_cast<float*>(s_dst + kTileTokens / 2);
+    uint32_t tcount = 0, returned = 0;
+    long long epi_wait = 0;
+    RowTile nxt = {};
+    if (first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, num_entries);
+    for (int t = first_tile; t < num_tiles; t += tile_step, ++tcount) {
+      const RowTile tl = nxt;
+      if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, num_entries);
+      const int as = tcount & 1;
+      const uint32_t aph = (tcount >> 1) & 1u;
+      int4 first[8];
+      if constexpr (Traits::kCombine) {
+        // Where the rows of this group's chunks go (thread = row), worked out while the accumulator is being made.
+        group_sync(c.h);  // the previous tile's table has been used up
+        const int row = (c.gt >> 5) * 64 + c.h * 32 + lane;  // entry gt: row of chunk 2 (gt / 32) + h
+        int src = -1, pos = 0;
+        if (row < tl.nrows) resolve_source(p, tl.g, tl.row0 + row, &src, &pos);
+        s_dst[c.gt] = src >= 0 ? (static_cast<uint32_t>(src) << 27) | static_cast<uint32_t>(pos) : ~0u;
+        if constexpr (MODE == kModeDownFwd) s_wts[c.gt] = row < tl.nrows ? p.row_w[tl.row0 + row] : 0.0f;
+        // Lane s keeps the count of row pieces this warp accounts for at source rank s (`flush_returned`).
+        for (int s = 0; s < p.lay.P; ++s) {
+          const uint32_t cnt = __popc(__ballot_sync(0xffffffffu, src == s));
+          if (lane == s) returned += cnt;
+        }
+      }
+      if constexpr (MODE == kModeDswiglu) {
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(
+            p.in0 + static_cast<size_t>(tl.row0 + c.h * 32) * p.ld0 + 2 * (tl.n * kBlockN + rank * kBlockM)) + lane * 16;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int row = c.q + 4 * i;
+          first[i] = make_int4(0, 0, 0, 0);
+          if (c.h * 32 + row < tl.nrows) first[i] = *reinterpret_cast<const int4*>(src + static_cast<size_t>(row) * p.ld0 * 2);
+        }
+      }
+      const long long w0 = counting ? clock64() : 0;
+      const bool reached_acc = mbar_wait(acc_full_bar(as), aph, p.mbar_limit, abort_flag);
+      if (counting) epi_wait += clock64() - w0;
+      if (!reached_acc && lane == 0) {
+        report_status(p.status, kStatusMbarTimeout, kKernelGemm, MODE, t, 1500 + as, 0, 0);
+        raise_abort();
+      }
+      // One decision for the whole group: nobody may be left alone at a group barrier.
+      if (!group_vote(c.h, reached_acc)) break;
+      tcgen05_fence_after_sync();
+      const uint32_t tacc = tmem_base + (static_cast<uint32_t>(c.q * 32) << 16) + as * kTileTokens;
+      auto release = [&]() {  // this warp has read its last accumulator value
+        tcgen05_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(leader_acc_empty0 + 8u * as);
+      };
+      if constexpr (MODE == kModeSwiglu) swiglu_epilogue(p, tl, tacc, c, release);
+      else if constexpr (MODE == kModeDswiglu) dswiglu_epilogue(p, tl, tacc, c, first, release);
+      else combine_epilogue<MODE>(p, tl, tacc, c, s_dst, s_wts, release);
+    }
+    if (counting && warp == 2 && lane == 0) prof_add(kProfEpiWait, epi_wait);
+    if constexpr (Traits::kCombine) {
+      // The group's stores are all issued before any of its warps releases its counts (also on the unwind path).
+      group_sync(c.h);
+      if (lane < p.lay.P && returned > 0) {
+        __threadfence_system();
+        red_add_release_sys(p.peer_count[lane], returned);
+      }
+    }
+  }
+
+  // ================================ teardown ================================================
+  tcgen05_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();  // nobody frees TMEM or leaves while its partner may still signal or compute
+  if (warp == 1) {
+    tcgen05_fence_after_sync();
+    tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
+}  // namespace
+
+int row_gemm_smem_bytes() { return kRowSmemBytes; }
+
+void launch_row_gemm(int mode, const GemmParams& p, const CUtensorMap& map_a, const TokenMaps& maps_b, int grid,
+                     cudaStream_t stream) {
+  grid &= ~1;  // whole pairs only
+#define CEM_LAUNCH_ROW(M)                                                                                          \
+  case M: {                                                                                                        \
+    static const int resident = resident_pair_grid(row_gemm_kernel<M>, kRowThreads, kRowSmemBytes);                \
+    const int g = grid < resident ? grid : resident;                                                               \
+    g_pair_grid_used = g;                                                                                          \
+    row_gemm_kernel<M><<<g, kRowThreads, kRowSmemBytes, stream>>>(p, map_a, maps_b);                               \
+    break;                                                                                                         \
+  }
+  switch (mode) {
+    CEM_LAUNCH_ROW(kModeSwiglu)
+    CEM_LAUNCH_ROW(kModeDownFwd)
+    CEM_LAUNCH_ROW(kModeDswiglu)
+    CEM_LAUNCH_ROW(kModeDx)
+    default:
+      break;
+  }
+#undef CEM_LAUNCH_ROW
+}
+
+}  // namespace cem

@@ -91,12 +91,11 @@ __device__ void plan_phase_b_warps(int* plan, const PlanLayout& y, const int* se
   int num_slices = plan[0];
   if (num_slices > y.max_slices) num_slices = y.max_slices;
   for (int j = warp; j < y.max_slices; j += nwarps) {
-    int num_m = 0, num_g = 0, num_p = 0, chunks = 0;
+    int num_t = 0, num_g = 0, chunks = 0;
     if (j < num_slices) {
       const int lo = j * S, hi = lo + S;
-      int* mt = plan + y.off_mtiles + 4 * y.max_mtiles * j;
+      int* tt = plan + y.off_tiles + 4 * y.max_tiles * j;
       int* gt = plan + y.off_gtiles + 4 * y.max_gtiles * j;
-      int* pt = plan + y.off_ptiles + 4 * y.max_ptiles * j;
       for (int l0 = 0; l0 < L; l0 += 32) {
         const int l = l0 + lane;
         int es = 0, er = -1, first = 0, rows = 0;
@@ -106,29 +105,21 @@ __device__ void plan_phase_b_warps(int* plan, const PlanLayout& y, const int* se
           first = plan_clip(lo, es, es + er);
           rows = plan_clip(hi, es, es + er) - first;
         }
-        const int cm = (rows + kTileM - 1) / kTileM, cp = (rows + 2 * kTileM - 1) / (2 * kTileM);
+        const int ct = plan_num_tiles(rows);
         const int cg = (rows > 0 || (j == 0 && er == 0)) ? 1 : 0;
-        int tm, tp, tg;
-        const int em = num_m + warp_exclusive_scan(cm, lane, &tm);
-        const int ep = num_p + warp_exclusive_scan(cp, lane, &tp);
+        int tt_total, tg;
+        const int et = num_t + warp_exclusive_scan(ct, lane, &tt_total);
         const int eg = num_g + warp_exclusive_scan(cg, lane, &tg);
-        for (int t = 0; t < cm; ++t) {
-          const int off = t * kTileM;
-          reinterpret_cast<int4*>(mt)[em + t] =
-              make_int4(l, first - lo + off, rows - off < kTileM ? rows - off : kTileM, 0);
-        }
-        for (int t = 0; t < cp; ++t) {
-          const int off = t * 2 * kTileM;
-          reinterpret_cast<int4*>(pt)[ep + t] =
-              make_int4(l, first - lo + off, rows - off < 2 * kTileM ? rows - off : 2 * kTileM, 0);
+        for (int k = 0; k < ct; ++k) {
+          const int at = plan_tile_begin(rows, ct, k), n = plan_tile_begin(rows, ct, k + 1) - at;
+          reinterpret_cast<int4*>(tt)[et + k] = make_int4(l, first - lo + at, n, (n + kTileUnit - 1) / kTileUnit * kTileUnit);
         }
         if (cg) {
           reinterpret_cast<int4*>(gt)[eg] =
               rows > 0 ? make_int4(l, first - lo, rows, (es >= lo ? kGroupFirst : 0) | (es + er <= hi ? kGroupFinal : 0))
                        : make_int4(l, 0, 0, kGroupFirst | kGroupFinal);
         }
-        num_m += tm;
-        num_p += tp;
+        num_t += tt_total;
         num_g += tg;
       }
       int* put = plan + y.off_put + 4 * n * j;
@@ -148,10 +139,9 @@ __device__ void plan_phase_b_warps(int* plan, const PlanLayout& y, const int* se
       }
     }
     if (lane == 0) {
-      plan[y.off_num_mtiles + j] = num_m;
+      plan[y.off_num_tiles + j] = num_t;
       plan[y.off_num_gtiles + j] = num_g;
       plan[y.off_num_chunks + j] = chunks;
-      plan[y.off_num_ptiles + j] = num_p;
     }
   }
 }

@@ -16,9 +16,9 @@
 //   in_size[P*L]          i = s*L+l : counts[s][me][l]
 //   src_send_start[P*L]   i = s*L+l : start of that segment in source s's send order (combine target)
 //   expert_start[L], expert_rows[L]   my experts in my stream
-//   per slice j:  num_mtiles[j], num_gtiles[j], num_chunks[j]
-//                 mtiles[j][max_mtiles]  {expert, row0 (slice-relative), nrows, 0}         GEMM row tiles
-//                 ptiles[j][max_ptiles]  {expert, row0, nrows (<= 256), 0}                 row-tile PAIRS (2-CTA GEMMs)
+//   per slice j:  num_tiles[j], num_gtiles[j], num_chunks[j]
+//                 tiles[j][max_tiles]    {expert, row0 (slice-relative), nrows, ncols}     GEMM row tiles: <= 256 rows of one
+//                                                                                          expert, ncols = nrows up to 32
 //                 gtiles[j][max_gtiles]  {expert, row0, nrows, flags}                      weight-grad groups
 //                 put[j][P*L]            {send-order offset, rows, dest row, chunk prefix} my outgoing segments
 #pragma once
@@ -34,7 +34,8 @@
 namespace cem {
 
 constexpr int kPlanHeaderInts = 16;
-constexpr int kTileM = 128;         // rows of one GEMM row tile
+constexpr int kTileTokens = 256;    // most rows of one GEMM row tile
+constexpr int kTileUnit = 32;       // granularity of its MMA width
 constexpr int kPutChunkRows = 4;    // rows one warp moves between two arrival signals
 
 // gtile flags
@@ -42,11 +43,11 @@ constexpr int kGroupFirst = 1;  // the expert's rows begin in this slice: overwr
 constexpr int kGroupFinal = 2;  // the expert's rows end in this slice: write the final gradient
 
 struct PlanLayout {
-  int P, L, S, max_slices, max_mtiles, max_gtiles, max_ptiles;
+  int P, L, S, max_slices, max_tiles, max_gtiles;
   int off_send_start, off_seg_start, off_seg_size, off_in_start, off_in_size, off_src_send_start;
   int off_expert_start, off_expert_rows;
-  int off_num_mtiles, off_num_gtiles, off_num_chunks, off_num_ptiles;
-  int off_mtiles, off_gtiles, off_put, off_ptiles;
+  int off_num_tiles, off_num_gtiles, off_num_chunks;
+  int off_tiles, off_gtiles, off_put;
   int total;
 };
 
@@ -55,9 +56,8 @@ CEM_HD inline int plan_align4(int v) { return (v + 3) & ~3; }
 CEM_HD inline PlanLayout make_plan_layout(int P, int L, int S, int max_slices) {
   PlanLayout y;
   y.P = P; y.L = L; y.S = S; y.max_slices = max_slices;
-  y.max_mtiles = (S + kTileM - 1) / kTileM + L;
+  y.max_tiles = (S + kTileTokens - 1) / kTileTokens + L;
   y.max_gtiles = L;
-  y.max_ptiles = (S + 2 * kTileM - 1) / (2 * kTileM) + L;
   const int n = P * L;
   int o = kPlanHeaderInts;
   y.off_send_start = o; o += plan_align4(n);
@@ -68,19 +68,29 @@ CEM_HD inline PlanLayout make_plan_layout(int P, int L, int S, int max_slices) {
   y.off_src_send_start = o; o += plan_align4(n);
   y.off_expert_start = o; o += plan_align4(L);
   y.off_expert_rows = o; o += plan_align4(L);
-  y.off_num_mtiles = o; o += plan_align4(max_slices);
+  y.off_num_tiles = o; o += plan_align4(max_slices);
   y.off_num_gtiles = o; o += plan_align4(max_slices);
   y.off_num_chunks = o; o += plan_align4(max_slices);
-  y.off_num_ptiles = o; o += plan_align4(max_slices);
-  y.off_mtiles = o; o += 4 * y.max_mtiles * max_slices;
+  y.off_tiles = o; o += 4 * y.max_tiles * max_slices;
   y.off_gtiles = o; o += 4 * y.max_gtiles * max_slices;
   y.off_put = o; o += 4 * n * max_slices;
-  y.off_ptiles = o; o += 4 * y.max_ptiles * max_slices;
   y.total = o;
   return y;
 }
 
 CEM_HD inline int plan_clip(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
+
+// An expert's `rows` rows of a slice are cut into the fewest tiles of at most 256 rows, as equal as multiples of 32 allow:
+// 270 rows are 160 + 110 (MMA widths 160 + 128), not 256 + 14. Equal tiles keep every tile's MMA time above the time its
+// weight columns take to load, and all tiles of a slice about the same length.
+CEM_HD inline int plan_num_tiles(int rows) { return (rows + kTileTokens - 1) / kTileTokens; }
+
+// First row of tile `k` (of `tiles`), k in [0, tiles]; the last tile ends at `rows`.
+CEM_HD inline int plan_tile_begin(int rows, int tiles, int k) {
+  const int units = (rows + kTileUnit - 1) / kTileUnit, base = units / tiles, rem = units - base * tiles;
+  const int at = kTileUnit * (k * base + (k < rem ? k : rem));
+  return at < rows ? at : rows;
+}
 
 // counts[s][r][l] -> count
 CEM_HD inline int plan_count(const int* counts, int P, int L, int s, int r, int l) {
@@ -151,32 +161,24 @@ CEM_HD inline void plan_phase_b(int* plan, const PlanLayout& y, int tid, int nth
   int num_slices = plan[0];
   if (num_slices > y.max_slices) num_slices = y.max_slices;
   for (int j = tid; j < y.max_slices; j += nthreads) {
-    int num_m = 0, num_g = 0, num_p = 0, chunks = 0;
+    int num_t = 0, num_g = 0, chunks = 0;
     if (j < num_slices) {
       const int lo = j * S, hi = lo + S;
-      int* mt = plan + y.off_mtiles + 4 * y.max_mtiles * j;
+      int* tt = plan + y.off_tiles + 4 * y.max_tiles * j;
       int* gt = plan + y.off_gtiles + 4 * y.max_gtiles * j;
-      int* pt = plan + y.off_ptiles + 4 * y.max_ptiles * j;
       for (int l = 0; l < L; ++l) {
         const int es = plan[y.off_expert_start + l], er = plan[y.off_expert_rows + l];
         const int first = plan_clip(lo, es, es + er), last = plan_clip(hi, es, es + er);
         const int rows = last - first;
         if (rows > 0) {
-          for (int off = 0; off < rows; off += kTileM) {
-            mt[4 * num_m + 0] = l;
-            mt[4 * num_m + 1] = first - lo + off;
-            mt[4 * num_m + 2] = rows - off < kTileM ? rows - off : kTileM;
-            mt[4 * num_m + 3] = 0;
-            ++num_m;
-          }
-          // Pairs of consecutive row tiles of one expert share its weights in a 2-CTA MMA; an odd
-          // last tile is a pair whose second half is empty.
-          for (int off = 0; off < rows; off += 2 * kTileM) {
-            pt[4 * num_p + 0] = l;
-            pt[4 * num_p + 1] = first - lo + off;
-            pt[4 * num_p + 2] = rows - off < 2 * kTileM ? rows - off : 2 * kTileM;
-            pt[4 * num_p + 3] = 0;
-            ++num_p;
+          const int tiles = plan_num_tiles(rows);
+          for (int k = 0; k < tiles; ++k) {
+            const int at = plan_tile_begin(rows, tiles, k), n = plan_tile_begin(rows, tiles, k + 1) - at;
+            tt[4 * num_t + 0] = l;
+            tt[4 * num_t + 1] = first - lo + at;
+            tt[4 * num_t + 2] = n;
+            tt[4 * num_t + 3] = (n + kTileUnit - 1) / kTileUnit * kTileUnit;
+            ++num_t;
           }
           gt[4 * num_g + 0] = l;
           gt[4 * num_g + 1] = first - lo;
@@ -203,10 +205,9 @@ CEM_HD inline void plan_phase_b(int* plan, const PlanLayout& y, int tid, int nth
         chunks += (last - first + kPutChunkRows - 1) / kPutChunkRows;
       }
     }
-    plan[y.off_num_mtiles + j] = num_m;
+    plan[y.off_num_tiles + j] = num_t;
     plan[y.off_num_gtiles + j] = num_g;
     plan[y.off_num_chunks + j] = chunks;
-    plan[y.off_num_ptiles + j] = num_p;
   }
 }
 

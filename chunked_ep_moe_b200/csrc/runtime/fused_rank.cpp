@@ -78,24 +78,20 @@ ArenaLayout make_arena_layout(int P, int L, int S, int D, int tk_cap, bool fp8) 
 
 FusedRank::FusedRank(int P, int L, int me, int S, int D, int F, int K, int stripe, int tk_cap, int max_slices,
                      int num_sms, bool fp8, int64_t arena, std::vector<int64_t> peer_arenas, bool use_comm_stream,
-                     int64_t spin_limit, int put_blocks, bool cta_pairs, bool tgmm_pairs)
+                     int64_t spin_limit, int put_blocks)
     : P_(P), L_(L), me_(me), S_(S), D_(D), F_(F), K_(K), stripe_(stripe), tk_cap_(tk_cap), max_slices_(max_slices),
-      num_sms_(num_sms), put_blocks_(put_blocks), fp8_(fp8), use_comm_stream_(use_comm_stream),
-      cta_pairs_(cta_pairs && num_sms >= 2), tgmm_pairs_(tgmm_pairs && num_sms >= 2) {
+      num_sms_(num_sms), put_blocks_(put_blocks), fp8_(fp8), use_comm_stream_(use_comm_stream) {
   expect(P >= 1 && L >= 1 && me >= 0 && me < P, "bad rank geometry");
   expect(static_cast<int>(peer_arenas.size()) == P, "need one arena pointer per rank");
   expect(P <= 32, "at most 32 expert-parallel ranks (one warp lane watches one source)");
   expect(P * L <= 1024, "at most 1024 experts");
+  expect(tk_cap < (1 << 27), "at most 2^27 token copies per rank (a returned row's position has 27 bits)");
   expect(D % 256 == 0, "fused kernels need D % 256 == 0");
   expect(F % 256 == 0, "fused kernels need F % 256 == 0");
   expect(stripe == 32 || stripe == 64 || stripe == 128, "fused kernels need stripe_width in {32, 64, 128}");
   expect(S % 8 == 0 && S >= 8, "fused kernels need slice_size % 8 == 0");
   expect(!fp8 || D % 128 == 0, "fp8 wire needs D % 128 == 0");
   spin_limit_ = static_cast<uint32_t>(spin_limit);
-  if (const char* v = std::getenv("CEM_GEMM_EXCLUSIVE_SM")) g_gemm_extra_smem = std::atoi(v) != 0 ? 1024 : 0;
-  if (const char* v = std::getenv("CEM_PAIR_SUSPEND")) g_pair_suspend_waits = std::atoi(v) != 0 ? 1 : 0;
-  if (const char* v = std::getenv("CEM_RET_BLOCKED")) ret_blocked_ = std::atoi(v) != 0;
-  if (const char* v = std::getenv("CEM_RET_LSU")) ret_lsu_ = std::atoi(v) != 0;
   mbar_limit_ = 20u * 1000u * 1000u;  // microseconds: longer than any legitimate wait on another rank
   lay_ = make_plan_layout(P, L, S, max_slices);
   arena_lay_ = make_arena_layout(P, L, S, D, tk_cap, fp8);
@@ -109,7 +105,7 @@ FusedRank::FusedRank(int P, int L, int me, int S, int D, int F, int K, int strip
     act_[q] = torch::zeros({S, F}, bf16);
     h_[q] = torch::zeros({S, 2 * F}, bf16);
     dh_[q] = torch::zeros({S, 2 * F}, bf16);
-    dwp_[q] = torch::zeros({S, F / 256}, f32);
+    dwp_[q] = torch::zeros({S, F / 32}, f32);
   }
   carry_up_ = torch::zeros({2, D, 2 * F}, f32);
   carry_down_ = torch::zeros({2, F, D}, f32);
@@ -146,22 +142,21 @@ FusedRank::FusedRank(int P, int L, int me, int S, int D, int F, int K, int strip
   }
   tables_ = torch::from_blob(host.data(), {static_cast<int64_t>(kNumTables), P}, torch::kInt64).clone().to(torch::kCUDA);
 
-  // TMA descriptors of the local buffers. K-major A tiles are 128 rows, MN-major tiles 64 rows (k) of several
-  // 64-column chunks brought by one 3-D copy (a CTA of a pair loads half of the 256-wide column tile).
-  const uint32_t mn_chunks_b = tgmm_pairs_ ? 2 : 4;  // the MN-major maps of local buffers feed the weight-gradient mode
+  // TMA descriptors of the local buffers: row-wise operands by tile width, weight-gradient operands as 64 rows of two
+  // 64-column chunks brought by one 3-D copy (what each CTA of a pair loads).
   for (int b = 0; b < 2; ++b) {
     const void* xb = arena_ + arena_lay_.xbuf + static_cast<size_t>(b) * S * D * 2;
-    map_x_k_[b] = make_bf16_map_2d(xb, S, D, 128);
-    map_x_mn_[b] = make_bf16_map_chunked(xb, S, D, 64, 2);  // weight-gradient lhs: 128 columns per tile
     const void* gb = arena_ + arena_lay_.gbuf + static_cast<size_t>(b) * S * D * 2;
-    map_g_k_[b] = make_bf16_map_2d(gb, S, D, 128);
-    map_g_mn_[b] = make_bf16_map_chunked(gb, S, D, 64, mn_chunks_b);  // weight-gradient rhs
+    map_x_[b] = make_token_maps(xb, S, D);
+    map_x_mn_[b] = make_bf16_map_chunked(xb, S, D, 64, 2);
+    map_g_[b] = make_token_maps(gb, S, D);
+    map_g_mn_[b] = make_bf16_map_chunked(gb, S, D, 64, 2);
   }
   for (int q = 0; q < 2; ++q) {
-    map_act_k_[q] = make_bf16_map_2d(act_[q].data_ptr(), S, F, 128);
+    map_act_[q] = make_token_maps(act_[q].data_ptr(), S, F);
     map_act_mn_[q] = make_bf16_map_chunked(act_[q].data_ptr(), S, F, 64, 2);
-    map_dh_k_[q] = make_bf16_map_2d(dh_[q].data_ptr(), S, 2 * F, 128);
-    map_dh_mn_[q] = make_bf16_map_chunked(dh_[q].data_ptr(), S, 2 * F, 64, mn_chunks_b);
+    map_dh_[q] = make_token_maps(dh_[q].data_ptr(), S, 2 * F);
+    map_dh_mn_[q] = make_bf16_map_chunked(dh_[q].data_ptr(), S, 2 * F, 64, 2);
   }
 
   if (use_comm_stream_) {
@@ -290,8 +285,8 @@ int64_t FusedRank::begin_forward_async(torch::Tensor expert_ids, torch::Tensor p
   cuda_check(cudaMemcpyAsync(host_header_ + 16, status_.data_ptr(), 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, st),
              "status copy");
   cuda_check(cudaEventRecord(ev_header_, st), "event record");
-  // any slice below the workspace's capacity may be launched until resolved; D/256 pieces per row come back
-  begin_pass(plan, max_slices_, tk, D_ / kBlockN);
+  // any slice below the workspace's capacity may be launched until resolved; D/128 pieces per row come back
+  begin_pass(plan, max_slices_, tk, D_ / kCombineCols);
   return last_slices_ < 0 ? -1 : std::min<int64_t>(last_slices_, max_slices_);
 }
 
@@ -349,7 +344,7 @@ int64_t FusedRank::begin_backward(torch::Tensor plan, int64_t known_slices, int6
     cur_slices_ = host_header_[0];
     cur_rows_ = host_header_[5];
   }
-  begin_pass(plan, cur_slices_, cur_rows_, D_ / kBlockN + 1);  // per row: the pieces of dx and the d_weight scalar
+  begin_pass(plan, cur_slices_, cur_rows_, D_ / kCombineCols + 1);  // per row: the pieces of dx and the d_weight scalar
   return cur_slices_;
 }
 
@@ -447,6 +442,8 @@ const CUtensorMap& FusedRank::weight_map(const torch::Tensor& w, uint32_t box_ro
   return it->second;
 }
 
+const CUtensorMap& FusedRank::up_map(const torch::Tensor& w_up) { return weight_map(w_up, 64, stripe_ == 128 ? 1 : 2); }
+
 void FusedRank::dequant(const int* plan, int j, int b, bool with_g, cudaStream_t st) {
   // Rows arrived as e4m3 + block scales: expand them into the bf16 slice buffers the GEMMs read.
   DequantParams d{};
@@ -484,16 +481,25 @@ void FusedRank::set_pipeline_counters(c10::optional<torch::Tensor> counters) {
   prof_ = t;
 }
 
-void FusedRank::launch_gemm(int mode, const GemmParams& p0, const CUtensorMap& a, const CUtensorMap& b,
-                            cudaStream_t st, const CUtensorMap* c, int spare_sms) {
-  GemmParams p = p0;
+void FusedRank::count_pipeline(int mode, GemmParams* p) {
   if (prof_.defined())
-    p.prof = reinterpret_cast<unsigned long long*>(prof_.data_ptr<int64_t>()) +
-             static_cast<size_t>(mode) * prof_.size(1) * kProfSlots;
-  const CUtensorMap& out = c != nullptr ? *c : a;
-  const int grid = std::max(2, num_sms_ - spare_sms);
-  if (mode == kModeTgmm ? tgmm_pairs_ : cta_pairs_) launch_grouped_gemm_pair(mode, p, a, b, out, grid, st);
-  else launch_grouped_gemm(mode, p, a, b, out, grid, st);
+    p->prof = reinterpret_cast<unsigned long long*>(prof_.data_ptr<int64_t>()) +
+              static_cast<size_t>(mode) * prof_.size(1) * kProfSlots;
+}
+
+void FusedRank::row_gemm(int mode, const GemmParams& p0, const CUtensorMap& weights, const TokenMaps& rows,
+                         cudaStream_t st, int spare_sms) {
+  GemmParams p = p0;
+  count_pipeline(mode, &p);
+  launch_row_gemm(mode, p, weights, rows, std::max(2, num_sms_ - spare_sms), st);
+  ++launches_;
+}
+
+void FusedRank::weight_grad(const GemmParams& p0, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& out,
+                            cudaStream_t st) {
+  GemmParams p = p0;
+  count_pipeline(kModeTgmm, &p);
+  launch_weight_grad(p, a, b, out, std::max(2, num_sms_), st);
   ++launches_;
 }
 
@@ -546,8 +552,7 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
     // expansion kernel, and it only starts once the expansion of the PREVIOUS slice has finished, so that at most one
     // kernel is ever waiting for an expansion that still needs SMs.
     if (fp8_ && async && j >= 1) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(j - 1) % 4], 0), "wait expansion");
-    launch_gemm(kModeSwiglu, p, map_x_k_[b], weight_map(w_up, 64, cta_pairs_ ? 2 : 4), st, nullptr,
-                fp8_ && async ? kExpandSms : 0);
+    row_gemm(kModeSwiglu, p, up_map(w_up), map_x_[b], st, fp8_ && async ? kExpandSms : 0);
   }
   {
     GemmParams p = base_params(pl, static_cast<int>(j));
@@ -556,12 +561,9 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
     p.b_group_rows = F_;
     p.row_w = reinterpret_cast<const float*>(arena_ + arena_lay_.wbuf) + static_cast<size_t>(b) * S_;
     p.peer_rows = table<__nv_bfloat16>(kTabRet);
-    p.ret_blocked = ret_blocked_ ? 1 : 0;
-    p.ret_lsu = ret_lsu_ ? 1 : 0;
-    p.ret_rows = tk_cap_;
     p.peer_count = table<uint32_t>(kTabCount);
     p.ld0 = D_;
-    launch_gemm(kModeDownFwd, p, map_act_k_[q], weight_map(w_down, 64, cta_pairs_ ? 2 : 4), st);
+    row_gemm(kModeDownFwd, p, weight_map(w_down, 64, 2), map_act_[q], st);
   }
   if (async) {
     cuda_check(cudaEventRecord(ev_down_[q], st), "event record");
@@ -590,7 +592,7 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
   const int b = static_cast<int>(seq & 1u);
   const int* pl = plan.data_ptr<int>();
   const int par = static_cast<int>(j & 1);
-  const int dwp_tiles = F_ / kBlockN;
+  const int dwp_tiles = F_ / 32;
   if (fp8_ && !async) dequant(pl, static_cast<int>(j), b, /*with_g=*/true, st);  // lockstep: every put is done
   // Remat: h and w * act. y is not recomputed: d_weight = <g, act Wd> = <g Wd^T, act> is a by-product of the next GEMM, so
   // the down-projection GEMM that used to form <g, y> and w * g here (8 % of a step's FLOPs, 230 us per 8192-row slice at
@@ -614,8 +616,7 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     // expansion kernel, and it only starts once the expansion of the PREVIOUS slice has finished, so that at most one
     // kernel is ever waiting for an expansion that still needs SMs.
     if (fp8_ && async && j >= 1) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(j - 1) % 4], 0), "wait expansion");
-    launch_gemm(kModeSwiglu, p, map_x_k_[b], weight_map(w_up, 64, cta_pairs_ ? 2 : 4), st, nullptr,
-                fp8_ && async ? kExpandSms : 0);
+    row_gemm(kModeSwiglu, p, up_map(w_up), map_x_[b], st, fp8_ && async ? kExpandSms : 0);
   }
   if (async) {
     cuda_check(cudaEventRecord(ev_up_[q], st), "event record");
@@ -632,7 +633,7 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     p.ld0 = 2 * F_;
     p.dwp = dwp_[q].data_ptr<float>();
     p.dwp_tiles = dwp_tiles;
-    launch_gemm(kModeDswiglu, p, map_g_k_[b], weight_map(w_down, cta_pairs_ ? 128 : 256), st);
+    row_gemm(kModeDswiglu, p, weight_map(w_down, 128), map_g_[b], st);
   }
   if (async) {
     cuda_check(cudaEventRecord(ev_ds_[q], st), "event record");
@@ -645,7 +646,7 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     p.carry_in = carry_down_.data_ptr<float>() + static_cast<size_t>(par ^ 1) * F_ * D_;
     p.carry_out = carry_down_.data_ptr<float>() + static_cast<size_t>(par) * F_ * D_;
     p.grad_out = reinterpret_cast<__nv_bfloat16*>(dw_down.data_ptr());
-    launch_gemm(kModeTgmm, p, map_act_mn_[q], map_g_mn_[b], aux, &weight_map(dw_down, 32));
+    weight_grad(p, map_act_mn_[q], map_g_mn_[b], weight_map(dw_down, 32), aux);
   }
   if (async) {
     cuda_check(cudaEventRecord(ev_tgd_[q], aux), "event record");
@@ -670,12 +671,9 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     p.k_blocks = 2 * F_ / kBlockK;
     p.b_group_rows = D_;
     p.peer_rows = table<__nv_bfloat16>(kTabRet);
-    p.ret_blocked = ret_blocked_ ? 1 : 0;
-    p.ret_lsu = ret_lsu_ ? 1 : 0;
-    p.ret_rows = tk_cap_;
     p.peer_count = table<uint32_t>(kTabCount);
     p.ld0 = D_;
-    launch_gemm(kModeDx, p, map_dh_k_[q], weight_map(w_up, cta_pairs_ ? 128 : 256), st);
+    row_gemm(kModeDx, p, weight_map(w_up, 128), map_dh_[q], st);
   }
   if (async) cuda_check(cudaEventRecord(ev_dx_[q], st), "event record");
   {  // dW_up[g] = x^T dh
@@ -685,7 +683,7 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     p.carry_in = carry_up_.data_ptr<float>() + static_cast<size_t>(par ^ 1) * D_ * 2 * F_;
     p.carry_out = carry_up_.data_ptr<float>() + static_cast<size_t>(par) * D_ * 2 * F_;
     p.grad_out = reinterpret_cast<__nv_bfloat16*>(dw_up.data_ptr());
-    launch_gemm(kModeTgmm, p, map_x_mn_[b], map_dh_mn_[q], aux, &weight_map(dw_up, 32));
+    weight_grad(p, map_x_mn_[b], map_dh_mn_[q], weight_map(dw_up, 32), aux);
   }
   if (async) cuda_check(cudaEventRecord(ev_tgu_[q], aux), "event record");
   launch_slice_done(table<uint32_t>(kTabCredit), P_, me_, seq, aux);
@@ -722,8 +720,6 @@ void FusedRank::finish_forward(torch::Tensor inv_order, torch::Tensor out) {
   c.num_tokens = static_cast<int>(out.size(0));
   c.top_k = K_;
   c.hidden = D_;
-  c.blocked = ret_blocked_ ? 1 : 0;
-  c.ret_rows = tk_cap_;
   c.count = reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.ret_count);
   c.target = ret_target_;
   c.spin_limit = spin_limit_;
@@ -750,8 +746,6 @@ void FusedRank::finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch
   c.num_tokens = static_cast<int>(dx.size(0));
   c.top_k = K_;
   c.hidden = D_;
-  c.blocked = ret_blocked_ ? 1 : 0;
-  c.ret_rows = tk_cap_;
   c.count = reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.ret_count);
   c.target = ret_target_;
   c.spin_limit = spin_limit_;

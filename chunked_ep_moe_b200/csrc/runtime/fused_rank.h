@@ -41,7 +41,7 @@ class FusedRank {
  public:
   FusedRank(int P, int L, int me, int S, int D, int F, int K, int stripe, int tk_cap, int max_slices, int num_sms,
             bool fp8, int64_t arena, std::vector<int64_t> peer_arenas, bool use_comm_stream, int64_t spin_limit,
-            int put_blocks, bool cta_pairs, bool tgmm_pairs);
+            int put_blocks);
   ~FusedRank();
 
   // Forward pass set-up: sort, traffic exchange, plan tables, arrival targets. `plan`, `order`,
@@ -100,16 +100,15 @@ class FusedRank {
   // `chunks` > 0: the MN-major description (64-column chunks, `chunks` of them per copy); 0: plain 2-D boxes.
   const CUtensorMap& weight_map(const torch::Tensor& w, uint32_t box_rows, uint32_t chunks = 0);
   void dequant(const int* plan, int j, int b, bool with_g, cudaStream_t st);
-  // `c`: the output's tensor map (weight-gradient mode: tiled stores of the bf16 gradient); null otherwise.
-  void launch_gemm(int mode, const GemmParams& p, const CUtensorMap& a, const CUtensorMap& b, cudaStream_t st,
-                   const CUtensorMap* c = nullptr, int spare_sms = 0);
+  const CUtensorMap& up_map(const torch::Tensor& w_up);  // w_up as the SwiGLU mode reads it
+  void count_pipeline(int mode, GemmParams* p);
+  void row_gemm(int mode, const GemmParams& p, const CUtensorMap& weights, const TokenMaps& rows, cudaStream_t st,
+                int spare_sms = 0);
+  void weight_grad(const GemmParams& p, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& out,
+                   cudaStream_t st);
 
   int P_, L_, me_, S_, D_, F_, K_, stripe_, tk_cap_, max_slices_, num_sms_, put_blocks_;
-  // `cta_pairs_`: the row-wise GEMM modes run as CTA pairs (256-row tiles). `tgmm_pairs_`: the weight-gradient mode
-  // does; its pairs split the dense feature dimension, so they cost no token padding and are on by default.
-  bool fp8_, use_comm_stream_, cta_pairs_, tgmm_pairs_;
-  bool ret_lsu_ = false;      // CEM_RET_LSU: combine epilogues write staged rows with vector stores, not bulk stores
-  bool ret_blocked_ = false;  // CEM_RET_BLOCKED: return buffers kept column tile by column tile (every rank alike)
+  bool fp8_, use_comm_stream_;
   uint32_t spin_limit_, mbar_limit_;
   PlanLayout lay_;
   ArenaLayout arena_lay_;
@@ -127,8 +126,8 @@ class FusedRank {
   template <typename T>
   T* const* table(int t) const { return reinterpret_cast<T* const*>(tables_.data_ptr<int64_t>() + t * P_); }
 
-  CUtensorMap map_x_k_[2], map_x_mn_[2], map_act_k_[2], map_act_mn_[2], map_g_k_[2], map_g_mn_[2], map_dh_k_[2],
-      map_dh_mn_[2];
+  TokenMaps map_x_[2], map_g_[2], map_act_[2], map_dh_[2];
+  CUtensorMap map_x_mn_[2], map_g_mn_[2], map_act_mn_[2], map_dh_mn_[2];
   std::map<std::tuple<const void*, uint32_t, int64_t, int64_t>, CUtensorMap> weight_maps_;
 
   cudaStream_t comm_stream_ = nullptr, aux_stream_ = nullptr, chain_[2] = {};

@@ -2,6 +2,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 
@@ -32,8 +33,8 @@ cudaStream_t stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 }  // namespace
 
-KernelRunner::KernelRunner(int L, int S, int stripe, int num_sms, bool cta_pairs)
-    : L_(L), S_(S), stripe_(stripe), num_sms_(num_sms), pairs_(cta_pairs && num_sms >= 2) {
+KernelRunner::KernelRunner(int L, int S, int stripe, int num_sms)
+    : L_(L), S_(S), stripe_(stripe), num_sms_(std::max(2, num_sms)) {
   need(L >= 1 && L <= 1024, "1 <= L <= 1024");
   need(S >= 8 && S % 8 == 0, "S must be a positive multiple of 8");
   need(stripe == 32 || stripe == 64 || stripe == 128, "stripe must be 32, 64 or 128");
@@ -77,13 +78,6 @@ GemmParams KernelRunner::base() const {
   return p;
 }
 
-void KernelRunner::launch(int mode, const GemmParams& p, const CUtensorMap& a, const CUtensorMap& b,
-                          const CUtensorMap* c) {
-  const CUtensorMap& out = c != nullptr ? *c : a;
-  if (pairs_) launch_grouped_gemm_pair(mode, p, a, b, out, num_sms_, stream());
-  else launch_grouped_gemm(mode, p, a, b, out, num_sms_, stream());
-}
-
 void KernelRunner::gmm_swiglu(torch::Tensor x, torch::Tensor w_up, torch::Tensor act, c10::optional<torch::Tensor> h) {
   need_weights(w_up, L_, "w_up");
   const int64_t D = w_up.size(1), F2 = w_up.size(2);
@@ -99,9 +93,8 @@ void KernelRunner::gmm_swiglu(torch::Tensor x, torch::Tensor w_up, torch::Tensor
   p.ld0 = static_cast<int>(F2 / 2);
   p.out1 = h.has_value() ? reinterpret_cast<__nv_bfloat16*>(h->data_ptr()) : nullptr;
   p.ld1 = static_cast<int>(F2);
-  const CUtensorMap a = make_bf16_map_2d(x.data_ptr(), S_, D, 128);
-  const CUtensorMap b = make_bf16_map_chunked(w_up.data_ptr(), static_cast<uint64_t>(L_) * D, F2, 64, pairs_ ? 2 : 4);
-  launch(kModeSwiglu, p, a, b, nullptr);
+  const CUtensorMap w = make_bf16_map_chunked(w_up.data_ptr(), static_cast<uint64_t>(L_) * D, F2, 64, stripe_ == 128 ? 1 : 2);
+  launch_row_gemm(kModeSwiglu, p, w, make_token_maps(x.data_ptr(), S_, D), num_sms_, stream());
 }
 
 void KernelRunner::gmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out, bool transpose_rhs) {
@@ -119,16 +112,16 @@ void KernelRunner::gmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out, 
   p.ld0 = static_cast<int>(N);
   p.peer_rows = reinterpret_cast<__nv_bfloat16* const*>(table_.data_ptr<int64_t>());
   p.peer_count = reinterpret_cast<uint32_t* const*>(table_.data_ptr<int64_t>() + 1);
-  const CUtensorMap a = make_bf16_map_2d(lhs.data_ptr(), S_, K, 128);
+  const TokenMaps rows = make_token_maps(lhs.data_ptr(), S_, K);
   if (!transpose_rhs) {
     p.b_group_rows = static_cast<int>(K);
     p.row_w = ones_.data_ptr<float>();
-    const CUtensorMap b = make_bf16_map_chunked(rhs.data_ptr(), static_cast<uint64_t>(L_) * K, N, 64, pairs_ ? 2 : 4);
-    launch(kModeDownFwd, p, a, b, nullptr);
+    const CUtensorMap w = make_bf16_map_chunked(rhs.data_ptr(), static_cast<uint64_t>(L_) * K, N, 64, 2);
+    launch_row_gemm(kModeDownFwd, p, w, rows, num_sms_, stream());
   } else {
     p.b_group_rows = static_cast<int>(N);
-    const CUtensorMap b = make_bf16_map_2d(rhs.data_ptr(), static_cast<uint64_t>(L_) * N, K, pairs_ ? 128 : 256);
-    launch(kModeDx, p, a, b, nullptr);
+    const CUtensorMap w = make_bf16_map_2d(rhs.data_ptr(), static_cast<uint64_t>(L_) * N, K, 128);
+    launch_row_gemm(kModeDx, p, w, rows, num_sms_, stream());
   }
 }
 
@@ -145,19 +138,13 @@ void KernelRunner::gmm_down_dw(torch::Tensor act, torch::Tensor w_down, torch::T
   need(dwp.is_cuda() && dwp.scalar_type() == torch::kFloat32 && dwp.is_contiguous() && dwp.dim() == 2 &&
            dwp.size(0) == S_ && dwp.size(1) == D / kBlockN,
        "dwp must be a contiguous CUDA fp32 [S, D/256] tensor");
-  GemmParams p = base();
-  p.n_tiles = static_cast<int>(D / kBlockN);
-  p.k_blocks = static_cast<int>(F / kBlockK);
-  p.b_group_rows = static_cast<int>(F);
-  p.row_w = row_w.data_ptr<float>();
-  p.in0 = reinterpret_cast<const __nv_bfloat16*>(g.data_ptr());
-  p.out0 = reinterpret_cast<__nv_bfloat16*>(dy.data_ptr());
-  p.ld0 = static_cast<int>(D);
-  p.dwp = dwp.data_ptr<float>();
-  p.dwp_tiles = static_cast<int>(D / kBlockN);
-  const CUtensorMap a = make_bf16_map_2d(act.data_ptr(), S_, F, 128);
-  const CUtensorMap b = make_bf16_map_chunked(w_down.data_ptr(), static_cast<uint64_t>(L_) * F, D, 64, pairs_ ? 2 : 4);
-  launch(kModeDownDw, p, a, b, nullptr);
+  // The grouped GEMM, then plain tensor ops (the layer itself forms neither y nor w * g, see FusedRank::compute_backward).
+  torch::Tensor y = torch::zeros_like(g);
+  gmm(act, w_down, y, false);
+  const torch::Tensor live = (torch::arange(S_, counts_.options()) < counts_.sum()).unsqueeze(1);
+  const torch::Tensor gf = g.to(torch::kFloat32);
+  dy.copy_(torch::where(live, (row_w.unsqueeze(1) * gf).to(torch::kBFloat16), dy));
+  dwp.copy_(torch::where(live, (gf * y.to(torch::kFloat32)).view({S_, D / kBlockN, kBlockN}).sum(2), dwp));
 }
 
 void KernelRunner::gmm_dswiglu(torch::Tensor dy, torch::Tensor w_down, torch::Tensor h, torch::Tensor dh) {
@@ -174,9 +161,8 @@ void KernelRunner::gmm_dswiglu(torch::Tensor dy, torch::Tensor w_down, torch::Te
   p.in0 = reinterpret_cast<const __nv_bfloat16*>(h.data_ptr());
   p.out0 = reinterpret_cast<__nv_bfloat16*>(dh.data_ptr());
   p.ld0 = static_cast<int>(2 * F);
-  const CUtensorMap a = make_bf16_map_2d(dy.data_ptr(), S_, D, 128);
-  const CUtensorMap b = make_bf16_map_2d(w_down.data_ptr(), static_cast<uint64_t>(L_) * F, D, pairs_ ? 128 : 256);
-  launch(kModeDswiglu, p, a, b, nullptr);
+  const CUtensorMap w = make_bf16_map_2d(w_down.data_ptr(), static_cast<uint64_t>(L_) * F, D, 128);
+  launch_row_gemm(kModeDswiglu, p, w, make_token_maps(dy.data_ptr(), S_, D), num_sms_, stream());
 }
 
 void KernelRunner::tgmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out) {
@@ -195,9 +181,9 @@ void KernelRunner::tgmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out)
   p.carry_out = nullptr;
   p.grad_out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
   const CUtensorMap a = make_bf16_map_chunked(lhs.data_ptr(), S_, M, 64, 2);
-  const CUtensorMap b = make_bf16_map_chunked(rhs.data_ptr(), S_, N, 64, pairs_ ? 2 : 4);
+  const CUtensorMap b = make_bf16_map_chunked(rhs.data_ptr(), S_, N, 64, 2);
   const CUtensorMap c = make_bf16_map_2d(out.data_ptr(), static_cast<uint64_t>(L_) * M, N, 32);
-  launch(kModeTgmm, p, a, b, &c);
+  launch_weight_grad(p, a, b, c, num_sms_, stream());
 }
 
 void KernelRunner::check_status() {

@@ -1,6 +1,6 @@
 // One grouped-GEMM mode at a time on caller-owned tensors: the per-kernel entry points of the fused expert MLP.
 //
-// The layer executor (`FusedRank`) only ever runs the six modes as parts of a pass. This class launches ONE mode on
+// The layer executor (`FusedRank`) only ever runs the modes as parts of a pass. This class launches ONE mode on
 // tensors the caller provides, with the row groups of a single expert-major slice, so that every kernel can be
 // tested against a plain reference on its own and used as a building block (`ops/fused_expert.py`). It mirrors the
 // reference's kernel-level surface: gmm, gmm_swiglu, gmm_dswiglu, tgmm
@@ -23,7 +23,7 @@ namespace cem {
 
 class KernelRunner {
  public:
-  KernelRunner(int L, int S, int stripe, int num_sms, bool cta_pairs);
+  KernelRunner(int L, int S, int stripe, int num_sms);
 
   // rows per expert, int32 [L] on the device, sum <= S
   void set_groups(torch::Tensor group_rows);
@@ -31,7 +31,7 @@ class KernelRunner {
   void gmm_swiglu(torch::Tensor x, torch::Tensor w_up, torch::Tensor act, c10::optional<torch::Tensor> h);
   // out[S,N] = lhs[S,K] rhs[g]; rhs is [L,K,N], or [L,N,K] with transpose_rhs (no transpose is materialised)
   void gmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out, bool transpose_rhs);
-  // dy[S,D] = w * g and dwp[S, D/256] = partial sums of <g, act W_down> per 256-column tile (y is never stored)
+  // dy[S,D] = w * g and dwp[S, D/256] = partial sums of <g, act W_down> per 256 columns
   void gmm_down_dw(torch::Tensor act, torch::Tensor w_down, torch::Tensor g, torch::Tensor row_w, torch::Tensor dy,
                    torch::Tensor dwp);
   // dh[S,2F] = SwiGLU'(h) * (dy W_down^T), w_down [L,F,D]
@@ -43,9 +43,7 @@ class KernelRunner {
 
  private:
   GemmParams base() const;
-  void launch(int mode, const GemmParams& p, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap* c);
   int L_, S_, stripe_, num_sms_;
-  bool pairs_;
   PlanLayout lay_;
   torch::Tensor plan_, counts_, status_, ones_, counter_, table_;
 };

@@ -66,4 +66,10 @@ CUtensorMap make_bf16_map_chunked(const void* base, uint64_t rows, uint64_t cols
   return map;
 }
 
+TokenMaps make_token_maps(const void* base, uint64_t rows, uint64_t cols) {
+  TokenMaps maps;
+  for (uint32_t i = 0; i < 8; ++i) maps.by_width[i] = make_bf16_map_2d(base, rows, cols, 16 * (i + 1));
+  return maps;
+}
+
 }  // namespace cem

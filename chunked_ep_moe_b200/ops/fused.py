@@ -42,19 +42,6 @@ _retired: list = []  # workspaces replaced by `reserve()`; passes in flight may 
 SOLO = "solo"
 
 
-def use_cta_pairs(tokens_times_k: int, local_experts: int) -> bool:
-    """Which GEMM kernel family a workspace runs: CTA pairs (`cta_group::2`, 256-row tiles) or single CTAs.
-
-    The pair kernels are faster per tile but round every expert's rows in a slice up to 256 instead of 128, so they
-    win once an expert receives many rows per pass (measured cross-over: ~512 rows per expert is a draw, 1024 rows
-    +5 %, 2048 rows +8 %). `CEM_CTA_PAIRS=0/1` overrides the choice.
-    """
-    env = os.environ.get("CEM_CTA_PAIRS")
-    if env is not None:
-        return env != "0"
-    return tokens_times_k // max(local_experts, 1) >= 768
-
-
 class FusedWorkspace:
     """Symmetric arena + per-rank executor for one (geometry, process group)."""
 
@@ -80,9 +67,7 @@ class FusedWorkspace:
             stripe=cfg.stripe_width, tk_cap=tk_cap, max_slices=self.max_slices,
             num_sms=int(os.environ.get("CEM_GEMM_GRID", cfg.num_sms)), fp8=self.fp8,
             arena=self.arena.local, peer_arenas=self.arena.peers, use_comm_stream=True,
-            spin_limit=int(os.environ.get("CEM_SPIN_LIMIT", _DEFAULT_SPIN_LIMIT)), put_blocks=int(os.environ.get("CEM_PUT_BLOCKS", _PUT_BLOCKS)),
-            cta_pairs=use_cta_pairs(tk_cap, self.local_experts),
-            tgmm_pairs=os.environ.get("CEM_TGMM_PAIRS", "1") != "0")
+            spin_limit=int(os.environ.get("CEM_SPIN_LIMIT", _DEFAULT_SPIN_LIMIT)), put_blocks=int(os.environ.get("CEM_PUT_BLOCKS", _PUT_BLOCKS)))
         if "CEM_MBAR_LIMIT_US" in os.environ:
             self.rank.set_mbar_limit_us(int(os.environ["CEM_MBAR_LIMIT_US"]))
         self.plan_ints = self.rank.plan_ints()
@@ -198,7 +183,7 @@ def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidd
     tk = tokens_per_rank * top_k if tk_cap is None else tk_cap
     S, D, F = slice_size, hidden, ffn
     arena = int(ext.arena_bytes(world, L, S, D, tk, fp8))
-    scratch = 2 * (S * F * 2 + S * 2 * F * 2 + S * 2 * F * 2 + S * (F // 256) * 4)  # act, h, dh, d_weight shares, x2
+    scratch = 2 * (S * F * 2 + S * 2 * F * 2 + S * 2 * F * 2 + S * (F // 32) * 4)  # act, h, dh, d_weight shares, x2
     carry = 2 * (D * 2 * F + F * D) * 4
     weights = L * (D * 2 * F + F * D) * 2
     max_slices = max(1, math.ceil(world * tk / S)) + 1
@@ -218,7 +203,7 @@ def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidd
 
 PIPELINE_COUNTER_SLOTS = ("loop_cycles", "loop_ns", "producer_wait_free_stage", "mma_wait_filled_stage",
                           "mma_wait_accumulator", "k_blocks", "epilogue_wait_accumulator", "tiles")
-GEMM_MODE_NAMES = ("swiglu", "down_fwd", "down_dw", "dswiglu", "dx", "tgmm")
+GEMM_MODE_NAMES = ("swiglu", "down_fwd", "unused", "dswiglu", "dx", "tgmm")
 
 
 def pipeline_counters(enable: bool = True) -> list:

@@ -3,7 +3,7 @@
 
 Same kernel-level surface as the reference's fused backend (src/chunked_moe/kernels/fused_expert.py:102-366): every
 function takes an expert-major slice of at most S rows plus the rows per expert, runs ONE tcgen05 grouped-GEMM mode
-of `csrc/gemm/grouped_gemm.cu` on it, and returns tensors the caller owns. Rows past `sum(group_sizes)` are padding:
+of `csrc/gemm/` on it, and returns tensors the caller owns. Rows past `sum(group_sizes)` are padding:
 they are never read into a weight gradient and their outputs are left as allocated (zeros here).
 
 This is what `expert_compute="fused"` runs under a COLLECTIVE transport (`ragged_a2a`, `emulated` on a GPU): the
@@ -39,8 +39,7 @@ def _runner(num_groups: int, rows: int, stripe: int, device: torch.device):
     runner = _runners.get(key)
     if runner is None:
         ext = _build.load()
-        pairs = os.environ.get("CEM_CTA_PAIRS", "0") != "0"
-        runner = ext.KernelRunner(num_groups, rows, stripe, int(os.environ.get("CEM_GEMM_GRID", B200_NUM_SMS)), pairs)
+        runner = ext.KernelRunner(num_groups, rows, stripe, int(os.environ.get("CEM_GEMM_GRID", B200_NUM_SMS)))
         _runners[key] = runner
     return runner
 
