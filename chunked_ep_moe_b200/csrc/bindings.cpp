@@ -152,6 +152,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("put", &cem::FusedRank::put)
       .def("compute_forward", &cem::FusedRank::compute_forward)
       .def("compute_backward", &cem::FusedRank::compute_backward)
+      .def("forward_pass", &cem::FusedRank::forward_pass)
+      .def("backward_pass", &cem::FusedRank::backward_pass)
       .def("finish_forward", &cem::FusedRank::finish_forward)
       .def("finish_backward", &cem::FusedRank::finish_backward)
       .def("check_status", &cem::FusedRank::check_status)

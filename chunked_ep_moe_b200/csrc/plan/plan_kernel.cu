@@ -146,6 +146,16 @@ __device__ void plan_phase_b_warps(int* plan, const PlanLayout& y, const int* se
   }
 }
 
+// Header and status block straight into pinned host memory, as soon as the header stands (the per-slice tables are still
+// to come). One thread, after the block barrier that ends phase A.
+__device__ void publish_header(const PlanKernelParams& p) {
+  if (p.host_out == nullptr || threadIdx.x != 0) return;
+  for (int q = 0; q < kPlanHeaderInts; ++q) p.host_out[q] = p.plan[q];
+  const int* status = reinterpret_cast<const int*>(p.status);
+  for (int q = 0; q < 8; ++q) p.host_out[kPlanHeaderInts + q] = status != nullptr ? __ldcg(status + q) : 0;
+  st_release_sys(reinterpret_cast<uint32_t*>(p.host_out) + kPlanHeaderInts + 8, p.host_seq);
+}
+
 __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams p) {
   __shared__ int s_abort;
   const int P = p.lay.P, n = P * p.lay.L;
@@ -173,6 +183,7 @@ __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams 
   __syncthreads();
   if (s_abort) {
     if (threadIdx.x == 0) p.plan[0] = 0;  // zero slices: the pass launches nothing
+    publish_header(p);
     return;
   }
   // 3. tables. When the traffic matrix and the per-segment sums fit into shared memory (always, at real sizes) the block
@@ -186,6 +197,7 @@ __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams 
     // scratch of the per-pass sums: rowsum [n], ebegin [n], prefix [P * n]; the same space holds phase B's inputs after
     plan_phase_a_block(s_counts, p.plan, p.lay, p.me, s_counts + P * n, s_counts + P * n + n, s_counts + P * n + 2 * n);
     __syncthreads();
+    publish_header(p);
     int* s_seg_start = s_counts + P * n;
     int* s_seg_size = s_seg_start + n;
     int* s_send_start = s_seg_size + n;
@@ -206,6 +218,7 @@ __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams 
   }
   plan_phase_a(p.counts, p.plan, p.lay, p.me, threadIdx.x, blockDim.x);
   __syncthreads();
+  publish_header(p);
   plan_phase_b(p.plan, p.lay, threadIdx.x, blockDim.x);
 }
 

@@ -22,6 +22,8 @@ struct PlanKernelParams {
   int* plan;                       // output tables
   uint32_t spin_limit;
   StatusBlock* status;
+  int32_t* host_out = nullptr;     // pinned host words: header (16), status block (8), sequence number; or null
+  uint32_t host_seq = 0;           // stored last: the host polls for it
   int use_smem = 0;                // set by the launcher: the tables are built from a shared-memory copy of the matrix
 };
 

@@ -2,8 +2,12 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <nvtx3/nvToolsExt.h>
+#include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -16,6 +20,19 @@ namespace cem {
 namespace {
 
 constexpr int kExpandSms = 12;  // SMs the up-projection GEMM leaves to the fp8 expansion kernel
+// Pinned words: 16 of the plan header, 8 of the status block and their sequence number (written by the plan kernel), then
+// a second status block for `check_status`.
+constexpr int kHostSeq = kPlanHeaderInts + 8, kHostStatus = 32, kHostInts = 40;
+
+struct NvtxRange {
+  explicit NvtxRange(const char* name) { nvtxRangePushA(name); }
+  NvtxRange(const char* name, int64_t j) {
+    char buf[48];
+    std::snprintf(buf, sizeof(buf), "%s %lld", name, static_cast<long long>(j));
+    nvtxRangePushA(buf);
+  }
+  ~NvtxRange() { nvtxRangePop(); }
+};
 
 inline void cuda_check(cudaError_t err, const char* what) {
   if (err != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(err));
@@ -25,9 +42,11 @@ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 inline cudaStream_t current_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
-void expect(bool cond, const std::string& msg) {
-  if (!cond) throw std::runtime_error(msg);
-}
+// (A macro: the message of a check that holds is never put together.)
+#define expect(cond, msg)                            \
+  do {                                               \
+    if (!(cond)) throw std::runtime_error(msg);      \
+  } while (0)
 
 void expect_bf16_2d(const torch::Tensor& t, int64_t cols, const char* name) {
   expect(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 2 && t.size(1) == cols && t.is_contiguous(),
@@ -176,13 +195,12 @@ FusedRank::FusedRank(int P, int L, int me, int S, int D, int F, int K, int strip
     for (cudaEvent_t* e : {&ev_down_[q], &ev_up_[q], &ev_ds_[q], &ev_dx_[q], &ev_tgd_[q], &ev_tgu_[q]})
       cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "event");
   cuda_check(cudaEventCreateWithFlags(&ev_pass_, cudaEventDisableTiming), "event");
-  cuda_check(cudaEventCreateWithFlags(&ev_header_, cudaEventDisableTiming | cudaEventBlockingSync), "event");
   for (int i = 0; i < 4; ++i) {
     cuda_check(cudaEventCreateWithFlags(&ev_put_[i], cudaEventDisableTiming), "event");
     cuda_check(cudaEventCreateWithFlags(&ev_done_[i], cudaEventDisableTiming), "event");
   }
-  cuda_check(cudaMallocHost(reinterpret_cast<void**>(&host_header_), 24 * sizeof(int32_t)), "pinned header");
-  std::memset(host_header_, 0, 24 * sizeof(int32_t));
+  cuda_check(cudaMallocHost(reinterpret_cast<void**>(&host_header_), kHostInts * sizeof(int32_t)), "pinned header");
+  std::memset(host_header_, 0, kHostInts * sizeof(int32_t));
 }
 
 FusedRank::~FusedRank() {
@@ -197,7 +215,6 @@ FusedRank::~FusedRank() {
       if (e) cudaEventDestroy(e);
   }
   if (ev_pass_) cudaEventDestroy(ev_pass_);
-  if (ev_header_) cudaEventDestroy(ev_header_);
   for (int i = 0; i < 4; ++i) {
     if (ev_put_[i]) cudaEventDestroy(ev_put_[i]);
     if (ev_done_[i]) cudaEventDestroy(ev_done_[i]);
@@ -207,10 +224,11 @@ FusedRank::~FusedRank() {
 
 void FusedRank::check_status() {
   cudaStream_t st = current_stream();
-  cuda_check(cudaMemcpyAsync(host_header_ + 16, status_.data_ptr(), 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, st),
+  cuda_check(cudaMemcpyAsync(host_header_ + kHostStatus, status_.data_ptr(), 8 * sizeof(int32_t),
+                             cudaMemcpyDeviceToHost, st),
              "status copy");
   cuda_check(cudaStreamSynchronize(st), "status sync");
-  const int32_t* s = host_header_ + 16;
+  const int32_t* s = host_header_ + kHostStatus;
   if (s[0] != 0) {
     const std::string message = format_status(std::vector<int64_t>(s, s + 8), me_);
     cuda_check(cudaMemsetAsync(status_.data_ptr(), 0, 8 * sizeof(int32_t), st), "status clear");
@@ -277,21 +295,45 @@ int64_t FusedRank::begin_forward_async(torch::Tensor expert_ids, torch::Tensor p
     pp.flags = reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.traffic_flags + static_cast<size_t>(parity) * P_ * 4);
     pp.epoch = epoch;
   }
+  // The plan kernel itself stores header and status to the pinned words as soon as it knows them; nobody waits here.
+  pp.host_out = host_header_;
+  pp.host_seq = ++host_seq_;
   launch_plan_build(pp, st);
   ++launches_;
-  // Header and status follow the plan kernel to the host; nobody waits here.
-  cuda_check(cudaMemcpyAsync(host_header_, plan.data_ptr(), 16 * sizeof(int32_t), cudaMemcpyDeviceToHost, st),
-             "plan header copy");
-  cuda_check(cudaMemcpyAsync(host_header_ + 16, status_.data_ptr(), 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, st),
-             "status copy");
-  cuda_check(cudaEventRecord(ev_header_, st), "event record");
   // any slice below the workspace's capacity may be launched until resolved; D/128 pieces per row come back
   begin_pass(plan, max_slices_, tk, D_ / kCombineCols);
   return last_slices_ < 0 ? -1 : std::min<int64_t>(last_slices_, max_slices_);
 }
 
+// Waits for the plan kernel's stores to the pinned words. Polling memory notices them in well under a microsecond (a
+// blocking event wait and the two copies it followed took 25-40 us on the way of a one-token decode); a wait that turns
+// out long, behind a stream full of earlier work, sleeps between polls.
+void FusedRank::wait_header() {
+  const volatile uint32_t* seq = reinterpret_cast<const volatile uint32_t*>(host_header_ + kHostSeq);
+  cudaStream_t st = current_stream();
+  const auto arrived = [&]() { return *seq == host_seq_; };
+  const auto spin = [&](bool sleeping) {  // true: arrived, false: the time for busy polling is over
+    const auto t0 = std::chrono::steady_clock::now();
+    for (uint32_t i = 1; !arrived(); ++i) {
+      if (sleeping) {
+        usleep(20);
+      } else if (i % 256 != 0) {
+        continue;
+      }
+      // A stream that has failed, or is done without the store having become visible, ends the wait.
+      const cudaError_t state = cudaStreamQuery(st);
+      if (state == cudaSuccess && !arrived()) throw std::runtime_error("plan header wait: the plan kernel did not report");
+      if (state != cudaSuccess && state != cudaErrorNotReady) cuda_check(state, "plan header wait");
+      if (!sleeping && std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(150)) return false;
+    }
+    return true;
+  };
+  if (!spin(false)) spin(true);
+  std::atomic_thread_fence(std::memory_order_acquire);
+}
+
 int64_t FusedRank::resolve_slices() {
-  cuda_check(cudaEventSynchronize(ev_header_), "plan header wait");
+  wait_header();
   const int32_t* st = host_header_ + 16;
   if (st[0] != 0) {
     const std::string message = format_status(std::vector<int64_t>(st, st + 8), me_);
@@ -358,7 +400,7 @@ void FusedRank::begin_pass(const torch::Tensor& plan, int64_t slices, int64_t ro
                     fp8_ ? reinterpret_cast<uint32_t*>(ready_base_.data_ptr()) : nullptr, st);
   ++launches_;
   ret_target_ += static_cast<uint32_t>(cur_rows_) * static_cast<uint32_t>(pieces_per_row);
-  if (use_comm_stream_) cuda_check(cudaEventRecord(ev_pass_, st), "event record");
+  if (overlapped()) cuda_check(cudaEventRecord(ev_pass_, st), "event record");
 }
 
 void FusedRank::put(int64_t j, torch::Tensor plan, torch::Tensor order, torch::Tensor x,
@@ -370,8 +412,8 @@ void FusedRank::put(int64_t j, torch::Tensor plan, torch::Tensor order, torch::T
              w_flat.numel() == cur_rows_,
          "router weights must be a contiguous CUDA fp32 tensor of T*K elements");
   expect_i32(order, cur_rows_, "order");
-  cudaStream_t st = use_comm_stream_ ? comm_stream_ : current_stream();
-  if (use_comm_stream_) {
+  cudaStream_t st = overlapped() ? comm_stream_ : current_stream();
+  if (overlapped()) {
     if (j == 0) cuda_check(cudaStreamWaitEvent(comm_stream_, ev_pass_, 0), "wait pass event");
     if (j >= 2) cuda_check(cudaStreamWaitEvent(comm_stream_, ev_done_[(j - 2) % 4], 0), "wait slice event");
   }
@@ -403,8 +445,8 @@ void FusedRank::put(int64_t j, torch::Tensor plan, torch::Tensor order, torch::T
   }
   launch_dispatch_put(p, put_blocks_, st);
   ++launches_;
-  if (use_comm_stream_) cuda_check(cudaEventRecord(ev_put_[j % 4], comm_stream_), "event record");
-  if (fp8_ && use_comm_stream_) {
+  if (overlapped()) cuda_check(cudaEventRecord(ev_put_[j % 4], comm_stream_), "event record");
+  if (fp8_ && overlapped()) {
     // The expansion of slice j is issued together with its put, one slice ahead of the GEMMs: it waits for arrivals
     // expert by expert while slice j-1 computes. It may overwrite the bf16 slice buffer once slice j-2 is done with it.
     if (j == 0) cuda_check(cudaStreamWaitEvent(expand_stream_, ev_pass_, 0), "wait pass event");
@@ -522,13 +564,12 @@ void expect_weights(const torch::Tensor& w_up, const torch::Tensor& w_down, int 
 void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_up, torch::Tensor w_down) {
   expect(j >= 0 && j < cur_slices_, "slice index out of range");
   expect_weights(w_up, w_down, L_, D_, F_);
-  const bool async = use_comm_stream_;
+  const bool async = overlapped();
   const int q = static_cast<int>(j & 1);
   cudaStream_t st = async ? chain_[q] : current_stream();
   cudaStream_t aux = async ? aux_stream_ : st;
   if (async) {
-    if (j < 2) cuda_check(cudaStreamWaitEvent(st, ev_pass_, 0), "wait pass event");
-    cuda_check(cudaStreamWaitEvent(st, ev_put_[j % 4], 0), "wait put event");
+    cuda_check(cudaStreamWaitEvent(st, ev_put_[j % 4], 0), "wait put event");  // (behind the pass event)
   }
   const uint32_t seq = seq_ + static_cast<uint32_t>(j);
   const int b = static_cast<int>(seq & 1u);
@@ -579,13 +620,12 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
   expect(j >= 0 && j < cur_slices_, "slice index out of range");
   expect_weights(w_up, w_down, L_, D_, F_);
   expect_weights(dw_up, dw_down, L_, D_, F_);
-  const bool async = use_comm_stream_;
+  const bool async = overlapped();
   const int q = static_cast<int>(j & 1);
   cudaStream_t st = async ? chain_[q] : current_stream();
   cudaStream_t aux = async ? aux_stream_ : st;
   if (async) {
-    if (j < 2) cuda_check(cudaStreamWaitEvent(st, ev_pass_, 0), "wait pass event");
-    cuda_check(cudaStreamWaitEvent(st, ev_put_[j % 4], 0), "wait put event");
+    cuda_check(cudaStreamWaitEvent(st, ev_put_[j % 4], 0), "wait put event");  // (behind the pass event)
     if (j >= 2) cuda_check(cudaStreamWaitEvent(st, ev_tgd_[q], 0), "wait dW_down event");  // act of slice j-2
   }
   const uint32_t seq = seq_ + static_cast<uint32_t>(j);
@@ -693,7 +733,7 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
 
 // Makes the caller's stream wait for everything the pass issued on the chain and auxiliary streams.
 void FusedRank::join_streams(bool backward) {
-  if (!use_comm_stream_ || cur_slices_ <= 0) return;
+  if (!overlapped() || cur_slices_ <= 0) return;
   cudaStream_t st = current_stream();
   cuda_check(cudaStreamWaitEvent(st, ev_done_[(cur_slices_ - 1) % 4], 0), "join aux stream");
   if (fp8_) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(cur_slices_ - 1) % 4], 0), "join expand stream");
@@ -706,6 +746,7 @@ void FusedRank::join_streams(bool backward) {
 void FusedRank::end_pass(int64_t n_slices) {
   seq_ += static_cast<uint32_t>(n_slices);
   cur_slices_ = 0;
+  inline_ = false;
 }
 
 void FusedRank::finish_forward(torch::Tensor inv_order, torch::Tensor out) {
@@ -753,6 +794,84 @@ void FusedRank::finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch
   launch_combine_reduce(c, current_stream());
   ++launches_;
   end_pass(cur_slices_);
+}
+
+// ---------------------------------------------------------------------------------------------
+// whole passes
+// ---------------------------------------------------------------------------------------------
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> FusedRank::forward_pass(
+    torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down) {
+  const int64_t tk = expert_ids.numel();
+  expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
+  auto i32 = torch::TensorOptions().device(x.device()).dtype(torch::kInt32);
+  // (The send order needs no initial values: an id the sort leaves out is recorded in the status block first, and with
+  // that set every kernel that would read the order returns at once.)
+  torch::Tensor plan = torch::empty({lay_.total}, i32), order = torch::empty({tk}, i32),
+                inv_order = torch::empty({tk}, i32), out = torch::empty_like(x);
+  auto run_slices = [&](int64_t lo, int64_t hi) {
+    if (hi <= lo) return;
+    put(lo, plan, order, x, c10::nullopt, w_flat);
+    for (int64_t j = lo; j < hi; ++j) {
+      NvtxRange range("chunked_moe/fwd slice", j);
+      if (j + 1 < hi) put(j + 1, plan, order, x, c10::nullopt, w_flat);  // slice j+1 is in flight while slice j computes
+      compute_forward(j, plan, w_up, w_down);
+    }
+  };
+  // The slice count is a device value (it depends on the routing of every rank). The host does not wait for it: it
+  // launches as many slices as the previous pass of this workspace needed, THEN reads the real count (by then long on
+  // the host) and launches what is missing. Too many is harmless: a slice past the real count finds empty tables on
+  // every rank. Every rank guesses and learns the same numbers, so all ranks loop alike. One rank on its own receives
+  // exactly its own T*K copies and knows the count beforehand.
+  const int64_t known = P_ == 1 ? (tk + S_ - 1) / S_ : -1;
+  // A single slice of one rank: put, GEMMs and combine only follow one another, so they go to the caller's stream and the
+  // events that tie the streams together are saved (one-token decode 82 -> 77 us, 2000 tokens at D=2048 195 -> 190 us).
+  // The backward keeps its streams: its weight gradients fill the other GEMMs' tails (same layer 542 us, else 558 us). The
+  // fp8 wire keeps its expansion beside the GEMM.
+  inline_ = use_comm_stream_ && known == 1 && !fp8_;
+  int64_t guess;
+  {
+    NvtxRange range("chunked_moe/plan");
+    guess = std::max<int64_t>(0, begin_forward_async(expert_ids, plan, order, inv_order, plan, false));
+  }
+  if (known >= 0) guess = std::min<int64_t>(known, max_slices_);
+  run_slices(0, guess);
+  int64_t n = known;
+  if (known >= 0) {
+    set_pass_slices(guess);
+  } else {
+    n = resolve_slices();  // throws here if an earlier kernel recorded an error (bad expert id, timed-out wait)
+    run_slices(guess, n);
+    set_pass_slices(std::max(guess, n));
+  }
+  {
+    NvtxRange range("chunked_moe/combine");
+    finish_forward(inv_order, out);
+  }
+  if (known >= 0) n = resolve_slices();  // the same checks, with all of the pass on its way to the device
+  return std::make_tuple(out, plan, order, inv_order, n);
+}
+
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank::backward_pass(
+    torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
+    torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices) {
+  inline_ = false;  // (also behind a forward that threw)
+  // The slice count is the forward's: nothing is read back, the host never waits for the device here.
+  const int64_t n = begin_backward(plan, known_slices, order.numel());
+  torch::Tensor dw_up = torch::empty_like(w_up), dw_down = torch::empty_like(w_down), dx = torch::empty_like(x);
+  torch::Tensor d_weights = torch::empty({w_flat.numel()}, w_flat.options());
+  if (n > 0) {
+    put(0, plan, order, x, g, w_flat);
+  } else {
+    dw_up.zero_();
+    dw_down.zero_();
+  }
+  for (int64_t j = 0; j < n; ++j) {
+    NvtxRange range("chunked_moe/bwd slice", j);
+    if (j + 1 < n) put(j + 1, plan, order, x, g, w_flat);
+    compute_backward(j, plan, w_up, w_down, dw_up, dw_down);
+  }
+  finish_backward(inv_order, dx, d_weights);
+  return std::make_tuple(dx, d_weights, dw_up, dw_down);
 }
 
 // ---------------------------------------------------------------------------------------------

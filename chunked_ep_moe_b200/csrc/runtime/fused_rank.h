@@ -76,6 +76,15 @@ class FusedRank {
   void finish_forward(torch::Tensor inv_order, torch::Tensor out);
   void finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights);
 
+  // The two passes as one call each (what `chunked_moe` runs). Forward: (out, plan, order, inv_order, slice count); it
+  // throws a recorded kernel error. Backward: (dx, d_weights, dw_up, dw_down). Tensors are contiguous CUDA tensors of
+  // the workspace's geometry: x, g [T, D] bf16, expert_ids [T, K] int32, w_flat [T*K] fp32.
+  std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> forward_pass(
+      torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down);
+  std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> backward_pass(
+      torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
+      torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices);
+
   // Reads the status block (synchronises); throws std::runtime_error describing the first recorded error.
   void check_status();
   std::vector<int64_t> plan_header() const { return std::vector<int64_t>(host_header_, host_header_ + 16); }
@@ -95,6 +104,8 @@ class FusedRank {
   // Common start of a pass: counter targets on the device, what the pass will receive back (`pieces_per_row` of T*K rows).
   void begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row);
   void end_pass(int64_t n_slices);
+  void wait_header();
+  bool overlapped() const { return use_comm_stream_ && !inline_; }
   void join_streams(bool backward);
   GemmParams base_params(const int* plan, int j) const;
   // `chunks` > 0: the MN-major description (64-column chunks, `chunks` of them per copy); 0: plain 2-D boxes.
@@ -134,9 +145,11 @@ class FusedRank {
   cudaStream_t expand_stream_ = nullptr;  // fp8 wire: the expansion kernels run here, beside the GEMM chains
   cudaEvent_t ev_expand_[4] = {};  // expansion of slice j (mod 4) has finished
   cudaEvent_t ev_down_[2] = {}, ev_up_[2] = {}, ev_ds_[2] = {}, ev_dx_[2] = {}, ev_tgd_[2] = {}, ev_tgu_[2] = {};
-  cudaEvent_t ev_pass_ = nullptr, ev_put_[4] = {}, ev_done_[4] = {}, ev_header_ = nullptr;
+  cudaEvent_t ev_pass_ = nullptr, ev_put_[4] = {}, ev_done_[4] = {};
   int64_t last_slices_ = -1;  // slice count of the previous forward pass (the next pass's guess)
-  int32_t* host_header_ = nullptr;  // pinned: 16 plan header ints + 8 status ints
+  int32_t* host_header_ = nullptr;  // pinned: 16 plan header ints + 8 status ints + their sequence number, see the .cpp
+  uint32_t host_seq_ = 0;     // headers asked for so far
+  bool inline_ = false;       // the current pass runs on the caller's stream alone
 
   uint32_t seq_ = 0;          // global slice sequence number of the next pass's first slice
   uint32_t fwd_epoch_ = 0;    // forward passes started (traffic exchange epoch)

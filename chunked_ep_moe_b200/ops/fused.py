@@ -228,12 +228,6 @@ def pipeline_counters(enable: bool = True) -> list:
     return out
 
 
-def nvtx(name: str):
-    from ..utils.nvtx import nvtx_range
-
-    return nvtx_range(name)
-
-
 def _require(cond: bool, msg: str) -> None:
     if not cond:
         raise ValueError("chunked_moe fused path: " + msg)
@@ -245,39 +239,12 @@ class _ChunkedMoEFused(torch.autograd.Function):
         tokens, hidden = x.shape
         ffn = w_down.shape[1]
         ws = get_workspace(cfg, group, hidden, ffn, tokens * cfg.top_k)
-        rank = ws.rank
-        dev = x.device
-        plan = torch.empty(ws.plan_ints, dtype=torch.int32, device=dev)
-        order = torch.zeros(tokens * cfg.top_k, dtype=torch.int32, device=dev)  # no stray indices if an id is invalid
-        inv_order = torch.zeros_like(order)
         ids32 = expert_ids.to(torch.int32).contiguous()
         w_flat = weights.detach().float().reshape(-1).contiguous()
         xc, w_up_c, w_down_c = x.detach().contiguous(), w_up.detach().contiguous(), w_down.detach().contiguous()
-        def run_slices(lo: int, hi: int) -> None:
-            if hi <= lo:
-                return
-            rank.put(lo, plan, order, xc, None, w_flat)
-            for j in range(lo, hi):
-                with nvtx(f"chunked_moe/fwd slice {j}"):
-                    if j + 1 < hi:
-                        rank.put(j + 1, plan, order, xc, None, w_flat)  # slice j+1 is in flight while slice j computes
-                    rank.compute_forward(j, plan, w_up_c, w_down_c)
-
-        # The slice count is a device value (it depends on the routing). The host does not wait for it: it launches
-        # as many slices as the previous pass of this workspace needed, THEN reads the real count (by then long on
-        # the host) and launches what is missing. Too many is harmless: a slice past the real count finds empty
-        # tables on every rank. Every rank guesses and learns the same numbers, so all ranks loop alike.
-        with nvtx("chunked_moe/plan"):
-            guess = max(0, rank.begin_forward_async(ids32, plan, order, inv_order, ws.dummy_counts, False))
-        out = torch.empty_like(xc)
-        run_slices(0, guess)
-        n = rank.resolve_slices()  # raises here if an earlier kernel recorded an error (bad expert id, timed-out wait)
-        run_slices(guess, n)
-        rank.set_pass_slices(max(guess, n))
-        with nvtx("chunked_moe/combine"):
-            rank.finish_forward(inv_order, out)
+        out, plan, order, inv_order, n = ws.rank.forward_pass(xc, ids32, w_flat, w_up_c, w_down_c)
         ctx.save_for_backward(xc, weights, w_up_c, w_down_c, plan, order, inv_order)
-        ctx.cfg, ctx.group, ctx.ws, ctx.num_slices = cfg, group, ws, int(n)
+        ctx.ws, ctx.num_slices = ws, n
         ctx.mark_non_differentiable(expert_ids)
         return out
 
@@ -289,22 +256,8 @@ class _ChunkedMoEFused(torch.autograd.Function):
             raise RuntimeError("chunked_moe fused path: the workspace of this pass was released before its backward")
         g = g_out.to(x.dtype).contiguous()
         w_flat = weights.detach().float().reshape(-1).contiguous()
-        # The slice count is the forward's: nothing is read back, the host never waits for the device here.
-        n = rank.begin_backward(plan, ctx.num_slices, order.numel())
-        dw_up, dw_down = torch.empty_like(w_up), torch.empty_like(w_down)
-        if n > 0:
-            rank.put(0, plan, order, x, g, w_flat)
-        else:
-            dw_up.zero_()
-            dw_down.zero_()
-        for j in range(n):
-            with nvtx(f"chunked_moe/bwd slice {j}"):
-                if j + 1 < n:
-                    rank.put(j + 1, plan, order, x, g, w_flat)
-                rank.compute_backward(j, plan, w_up, w_down, dw_up, dw_down)
-        dx = torch.empty_like(x)
-        d_weights = torch.empty(weights.numel(), dtype=torch.float32, device=x.device)
-        rank.finish_backward(inv_order, dx, d_weights)
+        dx, d_weights, dw_up, dw_down = rank.backward_pass(x, g, w_flat, w_up, w_down, plan, order, inv_order,
+                                                           ctx.num_slices)
         return dx, None, d_weights.reshape(weights.shape).to(weights.dtype), dw_up, dw_down, None, None
 
 

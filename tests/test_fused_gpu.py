@@ -261,6 +261,24 @@ def test_slice_count_guess_is_corrected_in_both_directions():
             _close(ds.grad.cpu(), want["dw_down"], f"dw_down ({keep} tokens)")
 
 
+@pytest.mark.parametrize("tokens", [0, 1, 17, 64, 65])
+def test_one_slice_forward_equals_several_slices(tokens):
+    """A forward of one slice runs on the caller's stream, a longer one on the workspace's: 2 * tokens rows against slices
+    of 128 (one up to 64 tokens) and of 8 rows. A row's result does not depend on the slice it is in: equal bit for bit."""
+    gen = torch.Generator().manual_seed(11)
+    E, K, D, F = 4, 2, 256, 256
+    bf = lambda t: t.cuda().to(torch.bfloat16)
+    x = bf(torch.randn(tokens, D, generator=gen))
+    ids = torch.stack([torch.randperm(E, generator=gen)[:K] for _ in range(tokens)] or [torch.zeros(K)])[:tokens].int().cuda()
+    weights = (torch.rand(tokens, K, generator=gen) + 0.1).cuda()
+    w_up = bf(torch.randn(E, D, 2 * F, generator=gen) / math.sqrt(D))
+    w_down = bf(torch.randn(E, F, D, generator=gen) / math.sqrt(F))
+    outs = [chunked_moe(x, ids, weights, w_up, w_down,
+                        ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=s, transport="nvshmem", expert_compute="fused",
+                                         stripe_width=64)) for s in (128, 8)]
+    assert outs[0].shape == x.shape and torch.equal(*outs)
+
+
 def test_gemm_whose_rows_never_arrive_gives_up_and_reports(monkeypatch):
     """The real swiglu kernel waiting for rows nobody sends: its bounded wait runs out, every warp unwinds promptly
     (the barrier waits watch the CTA's abort flag), later kernels of the pass return at once, the host raises."""
