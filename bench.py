@@ -516,7 +516,7 @@ def main():
                "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 4}
 
     if rank == 0:
-        flops = 24.0 * D * F * T * K  # per rank, fwd + bwd with full remat
+        flops = 18.0 * D * F * T * K  # per rank, what fwd + bwd cannot do without (recomputation is not counted)
         peaks = {}
         try:
             peaks = json.load(open(os.path.join(REPO, "MEASURED_PEAKS.json")))

@@ -13,7 +13,8 @@ Per rank (one process per GPU, `group` is the expert-parallel process group):
 Same surface and gradient set as the reference's `custom_vjp`
 (src/chunked_moe/moe.py:122-209): gradients flow to x, router_weights, w_up and
 w_down; the backward is communicating (every rank of the group must call it).
-Only the inputs and the integer routing plan are saved between the passes.
+The inputs and the integer routing plan are saved between the passes; the fused path also keeps the up-projection's
+activations of large slices while the device has memory to spare.
 
 Backend selection: `transport="nvshmem"` + `expert_compute="fused"` runs the
 fused sm_100a executor; every other combination runs the torch slice loops on

@@ -29,7 +29,7 @@ __device__ __forceinline__ void resolve_source(const GemmParams& p, int g, int g
 // Dispatch consumer: waits until the rows of local expert `g` that belong to slices <= p.slice have arrived from every
 // source rank (lane s watches source s), then orders the async proxy behind what was observed, because the rows were
 // written through the generic proxy and TMA reads them next. Returns false on expiry (status recorded, abort set).
-__device__ __forceinline__ bool wait_expert_rows(const GemmParams& p, int g, int lane, volatile int* abort_flag) {
+__device__ __forceinline__ bool wait_expert_rows(const GemmParams& p, int mode, int g, int lane, volatile int* abort_flag) {
   bool ok = true;
   if (p.ready != nullptr) {
     // fp8 wire: the expansion kernel releases an expert's rows (bf16, local) once they have arrived and been expanded.
@@ -40,7 +40,7 @@ __device__ __forceinline__ bool wait_expert_rows(const GemmParams& p, int g, int
       uint32_t seen = 0;
       ok = spin_until_reached(p.ready + g, target, p.spin_limit, &seen);
       if (!ok) {
-        report_status(p.status, kStatusArrivalTimeout, kKernelGemm, kModeSwiglu, p.slice, 10000 + g, target, seen);
+        report_status(p.status, kStatusArrivalTimeout, kKernelGemm, mode, p.slice, 10000 + g, target, seen);
         *abort_flag = 1;
       }
     }
@@ -52,7 +52,7 @@ __device__ __forceinline__ bool wait_expert_rows(const GemmParams& p, int g, int
     uint32_t seen = 0;
     ok = spin_until_reached(p.arrive + i, target, p.spin_limit, &seen);
     if (!ok) {
-      report_status(p.status, kStatusArrivalTimeout, kKernelGemm, kModeSwiglu, p.slice, i, target, seen);
+      report_status(p.status, kStatusArrivalTimeout, kKernelGemm, mode, p.slice, i, target, seen);
       *abort_flag = 1;
     }
   }

@@ -21,8 +21,8 @@ constexpr int kSmemTailBytes = 256;   // barriers, TMEM slot, flags
 constexpr int kCombineCols = kBlockM; // columns of one returned row piece (what the returned-piece counters count)
 
 enum GemmMode : int {
-  kModeSwiglu = 0,   // act = silu(x Wg) * (x Wu) from striped w_up; optional h          (replaces gmm_swiglu)
-  kModeDownFwd = 1,  // y = act Wd; epilogue x router weight, rows stored to their source rank (gmm + combine)
+  kModeSwiglu = 0,   // act = w * silu(x Wg) * (x Wu) from striped w_up; optional h      (replaces gmm_swiglu)
+  kModeDownFwd = 1,  // y = act Wd, rows stored to their source rank                         (gmm + combine)
   // (2 is not used: the slot numbering of the pipeline counters is public)
   kModeDswiglu = 3,  // d_act = w * (g Wd^T); epilogue SwiGLU' with h -> dh, d_weight partials (gmm_dswiglu)
   kModeDx = 4,       // dx = dh Wu^T; rows stored to their source rank                      (gmm^T + combine)
@@ -58,7 +58,7 @@ struct GemmParams {
   StatusBlock* status;
   // Optional pipeline counters of this mode, [grid][kProfSlots] summed over launches; null = not counted.
   unsigned long long* prof;
-  // --- arrival flags (swiglu consumer) -----------------------------------------------------
+  // --- arrival flags (swiglu and dswiglu: the first consumer of a slice's rows) -----------------------------------------------------
   const uint32_t* arrive;     // [P*L] cumulative rows received per (source, local expert); null = no wait
   const uint32_t* pass_base;  // [P*L] value of `arrive` when this pass began
   // fp8 wire: rows are usable once the expansion kernel has released them, per local expert (replaces `arrive`)

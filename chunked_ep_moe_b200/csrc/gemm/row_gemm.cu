@@ -162,6 +162,16 @@ __device__ __forceinline__ void swiglu_epilogue(const GemmParams& p, const RowTi
   const int h_col1 = h_col0 + (p.stripe == 128 ? 128 : 64);
   for (int ch = c.h; ch < chunks; ch += 2) {
     const int row0 = tl.row0 + ch * 32, nvalid = tl.nrows - ch * 32;
+    // Router weights of this thread's four rows, asked for before anything else: they come from L2 (read past L1: the line
+    // may also hold weights of rows that had not arrived when another tile read it).
+    float w[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+    if (p.row_w != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = (is_gate ? 0 : 16) + 8 * (i >> 1) + 2 * (c.lane & 3) + (i & 1);
+        if (t < nvalid) w[i] = __ldcg(p.row_w + row0 + t);
+      }
+    }
     uint32_t r[32];
     load_fragment(tacc + ch * 32, r);
     if (ch + 2 >= chunks) release();
@@ -199,14 +209,6 @@ __device__ __forceinline__ void swiglu_epilogue(const GemmParams& p, const RowTi
 #pragma unroll
     for (int jj = 0; jj < 2; ++jj) {
       const int trow = (is_gate ? 0 : 16) + 8 * jj;
-      float w0 = 1.0f, w1 = 1.0f;
-      if (p.row_w != nullptr) {
-        // (Read past L1: the line may also hold weights of rows that had not arrived when another tile read it. Rows
-        // past the tile's end read their neighbours' weights or, at the end of the slice, nothing; they are not stored.)
-        const int t0 = trow + 2 * (c.lane & 3);
-        if (t0 < nvalid) w0 = __ldcg(p.row_w + row0 + t0);
-        if (t0 + 1 < nvalid) w1 = __ldcg(p.row_w + row0 + t0 + 1);
-      }
       uint32_t o[4];
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
@@ -219,7 +221,7 @@ __device__ __forceinline__ void swiglu_epilogue(const GemmParams& p, const RowTi
           const float gate = __uint_as_float(is_gate ? own : other), up = __uint_as_float(is_gate ? other : own);
           a[e] = silu_f(gate) * up;
         }
-        o[s] = pack_bf16(a[0] * w0, a[1] * w1);
+        o[s] = pack_bf16(a[0] * w[2 * jj], a[1] * w[2 * jj + 1]);
       }
       stmatrix_x4_trans(staged<128>(abuf, trow + (c.lane & 7), act_piece + (c.lane >> 3)), o);
     }
@@ -242,12 +244,10 @@ __device__ __forceinline__ void swiglu_epilogue(const GemmParams& p, const RowTi
 }
 
 // Down-projection / dX: every row's 128 columns go to the rank the row came from, at its send-order position.
-// `dst` (shared memory, one entry per row of this group's chunks): source << 27 | position, or ~0 for rows past the tile;
-// `wts`: the rows' router weights (down-projection).
-template <int MODE, typename Release>
+// `dst` (shared memory, one entry per row of this group's chunks): source << 27 | position, or ~0 for rows past the tile.
+template <typename Release>
 __device__ __forceinline__ void combine_epilogue(const GemmParams& p, const RowTile& tl, uint32_t tacc,
-                                                 const GroupCtx& c, const uint32_t* dst, const float* wts,
-                                                 Release&& release) {
+                                                 const GroupCtx& c, const uint32_t* dst, Release&& release) {
   const int chunks = (tl.nrows + 31) >> 5;
   const int col = tl.n * kBlockN + c.rank * kBlockM;
   for (int ch = c.h; ch < chunks; ch += 2) {
@@ -258,12 +258,10 @@ __device__ __forceinline__ void combine_epilogue(const GemmParams& p, const RowT
     uint32_t o[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float2 w = make_float2(1.0f, 1.0f);
-      if constexpr (MODE == kModeDownFwd) w = *reinterpret_cast<const float2*>(wts + list0 + 8 * j + 2 * (c.lane & 3));
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
         const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
-        o[j][s] = pack_bf16(__uint_as_float(r[b]) * w.x, __uint_as_float(r[b + 1]) * w.y);
+        o[j][s] = pack_bf16(__uint_as_float(r[b]), __uint_as_float(r[b + 1]));
       }
     }
     const uint32_t buf = c.staging;
@@ -303,6 +301,12 @@ __device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowT
   for (int i = 0; i < 8; ++i) v[i] = first[i];
   for (int ch = c.h; ch < chunks; ch += 2) {
     const int row0 = tl.row0 + ch * 32, nvalid = tl.nrows - ch * 32;
+    float w[8];  // this thread's rows' router weights (past L1 and ahead of time, as in the up-projection)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = 8 * (i >> 1) + 2 * (c.lane & 3) + (i & 1);
+      w[i] = p.row_w != nullptr && t < nvalid ? __ldcg(p.row_w + row0 + t) : 1.0f;
+    }
     group_sync(c.h);  // the previous chunk has left the buffer
 #pragma unroll
     for (int i = 0; i < 8; ++i) st_shared_v4(staged<512>(c.staging, prow + 4 * i, piece), v[i].x, v[i].y, v[i].z, v[i].w);
@@ -319,12 +323,6 @@ __device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowT
     float part[8];  // <acc, act> over this thread's columns, rows 8 j + 2 (lane & 3) + e
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int t0 = 8 * j + 2 * (c.lane & 3);
-      float w[2] = {1.0f, 1.0f};
-      if (p.row_w != nullptr) {
-        if (t0 < nvalid) w[0] = p.row_w[row0 + t0];
-        if (t0 + 1 < nvalid) w[1] = p.row_w[row0 + t0 + 1];
-      }
       const uint32_t ga = staged<512>(c.staging, 8 * j + (c.lane & 7), gpiece);
       const uint32_t ua = staged<512>(c.staging, 8 * j + (c.lane & 7), upiece);
       uint32_t g[4], u[4];
@@ -336,7 +334,7 @@ __device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowT
         const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
         const float a[2] = {__uint_as_float(r[b]), __uint_as_float(r[b + 1])};
         // d_act is rounded to bf16 first, as the unfused reference stores it.
-        const uint32_t db = pack_bf16(w[0] * a[0], w[1] * a[1]);
+        const uint32_t db = pack_bf16(w[2 * j] * a[0], w[2 * j + 1] * a[1]);
         float dg[2], du[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -481,9 +479,9 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     for (int t = first_tile; t < num_tiles && !dead && !*abort_flag; t += tile_step) {
       const RowTile tl = nxt;
       if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, num_entries);
-      if constexpr (MODE == kModeSwiglu) {
+      if constexpr (MODE == kModeSwiglu || MODE == kModeDswiglu) {  // whichever reads a slice's dispatched rows first
         if ((p.arrive != nullptr || p.ready != nullptr) && tl.g != waited_expert) {
-          if (!wait_expert_rows(p, tl.g, lane, abort_flag)) {
+          if (!wait_expert_rows(p, MODE, tl.g, lane, abort_flag)) {
             if (lane == 0) raise_abort();
             break;
           }
@@ -602,9 +600,8 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     c.rank = rank;
     c.staging = staging_base + c.h * kGroupStaging;
     const uint32_t leader_acc_empty0 = map_to_cta(acc_empty_bar(0), 0);
-    // Combine modes: the row tables sit behind the 8 KB that a chunk is staged in.
+    // Combine modes: the row table sits behind the 8 KB that a chunk is staged in.
     uint32_t* s_dst = reinterpret_cast<uint32_t*>(staging_gen + c.h * kGroupStaging + 8192);
-    float* s_wts = reinterpret_cast<float*>(s_dst + kTileTokens / 2);
     uint32_t tcount = 0, returned = 0;
     long long epi_wait = 0;
     RowTile nxt = {};
@@ -622,7 +619,6 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
         int src = -1, pos = 0;
         if (row < tl.nrows) resolve_source(p, tl.g, tl.row0 + row, &src, &pos);
         s_dst[c.gt] = src >= 0 ? (static_cast<uint32_t>(src) << 27) | static_cast<uint32_t>(pos) : ~0u;
-        if constexpr (MODE == kModeDownFwd) s_wts[c.gt] = row < tl.nrows ? p.row_w[tl.row0 + row] : 0.0f;
         // Lane s keeps the count of row pieces this warp accounts for at source rank s (`flush_returned`).
         for (int s = 0; s < p.lay.P; ++s) {
           const uint32_t cnt = __popc(__ballot_sync(0xffffffffu, src == s));
@@ -657,7 +653,7 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
       };
       if constexpr (MODE == kModeSwiglu) swiglu_epilogue(p, tl, tacc, c, release);
       else if constexpr (MODE == kModeDswiglu) dswiglu_epilogue(p, tl, tacc, c, first, release);
-      else combine_epilogue<MODE>(p, tl, tacc, c, s_dst, s_wts, release);
+      else combine_epilogue(p, tl, tacc, c, s_dst, release);
     }
     if (counting && warp == 2 && lane == 0) prof_add(kProfEpiWait, epi_wait);
     if constexpr (Traits::kCombine) {

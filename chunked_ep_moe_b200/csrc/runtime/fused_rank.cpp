@@ -1,6 +1,7 @@
 #include "fused_rank.h"
 
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <nvtx3/nvToolsExt.h>
 #include <unistd.h>
@@ -23,6 +24,13 @@ constexpr int kExpandSms = 12;  // SMs the up-projection GEMM leaves to the fp8 
 // Pinned words: 16 of the plan header, 8 of the status block and their sequence number (written by the plan kernel), then
 // a second status block for `check_status`.
 constexpr int kHostSeq = kPlanHeaderInts + 8, kHostStatus = 32, kHostInts = 40;
+
+// Rows of a slice x D x F from which a training forward keeps h and w * act. Measured, forward + backward, keeping against
+// recomputing: 16384-row slices at D=1024, F=512 (2^33) 1026 against 1072 us, 7996 rows at D=2048, F=1024 (2^34) 503 against
+// 530 us; 1024-row slices at D=2048, F=1024 (2^31) 1133 against 1126 us (the GEMM it saves runs in the shadow of the next
+// put there), 1024 rows at D=F=512 204 us both ways (a kernel takes 8 us however little it does, and two allocations and a
+// slice's tensor maps cost the host what its launch does).
+constexpr int64_t kKeepWork = int64_t{1} << 32;
 
 struct NvtxRange {
   explicit NvtxRange(const char* name) { nvtxRangePushA(name); }
@@ -115,6 +123,12 @@ FusedRank::FusedRank(int P, int L, int me, int S, int D, int F, int K, int strip
   lay_ = make_plan_layout(P, L, S, max_slices);
   arena_lay_ = make_arena_layout(P, L, S, D, tk_cap, fp8);
   arena_ = reinterpret_cast<uint8_t*>(arena);
+  cudaDeviceProp prop;
+  int device = 0;
+  cuda_check(cudaGetDevice(&device), "device");
+  cuda_check(cudaGetDeviceProperties(&prop, device), "device properties");
+  device_bytes_ = prop.totalGlobalMem;
+  if (const char* v = std::getenv("CEM_KEEP_ACTIVATIONS")) keep_activations_ = std::atoi(v) != 0;
   for (int64_t p : peer_arenas) peers_.push_back(reinterpret_cast<uint8_t*>(p));
 
   auto bf16 = torch::TensorOptions().device(torch::kCUDA).dtype(torch::kBFloat16);
@@ -574,6 +588,7 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
   const uint32_t seq = seq_ + static_cast<uint32_t>(j);
   const int b = static_cast<int>(seq & 1u);
   const int* pl = plan.data_ptr<int>();
+  const bool keep = j < kept_slices_;
   if (fp8_ && !async) dequant(pl, static_cast<int>(j), b, /*with_g=*/false, st);  // lockstep: every put is done
   {
     GemmParams p = base_params(pl, static_cast<int>(j));
@@ -584,9 +599,10 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
     p.pass_base = reinterpret_cast<const uint32_t*>(pass_base_.data_ptr());
     p.ready = fp8_ ? reinterpret_cast<const uint32_t*>(ready_.data_ptr()) : nullptr;
     p.ready_base = reinterpret_cast<const uint32_t*>(ready_base_.data_ptr());
-    p.out0 = reinterpret_cast<__nv_bfloat16*>(act_[q].data_ptr());
+    p.row_w = reinterpret_cast<const float*>(arena_ + arena_lay_.wbuf) + static_cast<size_t>(b) * S_;
+    p.out0 = keep ? kept_act(j) : reinterpret_cast<__nv_bfloat16*>(act_[q].data_ptr());
     p.ld0 = F_;
-    p.out1 = nullptr;
+    p.out1 = keep ? kept_h(j) : nullptr;
     p.ld1 = 2 * F_;
     // fp8 wire: this kernel waits (in its producer warp) for the expansion kernel of the same slice. A persistent CTA
     // takes all of an SM's shared memory, so nothing else can start beside it: the kernel leaves a few SMs free for the
@@ -600,11 +616,11 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
     p.n_tiles = D_ / kBlockN;
     p.k_blocks = F_ / kBlockK;
     p.b_group_rows = F_;
-    p.row_w = reinterpret_cast<const float*>(arena_ + arena_lay_.wbuf) + static_cast<size_t>(b) * S_;
     p.peer_rows = table<__nv_bfloat16>(kTabRet);
     p.peer_count = table<uint32_t>(kTabCount);
     p.ld0 = D_;
-    row_gemm(kModeDownFwd, p, weight_map(w_down, 64, 2), map_act_[q], st);
+    row_gemm(kModeDownFwd, p, weight_map(w_down, 64, 2),
+             keep ? make_token_maps(kept_act(j), kept_slice_rows(j), F_) : map_act_[q], st);
   }
   if (async) {
     cuda_check(cudaEventRecord(ev_down_[q], st), "event record");
@@ -624,9 +640,10 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
   const int q = static_cast<int>(j & 1);
   cudaStream_t st = async ? chain_[q] : current_stream();
   cudaStream_t aux = async ? aux_stream_ : st;
+  const bool keep = j < kept_slices_;
   if (async) {
     cuda_check(cudaStreamWaitEvent(st, ev_put_[j % 4], 0), "wait put event");  // (behind the pass event)
-    if (j >= 2) cuda_check(cudaStreamWaitEvent(st, ev_tgd_[q], 0), "wait dW_down event");  // act of slice j-2
+    if (!keep && j >= 2) cuda_check(cudaStreamWaitEvent(st, ev_tgd_[q], 0), "wait dW_down event");  // act of slice j-2
   }
   const uint32_t seq = seq_ + static_cast<uint32_t>(j);
   const int b = static_cast<int>(seq & 1u);
@@ -634,50 +651,54 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
   const int par = static_cast<int>(j & 1);
   const int dwp_tiles = F_ / 32;
   if (fp8_ && !async) dequant(pl, static_cast<int>(j), b, /*with_g=*/true, st);  // lockstep: every put is done
-  // Remat: h and w * act. y is not recomputed: d_weight = <g, act Wd> = <g Wd^T, act> is a by-product of the next GEMM, so
+  // fp8 wire: the slice's first GEMM waits (in its producer warp) for the expansion kernel of the same slice. A persistent
+  // CTA takes all of an SM's shared memory, so nothing else can start beside it: that GEMM leaves a few SMs free for the
+  // expansion kernel, and it only starts once the expansion of the PREVIOUS slice has finished, so that at most one kernel
+  // is ever waiting for an expansion that still needs SMs.
+  if (fp8_ && async && j >= 1) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(j - 1) % 4], 0), "wait expansion");
+  const int spare = fp8_ && async ? kExpandSms : 0;
+  auto wait_for_rows = [&](GemmParams* p) {
+    p->arrive = fp8_ ? nullptr : reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.arrive);
+    p->pass_base = reinterpret_cast<const uint32_t*>(pass_base_.data_ptr());
+    p->ready = fp8_ ? reinterpret_cast<const uint32_t*>(ready_.data_ptr()) : nullptr;
+    p->ready_base = reinterpret_cast<const uint32_t*>(ready_base_.data_ptr());
+  };
+  // Unless the forward kept them: h and w * act again. y is not recomputed: d_weight = <g, act Wd> = <g Wd^T, act> is a by-product of the next GEMM, so
   // the down-projection GEMM that used to form <g, y> and w * g here (8 % of a step's FLOPs, 230 us per 8192-row slice at
   // D=7168, F=2048) and the w * g matrix are gone: 23.1 -> 21.4 ms per forward + backward at 32 experts, 65,536 rows.
-  {
+  if (!keep) {
     GemmParams p = base_params(pl, static_cast<int>(j));
     p.row_w = reinterpret_cast<const float*>(arena_ + arena_lay_.wbuf) + static_cast<size_t>(b) * S_;
     p.n_tiles = 2 * F_ / kBlockN;
     p.k_blocks = D_ / kBlockK;
     p.b_group_rows = D_;
-    p.arrive = fp8_ ? nullptr : reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.arrive);
-    p.pass_base = reinterpret_cast<const uint32_t*>(pass_base_.data_ptr());
-    p.ready = fp8_ ? reinterpret_cast<const uint32_t*>(ready_.data_ptr()) : nullptr;
-    p.ready_base = reinterpret_cast<const uint32_t*>(ready_base_.data_ptr());
+    wait_for_rows(&p);
     p.out0 = reinterpret_cast<__nv_bfloat16*>(act_[q].data_ptr());
     p.ld0 = F_;
     p.out1 = reinterpret_cast<__nv_bfloat16*>(h_[q].data_ptr());
     p.ld1 = 2 * F_;
-    // fp8 wire: this kernel waits (in its producer warp) for the expansion kernel of the same slice. A persistent CTA
-    // takes all of an SM's shared memory, so nothing else can start beside it: the kernel leaves a few SMs free for the
-    // expansion kernel, and it only starts once the expansion of the PREVIOUS slice has finished, so that at most one
-    // kernel is ever waiting for an expansion that still needs SMs.
-    if (fp8_ && async && j >= 1) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(j - 1) % 4], 0), "wait expansion");
-    row_gemm(kModeSwiglu, p, up_map(w_up), map_x_[b], st, fp8_ && async ? kExpandSms : 0);
+    row_gemm(kModeSwiglu, p, up_map(w_up), map_x_[b], st, spare);
+    if (async) cuda_check(cudaEventRecord(ev_up_[q], st), "event record");
   }
-  if (async) {
-    cuda_check(cudaEventRecord(ev_up_[q], st), "event record");
-    if (j >= 2) cuda_check(cudaStreamWaitEvent(st, ev_tgu_[q], 0), "wait dW_up event");  // dh, d_weight shares of slice j-2
-  }
+  if (async && j >= 2) cuda_check(cudaStreamWaitEvent(st, ev_tgu_[q], 0), "wait dW_up event");  // dh, d_weight shares of slice j-2
   {  // acc = g Wd^T; dh = SwiGLU'(h) * (w * acc), d_weight shares <acc, act>
     GemmParams p = base_params(pl, static_cast<int>(j));
     p.n_tiles = F_ / kBlockN;
     p.k_blocks = D_ / kBlockK;
     p.b_group_rows = F_;
     p.row_w = reinterpret_cast<const float*>(arena_ + arena_lay_.wbuf) + static_cast<size_t>(b) * S_;
-    p.in0 = reinterpret_cast<const __nv_bfloat16*>(h_[q].data_ptr());
+    if (keep) wait_for_rows(&p);
+    p.in0 = keep ? kept_h(j) : reinterpret_cast<const __nv_bfloat16*>(h_[q].data_ptr());
     p.out0 = reinterpret_cast<__nv_bfloat16*>(dh_[q].data_ptr());
     p.ld0 = 2 * F_;
     p.dwp = dwp_[q].data_ptr<float>();
     p.dwp_tiles = dwp_tiles;
-    row_gemm(kModeDswiglu, p, weight_map(w_down, 128), map_g_[b], st);
+    row_gemm(kModeDswiglu, p, weight_map(w_down, 128), map_g_[b], st, keep ? spare : 0);
   }
   if (async) {
     cuda_check(cudaEventRecord(ev_ds_[q], st), "event record");
-    cuda_check(cudaStreamWaitEvent(aux, ev_up_[q], 0), "wait up event");
+    // (The first GEMM of the slice saw every row arrive.)
+    cuda_check(cudaStreamWaitEvent(aux, keep ? ev_ds_[q] : ev_up_[q], 0), "wait for the first GEMM");
   }
   {  // dW_down[g] = (w act)^T g   (auxiliary stream; the fp32 carry chains slice to slice there)
     GemmParams p = base_params(pl, static_cast<int>(j));
@@ -686,9 +707,10 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     p.carry_in = carry_down_.data_ptr<float>() + static_cast<size_t>(par ^ 1) * F_ * D_;
     p.carry_out = carry_down_.data_ptr<float>() + static_cast<size_t>(par) * F_ * D_;
     p.grad_out = reinterpret_cast<__nv_bfloat16*>(dw_down.data_ptr());
-    weight_grad(p, map_act_mn_[q], map_g_mn_[b], weight_map(dw_down, 32), aux);
+    weight_grad(p, keep ? make_bf16_map_chunked(kept_act(j), kept_slice_rows(j), F_, 64, 2) : map_act_mn_[q],
+                map_g_mn_[b], weight_map(dw_down, 32), aux);
   }
-  if (async) {
+  if (async && !keep) {
     cuda_check(cudaEventRecord(ev_tgd_[q], aux), "event record");
     cuda_check(cudaStreamWaitEvent(aux, ev_ds_[q], 0), "wait dswiglu event");
   }
@@ -747,6 +769,43 @@ void FusedRank::end_pass(int64_t n_slices) {
   seq_ += static_cast<uint32_t>(n_slices);
   cur_slices_ = 0;
   inline_ = false;
+  release_kept();
+}
+
+// What a training forward keeps for its backward: h and w * act of its first `kept_slices_` slices (12 KB a row at F = 2048),
+// so that the backward starts from them instead of running the up-projection GEMM again (4 of its 16 D x F products per
+// row). Results do not change by it: the backward recomputes the same bits when it has to. Forward + backward, D=7168,
+// F=2048: 64 experts of 256 rows 7.10 -> 6.09 ms, Zipf routing in slices of 2048 rows 9.05 -> 7.80 ms, 32 experts of 1024
+// rows on the fp8 wire 12.0 -> 10.8 ms.
+void FusedRank::keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices) {
+  expect(h.is_cuda() && h.is_contiguous() && h.scalar_type() == torch::kBFloat16 && h.dim() == 2 && h.size(1) == 2 * F_ &&
+             act.is_cuda() && act.is_contiguous() && act.scalar_type() == torch::kBFloat16 && act.dim() == 2 &&
+             act.size(1) == F_ && act.size(0) == h.size(0) && act.size(0) > (slices - 1) * S_,
+         "kept activations must be contiguous CUDA bf16 [rows, 2F] and [rows, F] matrices that reach into every slice");
+  kept_h_ = h;
+  kept_act_ = act;
+  kept_slices_ = slices;
+}
+
+void FusedRank::release_kept() {
+  kept_h_ = torch::Tensor();
+  kept_act_ = torch::Tensor();
+  kept_slices_ = 0;
+}
+
+// Keeping pays once the GEMM that it saves is longer than a launch, and only while there is memory to spare: live tensors
+// and arenas, these included, stay within half of the device, else (or when the allocation fails) the backward recomputes.
+// (What the caching allocator knows, not `cudaMemGetInfo`: that call takes 2 ms with a busy device.)
+std::vector<torch::Tensor> FusedRank::allocate_kept(int64_t rows, const torch::TensorOptions& bf16) const {
+  if (std::min<int64_t>(rows, S_) * D_ * F_ < kKeepWork || !keep_activations_) return {};
+  try {
+    const auto pool = c10::cuda::CUDACachingAllocator::getDeviceStats(bf16.device().index());
+    const size_t live = static_cast<size_t>(pool.allocated_bytes[0].current) + arena_lay_.total;
+    if (live + static_cast<size_t>(rows) * 3 * F_ * 2 > device_bytes_ / 2) return {};
+    return {torch::empty({rows, 2 * F_}, bf16), torch::empty({rows, F_}, bf16)};
+  } catch (const c10::Error&) {  // no memory, or an allocator that keeps no statistics
+    return {};
+  }
 }
 
 void FusedRank::finish_forward(torch::Tensor inv_order, torch::Tensor out) {
@@ -799,9 +858,11 @@ void FusedRank::finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch
 // ---------------------------------------------------------------------------------------------
 // whole passes
 // ---------------------------------------------------------------------------------------------
-std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> FusedRank::forward_pass(
-    torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down) {
+std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass(
+    torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
+    bool training) {
   const int64_t tk = expert_ids.numel();
+  release_kept();  // (of a pass that threw)
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
   auto i32 = torch::TensorOptions().device(x.device()).dtype(torch::kInt32);
   // (The send order needs no initial values: an id the sort leaves out is recorded in the status block first, and with
@@ -834,6 +895,15 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> 
     guess = std::max<int64_t>(0, begin_forward_async(expert_ids, plan, order, inv_order, plan, false));
   }
   if (known >= 0) guess = std::min<int64_t>(known, max_slices_);
+  std::vector<torch::Tensor> kept;
+  int64_t kept_slices = 0;
+  if (training && guess > 0) {  // slices past the guess are recomputed
+    kept = allocate_kept(known >= 0 ? tk : guess * S_, x.options());
+    if (!kept.empty()) {
+      kept_slices = guess;
+      keep_rows(kept[0], kept[1], kept_slices);
+    }
+  }
   run_slices(0, guess);
   int64_t n = known;
   if (known >= 0) {
@@ -848,13 +918,18 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> 
     finish_forward(inv_order, out);
   }
   if (known >= 0) n = resolve_slices();  // the same checks, with all of the pass on its way to the device
-  return std::make_tuple(out, plan, order, inv_order, n);
+  std::vector<torch::Tensor> result{out, plan, order, inv_order};
+  result.insert(result.end(), kept.begin(), kept.end());
+  return std::make_tuple(result, n, kept_slices);
 }
 
 std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank::backward_pass(
     torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
-    torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices) {
+    torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
+    const std::vector<torch::Tensor>& kept, int64_t kept_slices) {
   inline_ = false;  // (also behind a forward that threw)
+  release_kept();
+  if (kept.size() == 2) keep_rows(kept[0], kept[1], kept_slices);
   // The slice count is the forward's: nothing is read back, the host never waits for the device here.
   const int64_t n = begin_backward(plan, known_slices, order.numel());
   torch::Tensor dw_up = torch::empty_like(w_up), dw_down = torch::empty_like(w_down), dx = torch::empty_like(x);

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <map>
+#include <algorithm>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -76,14 +77,17 @@ class FusedRank {
   void finish_forward(torch::Tensor inv_order, torch::Tensor out);
   void finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights);
 
-  // The two passes as one call each (what `chunked_moe` runs). Forward: (out, plan, order, inv_order, slice count); it
-  // throws a recorded kernel error. Backward: (dx, d_weights, dw_up, dw_down). Tensors are contiguous CUDA tensors of
-  // the workspace's geometry: x, g [T, D] bf16, expert_ids [T, K] int32, w_flat [T*K] fp32.
-  std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> forward_pass(
-      torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down);
+  // The two passes as one call each (what `chunked_moe` runs). Forward: ([out, plan, order, inv_order] and, when a
+  // `training` pass keeps them, [h, w * act]; slice count; slices kept); it throws a recorded kernel error. Backward:
+  // (dx, d_weights, dw_up, dw_down). Tensors are contiguous CUDA tensors of the workspace's geometry: x, g [T, D] bf16,
+  // expert_ids [T, K] int32, w_flat [T*K] fp32.
+  std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> forward_pass(
+      torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
+      bool training);
   std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> backward_pass(
       torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
-      torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices);
+      torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
+      const std::vector<torch::Tensor>& kept, int64_t kept_slices);
 
   // Reads the status block (synchronises); throws std::runtime_error describing the first recorded error.
   void check_status();
@@ -105,6 +109,16 @@ class FusedRank {
   void begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row);
   void end_pass(int64_t n_slices);
   void wait_header();
+  void keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices);
+  void release_kept();
+  std::vector<torch::Tensor> allocate_kept(int64_t rows, const torch::TensorOptions& bf16) const;
+  __nv_bfloat16* kept_h(int64_t j) const {
+    return reinterpret_cast<__nv_bfloat16*>(kept_h_.data_ptr()) + static_cast<size_t>(j) * S_ * 2 * F_;
+  }
+  __nv_bfloat16* kept_act(int64_t j) const {
+    return reinterpret_cast<__nv_bfloat16*>(kept_act_.data_ptr()) + static_cast<size_t>(j) * S_ * F_;
+  }
+  uint64_t kept_slice_rows(int64_t j) const { return std::min<int64_t>(S_, kept_act_.size(0) - j * S_); }
   bool overlapped() const { return use_comm_stream_ && !inline_; }
   void join_streams(bool backward);
   GemmParams base_params(const int* plan, int j) const;
@@ -128,6 +142,10 @@ class FusedRank {
 
   // local scratch (torch-owned)
   torch::Tensor act_[2], h_[2], dh_[2], dwp_[2];
+  torch::Tensor kept_h_, kept_act_;  // of the current pass: [rows, 2F], [rows, F] of its first kept_slices_ slices
+  int64_t kept_slices_ = 0;
+  size_t device_bytes_ = 0;
+  bool keep_activations_ = true;  // CEM_KEEP_ACTIVATIONS=0: always recompute (least memory)
   torch::Tensor carry_up_, carry_down_, pass_base_, expected_total_, status_, tables_,
       sort_scratch_, my_counts_;
   torch::Tensor ready_, ready_base_, ready_total_;  // fp8 wire: per-expert "rows expanded" counter, its base, its target

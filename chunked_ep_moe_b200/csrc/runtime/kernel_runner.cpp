@@ -40,11 +40,9 @@ KernelRunner::KernelRunner(int L, int S, int stripe, int num_sms)
   need(stripe == 32 || stripe == 64 || stripe == 128, "stripe must be 32, 64 or 128");
   lay_ = make_plan_layout(1, L, S, 1);
   auto i32 = torch::TensorOptions().device(torch::kCUDA).dtype(torch::kInt32);
-  auto f32 = torch::TensorOptions().device(torch::kCUDA).dtype(torch::kFloat32);
   plan_ = torch::zeros({lay_.total}, i32);
   counts_ = torch::zeros({L}, i32);
   status_ = torch::zeros({8}, i32);
-  ones_ = torch::ones({S}, f32);
   counter_ = torch::zeros({4}, i32);
   table_ = torch::zeros({2}, torch::TensorOptions().device(torch::kCUDA).dtype(torch::kInt64));
 }
@@ -115,7 +113,6 @@ void KernelRunner::gmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out, 
   const TokenMaps rows = make_token_maps(lhs.data_ptr(), S_, K);
   if (!transpose_rhs) {
     p.b_group_rows = static_cast<int>(K);
-    p.row_w = ones_.data_ptr<float>();
     const CUtensorMap w = make_bf16_map_chunked(rhs.data_ptr(), static_cast<uint64_t>(L_) * K, N, 64, 2);
     launch_row_gemm(kModeDownFwd, p, w, rows, num_sms_, stream());
   } else {

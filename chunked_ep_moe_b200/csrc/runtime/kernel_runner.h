@@ -45,7 +45,7 @@ class KernelRunner {
   GemmParams base() const;
   int L_, S_, stripe_, num_sms_;
   PlanLayout lay_;
-  torch::Tensor plan_, counts_, status_, ones_, counter_, table_;
+  torch::Tensor plan_, counts_, status_, counter_, table_;
 };
 
 }  // namespace cem

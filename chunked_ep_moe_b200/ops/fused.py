@@ -8,14 +8,16 @@ reached the host. Compared with the reference's loop
 (src/chunked_moe/moe.py:96-119, :148-206):
 
   * no `[T*K, D]` send buffer: the put kernel gathers rows straight from `x[token]`;
-  * the router weight is applied in the down-projection epilogue, which stores every finished
+  * the router weight is applied in the up-projection epilogue (`w * act`); the down-projection's stores every finished
     row into the source rank's return buffer; a local K-way fixed-order sum finishes the token;
-  * the backward recomputes the up-projection only: `d_weight = <g, act Wd>` is `<g Wd^T, act>`, a by-product of the
-    GEMM that yields `d_act = w * (g Wd^T)`, and `dW_down` contracts `w * act` with `g`; neither `y` nor `w * g` exists;
+  * `d_weight = <g, act Wd>` is `<g Wd^T, act>`, a by-product of the GEMM that yields `d_act = w * (g Wd^T)`, and
+    `dW_down` contracts `w * act` with `g`; neither `y` nor `w * g` exists;
+  * the backward starts from `h` and `w * act` where the forward could keep them (large slices, memory to spare,
+    `CEM_KEEP_ACTIVATIONS=0` never) and recomputes them, slice by slice, where it could not: the same bits either way;
   * weight gradients are written once per expert in bf16; only the (at most one) expert that
     straddles a slice boundary carries an fp32 partial to the next slice.
 
-Only the inputs and the integer plan (tables, send order, its inverse) are kept for the backward.
+Everything else the backward needs are the inputs and the integer plan (tables, send order, its inverse).
 """
 
 from __future__ import annotations
@@ -161,15 +163,16 @@ def launches() -> int:
     return sum(int(ws.rank.launches()) for ws in _workspaces.values() if ws.rank is not None)
 
 
-def expected_launches(num_slices: int, fp8: bool = False) -> int:
+def expected_launches(num_slices: int, fp8: bool = False, kept_slices: int = 0) -> int:
     """Kernels one forward+backward of the fused layer launches on a rank that loops `num_slices` slices.
 
     Forward: sort (3) + plan build + pass begin + per slice (put, swiglu, down+combine, slice done) + combine reduce.
     Backward: pass begin + per slice (put, swiglu+h, dswiglu, dW_down, d_weight return, dx+combine, dW_up, slice done)
-    + combine reduce. The fp8 wire adds one dequantisation kernel per slice and pass.
+    + combine reduce. The fp8 wire adds one dequantisation kernel per slice and pass. A slice whose activations the
+    forward kept needs no swiglu+h in the backward.
     """
     per_slice = 12 + (2 if fp8 else 0)
-    return 8 + per_slice * num_slices
+    return 8 + per_slice * num_slices - kept_slices
 
 
 def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidden: int, ffn: int, slice_size: int,
@@ -196,6 +199,7 @@ def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidd
         "expert weights (bf16)": weights,
         "expert weight gradients (bf16)": weights,
         "saved for backward (x, router weights, sort order, plan)": saved,
+        "kept for backward while memory allows (h, w * act; rows balanced over the ranks)": tk * 3 * F * 2,
     }
     out["total"] = sum(out.values())
     return out
@@ -235,30 +239,30 @@ def _require(cond: bool, msg: str) -> None:
 
 class _ChunkedMoEFused(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, expert_ids, weights, w_up, w_down, cfg, group):
+    def forward(ctx, x, expert_ids, weights, w_up, w_down, cfg, group, training):
         tokens, hidden = x.shape
         ffn = w_down.shape[1]
         ws = get_workspace(cfg, group, hidden, ffn, tokens * cfg.top_k)
         ids32 = expert_ids.to(torch.int32).contiguous()
         w_flat = weights.detach().float().reshape(-1).contiguous()
         xc, w_up_c, w_down_c = x.detach().contiguous(), w_up.detach().contiguous(), w_down.detach().contiguous()
-        out, plan, order, inv_order, n = ws.rank.forward_pass(xc, ids32, w_flat, w_up_c, w_down_c)
-        ctx.save_for_backward(xc, weights, w_up_c, w_down_c, plan, order, inv_order)
-        ctx.ws, ctx.num_slices = ws, n
+        (out, *saved), n, kept_slices = ws.rank.forward_pass(xc, ids32, w_flat, w_up_c, w_down_c, training)
+        ctx.save_for_backward(xc, weights, w_up_c, w_down_c, *saved)
+        ctx.ws, ctx.num_slices, ctx.kept_slices = ws, n, kept_slices
         ctx.mark_non_differentiable(expert_ids)
         return out
 
     @staticmethod
     def backward(ctx, g_out):
-        x, weights, w_up, w_down, plan, order, inv_order = ctx.saved_tensors
+        x, weights, w_up, w_down, plan, order, inv_order, *kept = ctx.saved_tensors
         rank = ctx.ws.rank
         if rank is None or ctx.ws.arena.local == 0:
             raise RuntimeError("chunked_moe fused path: the workspace of this pass was released before its backward")
         g = g_out.to(x.dtype).contiguous()
         w_flat = weights.detach().float().reshape(-1).contiguous()
         dx, d_weights, dw_up, dw_down = rank.backward_pass(x, g, w_flat, w_up, w_down, plan, order, inv_order,
-                                                           ctx.num_slices)
-        return dx, None, d_weights.reshape(weights.shape).to(weights.dtype), dw_up, dw_down, None, None
+                                                           ctx.num_slices, kept, ctx.kept_slices)
+        return dx, None, d_weights.reshape(weights.shape).to(weights.dtype), dw_up, dw_down, None, None, None
 
 
 def unsupported_reason(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor,
@@ -290,4 +294,5 @@ def chunked_moe_fused(x: torch.Tensor, expert_ids: torch.Tensor, weights: torch.
     _require(cfg.stripe_width in (32, 64, 128), "needs stripe_width in {32, 64, 128}")
     _require(cfg.slice_size % 8 == 0, "needs slice_size % 8 == 0")
     _require(cfg.accum_dtype == "float32", "weight gradients are accumulated in float32 (accum_dtype)")
-    return _ChunkedMoEFused.apply(x, expert_ids, weights, w_up, w_down, cfg, group)
+    training = torch.is_grad_enabled() and any(t.requires_grad for t in (x, weights, w_up, w_down))
+    return _ChunkedMoEFused.apply(x, expert_ids, weights, w_up, w_down, cfg, group, training)

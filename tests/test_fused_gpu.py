@@ -279,6 +279,43 @@ def test_one_slice_forward_equals_several_slices(tokens):
     assert outs[0].shape == x.shape and torch.equal(*outs)
 
 
+@pytest.mark.parametrize("wire", [None, "float8_e4m3fn"])
+@pytest.mark.parametrize("tokens,stripe", [(2048, 64), (3001, 128), (4097, 32)])
+def test_kept_activations_give_the_same_bits(monkeypatch, tokens, stripe, wire):
+    """A backward that starts from the forward's h and w * act equals one that recomputes them: one full slice, a ragged
+    last slice, a last slice of two rows. 4096 rows at D=2048, F=512 is the least work for which they are kept."""
+    from chunked_ep_moe_b200.ops import fused
+
+    E, K, D, F = 8, 2, 2048, 512
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    args = [rnd(tokens, D).bfloat16(), rnd(tokens, K).sigmoid(), (rnd(E, D, 2 * F) / math.sqrt(D)).bfloat16(),
+            (rnd(E, F, D) / math.sqrt(F)).bfloat16()]
+    ids = torch.topk(rnd(tokens, E), K, dim=-1).indices.int()
+    g = rnd(tokens, D).bfloat16()
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=4096, transport="nvshmem", expert_compute="fused",
+                           stripe_width=stripe, comm_dtype=wire)
+    slices = -(-tokens * K // 4096)
+    results, launched = [], []
+    for keep in ("1", "0"):
+        fused.release_workspaces()
+        monkeypatch.setenv("CEM_KEEP_ACTIVATIONS", keep)
+        x, w, w_up, w_down = [t.clone().requires_grad_(True) for t in args]
+        out = chunked_moe(x, ids, w, w_up, w_down, cfg)
+        out.backward(g, retain_graph=True)
+        first = [t.grad.clone() for t in (x, w, w_up, w_down)]
+        before = fused.launches()
+        for t in (x, w, w_up, w_down):
+            t.grad = None
+        out.backward(g)  # again: what was kept is still as it was
+        launched.append(fused.launches() - before)
+        results.append([out] + first)
+        assert all(torch.equal(a, t.grad) for a, t in zip(first, (x, w, w_up, w_down)))
+    assert launched[1] - launched[0] == slices  # no up-projection GEMM in the backward
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    fused.release_workspaces()
+
+
 def test_gemm_whose_rows_never_arrive_gives_up_and_reports(monkeypatch):
     """The real swiglu kernel waiting for rows nobody sends: its bounded wait runs out, every warp unwinds promptly
     (the barrier waits watch the CTA's abort flag), later kernels of the pass return at once, the host raises."""
