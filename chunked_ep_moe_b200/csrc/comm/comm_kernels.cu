@@ -9,6 +9,11 @@
 // the row count to the receiver's per-(source, expert) arrival counter. Receivers never take
 // part in the transfer; their GEMM producer warps acquire the counters.
 //
+// What bounds the put is the chain of dependent accesses in front of each copy (segment, send order, row), 0.6 us each with
+// 128 blocks on the device: the warp searches the segments 32 at a time, fetches its rows' send-order entries together and
+// keeps eight 16-byte loads per lane in flight. 1024 rows of x (and, in the backward, g) at D=2048, beside GEMMs: 25 -> 14.5 us
+// on average; forward + backward of eight such slices 1133 -> 977 us, 8192 tokens at D=1024 1026 -> 894 us.
+//
 // Protocol invariants:
 //   * arrival counters only grow (cumulative rows per (source, expert)); a pass's targets are
 //     base + rows expected so far, so nothing is ever reset and stale values are detectable;
@@ -27,68 +32,129 @@ namespace {
 
 constexpr int kPutThreads = 256;  // with 64 registers each it fits beside a GEMM CTA (see row_gemm.cu)
 
-__device__ __forceinline__ int find_segment(const int4* put, int n, int chunk) {
-  // Last segment whose chunk prefix is <= chunk (empty segments share a prefix with their successor).
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (put[mid].w <= chunk) lo = mid; else hi = mid - 1;
+// Last segment whose chunk prefix is <= chunk (empty segments share a prefix with their successor), for the whole warp: 32
+// prefixes at a time, two rounds for up to 1024 segments. (The first prefix is 0 and prefixes ascend.)
+__device__ __forceinline__ int find_segment(const int4* put, int n, int chunk, int lane) {
+  int lo = 0, len = n;
+  while (len > 1) {
+    const int step = (len + 31) >> 5, at = lane * step;
+    const unsigned below = __ballot_sync(0xffffffffu, at < len && put[lo + at].w <= chunk);
+    const int k = (31 - __clz(below)) * step;
+    lo += k;
+    len = len - k < step ? len - k : step;
   }
   return lo;
 }
 
-__device__ __forceinline__ void copy_row_bf16(const __nv_bfloat16* src, __nv_bfloat16* dst, int hidden, int lane) {
-  const int units = hidden >> 3;  // 16-byte units
+// Eight bf16 columns to e4m3 with one scale per 128 columns (the 16 lanes that share a block); all lanes take part.
+__device__ __forceinline__ uint2 quantise_e4m3(const int4& raw, float* scale_out) {
+  const uint32_t wds[4] = {static_cast<uint32_t>(raw.x), static_cast<uint32_t>(raw.y), static_cast<uint32_t>(raw.z),
+                           static_cast<uint32_t>(raw.w)};
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { v[2 * i] = bf16_lo(wds[i]); v[2 * i + 1] = bf16_hi(wds[i]); }
+  float amax = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+#pragma unroll
+  for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float scale = fmaxf(amax, 1e-12f) * (1.0f / 448.0f);
+  const float inv = 1.0f / scale;
+  uint32_t lo = 0, hi = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t b0 = __nv_cvt_float_to_fp8(v[i] * inv, __NV_SATFINITE, __NV_E4M3);
+    const uint32_t b1 = __nv_cvt_float_to_fp8(v[4 + i] * inv, __NV_SATFINITE, __NV_E4M3);
+    lo |= b0 << (8 * i);
+    hi |= b1 << (8 * i);
+  }
+  *scale_out = scale;
+  return make_uint2(lo, hi);
+}
+
+__device__ __forceinline__ int4 expand_e4m3(const uint2& raw, float scale) {
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half_raw h0 = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>((raw.x >> (8 * i)) & 0xFF), __NV_E4M3);
+    const __half_raw h1 = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>((raw.y >> (8 * i)) & 0xFF), __NV_E4M3);
+    v[i] = __half2float(*reinterpret_cast<const __half*>(&h0)) * scale;
+    v[4 + i] = __half2float(*reinterpret_cast<const __half*>(&h1)) * scale;
+  }
+  return make_int4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+}
+
+// Copies a chunk's rows to consecutive rows at `dst`, two rows side by side, eight 16-byte loads per lane in flight. Lane r
+// holds the token of row r, or -1 for a row that is left out.
+__device__ __forceinline__ void copy_rows(const __nv_bfloat16* src, __nv_bfloat16* dst, int lane_token, int rows,
+                                          int hidden, int lane) {
+  constexpr int kAhead = 4;
+  const int units = hidden >> 3;  // 16-byte units of a row, a multiple of 32
+#pragma unroll 1
+  for (int r = 0; r < rows; r += 2) {
+    const int t0 = __shfl_sync(0xffffffffu, lane_token, r), t1 = __shfl_sync(0xffffffffu, lane_token, r + 1);
+    const bool live0 = t0 >= 0, live1 = t1 >= 0;  // (lanes past `rows` hold -1)
+    const int4* s0 = reinterpret_cast<const int4*>(src + static_cast<size_t>(live0 ? t0 : 0) * hidden);
+    const int4* s1 = reinterpret_cast<const int4*>(src + static_cast<size_t>(live1 ? t1 : 0) * hidden);
+    int4* d = reinterpret_cast<int4*>(dst) + r * units;
+#pragma unroll 1
+    for (int u = lane; u < units; u += 32 * kAhead) {
+      int4 v0[kAhead], v1[kAhead];
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        if (u + 32 * k < units) {
+          if (live0) v0[k] = ld_nc_v4(s0 + u + 32 * k);
+          if (live1) v1[k] = ld_nc_v4(s1 + u + 32 * k);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        if (u + 32 * k < units) {
+          if (live0) d[u + 32 * k] = v0[k];
+          if (live1) d[units + u + 32 * k] = v1[k];
+        }
+      }
+    }
+  }
+}
+
+// Quantises one row to e4m3 with a scale per 128 columns.
+__device__ __forceinline__ void put_row_fp8(const __nv_bfloat16* src, uint8_t* dq, float* ds, int hidden, int lane) {
+  const int units = hidden >> 3;  // a multiple of 32
+  const int4* s = reinterpret_cast<const int4*>(src);
+  for (int u = lane; u < units; u += 32) {
+    float scale;
+    const uint2 q = quantise_e4m3(ld_nc_v4(s + u), &scale);
+    *reinterpret_cast<uint2*>(dq + static_cast<size_t>(u) * 8) = q;
+    if ((lane & 15) == 0) ds[u >> 4] = scale;
+  }
+}
+
+// One row over the fp8 wire without leaving this GPU: quantised and expanded again.
+__device__ __forceinline__ void put_row_rounded(const __nv_bfloat16* src, __nv_bfloat16* dst, int hidden, int lane) {
+  const int units = hidden >> 3;  // a multiple of 32
   const int4* s = reinterpret_cast<const int4*>(src);
   int4* d = reinterpret_cast<int4*>(dst);
-  int u = lane;
-  for (; u + 96 < units; u += 128) {
-    const int4 a = ld_nc_v4(s + u), b = ld_nc_v4(s + u + 32), c = ld_nc_v4(s + u + 64), e = ld_nc_v4(s + u + 96);
-    d[u] = a; d[u + 32] = b; d[u + 64] = c; d[u + 96] = e;
-  }
-  for (; u < units; u += 32) d[u] = ld_nc_v4(s + u);
-}
-
-// Quantises one row to e4m3 with a scale per 128 columns. 16 lanes cover one block (8 values each).
-__device__ __forceinline__ void put_row_fp8(const __nv_bfloat16* src, uint8_t* dq, float* ds, int hidden, int lane) {
-  const int units = hidden >> 3;
-  const int4* s = reinterpret_cast<const int4*>(src);
-  for (int u0 = 0; u0 < units; u0 += 32) {
-    const int u = u0 + lane;
-    float v[8];
-    if (u < units) {
-      const int4 raw = ld_nc_v4(s + u);
-      const uint32_t wds[4] = {static_cast<uint32_t>(raw.x), static_cast<uint32_t>(raw.y),
-                               static_cast<uint32_t>(raw.z), static_cast<uint32_t>(raw.w)};
+  for (int u = lane; u < units; u += 128) {
+    int4 v[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) { v[2 * i] = bf16_lo(wds[i]); v[2 * i + 1] = bf16_hi(wds[i]); }
-    } else {
+    for (int k = 0; k < 4; ++k)
+      if (u + 32 * k < units) v[k] = ld_nc_v4(s + u + 32 * k);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = 0.0f;
-    }
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
-#pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float scale = fmaxf(amax, 1e-12f) * (1.0f / 448.0f);
-    const float inv = 1.0f / scale;
-    if (u < units) {
-      uint32_t lo = 0, hi = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t b0 = __nv_cvt_float_to_fp8(v[i] * inv, __NV_SATFINITE, __NV_E4M3);
-        const uint32_t b1 = __nv_cvt_float_to_fp8(v[4 + i] * inv, __NV_SATFINITE, __NV_E4M3);
-        lo |= b0 << (8 * i);
-        hi |= b1 << (8 * i);
+    for (int k = 0; k < 4; ++k) {
+      if (u + 32 * k < units) {  // (the same in all lanes)
+        float scale;
+        const uint2 q = quantise_e4m3(v[k], &scale);
+        d[u + 32 * k] = expand_e4m3(q, scale);
       }
-      *reinterpret_cast<uint2*>(dq + static_cast<size_t>(u) * 8) = make_uint2(lo, hi);
-      if ((lane & 15) == 0) ds[u >> 4] = scale;
     }
   }
 }
 
-__global__ void __launch_bounds__(kPutThreads) dispatch_put_kernel(const PutParams p) {
+enum Wire { kWireBf16, kWireFp8, kWireRounded };
+
+template <int WIRE>
+__global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutParams p) {
   __shared__ int s_abort;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_seg = p.lay.P * p.lay.L;
@@ -119,40 +185,52 @@ __global__ void __launch_bounds__(kPutThreads) dispatch_put_kernel(const PutPara
   int pending = 0;
   auto flush = [&]() {
     __syncwarp();
-    if (lane < pending) {
-      __threadfence_system();
-      red_add_release_sys(pend_ptr, pend_cnt);
-    }
+    if (lane < pending) release_count(pend_ptr, pend_cnt, p.lay.P);
     pending = 0;
   };
   for (int c = blockIdx.x * (kPutThreads / 32) + warp; c < num_chunks; c += warps_total) {
-    const int seg = find_segment(put, n_seg, c);
+    const int seg = find_segment(put, n_seg, c, lane);
     const int4 e = put[seg];  // {send-order offset, rows, dest row, chunk prefix}
     const int r = seg / p.lay.L, l = seg - r * p.lay.L;
     const int first = (c - e.w) * kPutChunkRows;
     const int rows = min(kPutChunkRows, e.y - first);
-    for (int rr = 0; rr < rows; ++rr) {
-      const int flat = p.order[e.x + first + rr];
-      const int token = flat / p.top_k;
-      // Index check (warp-uniform): a send-order entry outside the token range or a destination row outside the
-      // slice buffer is recorded and the row is skipped, never dereferenced. The arrival is still signalled, so
-      // nothing waits for the row; the recorded status tells the host that the pass is invalid.
-      if (flat < 0 || token >= p.num_tokens || e.z + first + rr >= S) {
-        if (lane == 0)
-          report_status(p.status, kStatusBadIndex, kKernelPut, 0, p.slice, e.x + first + rr,
-                        static_cast<uint32_t>(p.num_tokens), static_cast<uint32_t>(token));
-        continue;
-      }
-      const size_t drow = static_cast<size_t>(buf) * S + e.z + first + rr;
-      if (p.peer_xq == nullptr) {
-        copy_row_bf16(p.x + static_cast<size_t>(token) * D, p.peer_x[r] + drow * D, D, lane);
-        if (p.g != nullptr) copy_row_bf16(p.g + static_cast<size_t>(token) * D, p.peer_g[r] + drow * D, D, lane);
+    const size_t drow = static_cast<size_t>(buf) * S + e.z + first;
+    int token = -1;  // of row `lane`
+    if (lane < rows) {
+      const int flat = p.order[e.x + first + lane];
+      token = flat / p.top_k;
+      // Index check: a send-order entry outside the token range or a destination row outside the slice buffer is recorded
+      // and the row is skipped, never dereferenced. The arrival is still signalled, so nothing waits for the row; the
+      // recorded status tells the host that the pass is invalid.
+      if (flat < 0 || token >= p.num_tokens || e.z + first + lane >= S) {
+        report_status(p.status, kStatusBadIndex, kKernelPut, 0, p.slice, e.x + first + lane,
+                      static_cast<uint32_t>(p.num_tokens), static_cast<uint32_t>(token));
+        token = -1;
       } else {
-        put_row_fp8(p.x + static_cast<size_t>(token) * D, p.peer_xq[r] + drow * D, p.peer_xs[r] + drow * (D >> 7), D, lane);
-        if (p.g != nullptr)
-          put_row_fp8(p.g + static_cast<size_t>(token) * D, p.peer_gq[r] + drow * D, p.peer_gs[r] + drow * (D >> 7), D, lane);
+        p.peer_w[r][drow + lane] = p.w_flat[flat];
       }
-      if (lane == 0) p.peer_w[r][drow] = p.w_flat[flat];
+    }
+    __syncwarp();
+    if constexpr (WIRE == kWireBf16) {
+#pragma unroll 1
+      for (int what = 0; what < (p.g != nullptr ? 2 : 1); ++what)  // (one copy of the loop: it fills the registers)
+        copy_rows(what ? p.g : p.x, (what ? p.peer_g[r] : p.peer_x[r]) + drow * D, token, rows, D, lane);
+    } else {
+      for (int rr = 0; rr < rows; ++rr) {
+        const int t = __shfl_sync(0xffffffffu, token, rr);
+        if (t < 0) continue;
+        const __nv_bfloat16* x = p.x + static_cast<size_t>(t) * D;
+        const __nv_bfloat16* g = p.g != nullptr ? p.g + static_cast<size_t>(t) * D : nullptr;
+        const size_t to = drow + rr;
+        if constexpr (WIRE == kWireFp8) {
+          put_row_fp8(x, p.peer_xq[r] + to * D, p.peer_xs[r] + to * (D >> 7), D, lane);
+          if (g != nullptr) put_row_fp8(g, p.peer_gq[r] + to * D, p.peer_gs[r] + to * (D >> 7), D, lane);
+        } else {
+#pragma unroll 1
+          for (int what = 0; what < (g != nullptr ? 2 : 1); ++what)
+            put_row_rounded(what ? g : x, (what ? p.peer_g[r] : p.peer_x[r]) + to * D, D, lane);
+        }
+      }
     }
     if (lane == pending) {
       pend_ptr = p.peer_arrive[r] + p.me * p.lay.L + l;
@@ -219,10 +297,7 @@ __global__ void __launch_bounds__(256) return_dw_kernel(const ReturnDwParams p) 
     if (lane == s) sent = cnt;
   }
   __syncwarp();
-  if (sent > 0) {
-    __threadfence_system();
-    red_add_release_sys(p.peer_count[lane], sent);
-  }
+  if (sent > 0) release_count(p.peer_count[lane], sent, p.lay.P);
 }
 
 __global__ void __launch_bounds__(256) combine_reduce_kernel(const CombineParams p) {
@@ -271,17 +346,7 @@ __device__ __forceinline__ void dequant_row(const uint8_t* q, const float* scale
   __nv_bfloat16* orow = out + static_cast<size_t>(row) * hidden;
   for (int u = threadIdx.x; u < units; u += blockDim.x) {
     const uint2 raw = *reinterpret_cast<const uint2*>(qrow + static_cast<size_t>(u) * 8);
-    const float scale = srow[u >> 4];
-    float v[8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const __half_raw h0 = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>((raw.x >> (8 * i)) & 0xFF), __NV_E4M3);
-      const __half_raw h1 = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>((raw.y >> (8 * i)) & 0xFF), __NV_E4M3);
-      v[i] = __half2float(*reinterpret_cast<const __half*>(&h0)) * scale;
-      v[4 + i] = __half2float(*reinterpret_cast<const __half*>(&h1)) * scale;
-    }
-    *reinterpret_cast<int4*>(orow + static_cast<size_t>(u) * 8) =
-        make_int4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+    *reinterpret_cast<int4*>(orow + static_cast<size_t>(u) * 8) = expand_e4m3(raw, srow[u >> 4]);
   }
 }
 
@@ -331,7 +396,9 @@ __global__ void wait_probe_kernel(const uint32_t* flag, uint32_t target, uint32_
 }  // namespace
 
 void launch_dispatch_put(const PutParams& p, int grid, cudaStream_t stream) {
-  dispatch_put_kernel<<<grid, kPutThreads, 0, stream>>>(p);
+  if (p.peer_xq != nullptr) dispatch_put_kernel<kWireFp8><<<grid, kPutThreads, 0, stream>>>(p);
+  else if (p.round_fp8) dispatch_put_kernel<kWireRounded><<<grid, kPutThreads, 0, stream>>>(p);
+  else dispatch_put_kernel<kWireBf16><<<grid, kPutThreads, 0, stream>>>(p);
 }
 
 void launch_slice_done(uint32_t* const* peer_credit, int num_ranks, int me, uint32_t seq, cudaStream_t stream) {

@@ -28,7 +28,9 @@ struct PutParams {
   const uint32_t* credit;           // [P] local: slices receiver r has finished with (written by r)
   uint32_t spin_limit;
   StatusBlock* status;
-  // fp8 wire (comm_dtype=float8_e4m3fn): rows travel as e4m3 + one fp32 scale per 128 columns
+  // fp8 wire (comm_dtype=float8_e4m3fn): rows travel as e4m3 + one fp32 scale per 128 columns. A rank on its own has no wire:
+  // `round_fp8` stores the values that expansion would yield, as bf16.
+  int round_fp8;
   uint8_t* const* peer_xq;          // [P] [2][S][D] e4m3, or null when rows travel in bf16
   uint8_t* const* peer_gq;
   float* const* peer_xs;            // [P] [2][S][D/128] scales

@@ -401,6 +401,18 @@ __device__ __forceinline__ void red_add_release_sys(uint32_t* p, uint32_t v) {
   asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Publishes everything this thread (and, behind a warp or block barrier, its neighbours) has stored, then adds to a counter.
+// A single rank's readers are all on this GPU: the fence need not reach the system.
+__device__ __forceinline__ void release_count(uint32_t* p, uint32_t v, int ranks) {
+  if (ranks == 1) {
+    __threadfence();
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+  } else {
+    __threadfence_system();
+    red_add_release_sys(p, v);
+  }
+}
+
 // Wrap-safe "counter has reached target" for monotonically increasing 32-bit counters.
 __device__ __forceinline__ bool reached(uint32_t seen, uint32_t target) {
   return static_cast<int32_t>(seen - target) >= 0;

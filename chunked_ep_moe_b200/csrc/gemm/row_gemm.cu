@@ -659,10 +659,7 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     if constexpr (Traits::kCombine) {
       // The group's stores are all issued before any of its warps releases its counts (also on the unwind path).
       group_sync(c.h);
-      if (lane < p.lay.P && returned > 0) {
-        __threadfence_system();
-        red_add_release_sys(p.peer_count[lane], returned);
-      }
+      if (lane < p.lay.P && returned > 0) release_count(p.peer_count[lane], returned, p.lay.P);
     }
   }
 

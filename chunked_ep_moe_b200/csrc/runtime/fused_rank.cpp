@@ -82,6 +82,7 @@ const char* status_name(int code) {
 }  // namespace
 
 ArenaLayout make_arena_layout(int P, int L, int S, int D, int tk_cap, bool fp8) {
+  fp8 = fp8 && P > 1;  // a rank on its own receives nothing over the wire (`FusedRank::expands`)
   ArenaLayout a{};
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes, 1024); return at; };
@@ -202,7 +203,7 @@ FusedRank::FusedRank(int P, int L, int me, int S, int D, int F, int K, int strip
     cuda_check(cudaStreamCreateWithPriority(&comm_stream_, cudaStreamNonBlocking, prio_high), "comm stream");
     cuda_check(cudaStreamCreateWithFlags(&aux_stream_, cudaStreamNonBlocking), "aux stream");
     for (int q = 0; q < 2; ++q) cuda_check(cudaStreamCreateWithFlags(&chain_[q], cudaStreamNonBlocking), "chain stream");
-    if (fp8_) cuda_check(cudaStreamCreateWithPriority(&expand_stream_, cudaStreamNonBlocking, prio_high), "expand stream");
+    if (expands()) cuda_check(cudaStreamCreateWithPriority(&expand_stream_, cudaStreamNonBlocking, prio_high), "expand stream");
   }
   for (int i = 0; i < 4; ++i) cuda_check(cudaEventCreateWithFlags(&ev_expand_[i], cudaEventDisableTiming), "event");
   for (int q = 0; q < 2; ++q)
@@ -410,8 +411,8 @@ void FusedRank::begin_pass(const torch::Tensor& plan, int64_t slices, int64_t ro
   cur_rows_ = rows;
   launch_pass_begin(plan.data_ptr<int>(), lay_, reinterpret_cast<uint32_t*>(expected_total_.data_ptr()),
                     reinterpret_cast<uint32_t*>(pass_base_.data_ptr()),
-                    fp8_ ? reinterpret_cast<uint32_t*>(ready_total_.data_ptr()) : nullptr,
-                    fp8_ ? reinterpret_cast<uint32_t*>(ready_base_.data_ptr()) : nullptr, st);
+                    expands() ? reinterpret_cast<uint32_t*>(ready_total_.data_ptr()) : nullptr,
+                    expands() ? reinterpret_cast<uint32_t*>(ready_base_.data_ptr()) : nullptr, st);
   ++launches_;
   ret_target_ += static_cast<uint32_t>(cur_rows_) * static_cast<uint32_t>(pieces_per_row);
   if (overlapped()) cuda_check(cudaEventRecord(ev_pass_, st), "event record");
@@ -451,7 +452,8 @@ void FusedRank::put(int64_t j, torch::Tensor plan, torch::Tensor order, torch::T
   p.credit = reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.credit);
   p.spin_limit = spin_limit_;
   p.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
-  if (fp8_) {
+  p.round_fp8 = fp8_ && !expands();
+  if (expands()) {
     p.peer_xq = table<uint8_t>(kTabXq);
     p.peer_gq = table<uint8_t>(kTabGq);
     p.peer_xs = table<float>(kTabXs);
@@ -460,7 +462,7 @@ void FusedRank::put(int64_t j, torch::Tensor plan, torch::Tensor order, torch::T
   launch_dispatch_put(p, put_blocks_, st);
   ++launches_;
   if (overlapped()) cuda_check(cudaEventRecord(ev_put_[j % 4], comm_stream_), "event record");
-  if (fp8_ && overlapped()) {
+  if (expands() && overlapped()) {
     // The expansion of slice j is issued together with its put, one slice ahead of the GEMMs: it waits for arrivals
     // expert by expert while slice j-1 computes. It may overwrite the bf16 slice buffer once slice j-2 is done with it.
     if (j == 0) cuda_check(cudaStreamWaitEvent(expand_stream_, ev_pass_, 0), "wait pass event");
@@ -589,15 +591,15 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
   const int b = static_cast<int>(seq & 1u);
   const int* pl = plan.data_ptr<int>();
   const bool keep = j < kept_slices_;
-  if (fp8_ && !async) dequant(pl, static_cast<int>(j), b, /*with_g=*/false, st);  // lockstep: every put is done
+  if (expands() && !async) dequant(pl, static_cast<int>(j), b, /*with_g=*/false, st);  // lockstep: every put is done
   {
     GemmParams p = base_params(pl, static_cast<int>(j));
     p.n_tiles = 2 * F_ / kBlockN;
     p.k_blocks = D_ / kBlockK;
     p.b_group_rows = D_;
-    p.arrive = fp8_ ? nullptr : reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.arrive);
+    p.arrive = expands() ? nullptr : reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.arrive);
     p.pass_base = reinterpret_cast<const uint32_t*>(pass_base_.data_ptr());
-    p.ready = fp8_ ? reinterpret_cast<const uint32_t*>(ready_.data_ptr()) : nullptr;
+    p.ready = expands() ? reinterpret_cast<const uint32_t*>(ready_.data_ptr()) : nullptr;
     p.ready_base = reinterpret_cast<const uint32_t*>(ready_base_.data_ptr());
     p.row_w = reinterpret_cast<const float*>(arena_ + arena_lay_.wbuf) + static_cast<size_t>(b) * S_;
     p.out0 = keep ? kept_act(j) : reinterpret_cast<__nv_bfloat16*>(act_[q].data_ptr());
@@ -608,8 +610,8 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
     // takes all of an SM's shared memory, so nothing else can start beside it: the kernel leaves a few SMs free for the
     // expansion kernel, and it only starts once the expansion of the PREVIOUS slice has finished, so that at most one
     // kernel is ever waiting for an expansion that still needs SMs.
-    if (fp8_ && async && j >= 1) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(j - 1) % 4], 0), "wait expansion");
-    row_gemm(kModeSwiglu, p, up_map(w_up), map_x_[b], st, fp8_ && async ? kExpandSms : 0);
+    if (expands() && async && j >= 1) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(j - 1) % 4], 0), "wait expansion");
+    row_gemm(kModeSwiglu, p, up_map(w_up), map_x_[b], st, expands() && async ? kExpandSms : 0);
   }
   {
     GemmParams p = base_params(pl, static_cast<int>(j));
@@ -650,17 +652,17 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
   const int* pl = plan.data_ptr<int>();
   const int par = static_cast<int>(j & 1);
   const int dwp_tiles = F_ / 32;
-  if (fp8_ && !async) dequant(pl, static_cast<int>(j), b, /*with_g=*/true, st);  // lockstep: every put is done
+  if (expands() && !async) dequant(pl, static_cast<int>(j), b, /*with_g=*/true, st);  // lockstep: every put is done
   // fp8 wire: the slice's first GEMM waits (in its producer warp) for the expansion kernel of the same slice. A persistent
   // CTA takes all of an SM's shared memory, so nothing else can start beside it: that GEMM leaves a few SMs free for the
   // expansion kernel, and it only starts once the expansion of the PREVIOUS slice has finished, so that at most one kernel
   // is ever waiting for an expansion that still needs SMs.
-  if (fp8_ && async && j >= 1) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(j - 1) % 4], 0), "wait expansion");
-  const int spare = fp8_ && async ? kExpandSms : 0;
+  if (expands() && async && j >= 1) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(j - 1) % 4], 0), "wait expansion");
+  const int spare = expands() && async ? kExpandSms : 0;
   auto wait_for_rows = [&](GemmParams* p) {
-    p->arrive = fp8_ ? nullptr : reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.arrive);
+    p->arrive = expands() ? nullptr : reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.arrive);
     p->pass_base = reinterpret_cast<const uint32_t*>(pass_base_.data_ptr());
-    p->ready = fp8_ ? reinterpret_cast<const uint32_t*>(ready_.data_ptr()) : nullptr;
+    p->ready = expands() ? reinterpret_cast<const uint32_t*>(ready_.data_ptr()) : nullptr;
     p->ready_base = reinterpret_cast<const uint32_t*>(ready_base_.data_ptr());
   };
   // Unless the forward kept them: h and w * act again. y is not recomputed: d_weight = <g, act Wd> = <g Wd^T, act> is a by-product of the next GEMM, so
@@ -758,7 +760,7 @@ void FusedRank::join_streams(bool backward) {
   if (!overlapped() || cur_slices_ <= 0) return;
   cudaStream_t st = current_stream();
   cuda_check(cudaStreamWaitEvent(st, ev_done_[(cur_slices_ - 1) % 4], 0), "join aux stream");
-  if (fp8_) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(cur_slices_ - 1) % 4], 0), "join expand stream");
+  if (expands()) cuda_check(cudaStreamWaitEvent(st, ev_expand_[(cur_slices_ - 1) % 4], 0), "join expand stream");
   if (backward) {
     cuda_check(cudaStreamWaitEvent(st, ev_dx_[(cur_slices_ - 1) & 1], 0), "join chain stream");
     if (cur_slices_ >= 2) cuda_check(cudaStreamWaitEvent(st, ev_dx_[cur_slices_ & 1], 0), "join chain stream");
@@ -886,9 +888,8 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
   const int64_t known = P_ == 1 ? (tk + S_ - 1) / S_ : -1;
   // A single slice of one rank: put, GEMMs and combine only follow one another, so they go to the caller's stream and the
   // events that tie the streams together are saved (one-token decode 82 -> 77 us, 2000 tokens at D=2048 195 -> 190 us).
-  // The backward keeps its streams: its weight gradients fill the other GEMMs' tails (same layer 542 us, else 558 us). The
-  // fp8 wire keeps its expansion beside the GEMM.
-  inline_ = use_comm_stream_ && known == 1 && !fp8_;
+  // The backward keeps its streams: its weight gradients fill the other GEMMs' tails (same layer 542 us, else 558 us).
+  inline_ = use_comm_stream_ && known == 1;
   int64_t guess;
   {
     NvtxRange range("chunked_moe/plan");

@@ -316,6 +316,39 @@ def test_kept_activations_give_the_same_bits(monkeypatch, tokens, stripe, wire):
     fused.release_workspaces()
 
 
+@pytest.mark.parametrize("hidden", [256, 768, 1280])
+@pytest.mark.parametrize("group_rows", [[1, 2, 3, 4], [5, 0, 7, 64], [0, 0, 0, 130]], ids=str)
+def test_one_rank_fp8_wire_rounds_like_the_wire(group_rows, hidden):
+    """One rank's fp8 wire stores expanded rows at once: bit for bit the bf16 wire on rows that were quantised and expanded
+    beforehand, forward and backward. Segments around the put's chunks of four rows, rows of 1, 3 and 5 x 256 columns."""
+    gen = torch.Generator().manual_seed(hidden)
+    E, K, D, F = 4, 2, hidden, 256
+    ids = _ids_with_groups(group_rows, K, E, gen).cuda()
+    T = ids.shape[0]
+    bf = lambda t: t.cuda().to(torch.bfloat16)
+    x, g = bf(torch.randn(T, D, generator=gen)), bf(torch.randn(T, D, generator=gen))
+    x[0, :128] = 0.0  # a block of zeros takes the smallest scale
+    weights = (torch.rand(T, K, generator=gen) + 0.1).cuda()
+    w_up = bf(torch.randn(E, D, 2 * F, generator=gen) / math.sqrt(D))
+    w_down = bf(torch.randn(E, F, D, generator=gen) / math.sqrt(F))
+
+    def rounded(t):  # the kernels' arithmetic, step by step in fp32
+        v = t.float().reshape(T, -1, 128)
+        scale = v.abs().amax(-1, keepdim=True).clamp_min(1e-12) * torch.tensor(1.0 / 448.0, device="cuda")
+        q = (v * scale.reciprocal()).clamp(-448.0, 448.0).to(torch.float8_e4m3fn)
+        return (q.float() * scale).reshape(T, -1).bfloat16()
+
+    results = []
+    for wire, xi, gi in (("float8_e4m3fn", x, g), (None, rounded(x), rounded(g))):
+        cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=64, transport="nvshmem", expert_compute="fused",
+                               stripe_width=64, comm_dtype=wire)
+        leaves = [t.clone().requires_grad_(True) for t in (xi, weights, w_up, w_down)]
+        out = chunked_moe(leaves[0], ids, *leaves[1:], cfg)
+        out.backward(gi)
+        results.append([out.detach()] + [t.grad for t in leaves])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
 def test_gemm_whose_rows_never_arrive_gives_up_and_reports(monkeypatch):
     """The real swiglu kernel waiting for rows nobody sends: its bounded wait runs out, every warp unwinds promptly
     (the barrier waits watch the CTA's abort flag), later kernels of the pass return at once, the host raises."""
