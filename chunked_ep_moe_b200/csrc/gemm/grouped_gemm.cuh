@@ -73,8 +73,11 @@ struct GemmParams {
   int dwp_tiles;
   int ld0, ld1;
   // --- combine targets (down_fwd, dx) --------------------------------------------------------
-  __nv_bfloat16* const* peer_rows;   // [P] base of each source rank's [T*K, ld] return buffer
-  uint32_t* const* peer_count;       // [P] each source rank's returned-row counter
+  __nv_bfloat16* const* peer_rows;   // [P] base of each source rank's [T*K, ld] return buffer; null: rows go to out0
+  uint32_t* const* peer_count;       // [P] each source rank's returned-row counter; null: nobody waits for the rows
+  // --- kernel-level entry points: rows of an output past the groups' last one (up to S) are set to zero -----------
+  __nv_bfloat16* tail[2];            // base of an output, or null
+  int tail_cols[2];
   // --- tgmm ---------------------------------------------------------------------------------
   const float* carry_in;   // [M, N] fp32 partial of the expert that straddles the previous slice boundary
   float* carry_out;        // [M, N] fp32 partial of the expert that straddles the next slice boundary

@@ -276,9 +276,10 @@ __device__ __forceinline__ void combine_epilogue(const GemmParams& p, const RowT
       const int row = (c.gt >> 4) + i * 8;
       const int4 v = ld_shared_v4(staged<256>(buf, row, piece));
       const uint32_t d = dst[list0 + row];
-      if (d != ~0u)
-        *reinterpret_cast<int4*>(p.peer_rows[d >> 27] + static_cast<size_t>(d & ((1u << 27) - 1)) * p.ld0 + col +
-                                 piece * 8) = v;
+      if (d != ~0u) {
+        __nv_bfloat16* base = p.peer_rows != nullptr ? p.peer_rows[d >> 27] : p.out0;
+        *reinterpret_cast<int4*>(base + static_cast<size_t>(d & ((1u << 27) - 1)) * p.ld0 + col + piece * 8) = v;
+      }
     }
   }
   if (c.h >= chunks) release();
@@ -375,6 +376,19 @@ __device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowT
                     ld_bytes, nvalid);
   }
   if (c.h >= chunks) release();
+}
+
+// Zeroes an output's rows past the groups' last one, a row per CTA and turn, by the epilogue warps while the first tile is
+// being made. (A fill of the whole output in front of the kernel took 6 us and a launch per output of 4096 x 4096.)
+__device__ __forceinline__ void zero_tail(const GemmParams& p, int thread) {
+  for (int i = 0; i < 2; ++i) {
+    if (p.tail[i] == nullptr) continue;
+    const int units = p.tail_cols[i] >> 3;
+    for (int row = p.plan[1] + blockIdx.x; row < p.lay.S; row += gridDim.x) {
+      int4* at = reinterpret_cast<int4*>(p.tail[i] + static_cast<size_t>(row) * p.tail_cols[i]);
+      for (int u = thread; u < units; u += 8 * 32) at[u] = make_int4(0, 0, 0, 0);
+    }
+  }
 }
 
 // 152 registers per thread: 320 threads x 152 leave room in the register file for a 256-thread, 64-register copy CTA (the
@@ -604,6 +618,7 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     uint32_t* s_dst = reinterpret_cast<uint32_t*>(staging_gen + c.h * kGroupStaging + 8192);
     uint32_t tcount = 0, returned = 0;
     long long epi_wait = 0;
+    zero_tail(p, (warp - 2) * 32 + lane);
     RowTile nxt = {};
     if (first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, num_entries);
     for (int t = first_tile; t < num_tiles; t += tile_step, ++tcount) {
@@ -659,7 +674,7 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     if constexpr (Traits::kCombine) {
       // The group's stores are all issued before any of its warps releases its counts (also on the unwind path).
       group_sync(c.h);
-      if (lane < p.lay.P && returned > 0) release_count(p.peer_count[lane], returned, p.lay.P);
+      if (p.peer_count != nullptr && lane < p.lay.P && returned > 0) release_count(p.peer_count[lane], returned, p.lay.P);
     }
   }
 

@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams 
   // 1. publish my histogram row into every rank's traffic matrix (row index = me)
   for (int r = 0; r < P; ++r) {
     int* dst = (p.peer_counts != nullptr ? p.peer_counts[r] : p.counts) + p.me * n;
+    if (dst == p.my_counts) continue;  // the caller's histogram is the matrix
     for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = p.my_counts[i];
   }
   __syncthreads();

@@ -41,17 +41,14 @@ KernelRunner::KernelRunner(int L, int S, int stripe, int num_sms)
   lay_ = make_plan_layout(1, L, S, 1);
   auto i32 = torch::TensorOptions().device(torch::kCUDA).dtype(torch::kInt32);
   plan_ = torch::zeros({lay_.total}, i32);
-  counts_ = torch::zeros({L}, i32);
   status_ = torch::zeros({8}, i32);
-  counter_ = torch::zeros({4}, i32);
-  table_ = torch::zeros({2}, torch::TensorOptions().device(torch::kCUDA).dtype(torch::kInt64));
 }
 
 void KernelRunner::set_groups(torch::Tensor group_rows) {
   need(group_rows.is_cuda() && group_rows.scalar_type() == torch::kInt32 && group_rows.is_contiguous() &&
            group_rows.numel() == L_,
        "group_rows must be a contiguous CUDA int32 tensor of L elements");
-  counts_.copy_(group_rows, /*non_blocking=*/true);
+  counts_ = group_rows;  // read by the plan kernel on this stream
   PlanKernelParams pp{};
   pp.lay = lay_;
   pp.me = 0;
@@ -91,6 +88,10 @@ void KernelRunner::gmm_swiglu(torch::Tensor x, torch::Tensor w_up, torch::Tensor
   p.ld0 = static_cast<int>(F2 / 2);
   p.out1 = h.has_value() ? reinterpret_cast<__nv_bfloat16*>(h->data_ptr()) : nullptr;
   p.ld1 = static_cast<int>(F2);
+  p.tail[0] = p.out0;
+  p.tail_cols[0] = p.ld0;
+  p.tail[1] = p.out1;
+  p.tail_cols[1] = p.ld1;
   const CUtensorMap w = make_bf16_map_chunked(w_up.data_ptr(), static_cast<uint64_t>(L_) * D, F2, 64, stripe_ == 128 ? 1 : 2);
   launch_row_gemm(kModeSwiglu, p, w, make_token_maps(x.data_ptr(), S_, D), num_sms_, stream());
 }
@@ -101,15 +102,14 @@ void KernelRunner::gmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out, 
   need(K % 64 == 0 && N % 256 == 0, "needs K % 64 == 0 and N % 256 == 0");
   need_bf16(lhs, S_, K, "lhs");
   need_bf16(out, S_, N, "out");
-  // One "rank": rows go back to where they came from, which is their own position in `out`.
-  const int64_t ptrs[2] = {reinterpret_cast<int64_t>(out.data_ptr()), reinterpret_cast<int64_t>(counter_.data_ptr())};
-  cudaMemcpyAsync(table_.data_ptr(), ptrs, sizeof(ptrs), cudaMemcpyHostToDevice, stream());
+  // Rows go back to where they came from, which is their own position in `out`.
   GemmParams p = base();
   p.n_tiles = static_cast<int>(N / kBlockN);
   p.k_blocks = static_cast<int>(K / kBlockK);
   p.ld0 = static_cast<int>(N);
-  p.peer_rows = reinterpret_cast<__nv_bfloat16* const*>(table_.data_ptr<int64_t>());
-  p.peer_count = reinterpret_cast<uint32_t* const*>(table_.data_ptr<int64_t>() + 1);
+  p.out0 = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
+  p.tail[0] = p.out0;
+  p.tail_cols[0] = p.ld0;
   const TokenMaps rows = make_token_maps(lhs.data_ptr(), S_, K);
   if (!transpose_rhs) {
     p.b_group_rows = static_cast<int>(K);
@@ -136,7 +136,7 @@ void KernelRunner::gmm_down_dw(torch::Tensor act, torch::Tensor w_down, torch::T
            dwp.size(0) == S_ && dwp.size(1) == D / kBlockN,
        "dwp must be a contiguous CUDA fp32 [S, D/256] tensor");
   // The grouped GEMM, then plain tensor ops (the layer itself forms neither y nor w * g, see FusedRank::compute_backward).
-  torch::Tensor y = torch::zeros_like(g);
+  torch::Tensor y = torch::empty_like(g);
   gmm(act, w_down, y, false);
   const torch::Tensor live = (torch::arange(S_, counts_.options()) < counts_.sum()).unsqueeze(1);
   const torch::Tensor gf = g.to(torch::kFloat32);
@@ -158,6 +158,8 @@ void KernelRunner::gmm_dswiglu(torch::Tensor dy, torch::Tensor w_down, torch::Te
   p.in0 = reinterpret_cast<const __nv_bfloat16*>(h.data_ptr());
   p.out0 = reinterpret_cast<__nv_bfloat16*>(dh.data_ptr());
   p.ld0 = static_cast<int>(2 * F);
+  p.tail[0] = p.out0;
+  p.tail_cols[0] = p.ld0;
   const CUtensorMap w = make_bf16_map_2d(w_down.data_ptr(), static_cast<uint64_t>(L_) * F, D, 128);
   launch_row_gemm(kModeDswiglu, p, w, make_token_maps(dy.data_ptr(), S_, D), num_sms_, stream());
 }

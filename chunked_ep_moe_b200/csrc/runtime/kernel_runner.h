@@ -27,6 +27,7 @@ class KernelRunner {
 
   // rows per expert, int32 [L] on the device, sum <= S
   void set_groups(torch::Tensor group_rows);
+  // (Row-wise results: rows past the last group are set to zero.)
   // act[S,F] = silu(x Wg) * (x Wu) from striped w_up [L,D,2F]; h [S,2F] (the rounded pre-activation) is optional
   void gmm_swiglu(torch::Tensor x, torch::Tensor w_up, torch::Tensor act, c10::optional<torch::Tensor> h);
   // out[S,N] = lhs[S,K] rhs[g]; rhs is [L,K,N], or [L,N,K] with transpose_rhs (no transpose is materialised)
@@ -45,7 +46,7 @@ class KernelRunner {
   GemmParams base() const;
   int L_, S_, stripe_, num_sms_;
   PlanLayout lay_;
-  torch::Tensor plan_, counts_, status_, counter_, table_;
+  torch::Tensor plan_, counts_, status_;
 };
 
 }  // namespace cem

@@ -52,55 +52,73 @@ def _prepare(rows_tensor: torch.Tensor, num_groups: int, group_sizes, stripe: in
     return runner
 
 
-def gmm(lhs: torch.Tensor, rhs: torch.Tensor, group_sizes, *, transpose_rhs: bool = False,
-        stripe: int = 64) -> torch.Tensor:
-    """`out[rows_g] = lhs[rows_g] @ rhs[g]` (`rhs [L, K, N]`), or `@ rhs[g]^T` (`rhs [L, N, K]`) with `transpose_rhs`."""
-    runner = _prepare(lhs, rhs.shape[0], group_sizes, stripe)
-    out = lhs.new_zeros((lhs.shape[0], rhs.shape[1] if transpose_rhs else rhs.shape[2]))
+def _rows(runner, like: torch.Tensor, cols: int) -> torch.Tensor:
+    """An output of the runner's kernels: they write the groups' rows and set the rows past the last group to zero."""
+    return torch.empty((like.shape[0], cols), dtype=like.dtype, device=like.device)
+
+
+def _gmm(runner, lhs, rhs, transpose_rhs):
+    out = _rows(runner, lhs, rhs.shape[1] if transpose_rhs else rhs.shape[2])
     runner.gmm(lhs.contiguous(), rhs.contiguous(), out, transpose_rhs)
     return out
 
 
-def gmm_swiglu(x: torch.Tensor, w_up: torch.Tensor, group_sizes, *, stripe: int,
-               return_h: bool = False) -> tuple[torch.Tensor, Optional[torch.Tensor]]:
-    """`act = silu(x Wg) * (x Wu)` from the striped `w_up [L, D, 2F]`; with `return_h` also the rounded `h [S, 2F]`."""
-    runner = _prepare(x, w_up.shape[0], group_sizes, stripe)
-    act = x.new_zeros((x.shape[0], w_up.shape[2] // 2))
-    h = x.new_zeros((x.shape[0], w_up.shape[2])) if return_h else None
+def _gmm_swiglu(runner, x, w_up, return_h):
+    act = _rows(runner, x, w_up.shape[2] // 2)
+    h = _rows(runner, x, w_up.shape[2]) if return_h else None
     runner.gmm_swiglu(x.contiguous(), w_up.contiguous(), act, h)
     return act, h
 
 
-def gmm_dswiglu(dy: torch.Tensor, w_down: torch.Tensor, h: torch.Tensor, group_sizes, *, stripe: int) -> torch.Tensor:
-    """`dh = SwiGLU'(h) * (dy @ w_down[g]^T)`: the gradient of the striped pre-activation; `d_act` never leaves the SM."""
-    runner = _prepare(dy, w_down.shape[0], group_sizes, stripe)
-    dh = torch.zeros_like(h)
+def _gmm_dswiglu(runner, dy, w_down, h):
+    dh = _rows(runner, h, h.shape[1])
     runner.gmm_dswiglu(dy.contiguous(), w_down.contiguous(), h.contiguous(), dh)
     return dh
 
 
-def tgmm(lhs: torch.Tensor, rhs: torch.Tensor, group_sizes, *, stripe: int = 64) -> torch.Tensor:
-    """`out[g] = lhs[rows_g]^T @ rhs[rows_g]` -> `[L, lhs_cols, rhs_cols]` (bf16; fp32 accumulation over the rows)."""
-    num_groups = len(group_sizes)
-    runner = _prepare(lhs, num_groups, group_sizes, stripe)
+def _tgmm(runner, lhs, rhs, num_groups):
     out = lhs.new_empty((num_groups, lhs.shape[1], rhs.shape[1]))
     runner.tgmm(lhs.contiguous(), rhs.contiguous(), out)
     return out
 
 
+def gmm(lhs: torch.Tensor, rhs: torch.Tensor, group_sizes, *, transpose_rhs: bool = False,
+        stripe: int = 64) -> torch.Tensor:
+    """`out[rows_g] = lhs[rows_g] @ rhs[g]` (`rhs [L, K, N]`), or `@ rhs[g]^T` (`rhs [L, N, K]`) with `transpose_rhs`."""
+    return _gmm(_prepare(lhs, rhs.shape[0], group_sizes, stripe), lhs, rhs, transpose_rhs)
+
+
+def gmm_swiglu(x: torch.Tensor, w_up: torch.Tensor, group_sizes, *, stripe: int,
+               return_h: bool = False) -> tuple[torch.Tensor, Optional[torch.Tensor]]:
+    """`act = silu(x Wg) * (x Wu)` from the striped `w_up [L, D, 2F]`; with `return_h` also the rounded `h [S, 2F]`."""
+    return _gmm_swiglu(_prepare(x, w_up.shape[0], group_sizes, stripe), x, w_up, return_h)
+
+
+def gmm_dswiglu(dy: torch.Tensor, w_down: torch.Tensor, h: torch.Tensor, group_sizes, *, stripe: int) -> torch.Tensor:
+    """`dh = SwiGLU'(h) * (dy @ w_down[g]^T)`: the gradient of the striped pre-activation; `d_act` never leaves the SM."""
+    return _gmm_dswiglu(_prepare(dy, w_down.shape[0], group_sizes, stripe), dy, w_down, h)
+
+
+def tgmm(lhs: torch.Tensor, rhs: torch.Tensor, group_sizes, *, stripe: int = 64) -> torch.Tensor:
+    """`out[g] = lhs[rows_g]^T @ rhs[rows_g]` -> `[L, lhs_cols, rhs_cols]` (bf16; fp32 accumulation over the rows)."""
+    return _tgmm(_prepare(lhs, len(group_sizes), group_sizes, stripe), lhs, rhs, len(group_sizes))
+
+
 def expert_forward(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, group_sizes, *, stripe: int,
                    need_residuals: bool = True) -> tuple[torch.Tensor, Optional[ForwardResiduals]]:
-    act, h = gmm_swiglu(x, w_up, group_sizes, stripe=stripe, return_h=need_residuals)
-    y = gmm(act, w_down, group_sizes, stripe=stripe)
+    runner = _prepare(x, w_up.shape[0], group_sizes, stripe)  # one build of the tile tables for the call's kernels
+    act, h = _gmm_swiglu(runner, x, w_up, need_residuals)
+    y = _gmm(runner, act, w_down, False)
     return y, (ForwardResiduals(h=h, act=act) if need_residuals else None)
 
 
 def expert_backward(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, group_sizes, res: ForwardResiduals,
                     dy: torch.Tensor, *, stripe: int) -> ExpertGrads:
-    dh = gmm_dswiglu(dy, w_down, res.h, group_sizes, stripe=stripe)
-    return ExpertGrads(dx=gmm(dh, w_up, group_sizes, transpose_rhs=True, stripe=stripe),
-                       dw_up=tgmm(x, dh, group_sizes, stripe=stripe),
-                       dw_down=tgmm(res.act, dy, group_sizes, stripe=stripe))
+    groups = w_up.shape[0]
+    runner = _prepare(dy, groups, group_sizes, stripe)
+    dh = _gmm_dswiglu(runner, dy, w_down, res.h)
+    return ExpertGrads(dx=_gmm(runner, dh, w_up, True), dw_up=_tgmm(runner, x, dh, groups),
+                       dw_down=_tgmm(runner, res.act, dy, groups))
 
 
 def check_status() -> None:

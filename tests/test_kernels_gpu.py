@@ -133,3 +133,18 @@ def test_down_gemm_with_d_weight_epilogue():
     _close(dwp.sum(dim=1), (g[:rows].float() * y.float()).sum(dim=-1), "d_weight", rows)
     fx.check_status()
     del _build
+
+
+@pytest.mark.parametrize("groups", [[0, 0, 0], [0, 1, 0], [40, 0, 87], [64, 1, 63], [500, 7, 2]], ids=str)
+def test_rows_past_the_groups_are_zero(groups):
+    """The kernels write their outputs' padding rows themselves: none, all, and counts around the grid's CTAs."""
+    S, D, F = (128 if sum(groups) <= 128 else 1024), 256, 512
+    x, dy, w_up, w_down, rows = _inputs(S, D, F, groups)
+    junk = [torch.full((S, 2 * F), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(8)]
+    del junk  # the outputs are likely to land on these
+    y, res = fx.expert_forward(x, w_up, w_down, groups, stripe=64)
+    dh = fx.gmm_dswiglu(dy, w_down, res.h, groups, stripe=64)
+    grads = fx.expert_backward(x, w_up, w_down, groups, res, dy, stripe=64)
+    for name, t in (("y", y), ("h", res.h), ("act", res.act), ("dh", dh), ("dx", grads.dx)):
+        assert torch.count_nonzero(t[rows:]) == 0 and torch.isfinite(t).all(), name
+    fx.check_status()
