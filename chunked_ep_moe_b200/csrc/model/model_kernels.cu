@@ -7,6 +7,8 @@
 
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 namespace cem {
 
 namespace {
@@ -17,7 +19,6 @@ __device__ __forceinline__ uint32_t bf_pack(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-__device__ __forceinline__ float bf_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -28,37 +29,49 @@ __device__ __forceinline__ float warp_sum(float v) {
 constexpr int kNormThreads = 256;  // 8 warps, one row per warp at a time
 constexpr int kMaxNormUnits = 8;   // 16-byte units per lane: rows of up to 8 * 32 * 8 = 2048 columns
 
+// The norm kernels are instantiated per number of 16-byte units a lane holds of a row (UNITS): sized for 2048 columns, the
+// 1024-column norms of the decoder paid for twice the registers and ran with 8 warps per SM. All of a row's loads go out
+// before the first value is used. 8192 rows of 1024 columns: forward 18 -> 10.5 us,
+// backward 37 -> 13.4 us, its column sums 11.6 -> 4.6 us (67 MB take 10.2 us at the measured copy rate).
+
+__device__ __forceinline__ void unpack8(const int4& v, float (&f)[8]) {
+  const uint32_t w[4] = {(uint32_t)v.x, (uint32_t)v.y, (uint32_t)v.z, (uint32_t)v.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) { f[2 * e] = bf_lo(w[e]); f[2 * e + 1] = bf_hi(w[e]); }
+}
+
 // s = x + delta (rounded to bf16, as the unfused residual add stores it); y = s * rsqrt(mean(s^2) + eps) * w.
-__global__ void __launch_bounds__(kNormThreads) add_rms_norm_fwd_kernel(const __nv_bfloat16* x,
-                                                                        const __nv_bfloat16* delta,
-                                                                        const __nv_bfloat16* w, __nv_bfloat16* s_out,
-                                                                        __nv_bfloat16* y, float* rstd_out, int rows,
-                                                                        int cols, float eps) {
+template <int UNITS>
+__global__ void __launch_bounds__(kNormThreads, UNITS <= 4 ? 3 : 1)
+add_rms_norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* delta, const __nv_bfloat16* w,
+                        __nv_bfloat16* s_out, __nv_bfloat16* y, float* rstd_out, int rows, int cols, float eps) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int units = cols >> 3, per_lane = (units + 31) >> 5;
+  const int units = cols >> 3;
+  const int4 zero = make_int4(0, 0, 0, 0);
   for (int row = blockIdx.x * (kNormThreads / 32) + warp; row < rows; row += gridDim.x * (kNormThreads / 32)) {
     const int4* xr = reinterpret_cast<const int4*>(x + static_cast<size_t>(row) * cols);
-    const int4* dr = delta ? reinterpret_cast<const int4*>(delta + static_cast<size_t>(row) * cols) : nullptr;
-    float v[kMaxNormUnits][8];
+    const int4* dr = reinterpret_cast<const int4*>(delta + static_cast<size_t>(row) * cols);
+    int4 a[UNITS], b[UNITS];
+#pragma unroll
+    for (int i = 0; i < UNITS; ++i) {
+      const int u = lane + 32 * i;
+      a[i] = u < units ? xr[u] : zero;
+      b[i] = delta != nullptr && u < units ? dr[u] : zero;
+    }
     float ss = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kMaxNormUnits; ++i) {
-      const int u = lane + 32 * i;
-      if (i < per_lane && u < units) {
-        const int4 a = xr[u];
-        const uint32_t aw[4] = {(uint32_t)a.x, (uint32_t)a.y, (uint32_t)a.z, (uint32_t)a.w};
-        uint32_t bw[4] = {0, 0, 0, 0};
-        if (dr) {
-          const int4 b = dr[u];
-          bw[0] = (uint32_t)b.x; bw[1] = (uint32_t)b.y; bw[2] = (uint32_t)b.z; bw[3] = (uint32_t)b.w;
-        }
+    for (int i = 0; i < UNITS; ++i) {
+      float av[8], bv[8];
+      unpack8(a[i], av);
+      unpack8(b[i], bv);
+      uint32_t so[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float lo = bf_round(bf_lo(aw[e]) + bf_lo(bw[e])), hi = bf_round(bf_hi(aw[e]) + bf_hi(bw[e]));
-          v[i][2 * e] = lo; v[i][2 * e + 1] = hi;
-          ss += lo * lo + hi * hi;
-        }
+      for (int e = 0; e < 4; ++e) {
+        so[e] = bf_pack(av[2 * e] + bv[2 * e], av[2 * e + 1] + bv[2 * e + 1]);
+        const float lo = bf_lo(so[e]), hi = bf_hi(so[e]);
+        ss += lo * lo + hi * hi;
       }
+      a[i] = make_int4(so[0], so[1], so[2], so[3]);
     }
     ss = warp_sum(ss);
     const float rstd = rsqrtf(ss / cols + eps);
@@ -67,18 +80,16 @@ __global__ void __launch_bounds__(kNormThreads) add_rms_norm_fwd_kernel(const __
     int4* sr = reinterpret_cast<int4*>(s_out + static_cast<size_t>(row) * cols);
     int4* yr = reinterpret_cast<int4*>(y + static_cast<size_t>(row) * cols);
 #pragma unroll
-    for (int i = 0; i < kMaxNormUnits; ++i) {
+    for (int i = 0; i < UNITS; ++i) {
       const int u = lane + 32 * i;
-      if (i < per_lane && u < units) {
-        const int4 wv = wr[u];
-        const uint32_t ww[4] = {(uint32_t)wv.x, (uint32_t)wv.y, (uint32_t)wv.z, (uint32_t)wv.w};
-        uint32_t so[4], yo[4];
+      if (u < units) {
+        float v[8], wv[8];
+        unpack8(a[i], v);
+        unpack8(wr[u], wv);
+        uint32_t yo[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          so[e] = bf_pack(v[i][2 * e], v[i][2 * e + 1]);
-          yo[e] = bf_pack(v[i][2 * e] * rstd * bf_lo(ww[e]), v[i][2 * e + 1] * rstd * bf_hi(ww[e]));
-        }
-        if (delta) sr[u] = make_int4(so[0], so[1], so[2], so[3]);
+        for (int e = 0; e < 4; ++e) yo[e] = bf_pack(v[2 * e] * rstd * wv[2 * e], v[2 * e + 1] * rstd * wv[2 * e + 1]);
+        if (delta) sr[u] = a[i];
         yr[u] = make_int4(yo[0], yo[1], yo[2], yo[3]);
       }
     }
@@ -87,73 +98,76 @@ __global__ void __launch_bounds__(kNormThreads) add_rms_norm_fwd_kernel(const __
 
 // ds = ds_in + rstd * (dy * w) - s * rstd^3 / D * sum(dy * w * s);  dw partial = sum over this block's rows of
 // dy * s * rstd, one fp32 row per block (summed afterwards in fixed order).
-__global__ void __launch_bounds__(kNormThreads) add_rms_norm_bwd_kernel(const __nv_bfloat16* dy,
-                                                                        const __nv_bfloat16* ds_in,
-                                                                        const __nv_bfloat16* s,
-                                                                        const __nv_bfloat16* w, const float* rstd_in,
-                                                                        __nv_bfloat16* ds_out, float* dw_partial,
-                                                                        int rows, int cols) {
+template <int UNITS>
+__global__ void __launch_bounds__(kNormThreads, UNITS <= 4 ? 2 : 1)
+add_rms_norm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* ds_in, const __nv_bfloat16* s,
+                        const __nv_bfloat16* w, const float* rstd_in, __nv_bfloat16* ds_out, float* dw_partial,
+                        int rows, int cols) {
   extern __shared__ float s_dw[];  // [8 warps][cols]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int units = cols >> 3, per_lane = (units + 31) >> 5;
-  float dw_acc[kMaxNormUnits][8];
+  const int units = cols >> 3;
+  const int4 zero = make_int4(0, 0, 0, 0);
+  float dw_acc[UNITS][8];
+  const int4* wr = reinterpret_cast<const int4*>(w);
 #pragma unroll
-  for (int i = 0; i < kMaxNormUnits; ++i)
+  for (int i = 0; i < UNITS; ++i) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) dw_acc[i][e] = 0.0f;
-  const int4* wr = reinterpret_cast<const int4*>(w);
+  }
   for (int row = blockIdx.x * (kNormThreads / 32) + warp; row < rows; row += gridDim.x * (kNormThreads / 32)) {
     const int4* gr = reinterpret_cast<const int4*>(dy + static_cast<size_t>(row) * cols);
     const int4* sr = reinterpret_cast<const int4*>(s + static_cast<size_t>(row) * cols);
-    const int4* ir = ds_in ? reinterpret_cast<const int4*>(ds_in + static_cast<size_t>(row) * cols) : nullptr;
+    const int4* ir = reinterpret_cast<const int4*>(ds_in + static_cast<size_t>(row) * cols);
     const float rstd = rstd_in[row];
-    float gw[kMaxNormUnits][8], sv[kMaxNormUnits][8];
+    int4 gq[UNITS], sq[UNITS], iq[UNITS];
+#pragma unroll
+    for (int i = 0; i < UNITS; ++i) {
+      const int u = lane + 32 * i;
+      gq[i] = u < units ? gr[u] : zero;
+      sq[i] = u < units ? sr[u] : zero;
+      iq[i] = ds_in != nullptr && u < units ? ir[u] : zero;
+    }
     float dot = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kMaxNormUnits; ++i) {
+    for (int i = 0; i < UNITS; ++i) {
+      float g[8], sv[8], wv[8];
+      unpack8(gq[i], g);
+      unpack8(sq[i], sv);
       const int u = lane + 32 * i;
-      if (i < per_lane && u < units) {
-        const int4 g = gr[u], sx = sr[u], wv = wr[u];
-        const uint32_t gq[4] = {(uint32_t)g.x, (uint32_t)g.y, (uint32_t)g.z, (uint32_t)g.w};
-        const uint32_t sq[4] = {(uint32_t)sx.x, (uint32_t)sx.y, (uint32_t)sx.z, (uint32_t)sx.w};
-        const uint32_t wq[4] = {(uint32_t)wv.x, (uint32_t)wv.y, (uint32_t)wv.z, (uint32_t)wv.w};
+      unpack8(u < units ? wr[u] : zero, wv);  // (from L1: kept in registers they would spill)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float g0 = bf_lo(gq[e]), g1 = bf_hi(gq[e]), s0 = bf_lo(sq[e]), s1 = bf_hi(sq[e]);
-          dw_acc[i][2 * e] += g0 * s0 * rstd;
-          dw_acc[i][2 * e + 1] += g1 * s1 * rstd;
-          gw[i][2 * e] = g0 * bf_lo(wq[e]); gw[i][2 * e + 1] = g1 * bf_hi(wq[e]);
-          sv[i][2 * e] = s0; sv[i][2 * e + 1] = s1;
-          dot += gw[i][2 * e] * s0 + gw[i][2 * e + 1] * s1;
-        }
+      for (int e = 0; e < 4; ++e) {
+        dw_acc[i][2 * e] += g[2 * e] * sv[2 * e] * rstd;
+        dw_acc[i][2 * e + 1] += g[2 * e + 1] * sv[2 * e + 1] * rstd;
+        dot += g[2 * e] * wv[2 * e] * sv[2 * e] + g[2 * e + 1] * wv[2 * e + 1] * sv[2 * e + 1];
       }
     }
     dot = warp_sum(dot);
     const float coef = dot * rstd * rstd * rstd / cols;
     int4* outr = reinterpret_cast<int4*>(ds_out + static_cast<size_t>(row) * cols);
 #pragma unroll
-    for (int i = 0; i < kMaxNormUnits; ++i) {
+    for (int i = 0; i < UNITS; ++i) {
       const int u = lane + 32 * i;
-      if (i < per_lane && u < units) {
-        uint32_t iq[4] = {0, 0, 0, 0};
-        if (ir) {
-          const int4 t = ir[u];
-          iq[0] = (uint32_t)t.x; iq[1] = (uint32_t)t.y; iq[2] = (uint32_t)t.z; iq[3] = (uint32_t)t.w;
-        }
+      if (u < units) {
+        float g[8], sv[8], wv[8], in[8];
+        unpack8(gq[i], g);
+        unpack8(sq[i], sv);
+        unpack8(wr[u], wv);
+        unpack8(iq[i], in);
         uint32_t o[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          o[e] = bf_pack(bf_lo(iq[e]) + gw[i][2 * e] * rstd - sv[i][2 * e] * coef,
-                         bf_hi(iq[e]) + gw[i][2 * e + 1] * rstd - sv[i][2 * e + 1] * coef);
+          o[e] = bf_pack(in[2 * e] + g[2 * e] * wv[2 * e] * rstd - sv[2 * e] * coef,
+                         in[2 * e + 1] + g[2 * e + 1] * wv[2 * e + 1] * rstd - sv[2 * e + 1] * coef);
         outr[u] = make_int4(o[0], o[1], o[2], o[3]);
       }
     }
   }
   // Block-level sum of the eight warps' weight-gradient rows, then one row of partials per block.
 #pragma unroll
-  for (int i = 0; i < kMaxNormUnits; ++i) {
+  for (int i = 0; i < UNITS; ++i) {
     const int u = lane + 32 * i;
-    if (i < per_lane && u < units)
+    if (u < units)
 #pragma unroll
       for (int e = 0; e < 8; ++e) s_dw[warp * cols + u * 8 + e] = dw_acc[i][e];
   }
@@ -163,6 +177,24 @@ __global__ void __launch_bounds__(kNormThreads) add_rms_norm_bwd_kernel(const __
 #pragma unroll
     for (int wi = 0; wi < kNormThreads / 32; ++wi) t += s_dw[wi * cols + c];
     dw_partial[static_cast<size_t>(blockIdx.x) * cols + c] = t;
+  }
+}
+
+// dW = column sums of the blocks' partials, fp32 in fixed order, rounded once. Eight warps take every eighth row of 32
+// columns each.
+__global__ void __launch_bounds__(256) norm_dw_kernel(const float* partial, int blocks, int cols, __nv_bfloat16* dw) {
+  __shared__ float sums[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
+  float t = 0.0f;
+  if (c < cols) {
+#pragma unroll 8
+    for (int r = warp; r < blocks; r += 8) t += partial[static_cast<size_t>(r) * cols + c];
+  }
+  sums[warp][lane] = t;
+  __syncthreads();
+  if (warp == 0 && c < cols) {
+    for (int i = 1; i < 8; ++i) t += sums[i][lane];
+    dw[c] = __float2bfloat16_rn(t);
   }
 }
 
@@ -338,15 +370,28 @@ __global__ void __launch_bounds__(256) dense_swiglu_bwd_kernel(const __nv_bfloat
 
 }  // namespace
 
+// Calls `f` with the smallest instantiated number of units per lane that holds a row.
+template <typename F>
+static void for_norm_units(int cols, F&& f) {
+  const int per_lane = ((cols >> 3) + 31) >> 5;
+  if (per_lane <= 1) f(std::integral_constant<int, 1>{});
+  else if (per_lane == 2) f(std::integral_constant<int, 2>{});
+  else if (per_lane == 3) f(std::integral_constant<int, 3>{});
+  else if (per_lane == 4) f(std::integral_constant<int, 4>{});
+  else f(std::integral_constant<int, kMaxNormUnits>{});
+}
+
 void launch_add_rms_norm_fwd(const void* x, const void* delta, const void* w, void* s_out, void* y, float* rstd,
                              int rows, int cols, float eps, cudaStream_t stream) {
   int grid = (rows + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
   if (grid < 1) grid = 1;
-  add_rms_norm_fwd_kernel<<<grid, kNormThreads, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(delta),
-      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(s_out), static_cast<__nv_bfloat16*>(y), rstd,
-      rows, cols, eps);
+  for_norm_units(cols, [&](auto units) {
+    add_rms_norm_fwd_kernel<decltype(units)::value><<<grid, kNormThreads, 0, stream>>>(
+        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(delta),
+        static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(s_out), static_cast<__nv_bfloat16*>(y), rstd,
+        rows, cols, eps);
+  });
 }
 
 int add_rms_norm_bwd_blocks(int rows) {
@@ -356,18 +401,21 @@ int add_rms_norm_bwd_blocks(int rows) {
 }
 
 void launch_add_rms_norm_bwd(const void* dy, const void* ds_in, const void* s, const void* w, const float* rstd,
-                             void* ds_out, float* dw_partial, int rows, int cols, cudaStream_t stream) {
+                             void* ds_out, float* dw_partial, void* dw, int rows, int cols, cudaStream_t stream) {
   const int grid = add_rms_norm_bwd_blocks(rows);
   const size_t smem = static_cast<size_t>(kNormThreads / 32) * cols * sizeof(float);
-  static bool configured = false;
-  if (!configured) {  // 64 KB at 2048 columns: above the default limit
-    cudaFuncSetAttribute(add_rms_norm_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536);
-    configured = true;
-  }
-  add_rms_norm_bwd_kernel<<<grid, kNormThreads, smem, stream>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(ds_in),
-      static_cast<const __nv_bfloat16*>(s), static_cast<const __nv_bfloat16*>(w), rstd,
-      static_cast<__nv_bfloat16*>(ds_out), dw_partial, rows, cols);
+  for_norm_units(cols, [&](auto units) {
+    constexpr int kUnits = decltype(units)::value;
+    // (64 KB at 2048 columns: above the default limit)
+    static const cudaError_t configured = cudaFuncSetAttribute(
+        add_rms_norm_bwd_kernel<kUnits>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUnits * 8192);
+    (void)configured;
+    add_rms_norm_bwd_kernel<kUnits><<<grid, kNormThreads, smem, stream>>>(
+        static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(ds_in),
+        static_cast<const __nv_bfloat16*>(s), static_cast<const __nv_bfloat16*>(w), rstd,
+        static_cast<__nv_bfloat16*>(ds_out), dw_partial, rows, cols);
+  });
+  norm_dw_kernel<<<(cols + 31) / 32, 256, 0, stream>>>(dw_partial, grid, cols, static_cast<__nv_bfloat16*>(dw));
 }
 
 void launch_rope_qkv(void* qkv, void* q, void* k, void* v, const float* cos_t, const float* sin_t, int B, int S, int H,

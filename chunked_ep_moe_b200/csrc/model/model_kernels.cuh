@@ -10,10 +10,10 @@ namespace cem {
 // is then not written); `rstd` [rows] fp32.
 void launch_add_rms_norm_fwd(const void* x, const void* delta, const void* w, void* s_out, void* y, float* rstd,
                              int rows, int cols, float eps, cudaStream_t stream);
-// `ds_in` may be null. `dw_partial` is [add_rms_norm_bwd_blocks(rows), cols] fp32; its column sums are dW.
+// `ds_in` may be null. `dw_partial` is [add_rms_norm_bwd_blocks(rows), cols] fp32 scratch; its column sums go to `dw` (bf16).
 int add_rms_norm_bwd_blocks(int rows);
 void launch_add_rms_norm_bwd(const void* dy, const void* ds_in, const void* s, const void* w, const float* rstd,
-                             void* ds_out, float* dw_partial, int rows, int cols, cudaStream_t stream);
+                             void* ds_out, float* dw_partial, void* dw, int rows, int cols, cudaStream_t stream);
 // Forward: qkv [B,S,3,H,hd] -> q, k rotated, v copied, each contiguous [B,H,S,hd]. Backward: the three gradients in
 // [B,H,S,hd] -> d_qkv in the qkv layout (q and k rotated back). cos/sin: [S, hd/2] fp32; hd a multiple of 8.
 void launch_rope_qkv(void* qkv, void* q, void* k, void* v, const float* cos_t, const float* sin_t, int B, int S, int H,

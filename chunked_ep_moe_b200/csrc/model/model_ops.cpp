@@ -51,14 +51,17 @@ std::vector<torch::Tensor> add_rms_norm_bwd(torch::Tensor dy, c10::optional<torc
   const int64_t rows = s.size(0), cols = s.size(1);
   need(cols % 8 == 0 && cols <= 2048, "columns must be a multiple of 8, at most 2048");
   need(rstd.is_cuda() && rstd.scalar_type() == torch::kFloat32 && rstd.numel() == rows, "rstd must be fp32 [rows]");
+  need(weight.is_cuda() && weight.scalar_type() == torch::kBFloat16 && weight.is_contiguous() && weight.numel() == cols,
+       "weight must be a contiguous CUDA bf16 vector of `cols` elements");
   const c10::cuda::CUDAGuard guard(s.device());
   torch::Tensor ds = torch::empty_like(s);
   const int blocks = add_rms_norm_bwd_blocks(static_cast<int>(rows));
   torch::Tensor partial = torch::empty({blocks, cols}, s.options().dtype(torch::kFloat32));
+  torch::Tensor dw = torch::empty_like(weight);
   launch_add_rms_norm_bwd(dy.data_ptr(), ds_in.has_value() ? ds_in->data_ptr() : nullptr, s.data_ptr(),
                           weight.data_ptr(), rstd.data_ptr<float>(), ds.data_ptr(), partial.data_ptr<float>(),
-                          static_cast<int>(rows), static_cast<int>(cols), stream());
-  return {ds, partial.sum(0)};
+                          dw.data_ptr(), static_cast<int>(rows), static_cast<int>(cols), stream());
+  return {ds, dw};
 }
 
 std::vector<torch::Tensor> rope_qkv_fwd(torch::Tensor qkv, torch::Tensor cos_t, torch::Tensor sin_t) {

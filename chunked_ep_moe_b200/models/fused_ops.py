@@ -45,9 +45,8 @@ class _AddRMSNorm(torch.autograd.Function):
             dw = None
         else:
             ds_flat = ds_in.reshape(-1, cols).contiguous() if ds_in is not None else None
-            ds, dw = _ext().add_rms_norm_bwd(dy.reshape(-1, cols).contiguous(), ds_flat, s, weight, rstd)
+            ds, dw = _ext().add_rms_norm_bwd(dy.reshape(-1, cols).contiguous(), ds_flat, s, weight.contiguous(), rstd)
             ds = ds.reshape(ctx.shape)
-            dw = dw.to(weight.dtype)
         return ds, (ds if ctx.has_delta else None), dw, None
 
 

@@ -137,3 +137,23 @@ def test_dense_swiglu(rows, ffn):
     ref.backward(go.float())
     _close(out, ref, "act", 1e-2)
     _close(gu.grad, ref_in.grad, "d_gate_up", 1e-2)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (7, 248), (9, 256), (33, 264), (8, 768), (2369, 776), (5, 1032), (2, 2040)])
+def test_add_rms_norm_row_widths(rows, cols):
+    """Every number of 16-byte units per lane, with ragged last units, and more rows than the grid has warps."""
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    x, delta, gs, gy = [torch.randn(rows, cols, device="cuda", generator=gen).bfloat16() for _ in range(4)]
+    w = (1 + 0.1 * torch.randn(cols, device="cuda", generator=gen)).bfloat16()
+    leaves = [t.clone().requires_grad_(True) for t in (x, delta, w)]
+    s, y = fused_ops.add_rms_norm(*leaves, 1e-6)
+    torch.autograd.backward([s, y], [gs, gy])
+    sr = (x.float() + delta.float()).bfloat16().double().requires_grad_(True)
+    wr = w.double().requires_grad_(True)
+    yr = sr * torch.rsqrt(sr.pow(2).mean(-1, keepdim=True) + 1e-6) * wr
+    torch.autograd.backward([sr, yr], [gs.double(), gy.double()])
+    assert torch.equal(s.double(), sr.detach())
+    # one rounding to bf16 (2^-9 of the value) on top of fp32 arithmetic
+    for name, got, want in (("y", y, yr.detach()), ("dx", leaves[0].grad, sr.grad), ("dw", leaves[2].grad, wr.grad)):
+        assert (got.double() - want).abs().le(want.abs() * 2.0**-8 + 1e-5 * want.abs().max()).all(), name
+    assert torch.equal(leaves[0].grad, leaves[1].grad)
