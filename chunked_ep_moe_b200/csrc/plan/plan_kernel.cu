@@ -21,7 +21,7 @@ __device__ __forceinline__ int warp_exclusive_scan(int v, int lane, int* total) 
 
 // Per-pass sums on the device (what `plan_phase_a` computes with one loop nest per value): every sum the tables need is
 // a prefix of a row of the traffic matrix or of the per-receiver expert totals, so the block first builds those prefix
-// tables in shared memory (one thread per row, 2 P + 1 rows of at most P * L values), then every value is a lookup plus
+// tables in shared memory (one warp per row, 2 P + 1 rows of at most P * L values), then every value is a lookup plus
 // at most P additions. `rowsum[r][l]`: rows expert l of rank r receives; `ebegin[r][l]`: where they start in r's stream;
 // `prefix[s][q]`: copies of source s that sort before its q-th (receiver, expert) pair.
 __device__ void plan_phase_a_block(const int* counts, int* plan, const PlanLayout& y, int me, int* rowsum, int* ebegin,
@@ -34,14 +34,18 @@ __device__ void plan_phase_a_block(const int* counts, int* plan, const PlanLayou
     rowsum[i] = sum;
   }
   __syncthreads();
-  for (int row = tid; row < 2 * P; row += nthreads) {
-    if (row < P) {  // exclusive scan of one receiver's expert totals
-      int run = 0;
-      for (int l = 0; l < L; ++l) { ebegin[row * L + l] = run; run += rowsum[row * L + l]; }
-    } else {        // exclusive scan of one source's row of the traffic matrix
-      const int s = row - P;
-      int run = 0;
-      for (int q = 0; q < n; ++q) { prefix[s * n + q] = run; run += counts[s * n + q]; }
+  const int lane = tid & 31;
+  for (int row = tid >> 5; row < 2 * P; row += nthreads >> 5) {  // a warp per row
+    // exclusive scan of one receiver's expert totals, or of one source's row of the traffic matrix
+    const int* src = row < P ? rowsum + row * L : counts + (row - P) * n;
+    int* dst = row < P ? ebegin + row * L : prefix + (row - P) * n;
+    const int len = row < P ? L : n;
+    int run = 0;
+    for (int q0 = 0; q0 < len; q0 += 32) {
+      int total;
+      const int before = warp_exclusive_scan(q0 + lane < len ? src[q0 + lane] : 0, lane, &total);
+      if (q0 + lane < len) dst[q0 + lane] = run + before;
+      run += total;
     }
   }
   __syncthreads();
@@ -146,14 +150,22 @@ __device__ void plan_phase_b_warps(int* plan, const PlanLayout& y, const int* se
   }
 }
 
-// Header and status block straight into pinned host memory, as soon as the header stands (the per-slice tables are still
-// to come). One thread, after the block barrier that ends phase A.
+// Header and status block straight into pinned host memory, as soon as the header stands and a block barrier has passed. The
+// last warp does it beside the others, which go on to the per-slice tables: stores to the host and the fence behind them take
+// 4 us. (It has slices of its own only from eight on.) Together with the scans by warps: 64 experts, 15.3 -> 12.3 us.
 __device__ void publish_header(const PlanKernelParams& p) {
-  if (p.host_out == nullptr || threadIdx.x != 0) return;
-  for (int q = 0; q < kPlanHeaderInts; ++q) p.host_out[q] = p.plan[q];
-  const int* status = reinterpret_cast<const int*>(p.status);
-  for (int q = 0; q < 8; ++q) p.host_out[kPlanHeaderInts + q] = status != nullptr ? __ldcg(status + q) : 0;
-  st_release_sys(reinterpret_cast<uint32_t*>(p.host_out) + kPlanHeaderInts + 8, p.host_seq);
+  const int lane = threadIdx.x & 31;
+  if (p.host_out == nullptr || (threadIdx.x >> 5) != (blockDim.x >> 5) - 1) return;
+  if (lane < kPlanHeaderInts) {
+    p.host_out[lane] = p.plan[lane];
+  } else if (lane < kPlanHeaderInts + 8) {
+    p.host_out[lane] = p.status != nullptr ? __ldcg(reinterpret_cast<const int*>(p.status) + lane - kPlanHeaderInts) : 0;
+  }
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence_system();
+    st_release_sys(reinterpret_cast<uint32_t*>(p.host_out) + kPlanHeaderInts + 8, p.host_seq);
+  }
 }
 
 __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams p) {
@@ -184,6 +196,7 @@ __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams 
   __syncthreads();
   if (s_abort) {
     if (threadIdx.x == 0) p.plan[0] = 0;  // zero slices: the pass launches nothing
+    __syncthreads();
     publish_header(p);
     return;
   }
@@ -198,7 +211,6 @@ __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams 
     // scratch of the per-pass sums: rowsum [n], ebegin [n], prefix [P * n]; the same space holds phase B's inputs after
     plan_phase_a_block(s_counts, p.plan, p.lay, p.me, s_counts + P * n, s_counts + P * n + n, s_counts + P * n + 2 * n);
     __syncthreads();
-    publish_header(p);
     int* s_seg_start = s_counts + P * n;
     int* s_seg_size = s_seg_start + n;
     int* s_send_start = s_seg_size + n;
@@ -214,6 +226,7 @@ __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams 
       s_expert_rows[l] = p.plan[p.lay.off_expert_rows + l];
     }
     __syncthreads();
+    publish_header(p);
     plan_phase_b_warps(p.plan, p.lay, s_seg_start, s_seg_size, s_send_start, s_expert_start, s_expert_rows);
     return;
   }
