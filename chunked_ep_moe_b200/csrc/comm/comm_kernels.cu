@@ -24,6 +24,7 @@
 
 #include <cuda_fp8.h>
 
+#include "../common/pdl.cuh"
 #include "../common/umma.cuh"
 
 namespace cem {
@@ -247,6 +248,7 @@ __global__ void slice_done_kernel(uint32_t* const* peer_credit, int num_ranks, i
 
 __global__ void pass_begin_kernel(const int* plan, PlanLayout lay, uint32_t* expected_total, uint32_t* pass_base,
                                   uint32_t* ready_total, uint32_t* ready_base) {
+  wait_predecessor();
   const int n = lay.P * lay.L;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const uint32_t base = expected_total[i];
@@ -407,7 +409,7 @@ void launch_slice_done(uint32_t* const* peer_credit, int num_ranks, int me, uint
 
 void launch_pass_begin(const int* plan, PlanLayout lay, uint32_t* expected_total, uint32_t* pass_base,
                        uint32_t* ready_total, uint32_t* ready_base, cudaStream_t stream) {
-  pass_begin_kernel<<<1, 256, 0, stream>>>(plan, lay, expected_total, pass_base, ready_total, ready_base);
+  launch_behind(pass_begin_kernel, 1, 256, 0, stream, plan, lay, expected_total, pass_base, ready_total, ready_base);
 }
 
 void launch_return_dw(const ReturnDwParams& p, cudaStream_t stream) {
