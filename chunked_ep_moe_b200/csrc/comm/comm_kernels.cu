@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(256) return_dw_kernel(const ReturnDwParams p) 
 __global__ void __launch_bounds__(256) combine_reduce_kernel(const CombineParams p) {
   __shared__ int s_abort;
   if (threadIdx.x == 0) {
+    if (blockIdx.x == 0 && p.credit != nullptr) st_release_sys(p.credit, p.credit_value);  // (behind the GEMMs on this stream)
     s_abort = (p.status != nullptr && p.status->code != 0) ? 1 : 0;
     uint32_t seen = 0;
     if (!s_abort && !spin_until_reached(p.count, p.target, p.spin_limit, &seen)) {

@@ -72,6 +72,8 @@ struct CombineParams {
   int num_tokens, top_k, hidden;
   const uint32_t* count;      // returned-row counter on this rank
   uint32_t target;            // value the counter reaches when everything is back
+  uint32_t* credit;           // one-slice pass of one rank: its slice buffers are free again (what `launch_slice_done` tells), or null
+  uint32_t credit_value;
   uint32_t spin_limit;
   StatusBlock* status;
 };

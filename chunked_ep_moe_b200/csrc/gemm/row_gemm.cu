@@ -3,7 +3,7 @@
 //
 // A pair of CTAs drives one 256 x N x 16 tcgen05.mma (cta_group::2): M = 256 weight columns (128 per CTA), N = a tile of
 // up to 256 rows of ONE expert, in steps of 32. With tokens on the M side a tile is 128 or 256 rows whatever the expert
-// has left; here an expert's rows are cut into equal tiles of a multiple of 32 (`plan_tile_span`), so the padding is 16
+// has left; here an expert's rows are cut into equal tiles of a multiple of 32 (`plan_tile_begin`), so the padding is 16
 // rows per expert on average. Each CTA stages its 128 weight columns and half of the tile's rows: 32 KB per k-block at
 // N = 256 (the SM's L2 port carries one request per 128-byte line, see grouped_gemm_pair.cu), less for narrow tiles.
 //

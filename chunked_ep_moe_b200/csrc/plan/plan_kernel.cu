@@ -304,17 +304,9 @@ __global__ void __launch_bounds__(256) sort_scan_kernel(int* block_hist, int num
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortRankedMaxExperts = 1024;  // kSortWarps * experts ints of shared memory: 32 KB
 
-__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* ids, int n, int num_experts,
-                                                                  const int* block_off, int* order, int* inv_order) {
-  extern __shared__ int s_slot[];  // [kSortWarps][num_experts]
-  release_successor();
-  wait_predecessor();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int base = blockIdx.x * kSortThreads * kSortItems + warp * (kSortItems * 32);
-  for (int i = threadIdx.x; i < kSortWarps * num_experts; i += blockDim.x) s_slot[i] = 0;
-  __syncthreads();
-  int* mine = s_slot + warp * num_experts;
-  int e_of[kSortItems];
+// A warp's kSortItems * 32 consecutive ids from `base` on, counted into its slots (ids without an expert: -1).
+__device__ __forceinline__ void sort_count(const int* ids, int n, int num_experts, int base, int lane, int* mine,
+                                           int (&e_of)[kSortItems]) {
 #pragma unroll
   for (int g = 0; g < kSortItems; ++g) {
     const int idx = base + g * 32 + lane;
@@ -323,17 +315,11 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* i
     e_of[g] = e;
     if (e >= 0) atomicAdd(mine + e, 1);
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
-    int run = block_off[e * gridDim.x + blockIdx.x];
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
-      const int c = s_slot[w * num_experts + e];
-      s_slot[w * num_experts + e] = run;
-      run += c;
-    }
-  }
-  __syncthreads();
+}
+
+// The same ids, 32 at a time and in order, to their output slots.
+__device__ __forceinline__ void sort_walk(const int (&e_of)[kSortItems], int base, int lane, int* mine, int* order,
+                                          int* inv_order) {
 #pragma unroll
   for (int g = 0; g < kSortItems; ++g) {
     const int e = e_of[g];
@@ -353,6 +339,32 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* i
     }
     __syncwarp();  // the next group's leaders see this group's slot updates
   }
+}
+
+__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* ids, int n, int num_experts,
+                                                                  const int* block_off, int* order, int* inv_order) {
+  extern __shared__ int s_slot[];  // [kSortWarps][num_experts]
+  release_successor();
+  wait_predecessor();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int base = blockIdx.x * kSortThreads * kSortItems + warp * (kSortItems * 32);
+  for (int i = threadIdx.x; i < kSortWarps * num_experts; i += blockDim.x) s_slot[i] = 0;
+  __syncthreads();
+  int* mine = s_slot + warp * num_experts;
+  int e_of[kSortItems];
+  sort_count(ids, n, num_experts, base, lane, mine, e_of);
+  __syncthreads();
+  for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
+    int run = block_off[e * gridDim.x + blockIdx.x];
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) {
+      const int c = s_slot[w * num_experts + e];
+      s_slot[w * num_experts + e] = run;
+      run += c;
+    }
+  }
+  __syncthreads();
+  sort_walk(e_of, base, lane, mine, order, inv_order);
 }
 
 __global__ void __launch_bounds__(kSortThreads) sort_scatter_serial_kernel(const int* ids, int n, int num_experts,
@@ -382,7 +394,65 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_serial_kernel(const
   }
 }
 
+// One block: 2048 ids are what one block of the scatter takes. Five kernels in a row (sort, plan, arrival targets) took 23 us of a
+// one-token decode even with each launched behind the one before; together with the credit from the combine kernel the call
+// went from 61 to 46 us, a 64-token decode at D=7168 from 509 to 493 us.
+__global__ void __launch_bounds__(kSortThreads) plan_small_kernel(const PlanKernelParams p, const int* ids, int n, int* order,
+                                                                  int* inv_order, uint32_t* expected_total,
+                                                                  uint32_t* pass_base) {
+  extern __shared__ int s_small[];
+  const int L = p.lay.L, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int* s_counts = s_small;                   // [L]
+  int* s_scratch = s_counts + L;             // [3 L]: phase A's sums
+  int* s_slot = s_scratch + 3 * L;           // [kSortWarps][L]
+  for (int i = threadIdx.x; i < kSortWarps * L; i += blockDim.x) s_slot[i] = 0;
+  __syncthreads();
+  const int base = warp * (kSortItems * 32);
+  int* mine = s_slot + warp * L;
+  int e_of[kSortItems];
+  sort_count(ids, n, L, base, lane, mine, e_of);
+#pragma unroll
+  for (int g = 0; g < kSortItems; ++g) {
+    const int idx = base + g * 32 + lane;
+    if (idx < n && e_of[g] < 0)
+      report_status(p.status, kStatusBadIndex, kKernelPlan, 1, 0, idx, static_cast<uint32_t>(L), static_cast<uint32_t>(ids[idx]));
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < L; e += blockDim.x) {
+    int sum = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) sum += s_slot[w * L + e];
+    s_counts[e] = sum;
+  }
+  __syncthreads();
+  plan_phase_a_block(s_counts, p.plan, p.lay, 0, s_scratch, s_scratch + L, s_scratch + 2 * L);
+  __syncthreads();
+  const int* send_start = s_scratch + 2 * L;  // phase A's prefix: with one rank also every segment's place in the stream
+  for (int e = threadIdx.x; e < L; e += blockDim.x) {
+    int run = send_start[e];
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) {
+      const int c = s_slot[w * L + e];
+      s_slot[w * L + e] = run;
+      run += c;
+    }
+    const uint32_t total = expected_total[e];
+    pass_base[e] = total;
+    expected_total[e] = total + static_cast<uint32_t>(s_counts[e]);
+  }
+  __syncthreads();
+  publish_header(p);
+  sort_walk(e_of, base, lane, mine, order, inv_order);
+  plan_phase_b_warps(p.plan, p.lay, send_start, s_counts, send_start, send_start, s_counts);
+}
+
 }  // namespace
+
+void launch_plan_small(const PlanKernelParams& p, const int* expert_ids, int n, int* order, int* inv_order,
+                       uint32_t* expected_total, uint32_t* pass_base, cudaStream_t stream) {
+  const size_t smem = sizeof(int) * (4 + kSortWarps) * static_cast<size_t>(p.lay.L);
+  plan_small_kernel<<<1, kSortThreads, smem, stream>>>(p, expert_ids, n, order, inv_order, expected_total, pass_base);
+}
 
 void launch_plan_build(const PlanKernelParams& p_in, cudaStream_t stream) {
   PlanKernelParams p = p_in;

@@ -32,6 +32,13 @@ struct PlanKernelParams {
 // prefix sums + per-slice argument builders (src/chunked_moe/plan.py:77-163).
 void launch_plan_build(const PlanKernelParams& p, cudaStream_t stream);
 
+// Everything that starts a pass of ONE rank with few ids, as one kernel: the stable sort (order, inv_order), the tables, header
+// and status to the host, and the arrival targets (`expected_total`, `pass_base`: as in `launch_pass_begin`). `p.counts`,
+// `p.my_counts` and the exchange's fields are not used. At most kPlanSmallIds ids and kPlanSmallExperts experts.
+constexpr int kPlanSmallIds = 2048, kPlanSmallExperts = 512;
+void launch_plan_small(const PlanKernelParams& p, const int* expert_ids, int n, int* order, int* inv_order,
+                       uint32_t* expected_total, uint32_t* pass_base, cudaStream_t stream);
+
 // Host restatement of the table build, for CPU tests of the shared arithmetic.
 void plan_build_host(const int* counts, int* plan, const PlanLayout& lay, int me);
 

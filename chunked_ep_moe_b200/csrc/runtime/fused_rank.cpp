@@ -291,6 +291,19 @@ int64_t FusedRank::begin_forward_async(torch::Tensor expert_ids, torch::Tensor p
   pp.plan = plan.data_ptr<int>();
   pp.spin_limit = spin_limit_;
   pp.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
+  pp.host_out = host_header_;
+  pp.host_seq = ++host_seq_;
+  if (short_pass_ && tk <= kPlanSmallIds && L_ <= kPlanSmallExperts) {
+    expect_i32(expert_ids, tk, "expert_ids");
+    expect_i32(order, tk, "order");
+    expect_i32(inv_order, tk, "inv_order");
+    launch_plan_small(pp, expert_ids.data_ptr<int>(), static_cast<int>(tk), order.data_ptr<int>(),
+                      inv_order.data_ptr<int>(), reinterpret_cast<uint32_t*>(expected_total_.data_ptr()),
+                      reinterpret_cast<uint32_t*>(pass_base_.data_ptr()), st);
+    ++launches_;
+    begin_pass(plan, max_slices_, tk, D_ / kCombineCols, /*targets_set=*/true);
+    return last_slices_;
+  }
   if (counts_prefilled) {
     expect_i32(counts, static_cast<int64_t>(P_) * P_ * L_, "counts");
     pp.counts = counts.data_ptr<int>();
@@ -311,8 +324,6 @@ int64_t FusedRank::begin_forward_async(torch::Tensor expert_ids, torch::Tensor p
     pp.epoch = epoch;
   }
   // The plan kernel itself stores header and status to the pinned words as soon as it knows them; nobody waits here.
-  pp.host_out = host_header_;
-  pp.host_seq = ++host_seq_;
   launch_plan_build(pp, st);
   ++launches_;
   // any slice below the workspace's capacity may be launched until resolved; D/128 pieces per row come back
@@ -405,15 +416,18 @@ int64_t FusedRank::begin_backward(torch::Tensor plan, int64_t known_slices, int6
   return cur_slices_;
 }
 
-void FusedRank::begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row) {
+void FusedRank::begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row,
+                           bool targets_set) {
   cudaStream_t st = current_stream();
   cur_slices_ = slices;
   cur_rows_ = rows;
-  launch_pass_begin(plan.data_ptr<int>(), lay_, reinterpret_cast<uint32_t*>(expected_total_.data_ptr()),
-                    reinterpret_cast<uint32_t*>(pass_base_.data_ptr()),
-                    expands() ? reinterpret_cast<uint32_t*>(ready_total_.data_ptr()) : nullptr,
-                    expands() ? reinterpret_cast<uint32_t*>(ready_base_.data_ptr()) : nullptr, st);
-  ++launches_;
+  if (!targets_set) {
+    launch_pass_begin(plan.data_ptr<int>(), lay_, reinterpret_cast<uint32_t*>(expected_total_.data_ptr()),
+                      reinterpret_cast<uint32_t*>(pass_base_.data_ptr()),
+                      expands() ? reinterpret_cast<uint32_t*>(ready_total_.data_ptr()) : nullptr,
+                      expands() ? reinterpret_cast<uint32_t*>(ready_base_.data_ptr()) : nullptr, st);
+    ++launches_;
+  }
   ret_target_ += static_cast<uint32_t>(cur_rows_) * static_cast<uint32_t>(pieces_per_row);
   if (overlapped()) cuda_check(cudaEventRecord(ev_pass_, st), "event record");
 }
@@ -628,8 +642,10 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
     cuda_check(cudaEventRecord(ev_down_[q], st), "event record");
     cuda_check(cudaStreamWaitEvent(aux, ev_down_[q], 0), "wait down event");
   }
-  launch_slice_done(table<uint32_t>(kTabCredit), P_, me_, seq, aux);  // credits leave in slice order
-  ++launches_;
+  if (!short_pass_) {  // (else the combine kernel gives the credit)
+    launch_slice_done(table<uint32_t>(kTabCredit), P_, me_, seq, aux);  // credits leave in slice order
+    ++launches_;
+  }
   if (async) cuda_check(cudaEventRecord(ev_done_[j % 4], aux), "event record");
 }
 
@@ -770,7 +786,7 @@ void FusedRank::join_streams(bool backward) {
 void FusedRank::end_pass(int64_t n_slices) {
   seq_ += static_cast<uint32_t>(n_slices);
   cur_slices_ = 0;
-  inline_ = false;
+  inline_ = short_pass_ = false;
   release_kept();
 }
 
@@ -824,6 +840,10 @@ void FusedRank::finish_forward(torch::Tensor inv_order, torch::Tensor out) {
   c.hidden = D_;
   c.count = reinterpret_cast<const uint32_t*>(arena_ + arena_lay_.ret_count);
   c.target = ret_target_;
+  if (short_pass_) {
+    c.credit = reinterpret_cast<uint32_t*>(arena_ + arena_lay_.credit);
+    c.credit_value = seq_ + 1;
+  }
   c.spin_limit = spin_limit_;
   c.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
   launch_combine_reduce(c, current_stream());
@@ -865,6 +885,7 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
     bool training) {
   const int64_t tk = expert_ids.numel();
   release_kept();  // (of a pass that threw)
+  short_pass_ = false;
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
   auto i32 = torch::TensorOptions().device(x.device()).dtype(torch::kInt32);
   // (The send order needs no initial values: an id the sort leaves out is recorded in the status block first, and with
@@ -890,6 +911,10 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
   // events that tie the streams together are saved (one-token decode 82 -> 77 us, 2000 tokens at D=2048 195 -> 190 us).
   // The backward keeps its streams: its weight gradients fill the other GEMMs' tails (same layer 542 us, else 558 us).
   inline_ = use_comm_stream_ && known == 1;
+  // Without autograd such a pass is also launched with as few kernels as it can do with: sort, plan and arrival targets as one
+  // (few ids), the slice's credit from the combine kernel. (Training passes keep the launches that `expected_launches` counts;
+  // a training step's forty launches hide what these five cost.) 61 -> 46 us for one token.
+  short_pass_ = inline_ && !training;
   int64_t guess;
   {
     NvtxRange range("chunked_moe/plan");
@@ -928,7 +953,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
     torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
     torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
     const std::vector<torch::Tensor>& kept, int64_t kept_slices) {
-  inline_ = false;  // (also behind a forward that threw)
+  inline_ = short_pass_ = false;  // (also behind a forward that threw)
   release_kept();
   if (kept.size() == 2) keep_rows(kept[0], kept[1], kept_slices);
   // The slice count is the forward's: nothing is read back, the host never waits for the device here.

@@ -106,7 +106,8 @@ class FusedRank {
 
  private:
   // Common start of a pass: counter targets on the device, what the pass will receive back (`pieces_per_row` of T*K rows).
-  void begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row);
+  void begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row,
+                  bool targets_set = false);
   void end_pass(int64_t n_slices);
   void wait_header();
   void keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices);
@@ -171,6 +172,7 @@ class FusedRank {
   int64_t last_slices_ = -1;  // slice count of the previous forward pass (the next pass's guess)
   int32_t* host_header_ = nullptr;  // pinned: 16 plan header ints + 8 status ints + their sequence number, see the .cpp
   uint32_t host_seq_ = 0;     // headers asked for so far
+  bool short_pass_ = false;   // an inline pass without autograd: fewer, larger kernels
   bool inline_ = false;       // the current pass runs on the caller's stream alone
 
   uint32_t seq_ = 0;          // global slice sequence number of the next pass's first slice

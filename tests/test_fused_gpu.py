@@ -349,6 +349,26 @@ def test_one_rank_fp8_wire_rounds_like_the_wire(group_rows, hidden):
     assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
+@pytest.mark.parametrize("experts", [4, 33, 512, 544])
+@pytest.mark.parametrize("tokens", [1, 127, 129, 1024, 1025])
+def test_forward_without_autograd_gives_the_same_bits(tokens, experts):
+    """One-slice forwards without autograd start with one kernel up to 2048 ids and 512 experts: equal to the pass that trains
+    (separate kernels), whichever came before it in the workspace."""
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    K, D, F = 2, 256, 256
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    w_up, w_down = (rnd(experts, D, 2 * F) / math.sqrt(D)).bfloat16(), (rnd(experts, F, D) / math.sqrt(F)).bfloat16()
+    cfg = ChunkedMoEConfig(num_experts=experts, top_k=K, slice_size=4096, transport="nvshmem", expert_compute="fused",
+                           stripe_width=64)
+    for step in range(3):  # free, training, free, training ... on one workspace
+        x, weights = rnd(tokens, D).bfloat16(), rnd(tokens, K).sigmoid()
+        ids = torch.topk(rnd(tokens, experts) + (torch.arange(experts, device="cuda") == 3) * 3.0 * step, K).indices.int()
+        free = chunked_moe(x, ids, weights, w_up, w_down, cfg)
+        trained = chunked_moe(x.clone().requires_grad_(True), ids, weights, w_up, w_down, cfg)
+        assert torch.equal(free, trained.detach()), step
+        trained.backward(x)
+
+
 def test_gemm_whose_rows_never_arrive_gives_up_and_reports(monkeypatch):
     """The real swiglu kernel waiting for rows nobody sends: its bounded wait runs out, every warp unwinds promptly
     (the barrier waits watch the CTA's abort flag), later kernels of the pass return at once, the host raises."""
