@@ -8,7 +8,8 @@ Sized so that a full-section profiler capture of a few launches ends in about a 
 D=2048, F=1024 (201 MB of bf16 expert weights, larger than the 126 MB L2), 16384 token copies in
 two 8192-row slices. Launch order of one pass: forward = sort x3, plan, pass_begin, put, put,
 [swiglu, down+combine, done] x2, combine_reduce; backward = pass_begin, put, put,
-[swiglu, down(d_weight), dswiglu, tgmm(dW_down), dx+combine, tgmm(dW_up), done] x2, combine_reduce.
+[swiglu unless the forward kept its results, dswiglu, tgmm(dW_down), return_dw, dx+combine, tgmm(dW_up), done] x2,
+combine_reduce.
 
     python bench/profile_case.py            # prints per-pass device times
 """

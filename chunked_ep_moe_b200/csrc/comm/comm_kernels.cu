@@ -157,6 +157,8 @@ enum Wire { kWireBf16, kWireFp8, kWireRounded };
 template <int WIRE>
 __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutParams p) {
   __shared__ int s_abort;
+  release_successor();
+  wait_predecessor();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_seg = p.lay.P * p.lay.L;
   if (threadIdx.x == 0) s_abort = (p.status != nullptr && p.status->code != 0) ? 1 : 0;
@@ -304,6 +306,7 @@ __global__ void __launch_bounds__(256) return_dw_kernel(const ReturnDwParams p) 
 
 __global__ void __launch_bounds__(256) combine_reduce_kernel(const CombineParams p) {
   __shared__ int s_abort;
+  wait_predecessor();
   if (threadIdx.x == 0) {
     if (blockIdx.x == 0 && p.credit != nullptr) st_release_sys(p.credit, p.credit_value);  // (behind the GEMMs on this stream)
     s_abort = (p.status != nullptr && p.status->code != 0) ? 1 : 0;
@@ -398,10 +401,10 @@ __global__ void wait_probe_kernel(const uint32_t* flag, uint32_t target, uint32_
 
 }  // namespace
 
-void launch_dispatch_put(const PutParams& p, int grid, cudaStream_t stream) {
-  if (p.peer_xq != nullptr) dispatch_put_kernel<kWireFp8><<<grid, kPutThreads, 0, stream>>>(p);
-  else if (p.round_fp8) dispatch_put_kernel<kWireRounded><<<grid, kPutThreads, 0, stream>>>(p);
-  else dispatch_put_kernel<kWireBf16><<<grid, kPutThreads, 0, stream>>>(p);
+void launch_dispatch_put(const PutParams& p, int grid, cudaStream_t stream, bool behind) {
+  if (p.peer_xq != nullptr) launch_maybe_behind(behind, dispatch_put_kernel<kWireFp8>, grid, kPutThreads, 0, stream, p);
+  else if (p.round_fp8) launch_maybe_behind(behind, dispatch_put_kernel<kWireRounded>, grid, kPutThreads, 0, stream, p);
+  else launch_maybe_behind(behind, dispatch_put_kernel<kWireBf16>, grid, kPutThreads, 0, stream, p);
 }
 
 void launch_slice_done(uint32_t* const* peer_credit, int num_ranks, int me, uint32_t seq, cudaStream_t stream) {
@@ -417,10 +420,10 @@ void launch_return_dw(const ReturnDwParams& p, cudaStream_t stream) {
   return_dw_kernel<<<(p.lay.S + 255) / 256, 256, 0, stream>>>(p);
 }
 
-void launch_combine_reduce(const CombineParams& p, cudaStream_t stream) {
+void launch_combine_reduce(const CombineParams& p, cudaStream_t stream, bool behind) {
   int grid = p.num_tokens < 1184 ? p.num_tokens : 1184;  // 8 CTAs per SM on 148 SMs
   if (grid < 1) grid = 1;
-  combine_reduce_kernel<<<grid, 256, 0, stream>>>(p);
+  launch_maybe_behind(behind, combine_reduce_kernel, grid, 256, 0, stream, p);
 }
 
 void launch_dequant_slice(const DequantParams& p, cudaStream_t stream) {

@@ -37,7 +37,8 @@ struct PutParams {
   float* const* peer_gs;
 };
 
-void launch_dispatch_put(const PutParams& p, int grid, cudaStream_t stream);
+// `behind`: may become resident in its predecessor's tail (see `launch_row_gemm`).
+void launch_dispatch_put(const PutParams& p, int grid, cudaStream_t stream, bool behind = false);
 
 // Tells every sender that this rank has finished reading the slice buffers of sequence `seq`.
 void launch_slice_done(uint32_t* const* peer_credit, int num_ranks, int me, uint32_t seq, cudaStream_t stream);
@@ -78,7 +79,7 @@ struct CombineParams {
   StatusBlock* status;
 };
 
-void launch_combine_reduce(const CombineParams& p, cudaStream_t stream);
+void launch_combine_reduce(const CombineParams& p, cudaStream_t stream, bool behind = false);
 
 // Receiver-side expansion of arrived fp8 rows (e4m3 + one fp32 scale per 128 columns) into the bf16 slice buffer
 // the GEMMs read, expert by expert: the kernel acquires the arrival counters of ONE expert's segments, expands that

@@ -26,4 +26,12 @@ void launch_behind(void (*kernel)(Params...), int grid, int block, size_t smem, 
   cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
+// `launch_behind` if `behind`, else an ordinary launch.
+template <typename... Params, typename... Args>
+void launch_maybe_behind(bool behind, void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream,
+                         Args&&... args) {
+  if (behind) launch_behind(kernel, grid, block, smem, stream, args...);
+  else kernel<<<grid, block, smem, stream>>>(args...);
+}
+
 }  // namespace cem

@@ -92,9 +92,13 @@ struct alignas(64) TokenMaps {
 
 // Row-wise modes (everything but kModeTgmm). `map_a`: the weights, for the modes that read them with K along rows the
 // chunked description with boxes of 64 rows x 2 chunks (1 chunk for SwiGLU with stripes of 128), else boxes of 128 rows.
-// `grid` is rounded down to an even number and clamped to what is resident at once.
+// `grid` is rounded down to an even number and clamped to what is resident at once. `behind`: the kernel may become resident in
+// its predecessor's tail (programmatic dependent launch). Only where nothing else wants the SMs meanwhile: a waiting CTA holds
+// one, which two slices in flight would miss, and which a kernel that the PREDECESSOR waits for (the expansion of the fp8
+// wire, a put to this rank) may need. So: one rank, one stream (one-slice forwards: one token 46.3 -> 43.1 us, 64 tokens at
+// D=7168 497 -> 487 us, 2000 tokens at D=2048 153 -> 147 us; a kernel-level forward + backward gained nothing, 248 against 251).
 void launch_row_gemm(int mode, const GemmParams& p, const CUtensorMap& map_a, const TokenMaps& maps_b, int grid,
-                     cudaStream_t stream);
+                     cudaStream_t stream, bool behind = false);
 
 // Weight gradients (kModeTgmm). `map_a`, `map_b`: chunked descriptions with boxes of 64 rows x 2 chunks; `map_c`: the bf16
 // gradient [L*M, N] with boxes of 32 rows x 64 columns (tiled stores).

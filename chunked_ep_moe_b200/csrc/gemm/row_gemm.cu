@@ -25,6 +25,7 @@
 // XOR-ed with the row number (mod 8): fragment and row accesses are both free of bank conflicts.
 #include "grouped_gemm.cuh"
 
+#include "../common/pdl.cuh"
 #include "../common/umma.cuh"
 #include "gemm_common.cuh"
 
@@ -441,14 +442,8 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
                                         smem_base - smem_u32(smem_raw));
     return;
   }
-  // An earlier kernel of this pass already gave up: both CTAs of the pair leave together (the leader decides).
-  if (threadIdx.x == 0 && leader) {
-    const uint32_t v = (p.status != nullptr && p.status->code != 0) ? 1u : 0u;
-    *early_flag = static_cast<int>(v);
-    st_shared_cluster_u32(map_to_cta(bar_base + kSlotOff + 8, 1), v);
-  }
-  cluster_sync_all();
-  if (*early_flag) return;
+  release_successor();
+  cluster_sync_all();  // both CTAs run
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kRowStages; ++s) {
@@ -469,13 +464,22 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     tmem_alloc_pair(tmem_slot, 512);
     tmem_relinquish_pair();
   }
+  // Launched behind its predecessor, the kernel has come this far in that one's tail; global memory from here on.
+  wait_predecessor();
+  // An earlier kernel of this pass already gave up: neither CTA of the pair does anything (the leader decides).
+  if (threadIdx.x == 0 && leader) {
+    const uint32_t v = (p.status != nullptr && p.status->code != 0) ? 1u : 0u;
+    *early_flag = static_cast<int>(v);
+    st_shared_cluster_u32(map_to_cta(bar_base + kSlotOff + 8, 1), v);
+  }
   tcgen05_fence_before_sync();
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers exist before anyone signals across the pair
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot_gen;
 
-  const int num_entries = p.plan[p.lay.off_num_tiles + p.slice];
+  const bool gave_up = *early_flag != 0;
+  const int num_entries = gave_up ? 0 : p.plan[p.lay.off_num_tiles + p.slice];
   const int num_tiles = num_entries * p.n_tiles;
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
 
@@ -618,7 +622,7 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     uint32_t* s_dst = reinterpret_cast<uint32_t*>(staging_gen + c.h * kGroupStaging + 8192);
     uint32_t tcount = 0, returned = 0;
     long long epi_wait = 0;
-    zero_tail(p, (warp - 2) * 32 + lane);
+    if (!gave_up) zero_tail(p, (warp - 2) * 32 + lane);
     RowTile nxt = {};
     if (first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, num_entries);
     for (int t = first_tile; t < num_tiles; t += tile_step, ++tcount) {
@@ -693,14 +697,14 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
 int row_gemm_smem_bytes() { return kRowSmemBytes; }
 
 void launch_row_gemm(int mode, const GemmParams& p, const CUtensorMap& map_a, const TokenMaps& maps_b, int grid,
-                     cudaStream_t stream) {
+                     cudaStream_t stream, bool behind) {
   grid &= ~1;  // whole pairs only
 #define CEM_LAUNCH_ROW(M)                                                                                          \
   case M: {                                                                                                        \
     static const int resident = resident_pair_grid(row_gemm_kernel<M>, kRowThreads, kRowSmemBytes);                \
     const int g = grid < resident ? grid : resident;                                                               \
     g_pair_grid_used = g;                                                                                          \
-    row_gemm_kernel<M><<<g, kRowThreads, kRowSmemBytes, stream>>>(p, map_a, maps_b);                               \
+    launch_maybe_behind(behind, row_gemm_kernel<M>, g, kRowThreads, kRowSmemBytes, stream, p, map_a, maps_b);      \
     break;                                                                                                         \
   }
   switch (mode) {

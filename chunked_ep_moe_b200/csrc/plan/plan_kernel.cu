@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(kSortThreads) plan_small_kernel(const PlanKern
                                                                   int* inv_order, uint32_t* expected_total,
                                                                   uint32_t* pass_base) {
   extern __shared__ int s_small[];
+  release_successor();
   const int L = p.lay.L, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int* s_counts = s_small;                   // [L]
   int* s_scratch = s_counts + L;             // [3 L]: phase A's sums

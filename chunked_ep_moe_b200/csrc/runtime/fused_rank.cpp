@@ -473,7 +473,7 @@ void FusedRank::put(int64_t j, torch::Tensor plan, torch::Tensor order, torch::T
     p.peer_xs = table<float>(kTabXs);
     p.peer_gs = table<float>(kTabGs);
   }
-  launch_dispatch_put(p, put_blocks_, st);
+  launch_dispatch_put(p, put_blocks_, st, inline_);
   ++launches_;
   if (overlapped()) cuda_check(cudaEventRecord(ev_put_[j % 4], comm_stream_), "event record");
   if (expands() && overlapped()) {
@@ -563,7 +563,7 @@ void FusedRank::row_gemm(int mode, const GemmParams& p0, const CUtensorMap& weig
                          cudaStream_t st, int spare_sms) {
   GemmParams p = p0;
   count_pipeline(mode, &p);
-  launch_row_gemm(mode, p, weights, rows, std::max(2, num_sms_ - spare_sms), st);
+  launch_row_gemm(mode, p, weights, rows, std::max(2, num_sms_ - spare_sms), st, inline_);
   ++launches_;
 }
 
@@ -846,7 +846,7 @@ void FusedRank::finish_forward(torch::Tensor inv_order, torch::Tensor out) {
   }
   c.spin_limit = spin_limit_;
   c.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
-  launch_combine_reduce(c, current_stream());
+  launch_combine_reduce(c, current_stream(), inline_);
   ++launches_;
   end_pass(cur_slices_);
 }
