@@ -210,6 +210,7 @@ FusedRank::FusedRank(int P, int L, int me, int S, int D, int F, int K, int strip
     for (cudaEvent_t* e : {&ev_down_[q], &ev_up_[q], &ev_ds_[q], &ev_dx_[q], &ev_tgd_[q], &ev_tgu_[q]})
       cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "event");
   cuda_check(cudaEventCreateWithFlags(&ev_pass_, cudaEventDisableTiming), "event");
+  cuda_check(cudaEventCreateWithFlags(&ev_end_, cudaEventDisableTiming), "event");
   for (int i = 0; i < 4; ++i) {
     cuda_check(cudaEventCreateWithFlags(&ev_put_[i], cudaEventDisableTiming), "event");
     cuda_check(cudaEventCreateWithFlags(&ev_done_[i], cudaEventDisableTiming), "event");
@@ -230,6 +231,7 @@ FusedRank::~FusedRank() {
       if (e) cudaEventDestroy(e);
   }
   if (ev_pass_) cudaEventDestroy(ev_pass_);
+  if (ev_end_) cudaEventDestroy(ev_end_);
   for (int i = 0; i < 4; ++i) {
     if (ev_put_[i]) cudaEventDestroy(ev_put_[i]);
     if (ev_done_[i]) cudaEventDestroy(ev_done_[i]);
@@ -285,6 +287,7 @@ int64_t FusedRank::begin_forward_async(torch::Tensor expert_ids, torch::Tensor p
   const int64_t tk = expert_ids.numel();
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
   expect_i32(plan, lay_.total, "plan");
+  enter_pass();
   PlanKernelParams pp{};
   pp.lay = lay_;
   pp.me = me_;
@@ -397,6 +400,7 @@ int64_t FusedRank::begin_forward(torch::Tensor expert_ids, torch::Tensor plan, t
 int64_t FusedRank::begin_backward(torch::Tensor plan, int64_t known_slices, int64_t known_rows) {
   cudaStream_t st = current_stream();
   expect_i32(plan, lay_.total, "plan");
+  enter_pass();
   if (known_slices >= 0 && known_rows >= 0) {
     // The caller kept what the forward of this plan read back: no device-to-host copy, no synchronisation, so the
     // host keeps running ahead of the device through the whole backward. (A recorded kernel error then surfaces at
@@ -414,6 +418,17 @@ int64_t FusedRank::begin_backward(torch::Tensor plan, int64_t known_slices, int6
   }
   begin_pass(plan, cur_slices_, cur_rows_, D_ / kCombineCols + 1);  // per row: the pieces of dx and the d_weight scalar
   return cur_slices_;
+}
+
+// Passes of a workspace share its scratch, its return buffer and its counters, whatever streams they come on: a pass on
+// another stream than the one before waits there for that one's end. (One event record per pass; nothing else as long as the
+// stream stays the same.)
+void FusedRank::enter_pass() {
+  cudaStream_t st = current_stream();
+  unsigned long long id = 0;
+  cuda_check(cudaStreamGetId(st, &id), "stream id");
+  if (passed_ && id != pass_stream_) cuda_check(cudaStreamWaitEvent(st, ev_end_, 0), "wait for the last pass");
+  pass_stream_ = id;
 }
 
 void FusedRank::begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row,
@@ -784,6 +799,8 @@ void FusedRank::join_streams(bool backward) {
 }
 
 void FusedRank::end_pass(int64_t n_slices) {
+  cuda_check(cudaEventRecord(ev_end_, current_stream()), "event record");
+  passed_ = true;
   seq_ += static_cast<uint32_t>(n_slices);
   cur_slices_ = 0;
   inline_ = short_pass_ = false;

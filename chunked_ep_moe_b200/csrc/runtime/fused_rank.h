@@ -108,6 +108,7 @@ class FusedRank {
   // Common start of a pass: counter targets on the device, what the pass will receive back (`pieces_per_row` of T*K rows).
   void begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row,
                   bool targets_set = false);
+  void enter_pass();
   void end_pass(int64_t n_slices);
   void wait_header();
   void keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices);
@@ -169,6 +170,9 @@ class FusedRank {
   cudaEvent_t ev_expand_[4] = {};  // expansion of slice j (mod 4) has finished
   cudaEvent_t ev_down_[2] = {}, ev_up_[2] = {}, ev_ds_[2] = {}, ev_dx_[2] = {}, ev_tgd_[2] = {}, ev_tgu_[2] = {};
   cudaEvent_t ev_pass_ = nullptr, ev_put_[4] = {}, ev_done_[4] = {};
+  cudaEvent_t ev_end_ = nullptr;           // the last pass's final kernel
+  unsigned long long pass_stream_ = 0;     // id of the stream that pass came on (ids are never used again, handles are)
+  bool passed_ = false;                    // there was one
   int64_t last_slices_ = -1;  // slice count of the previous forward pass (the next pass's guess)
   int32_t* host_header_ = nullptr;  // pinned: 16 plan header ints + 8 status ints + their sequence number, see the .cpp
   uint32_t host_seq_ = 0;     // headers asked for so far

@@ -279,6 +279,43 @@ def test_one_slice_forward_equals_several_slices(tokens):
     assert outs[0].shape == x.shape and torch.equal(*outs)
 
 
+@pytest.mark.parametrize("training", [False, True], ids=["forward", "training"])
+@pytest.mark.parametrize("slice_size", [4096, 512], ids=["one slice", "several slices"])
+def test_passes_on_several_streams_follow_one_another(slice_size, training):
+    """Passes of one workspace issued in turn on streams that the caller does not order: each equals, bit for bit, what it
+    gives alone. (At this size a pass runs for longer than the host takes to issue the next one.)"""
+    E, K, D, F, T = 8, 2, 2048, 1024, 1500
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    w_up, w_down = (rnd(E, D, 2 * F) / math.sqrt(D)).bfloat16(), (rnd(E, F, D) / math.sqrt(F)).bfloat16()
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=slice_size, transport="nvshmem", expert_compute="fused",
+                           stripe_width=64)
+    cases = [(rnd(T - 100 * i, D).bfloat16(), torch.topk(rnd(T - 100 * i, E), K).indices.int(), rnd(T - 100 * i, K).sigmoid())
+             for i in range(3)]
+
+    def one(case):
+        x, ids, w = case
+        leaves = [t.clone().requires_grad_(training) for t in (x, w, w_up, w_down)]
+        out = chunked_moe(leaves[0], ids, *leaves[1:], cfg)
+        if not training:
+            return [out]
+        out.backward(x)
+        return [out.detach()] + [t.grad for t in leaves]
+
+    want = []
+    for case in cases:
+        want.append(one(case))
+        torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in cases]
+    got = []
+    for i in range(12):
+        with torch.cuda.stream(streams[i % 3]):
+            got.append(one(cases[i % 3]))
+    torch.cuda.synchronize()
+    for i, g in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(g, want[i % 3])), f"pass {i}"
+
+
 @pytest.mark.parametrize("wire", [None, "float8_e4m3fn"])
 @pytest.mark.parametrize("tokens,stripe", [(2048, 64), (3001, 128), (4097, 32)])
 def test_kept_activations_give_the_same_bits(monkeypatch, tokens, stripe, wire):
