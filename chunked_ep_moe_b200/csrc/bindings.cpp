@@ -126,7 +126,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("router_bwd", &cem::router_bwd, "-> fp32 gradient of the logits");
   py::class_<cem::KernelRunner>(m, "KernelRunner")
       .def(py::init<int, int, int, int>(), py::arg("L"), py::arg("S"), py::arg("stripe"), py::arg("num_sms"))
-      .def("set_groups", &cem::KernelRunner::set_groups)
+      .def("with_groups", &cem::KernelRunner::with_groups)
       .def("gmm_swiglu", &cem::KernelRunner::gmm_swiglu, py::arg("x"), py::arg("w_up"), py::arg("act"),
            py::arg("h") = py::none())
       .def("gmm", &cem::KernelRunner::gmm)

@@ -39,28 +39,30 @@ KernelRunner::KernelRunner(int L, int S, int stripe, int num_sms)
   need(S >= 8 && S % 8 == 0, "S must be a positive multiple of 8");
   need(stripe == 32 || stripe == 64 || stripe == 128, "stripe must be 32, 64 or 128");
   lay_ = make_plan_layout(1, L, S, 1);
-  auto i32 = torch::TensorOptions().device(torch::kCUDA).dtype(torch::kInt32);
-  plan_ = torch::zeros({lay_.total}, i32);
-  status_ = torch::zeros({8}, i32);
+  status_ = torch::zeros({8}, torch::TensorOptions().device(torch::kCUDA).dtype(torch::kInt32));
 }
 
-void KernelRunner::set_groups(torch::Tensor group_rows) {
+KernelRunner KernelRunner::with_groups(torch::Tensor group_rows) const {
   need(group_rows.is_cuda() && group_rows.scalar_type() == torch::kInt32 && group_rows.is_contiguous() &&
            group_rows.numel() == L_,
        "group_rows must be a contiguous CUDA int32 tensor of L elements");
-  counts_ = group_rows;  // read by the plan kernel on this stream
+  KernelRunner bound = *this;
+  bound.counts_ = group_rows;  // read by the plan kernel on this stream
+  bound.plan_ = torch::empty({lay_.total}, group_rows.options());
   PlanKernelParams pp{};
   pp.lay = lay_;
   pp.me = 0;
-  pp.plan = plan_.data_ptr<int>();
-  pp.counts = counts_.data_ptr<int>();
-  pp.my_counts = counts_.data_ptr<int>();
+  pp.plan = bound.plan_.data_ptr<int>();
+  pp.counts = bound.counts_.data_ptr<int>();
+  pp.my_counts = bound.counts_.data_ptr<int>();
   pp.spin_limit = 1;
   pp.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
   launch_plan_build(pp, stream());
+  return bound;
 }
 
 GemmParams KernelRunner::base() const {
+  need(plan_.defined(), "no groups (with_groups)");
   GemmParams p{};
   p.plan = plan_.data_ptr<int>();
   p.lay = lay_;

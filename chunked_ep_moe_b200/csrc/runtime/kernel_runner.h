@@ -6,9 +6,9 @@
 // reference's kernel-level surface: gmm, gmm_swiglu, gmm_dswiglu, tgmm
 // (src/chunked_moe/kernels/fused_expert.py:102-352).
 //
-// Rows: a slice holds at most `S` rows, expert after expert; `set_groups` takes the rows per expert as a device
+// Rows: a slice holds at most `S` rows, expert after expert; `with_groups` takes the rows per expert as a device
 // tensor and builds the tile tables on the device (no host synchronisation). Rows past the groups' total are padding:
-// never read into a weight gradient, never written.
+// never read into a weight gradient; the row-wise modes set them to zero in their outputs.
 #pragma once
 
 #include <torch/extension.h>
@@ -25,9 +25,9 @@ class KernelRunner {
  public:
   KernelRunner(int L, int S, int stripe, int num_sms);
 
-  // rows per expert, int32 [L] on the device, sum <= S
-  void set_groups(torch::Tensor group_rows);
-  // (Row-wise results: rows past the last group are set to zero.)
+  // A runner with the tile tables of one slice: rows per expert, int32 [L] on the device, sum <= S. The tables are the
+  // result's own, so slices of several callers, on whatever streams and threads, have nothing in common but the status block.
+  KernelRunner with_groups(torch::Tensor group_rows) const;
   // act[S,F] = silu(x Wg) * (x Wu) from striped w_up [L,D,2F]; h [S,2F] (the rounded pre-activation) is optional
   void gmm_swiglu(torch::Tensor x, torch::Tensor w_up, torch::Tensor act, c10::optional<torch::Tensor> h);
   // out[S,N] = lhs[S,K] rhs[g]; rhs is [L,K,N], or [L,N,K] with transpose_rhs (no transpose is materialised)

@@ -34,7 +34,7 @@ def _group_tensor(group_sizes, device) -> torch.Tensor:
 
 
 def _runner(num_groups: int, rows: int, stripe: int, device: torch.device):
-    """The cached launcher for slices of `rows` rows and `num_groups` experts (tile tables live in it)."""
+    """The cached launcher for slices of `rows` rows and `num_groups` experts."""
     key = (num_groups, rows, stripe, device.index)
     runner = _runners.get(key)
     if runner is None:
@@ -45,11 +45,11 @@ def _runner(num_groups: int, rows: int, stripe: int, device: torch.device):
 
 
 def _prepare(rows_tensor: torch.Tensor, num_groups: int, group_sizes, stripe: int):
+    """A launcher with the tile tables of this slice (its own: calls on other streams or threads do not touch them)."""
     if rows_tensor.shape[0] % 8:
         raise ValueError(f"the fused kernels need a multiple of 8 rows per slice, got {rows_tensor.shape[0]}")
     runner = _runner(num_groups, rows_tensor.shape[0], stripe, rows_tensor.device)
-    runner.set_groups(_group_tensor(group_sizes, rows_tensor.device))
-    return runner
+    return runner.with_groups(_group_tensor(group_sizes, rows_tensor.device))
 
 
 def _rows(runner, like: torch.Tensor, cols: int) -> torch.Tensor:

@@ -148,3 +148,16 @@ def test_rows_past_the_groups_are_zero(groups):
     for name, t in (("y", y), ("h", res.h), ("act", res.act), ("dh", dh), ("dx", grads.dx)):
         assert torch.count_nonzero(t[rows:]) == 0 and torch.isfinite(t).all(), name
     fx.check_status()
+
+
+def test_slices_in_preparation_do_not_share_tables():
+    """Two slices of one geometry prepared before either runs (two threads, two streams): each keeps its own groups."""
+    S, D, F = 256, 256, 256
+    x, _, w_up, _, _ = _inputs(S, D, F, [256, 0, 0])
+    groups = [[100, 0, 90], [3, 200, 53]]
+    prepared = [fx._prepare(x, 3, g, 64) for g in groups]
+    for runner, g in zip(prepared, groups):
+        act, h = fx._gmm_swiglu(runner, x, w_up, True)
+        want = fx.gmm_swiglu(x, w_up, g, stripe=64, return_h=True)
+        assert torch.equal(act, want[0]) and torch.equal(h, want[1])
+    fx.check_status()
