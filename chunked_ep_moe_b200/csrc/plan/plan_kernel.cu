@@ -97,7 +97,7 @@ __device__ void plan_phase_b_warps(int* plan, const PlanLayout& y, const int* se
   if (num_slices > y.max_slices) num_slices = y.max_slices;
   for (int j = warp; j < y.max_slices; j += nwarps) {
     int num_t = 0, num_g = 0, chunks = 0;
-    if (j < num_slices) {
+    if (j < num_slices || j == 0) {
       const int lo = j * S, hi = lo + S;
       int* tt = plan + y.off_tiles + 4 * y.max_tiles * j;
       int* gt = plan + y.off_gtiles + 4 * y.max_gtiles * j;

@@ -162,7 +162,7 @@ CEM_HD inline void plan_phase_b(int* plan, const PlanLayout& y, int tid, int nth
   if (num_slices > y.max_slices) num_slices = y.max_slices;
   for (int j = tid; j < y.max_slices; j += nthreads) {
     int num_t = 0, num_g = 0, chunks = 0;
-    if (j < num_slices) {
+    if (j < num_slices || j == 0) {  // (slice 0 also without rows: that is where empty experts' gradients are written)
       const int lo = j * S, hi = lo + S;
       int* tt = plan + y.off_tiles + 4 * y.max_tiles * j;
       int* gt = plan + y.off_gtiles + 4 * y.max_gtiles * j;

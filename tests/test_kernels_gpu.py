@@ -161,3 +161,19 @@ def test_slices_in_preparation_do_not_share_tables():
         want = fx.gmm_swiglu(x, w_up, g, stripe=64, return_h=True)
         assert torch.equal(act, want[0]) and torch.equal(h, want[1])
     fx.check_status()
+
+
+@pytest.mark.parametrize("groups", [[0], [0, 0, 0], [0, 1, 0], [40, 0, 87]], ids=str)
+def test_gradients_of_experts_without_rows_are_zero(groups):
+    """Also when no expert has any (a rank's trailing slices under a collective transport)."""
+    S, D, F = 128, 256, 256
+    x, dy, w_up, w_down, _ = _inputs(S, D, F, groups)
+    _, res = fx.expert_forward(x, w_up, w_down, groups, stripe=64)
+    for t in (w_up, w_down):
+        junk = [torch.full_like(t, float("nan")) for _ in range(4)]
+        del junk  # the gradients are likely to land on these
+    grads = fx.expert_backward(x, w_up, w_down, groups, res, dy, stripe=64)
+    for name, t in (("dw_up", grads.dw_up), ("dw_down", grads.dw_down)):
+        for g, n in zip(t, groups):
+            assert torch.isfinite(g).all() and (n > 0 or torch.count_nonzero(g) == 0), name
+    fx.check_status()

@@ -110,6 +110,33 @@ def _check_tables(P, L, S, tokens, top_k, skew, seed):
         np.testing.assert_array_equal(seen_final, np.ones(L))  # every expert's gradient is finalised exactly once
 
 
+def _check_nothing_routed(tab, lay, P, L, max_slices):
+    """Slice 0 finalises every expert's (empty) gradient, nothing else is in the tables."""
+    assert tab[0] == 0 and tab[1] == 0
+    for j in range(max_slices):
+        assert tab[lay["num_mtiles"] + j] == 0 and tab[lay["num_chunks"] + j] == 0
+        assert tab[lay["num_gtiles"] + j] == (L if j == 0 else 0)
+    groups = tab[lay["gtiles"]: lay["gtiles"] + 4 * L].reshape(L, 4)
+    np.testing.assert_array_equal(groups, [[l, 0, 0, 3] for l in range(L)])
+
+
+@pytest.mark.parametrize("P,L,max_slices", [(1, 1, 1), (1, 5, 1), (1, 40, 2), (3, 33, 2)])
+def test_tables_without_a_single_row(P, L, max_slices):
+    """No expert has any row: the weight-gradient kernel still has to write all of them, as zeros."""
+    ext = _build.load()
+    tab = ext.plan_build_host(torch.zeros(P, P, L, dtype=torch.int32), 64, max_slices, P - 1).numpy()
+    _check_nothing_routed(tab, ext.plan_layout(P, L, 64, max_slices), P, L, max_slices)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("P,L,max_slices", [(1, 1, 1), (1, 5, 1), (1, 40, 2), (3, 33, 2), (8, 128, 2)])
+def test_plan_kernel_without_a_single_row(P, L, max_slices):
+    """The same from the plan kernel; 8 x 128 experts do not fit its shared memory (serial tables)."""
+    ext = _build.load()
+    tab = ext.plan_build_device(torch.zeros(P, P, L, dtype=torch.int32, device="cuda"), 64, max_slices, P - 1).cpu().numpy()
+    _check_nothing_routed(tab, ext.plan_layout(P, L, 64, max_slices), P, L, max_slices)
+
+
 def test_status_block_text():
     """The message `check_status` raises for a recorded kernel error (formatting runs without a GPU)."""
     from chunked_ep_moe_b200 import _build
