@@ -361,19 +361,29 @@ void FusedRank::wait_header() {
   std::atomic_thread_fence(std::memory_order_acquire);
 }
 
+// Waits until nothing that was launched for a pass runs any more: behind an error the pass's tensors are about to be released
+// and the status block, which makes its remaining kernels return at once, to be cleared. (Every wait in a kernel is bounded.)
+void FusedRank::quiesce() const {
+  for (cudaStream_t s : {comm_stream_, expand_stream_, chain_[0], chain_[1], aux_stream_})
+    if (s != nullptr) cudaStreamSynchronize(s);
+  cudaStreamSynchronize(current_stream());
+}
+
 int64_t FusedRank::resolve_slices() {
   wait_header();
+  std::string message;
   const int32_t* st = host_header_ + 16;
-  if (st[0] != 0) {
-    const std::string message = format_status(std::vector<int64_t>(st, st + 8), me_);
-    cudaStream_t cur = current_stream();
-    cuda_check(cudaStreamSynchronize(cur), "status sync");  // what was launched on the guess ends (at once) first
-    cuda_check(cudaMemsetAsync(status_.data_ptr(), 0, 8 * sizeof(int32_t), cur), "status clear");
-    cuda_check(cudaStreamSynchronize(cur), "status clear sync");
+  if (st[0] != 0) message = format_status(std::vector<int64_t>(st, st + 8), me_);
+  else if (host_header_[4] != 0) message = "routing needs more slices than the workspace was sized for (max_slices)";
+  else if (host_header_[5] != cur_rows_) message = "the routing plan does not account for every token copy";
+  if (!message.empty()) {
+    quiesce();  // what was launched on the guess ends (at once, if an error is recorded) before anything is cleared
+    if (st[0] != 0) {
+      cuda_check(cudaMemsetAsync(status_.data_ptr(), 0, 8 * sizeof(int32_t), current_stream()), "status clear");
+      cuda_check(cudaStreamSynchronize(current_stream()), "status clear sync");
+    }
     throw std::runtime_error(message);
   }
-  expect(host_header_[4] == 0, "routing needs more slices than the workspace was sized for (max_slices)");
-  expect(host_header_[5] == cur_rows_, "the routing plan does not account for every token copy");
   last_slices_ = host_header_[0];
   return last_slices_;
 }
@@ -909,6 +919,8 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
   // that set every kernel that would read the order returns at once.)
   torch::Tensor plan = torch::empty({lay_.total}, i32), order = torch::empty({tk}, i32),
                 inv_order = torch::empty({tk}, i32), out = torch::empty_like(x);
+  std::vector<torch::Tensor> kept;
+  const QuiesceOnError guard{this};
   auto run_slices = [&](int64_t lo, int64_t hi) {
     if (hi <= lo) return;
     put(lo, plan, order, x, c10::nullopt, w_flat);
@@ -938,7 +950,6 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
     guess = std::max<int64_t>(0, begin_forward_async(expert_ids, plan, order, inv_order, plan, false));
   }
   if (known >= 0) guess = std::min<int64_t>(known, max_slices_);
-  std::vector<torch::Tensor> kept;
   int64_t kept_slices = 0;
   if (training && guess > 0) {  // slices past the guess are recomputed
     kept = allocate_kept(known >= 0 ? tk : guess * S_, x.options());
@@ -977,6 +988,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
   const int64_t n = begin_backward(plan, known_slices, order.numel());
   torch::Tensor dw_up = torch::empty_like(w_up), dw_down = torch::empty_like(w_down), dx = torch::empty_like(x);
   torch::Tensor d_weights = torch::empty({w_flat.numel()}, w_flat.options());
+  const QuiesceOnError guard{this};
   if (n > 0) {
     put(0, plan, order, x, g, w_flat);
   } else {

@@ -18,6 +18,7 @@
 
 #include <map>
 #include <algorithm>
+#include <exception>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -111,6 +112,15 @@ class FusedRank {
   void enter_pass();
   void end_pass(int64_t n_slices);
   void wait_header();
+  void quiesce() const;
+  // Declared behind the tensors that a pass uses on the rank's streams: they are not released under it by an exception.
+  struct QuiesceOnError {
+    const FusedRank* rank;
+    const int before = std::uncaught_exceptions();
+    ~QuiesceOnError() {
+      if (std::uncaught_exceptions() > before) rank->quiesce();
+    }
+  };
   void keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices);
   void release_kept();
   std::vector<torch::Tensor> allocate_kept(int64_t rows, const torch::TensorOptions& bf16) const;

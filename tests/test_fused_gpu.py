@@ -230,6 +230,49 @@ def test_invalid_expert_id_is_reported_by_the_forward():
         fused.release_workspaces()  # the pass was abandoned half way: do not reuse this workspace
 
 
+def test_nothing_runs_any_more_when_an_error_is_raised():
+    """The pass behind an invalid expert id is launched on a guess, over many slices and the workspace's streams, before the
+    host learns of the id. When that raises, all of it has ended and ended unheard: a kernel that only started once the status
+    was cleared would have moved rows (and would work on tensors that the caller has released)."""
+    from chunked_ep_moe_b200 import _build
+    from chunked_ep_moe_b200.ops import fused
+
+    torch.manual_seed(0)
+    T, D, F, E, K, S = 256, 256, 256, 2, 2, 8
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=S, transport="nvshmem", expert_compute="fused",
+                           stripe_width=64)
+    ws = fused.get_workspace(cfg, None, D, F, T * K)
+    rank, slices = ws.rank, T * K // S
+    x = torch.randn(T, D, device="cuda").bfloat16()
+    ids = torch.stack([torch.randperm(E, device="cuda")[:K] for _ in range(T)]).int().contiguous()
+    ids[T - 1, 1] = E
+    w_flat = torch.rand(T * K, device="cuda")
+    w_up = (torch.randn(E, D, 2 * F, device="cuda") * 0.05).bfloat16()
+    w_down = (torch.randn(E, F, D, device="cuda") * 0.05).bfloat16()
+    plan = torch.zeros(ws.plan_ints, dtype=torch.int32, device="cuda")
+    order = torch.zeros(T * K, dtype=torch.int32, device="cuda")
+    inv_order = torch.zeros_like(order)
+    torch.cuda.synchronize()
+    try:
+        torch.cuda._sleep(40_000_000)  # some 20 ms: all of the pass is queued before the first kernel starts
+        rank.begin_forward_async(ids, plan, order, inv_order, ws.dummy_counts, False)
+        rank.put(0, plan, order, x, None, w_flat)
+        for j in range(slices):
+            if j + 1 < slices:
+                rank.put(j + 1, plan, order, x, None, w_flat)
+            rank.compute_forward(j, plan, w_up, w_down)
+        with pytest.raises(RuntimeError, match="index check failed"):
+            rank.resolve_slices()
+        torch.cuda.synchronize()
+        rank.check_status()
+        lay = _build.load().arena_layout(1, E, S, D, T * K, False)
+        arrived = _build.load().arena_read_i32(ws.arena.local, lay["arrive"], E)
+        assert torch.count_nonzero(arrived) == 0, arrived
+    finally:
+        torch.cuda.synchronize()
+        fused.release_workspaces()  # the pass was abandoned half way: do not reuse this workspace
+
+
 def test_slice_count_guess_is_corrected_in_both_directions():
     """The forward launches on the previous pass's slice count before it knows its own: passes that need more slices
     than the one before, and fewer, must both match the oracle (the same workspace throughout)."""
