@@ -200,14 +200,15 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
     const size_t drow = static_cast<size_t>(buf) * S + e.z + first;
     int token = -1;  // of row `lane`
     if (lane < rows) {
-      const int flat = p.order[e.x + first + lane];
+      const int at = e.x + first + lane, row = e.z + first + lane;
+      const int flat = at >= 0 && at < p.num_tokens * p.top_k ? p.order[at] : -1;
       token = flat / p.top_k;
-      // Index check: a send-order entry outside the token range or a destination row outside the slice buffer is recorded
-      // and the row is skipped, never dereferenced. The arrival is still signalled, so nothing waits for the row; the
-      // recorded status tells the host that the pass is invalid.
-      if (flat < 0 || token >= p.num_tokens || e.z + first + lane >= S) {
-        report_status(p.status, kStatusBadIndex, kKernelPut, 0, p.slice, e.x + first + lane,
-                      static_cast<uint32_t>(p.num_tokens), static_cast<uint32_t>(token));
+      // Index check: a segment outside the send order, an entry outside the token range or a destination row outside the slice
+      // buffer is recorded and the row is skipped, never dereferenced. The arrival is still signalled, so nothing waits for the
+      // row; the recorded status tells the host that the pass is invalid.
+      if (flat < 0 || token >= p.num_tokens || row < 0 || row >= S) {
+        report_status(p.status, kStatusBadIndex, kKernelPut, 0, p.slice, at, static_cast<uint32_t>(p.num_tokens),
+                      static_cast<uint32_t>(token));
         token = -1;
       } else {
         p.peer_w[r][drow + lane] = p.w_flat[flat];

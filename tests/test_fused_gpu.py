@@ -203,6 +203,39 @@ def test_bad_send_order_entry_is_reported_not_dereferenced():
         fused.release_workspaces()  # the pass was abandoned half way: do not reuse this workspace
 
 
+@pytest.mark.parametrize("field,value", [(2, -3), (2, 200), (0, -5), (0, 126)],
+                         ids=["row below", "row above", "segment below", "segment above"])
+def test_put_segment_out_of_range_is_reported_not_dereferenced(field, value):
+    """A put table whose destination rows or send-order entries leave their buffers: recorded, the rows are skipped."""
+    from chunked_ep_moe_b200 import _build
+    from chunked_ep_moe_b200.ops import fused
+
+    torch.manual_seed(0)
+    T, D, F, E, K, S = 64, 256, 256, 2, 2, 168  # a geometry no other test uses: the workspace is thrown away below
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=S, transport="nvshmem", expert_compute="fused",
+                           stripe_width=64)
+    ws = fused.get_workspace(cfg, None, D, F, T * K)
+    rank = ws.rank
+    x = torch.randn(T, D, device="cuda").bfloat16()
+    ids = torch.tensor([[0, 1]] * T, dtype=torch.int32, device="cuda")
+    plan = torch.empty(ws.plan_ints, dtype=torch.int32, device="cuda")
+    order = torch.empty(T * K, dtype=torch.int32, device="cuda")
+    inv_order = torch.empty_like(order)
+    lay = _build.load().plan_layout(1, E, S, ws.max_slices)
+    try:
+        assert rank.begin_forward(ids, plan, order, inv_order, ws.dummy_counts, False) == 1
+        plan[lay["put"] + 4 + field] = value  # {send-order offset, rows, destination row, ...} of the second expert
+        torch.cuda.synchronize()  # (the put runs on another stream)
+        rank.put(0, plan, order, x, None, torch.rand(T * K, device="cuda"))
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="index check failed"):
+            rank.check_status()
+        rank.check_status()
+    finally:
+        torch.cuda.synchronize()
+        fused.release_workspaces()  # the pass was abandoned half way: do not reuse this workspace
+
+
 def test_invalid_expert_id_is_reported_by_the_forward():
     """An expert id outside [0, E): the sort records it, every kernel launched on the guessed slice count returns at
     once, and the forward raises when it reads the pass's header (nothing is dereferenced, no wait runs out)."""
