@@ -1,5 +1,6 @@
 #include "fused_rank.h"
 
+#include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -951,7 +952,7 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
   }
   if (known >= 0) guess = std::min<int64_t>(known, max_slices_);
   int64_t kept_slices = 0;
-  if (training && guess > 0) {  // slices past the guess are recomputed
+  if (training && guess > 0 && !at::SavedTensorDefaultHooks::get_hooks().has_value()) {  // slices past the guess are recomputed
     kept = allocate_kept(known >= 0 ? tk : guess * S_, x.options());
     if (!kept.empty()) {
       kept_slices = guess;

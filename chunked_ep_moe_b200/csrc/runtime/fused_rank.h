@@ -79,7 +79,9 @@ class FusedRank {
   void finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights);
 
   // The two passes as one call each (what `chunked_moe` runs). Forward: ([out, plan, order, inv_order] and, when a
-  // `training` pass keeps them, [h, w * act]; slice count; slices kept); it throws a recorded kernel error. Backward:
+  // `training` pass keeps them, [h, w * act]; slice count; slices kept); it throws a recorded kernel error. Nothing is kept
+  // under saved-tensor hooks: what is saved may then not depend on how much memory is free (activation checkpointing wants
+  // the same tensors from the recomputation) and may be on its way to the host. Backward:
   // (dx, d_weights, dw_up, dw_down). Tensors are contiguous CUDA tensors of the workspace's geometry: x, g [T, D] bf16,
   // expert_ids [T, K] int32, w_flat [T*K] fp32.
   std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> forward_pass(

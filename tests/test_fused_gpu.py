@@ -429,6 +429,41 @@ def test_kept_activations_give_the_same_bits(monkeypatch, tokens, stripe, wire):
     fused.release_workspaces()
 
 
+def test_what_is_saved_under_hooks_does_not_depend_on_memory(monkeypatch):
+    """Activation checkpointing compares the tensors saved by the forward with those of its recomputation, when more or less
+    memory may be free: a layer large enough to keep activations saves the same ones whether it may keep any or not."""
+    from torch.utils.checkpoint import checkpoint
+
+    from chunked_ep_moe_b200.ops import fused
+
+    E, K, D, F, T = 8, 2, 2048, 512, 2048
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    args = [rnd(T, D).bfloat16(), rnd(T, K).sigmoid(), (rnd(E, D, 2 * F) / math.sqrt(D)).bfloat16(),
+            (rnd(E, F, D) / math.sqrt(F)).bfloat16()]
+    ids, g = torch.topk(rnd(T, E), K, dim=-1).indices.int(), rnd(T, D).bfloat16()
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=4096, transport="nvshmem", expert_compute="fused",
+                           stripe_width=64)
+    layer = lambda x, w, w_up, w_down: chunked_moe(x, ids, w, w_up, w_down, cfg)
+    saved, grads = {}, {}
+    for keep in ("1", "0"):
+        fused.release_workspaces()
+        monkeypatch.setenv("CEM_KEEP_ACTIVATIONS", keep)
+        shapes = []
+        leaves = [t.clone().requires_grad_(True) for t in args]
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: shapes.append((t.shape, t.dtype)) or t, lambda t: t):
+            out = layer(*leaves)
+        out.backward(g)
+        saved[keep], grads[keep] = shapes, [t.grad for t in leaves]
+    assert saved["1"] == saved["0"]
+    for reentrant in (False, True):
+        leaves = [t.clone().requires_grad_(True) for t in args]
+        checkpoint(layer, *leaves, use_reentrant=reentrant).backward(g)
+        assert all(torch.equal(a, b.grad) for a, b in zip(grads["1"], leaves))
+    assert all(torch.equal(a, b) for a, b in zip(grads["1"], grads["0"]))
+    fused.release_workspaces()
+
+
 @pytest.mark.parametrize("hidden", [256, 768, 1280])
 @pytest.mark.parametrize("group_rows", [[1, 2, 3, 4], [5, 0, 7, 64], [0, 0, 0, 130]], ids=str)
 def test_one_rank_fp8_wire_rounds_like_the_wire(group_rows, hidden):
