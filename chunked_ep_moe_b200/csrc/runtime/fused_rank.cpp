@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <stdexcept>
 
 #include "tensor_map.h"
@@ -840,13 +841,13 @@ void FusedRank::release_kept() {
 }
 
 // Keeping pays once the GEMM that it saves is longer than a launch, and only while there is memory to spare: live tensors
-// and arenas, these included, stay within half of the device, else (or when the allocation fails) the backward recomputes.
+// and all of the process's arenas, these included, stay within half of the device, else (or when the allocation fails) the backward recomputes.
 // (What the caching allocator knows, not `cudaMemGetInfo`: that call takes 2 ms with a busy device.)
 std::vector<torch::Tensor> FusedRank::allocate_kept(int64_t rows, const torch::TensorOptions& bf16) const {
   if (std::min<int64_t>(rows, S_) * D_ * F_ < kKeepWork || !keep_activations_) return {};
   try {
     const auto pool = c10::cuda::CUDACachingAllocator::getDeviceStats(bf16.device().index());
-    const size_t live = static_cast<size_t>(pool.allocated_bytes[0].current) + arena_lay_.total;
+    const size_t live = static_cast<size_t>(pool.allocated_bytes[0].current) + static_cast<size_t>(arenas_allocated());
     if (live + static_cast<size_t>(rows) * 3 * F_ * 2 > device_bytes_ / 2) return {};
     return {torch::empty({rows, 2 * F_}, bf16), torch::empty({rows, F_}, bf16)};
   } catch (const c10::Error&) {  // no memory, or an allocator that keeps no statistics
@@ -1008,15 +1009,46 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
 // ---------------------------------------------------------------------------------------------
 // symmetric arena: cudaMalloc + CUDA IPC handles
 // ---------------------------------------------------------------------------------------------
+namespace {
+std::mutex g_arena_mutex;
+std::map<int64_t, std::pair<int, int64_t>> g_arenas;  // address -> (device, bytes)
+
+int current_device() {
+  int device = 0;
+  cuda_check(cudaGetDevice(&device), "device");
+  return device;
+}
+}  // namespace
+
 int64_t arena_alloc(int64_t bytes) {
   void* p = nullptr;
   cuda_check(cudaMalloc(&p, static_cast<size_t>(bytes)), "arena cudaMalloc");
+  const int64_t ptr = reinterpret_cast<int64_t>(p);
+  {
+    std::lock_guard<std::mutex> lock(g_arena_mutex);
+    g_arenas[ptr] = {current_device(), bytes};
+  }
   cuda_check(cudaMemset(p, 0, static_cast<size_t>(bytes)), "arena memset");
   cuda_check(cudaDeviceSynchronize(), "arena sync");
-  return reinterpret_cast<int64_t>(p);
+  return ptr;
 }
 
-void arena_free(int64_t ptr) { cudaFree(reinterpret_cast<void*>(ptr)); }
+void arena_free(int64_t ptr) {
+  {
+    std::lock_guard<std::mutex> lock(g_arena_mutex);
+    g_arenas.erase(ptr);
+  }
+  cudaFree(reinterpret_cast<void*>(ptr));
+}
+
+int64_t arenas_allocated() {
+  const int device = current_device();
+  int64_t total = 0;
+  std::lock_guard<std::mutex> lock(g_arena_mutex);
+  for (const auto& [ptr, at] : g_arenas)
+    if (at.first == device) total += at.second;
+  return total;
+}
 
 py::bytes arena_export(int64_t ptr) {
   cudaIpcMemHandle_t h;

@@ -206,6 +206,8 @@ void arena_free(int64_t ptr);
 py::bytes arena_export(int64_t ptr);
 int64_t arena_import(py::bytes handle);
 void arena_close(int64_t ptr);
+// Bytes of this process's arenas on the current device (the caching allocator's statistics do not know them).
+int64_t arenas_allocated();
 void arena_zero(int64_t ptr, int64_t bytes);
 void arena_fill(int64_t ptr, int64_t bytes, int value);
 // Synchronises the device and copies `count` int32 values at `ptr + offset_bytes` to a CPU tensor (tests read counters).

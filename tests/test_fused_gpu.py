@@ -464,6 +464,38 @@ def test_what_is_saved_under_hooks_does_not_depend_on_memory(monkeypatch):
     fused.release_workspaces()
 
 
+def test_arenas_of_other_workspaces_count_against_the_kept_activations():
+    """Activations are kept while live tensors and arenas stay within half of the device; an arena is no tensor, and any
+    workspace's counts."""
+    from chunked_ep_moe_b200 import _build
+    from chunked_ep_moe_b200.ops import fused
+
+    ext = _build.load()
+    E, K, D, F, T = 8, 2, 2048, 512, 2048
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    x, ids = rnd(T, D).bfloat16(), torch.topk(rnd(T, E), K, dim=-1).indices.int()
+    w, w_up, w_down = rnd(T, K).sigmoid(), rnd(E, D, 2 * F).bfloat16(), rnd(E, F, D).bfloat16()
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=4096, transport="nvshmem", expert_compute="fused",
+                           stripe_width=64)
+    fused.release_workspaces()
+    assert ext.arenas_allocated() == 0
+    ws = fused.get_workspace(cfg, None, D, F, T * K)
+    own = ext.arenas_allocated()
+    assert own == ws.arena.nbytes
+    kept = lambda: ws.rank.forward_pass(x, ids, w.reshape(-1), w_up, w_down, True)[2]
+    assert kept() == 1
+    half = torch.cuda.get_device_properties(0).total_memory // 2
+    other = ext.arena_alloc(half - own // 2)
+    try:
+        assert ext.arenas_allocated() > half
+        assert kept() == 0
+    finally:
+        ext.arena_free(other)
+    assert ext.arenas_allocated() == own and kept() == 1
+    fused.release_workspaces()
+
+
 @pytest.mark.parametrize("hidden", [256, 768, 1280])
 @pytest.mark.parametrize("group_rows", [[1, 2, 3, 4], [5, 0, 7, 64], [0, 0, 0, 130]], ids=str)
 def test_one_rank_fp8_wire_rounds_like_the_wire(group_rows, hidden):
