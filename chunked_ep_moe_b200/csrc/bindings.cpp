@@ -103,6 +103,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("arena_bytes", &arena_bytes, "size of one rank's symmetric arena");
   m.def("arena_alloc", &cem::arena_alloc);
   m.def("arena_free", &cem::arena_free);
+  m.def("slices_to_keep", &cem::slices_to_keep, "slices whose activations a rank among several keeps");
   m.def("arenas_allocated", &cem::arenas_allocated, "bytes of this process's arenas on the current device");
   m.def("arena_export", &cem::arena_export);
   m.def("arena_import", &cem::arena_import);

@@ -387,6 +387,7 @@ int64_t FusedRank::resolve_slices() {
     throw std::runtime_error(message);
   }
   last_slices_ = host_header_[0];
+  last_rows_ = host_header_[1];
   return last_slices_;
 }
 
@@ -953,10 +954,11 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
   }
   if (known >= 0) guess = std::min<int64_t>(known, max_slices_);
   int64_t kept_slices = 0;
-  if (training && guess > 0 && !at::SavedTensorDefaultHooks::get_hooks().has_value()) {  // slices past the guess are recomputed
-    kept = allocate_kept(known >= 0 ? tk : guess * S_, x.options());
+  if (training && !at::SavedTensorDefaultHooks::get_hooks().has_value()) {
+    const int64_t slices = known >= 0 ? guess : slices_to_keep(guess, last_rows_, S_);  // the others are recomputed
+    if (slices > 0) kept = allocate_kept(known >= 0 ? tk : slices * S_, x.options());
     if (!kept.empty()) {
-      kept_slices = guess;
+      kept_slices = slices;
       keep_rows(kept[0], kept[1], kept_slices);
     }
   }

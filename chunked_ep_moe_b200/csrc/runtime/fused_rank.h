@@ -39,6 +39,13 @@ ArenaLayout make_arena_layout(int P, int L, int S, int D, int tk_cap, bool fp8);
 // Text of a recorded status block {code, kernel, mode, slice, detail, expected, seen, block} (what check_status raises).
 std::string format_status(const std::vector<int64_t>& status, int rank);
 
+// Slices of a training forward that a rank among several keeps h and w * act of: those that its own stream reached in the pass
+// before (`stream_rows`), at most the `guess` it launches. Every rank loops as often as the fullest one, but a rank only has
+// memory reserved for about the rows that come to it; slices past them hold none, and one that does after all is recomputed.
+inline int64_t slices_to_keep(int64_t guess, int64_t stream_rows, int64_t slice_rows) {
+  return std::min<int64_t>(guess, (stream_rows + slice_rows - 1) / slice_rows);
+}
+
 class FusedRank {
  public:
   FusedRank(int P, int L, int me, int S, int D, int F, int K, int stripe, int tk_cap, int max_slices, int num_sms,
@@ -186,6 +193,7 @@ class FusedRank {
   unsigned long long pass_stream_ = 0;     // id of the stream that pass came on (ids are never used again, handles are)
   bool passed_ = false;                    // there was one
   int64_t last_slices_ = -1;  // slice count of the previous forward pass (the next pass's guess)
+  int64_t last_rows_ = 0;     // rows that came to this rank in it
   int32_t* host_header_ = nullptr;  // pinned: 16 plan header ints + 8 status ints + their sequence number, see the .cpp
   uint32_t host_seq_ = 0;     // headers asked for so far
   bool short_pass_ = false;   // an inline pass without autograd: fewer, larger kernels

@@ -137,6 +137,13 @@ def test_plan_kernel_without_a_single_row(P, L, max_slices):
     _check_nothing_routed(tab, ext.plan_layout(P, L, 64, max_slices), P, L, max_slices)
 
 
+@pytest.mark.parametrize("guess,rows,want", [(5, 0, 0), (5, 1, 1), (5, 64, 1), (5, 65, 2), (5, 320, 5), (3, 320, 3),
+                                             (0, 320, 0)])
+def test_a_rank_keeps_the_slices_that_its_own_rows_reach(guess, rows, want):
+    """Not the fullest rank's: a rank that gets nothing reserves nothing. (Slices of 64 rows.)"""
+    assert _build.load().slices_to_keep(guess, rows, 64) == want
+
+
 def test_status_block_text():
     """The message `check_status` raises for a recorded kernel error (formatting runs without a GPU)."""
     from chunked_ep_moe_b200 import _build
