@@ -283,11 +283,13 @@ __global__ void __launch_bounds__(256) return_dw_kernel(const ReturnDwParams p) 
       if (expert_start[mid] <= at) lo = mid; else hi = mid - 1;
     }
     float sum = 0.0f;
+    const float w = p.row_w[row];
     const float4* parts = reinterpret_cast<const float4*>(p.dwp + static_cast<size_t>(row) * p.parts);
     for (int q = 0; q < p.parts / 4; ++q) {  // F / 32 of them: a multiple of eight
       const float4 v = parts[q];
       sum += (v.x + v.y) + (v.z + v.w);
     }
+    if (weight_divides(w)) sum /= w;
     for (int s = 0; s < p.lay.P; ++s) {
       const int i = s * p.lay.L + lo, off = at - p.plan[p.lay.off_in_start + i];
       if (off >= 0 && off < p.plan[p.lay.off_in_size + i]) {

@@ -413,6 +413,10 @@ __device__ __forceinline__ void release_count(uint32_t* p, uint32_t v, int ranks
   }
 }
 
+// Whether a row's router weight gradient is summed as <acc, w * act> and divided by w (else as <acc, act>): with w in this range
+// no w * act of a normal size has left the normal bf16 numbers. False for zero, infinities and NaN.
+__device__ __forceinline__ bool weight_divides(float w) { return fabsf(w) >= 0x1p-32f && fabsf(w) <= 0x1p32f; }
+
 // Wrap-safe "counter has reached target" for monotonically increasing 32-bit counters.
 __device__ __forceinline__ bool reached(uint32_t seen, uint32_t target) {
   return static_cast<int32_t>(seen - target) >= 0;

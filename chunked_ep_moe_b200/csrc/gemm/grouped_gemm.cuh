@@ -68,8 +68,10 @@ struct GemmParams {
   __nv_bfloat16* out0;        // swiglu: act [S,F]; dswiglu: dh [S,2F]
   __nv_bfloat16* out1;        // swiglu: h [S,2F] or null
   const __nv_bfloat16* in0;   // dswiglu: h [S,2F]
+  const __nv_bfloat16* in1;   // dswiglu: w * act [S,F], leading dimension ld1 (with dwp)
   const float* row_w;         // router weight per slice row [S]; swiglu / dswiglu: null = 1
-  float* dwp;                 // dswiglu: shares of the router weights' gradients, one per 32 columns [S, dwp_tiles], or null
+  float* dwp;                 // dswiglu: shares of the router weights' gradients (times the weight, see `weight_divides`), one per
+                              // 32 columns [S, dwp_tiles], or null
   int dwp_tiles;
   int ld0, ld1;
   // --- combine targets (down_fwd, dx) --------------------------------------------------------

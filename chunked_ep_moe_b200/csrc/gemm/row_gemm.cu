@@ -289,18 +289,67 @@ __device__ __forceinline__ void combine_epilogue(const GemmParams& p, const RowT
 // SwiGLU': 128 columns of d_act and the 256 striped columns of h / dh that belong to them (512 bytes of a row). The
 // group brings a chunk of h into its staging buffer (the next chunk's loads are in flight meanwhile), every warp turns
 // its own gate and up columns into gradients in place, the group writes the chunk out as dh.
+//
+// d_weight = <acc, act> is summed against the stored w * act and divided by w where the shares are added up
+// (`weight_divides`): one rounding of act away from exact. Against the act that h gives, two rounded factors, it is 8 % further
+// from 64 bits than a GEMM on the rounded act is (0.00253 against 0.00235 at D=7168, F=2048; this way 0.00167). A chunk of
+// w * act passes through the buffer that h goes into next, at two more group barriers.
+//
+// Nothing of this depends on the accumulator: the first chunk is staged while the tile's MMAs run. (The router weights are not
+// asked for before the accumulator is there: in a backward that starts with this GEMM they arrive with the rows it waits for.)
+struct DswigluLoads {
+  int4 h[8];    // this thread's 16-byte pieces of the chunk's 512-byte rows of h
+  int4 act[4];  // and of the 256-byte rows of w * act
+};
+
+// A chunk's loads; rows past the tile keep what the registers hold.
+__device__ __forceinline__ void load_dswiglu(const GemmParams& p, const RowTile& tl, const GroupCtx& c, int ch, DswigluLoads* v) {
+  const int row0 = tl.row0 + ch * 32, nvalid = tl.nrows - ch * 32, col = tl.n * kBlockN + c.rank * kBlockM;
+  const uint8_t* h = reinterpret_cast<const uint8_t*>(p.in0 + static_cast<size_t>(row0) * p.ld0 + 2 * col) + c.lane * 16;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = c.q + 4 * i;
+    if (row < nvalid) v->h[i] = *reinterpret_cast<const int4*>(h + static_cast<size_t>(row) * p.ld0 * 2);
+  }
+  if (p.dwp != nullptr) {
+    const __nv_bfloat16* act = p.in1 + static_cast<size_t>(row0) * p.ld1 + col + (c.gt & 15) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = (c.gt >> 4) + 8 * i;
+      if (row < nvalid) v->act[i] = *reinterpret_cast<const int4*>(act + static_cast<size_t>(row) * p.ld1);
+    }
+  }
+}
+
+// Loaded pieces of a chunk -> h in the group's buffer, w * act in the accumulator's fragment layout (m[j][s]: columns
+// 8 s + lane / 4, rows 8 j + 2 (lane & 3) + e).
+__device__ __forceinline__ void stage_dswiglu(const GemmParams& p, const GroupCtx& c, const DswigluLoads& v, uint32_t (&m)[4][4]) {
+  group_sync(c.h);  // the previous chunk has left the buffer
+  if (p.dwp != nullptr) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      st_shared_v4(staged<256>(c.staging, (c.gt >> 4) + 8 * i, c.gt & 15), v.act[i].x, v.act[i].y, v.act[i].z, v.act[i].w);
+    group_sync(c.h);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ldmatrix_x4_trans(staged<256>(c.staging, 8 * j + (c.lane & 7), c.q * 4 + (c.lane >> 3)), m[j]);
+    group_sync(c.h);  // every warp has read it: h goes over it
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    st_shared_v4(staged<512>(c.staging, c.q + 4 * i, c.lane), v.h[i].x, v.h[i].y, v.h[i].z, v.h[i].w);
+  group_sync(c.h);
+}
+
+// `v`, `m`: the first chunk's, staged.
 template <typename Release>
 __device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowTile& tl, uint32_t tacc,
-                                                 const GroupCtx& c, const int4 (&first)[8], Release&& release) {
+                                                 const GroupCtx& c, DswigluLoads& v, uint32_t (&m)[4][4],
+                                                 Release&& release) {
   const int chunks = (tl.nrows + 31) >> 5;
   const int col = 2 * (tl.n * kBlockN + c.rank * kBlockM);  // first striped column
   const int f = c.q * 32 + (c.lane >> 3) * 8;               // column (of 128) whose 16-byte piece this lane addresses
   const int gpiece = (2 * p.stripe * (f / p.stripe) + f % p.stripe) >> 3, upiece = gpiece + (p.stripe >> 3);
   const size_t ld_bytes = static_cast<size_t>(p.ld0) * 2;
-  const int piece = c.gt & 31, prow = c.gt >> 5;  // 32 threads per 512-byte row, four rows per sweep
-  int4 v[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = first[i];
   for (int ch = c.h; ch < chunks; ch += 2) {
     const int row0 = tl.row0 + ch * 32, nvalid = tl.nrows - ch * 32;
     float w[8];  // this thread's rows' router weights (past L1 and ahead of time, as in the up-projection)
@@ -309,20 +358,45 @@ __device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowT
       const int t = 8 * (i >> 1) + 2 * (c.lane & 3) + (i & 1);
       w[i] = p.row_w != nullptr && t < nvalid ? __ldcg(p.row_w + row0 + t) : 1.0f;
     }
-    group_sync(c.h);  // the previous chunk has left the buffer
-#pragma unroll
-    for (int i = 0; i < 8; ++i) st_shared_v4(staged<512>(c.staging, prow + 4 * i, piece), v[i].x, v[i].y, v[i].z, v[i].w);
-    if (ch + 2 < chunks) {
-      const uint8_t* src = reinterpret_cast<const uint8_t*>(p.in0 + static_cast<size_t>(row0 + 64) * p.ld0 + col) + piece * 16;
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (prow + 4 * i < nvalid - 64) v[i] = *reinterpret_cast<const int4*>(src + (prow + 4 * i) * ld_bytes);
-    }
-    group_sync(c.h);
+    if (ch != c.h) stage_dswiglu(p, c, v, m);
     uint32_t r[32];
     load_fragment(tacc + ch * 32, r);
     if (ch + 2 >= chunks) release();
-    float part[8];  // <acc, act> over this thread's columns, rows 8 j + 2 (lane & 3) + e
+    float part[8];      // <acc, w * act> over this thread's columns, rows 8 j + 2 (lane & 3) + e
+    if (p.dwp != nullptr) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        part[2 * j] = part[2 * j + 1] = 0.0f;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
+          part[2 * j] += __uint_as_float(r[b]) * bf16_lo(m[j][s]);
+          part[2 * j + 1] += __uint_as_float(r[b + 1]) * bf16_hi(m[j][s]);
+        }
+      }
+      uint32_t odd = 0;  // bit 2 j + e: the row's weight is nothing to divide by, its sum is <acc, act> with act from h
+#pragma unroll
+      for (int i = 0; i < 8; ++i) odd |= weight_divides(w[i]) ? 0u : 1u << i;
+      if (__any_sync(0xffffffffu, odd != 0)) {  // (rare: not in the loop below)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint32_t g[4], u[4];
+          ldmatrix_x4_trans(staged<512>(c.staging, 8 * j + (c.lane & 7), gpiece), g);
+          ldmatrix_x4_trans(staged<512>(c.staging, 8 * j + (c.lane & 7), upiece), u);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+              sum += __uint_as_float(r[(s >> 1) * 16 + j * 4 + (s & 1) * 2 + e]) *
+                     (silu_f(e ? bf16_hi(g[s]) : bf16_lo(g[s])) * (e ? bf16_hi(u[s]) : bf16_lo(u[s])));
+            if ((odd >> (2 * j + e)) & 1u) part[2 * j + e] = sum;
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (ch + 2 < chunks) load_dswiglu(p, tl, c, ch + 2, &v);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t ga = staged<512>(c.staging, 8 * j + (c.lane & 7), gpiece);
@@ -330,7 +404,6 @@ __device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowT
       uint32_t g[4], u[4];
       ldmatrix_x4_trans(ga, g);
       ldmatrix_x4_trans(ua, u);
-      part[2 * j] = part[2 * j + 1] = 0.0f;
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
         const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
@@ -345,7 +418,6 @@ __device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowT
           const float up = e ? bf16_hi(u[s]) : bf16_lo(u[s]);
           const float sig = sigmoid_f(gt);
           const float sl = gt * sig;
-          part[2 * j + e] += a[e] * (sl * up);
           dg[e] = d * up * (sig + sl * (1.0f - sig));
           du[e] = d * sl;
         }
@@ -630,7 +702,7 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
       if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, num_entries);
       const int as = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1u;
-      int4 first[8];
+      DswigluLoads first = {};  // (zeros: what rows past the tile are worked on with)
       if constexpr (Traits::kCombine) {
         // Where the rows of this group's chunks go (thread = row), worked out while the accumulator is being made.
         group_sync(c.h);  // the previous tile's table has been used up
@@ -644,15 +716,10 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
           if (lane == s) returned += cnt;
         }
       }
+      uint32_t first_act[4][4] = {};
       if constexpr (MODE == kModeDswiglu) {
-        const uint8_t* src = reinterpret_cast<const uint8_t*>(
-            p.in0 + static_cast<size_t>(tl.row0 + c.h * 32) * p.ld0 + 2 * (tl.n * kBlockN + rank * kBlockM)) + lane * 16;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int row = c.q + 4 * i;
-          first[i] = make_int4(0, 0, 0, 0);
-          if (c.h * 32 + row < tl.nrows) first[i] = *reinterpret_cast<const int4*>(src + static_cast<size_t>(row) * p.ld0 * 2);
-        }
+        load_dswiglu(p, tl, c, c.h, &first);
+        stage_dswiglu(p, c, first, first_act);
       }
       const long long w0 = counting ? clock64() : 0;
       const bool reached_acc = mbar_wait(acc_full_bar(as), aph, p.mbar_limit, abort_flag);
@@ -671,7 +738,7 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
         if (lane == 0) mbar_arrive_cluster(leader_acc_empty0 + 8u * as);
       };
       if constexpr (MODE == kModeSwiglu) swiglu_epilogue(p, tl, tacc, c, release);
-      else if constexpr (MODE == kModeDswiglu) dswiglu_epilogue(p, tl, tacc, c, first, release);
+      else if constexpr (MODE == kModeDswiglu) dswiglu_epilogue(p, tl, tacc, c, first, first_act, release);
       else combine_epilogue(p, tl, tacc, c, s_dst, release);
     }
     if (counting && warp == 2 && lane == 0) prof_add(kProfEpiWait, epi_wait);

@@ -727,7 +727,7 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     if (async) cuda_check(cudaEventRecord(ev_up_[q], st), "event record");
   }
   if (async && j >= 2) cuda_check(cudaStreamWaitEvent(st, ev_tgu_[q], 0), "wait dW_up event");  // dh, d_weight shares of slice j-2
-  {  // acc = g Wd^T; dh = SwiGLU'(h) * (w * acc), d_weight shares <acc, act>
+  {  // acc = g Wd^T; dh = SwiGLU'(h) * (w * acc), d_weight shares <acc, w * act>
     GemmParams p = base_params(pl, static_cast<int>(j));
     p.n_tiles = F_ / kBlockN;
     p.k_blocks = D_ / kBlockK;
@@ -735,6 +735,8 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     p.row_w = reinterpret_cast<const float*>(arena_ + arena_lay_.wbuf) + static_cast<size_t>(b) * S_;
     if (keep) wait_for_rows(&p);
     p.in0 = keep ? kept_h(j) : reinterpret_cast<const __nv_bfloat16*>(h_[q].data_ptr());
+    p.in1 = keep ? kept_act(j) : reinterpret_cast<const __nv_bfloat16*>(act_[q].data_ptr());
+    p.ld1 = F_;
     p.out0 = reinterpret_cast<__nv_bfloat16*>(dh_[q].data_ptr());
     p.ld0 = 2 * F_;
     p.dwp = dwp_[q].data_ptr<float>();
@@ -766,6 +768,7 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     r.lay = lay_;
     r.slice = static_cast<int>(j);
     r.dwp = dwp_[q].data_ptr<float>();
+    r.row_w = reinterpret_cast<const float*>(arena_ + arena_lay_.wbuf) + static_cast<size_t>(b) * S_;
     r.parts = dwp_tiles;
     r.peer_dw = table<float>(kTabDw);
     r.peer_count = table<uint32_t>(kTabCount);

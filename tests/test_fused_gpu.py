@@ -355,6 +355,46 @@ def test_one_slice_forward_equals_several_slices(tokens):
     assert outs[0].shape == x.shape and torch.equal(*outs)
 
 
+@pytest.mark.parametrize("tokens,stripe,slice_size", [(700, 64, 4096), (333, 128, 96), (131, 32, 8)])
+def test_router_weight_gradient_is_one_rounding_from_exact(tokens, stripe, slice_size):
+    """`d_weight = <g W_down^T, act>` with act rounded to bf16 once. A rounding is uniform within half a unit in the last place,
+    2^-8 of a value in [1, 2): at most 2^-8 / sqrt(3) of each term's value in the root mean square, and so of a row's sum of
+    1024 unrelated terms (and far above the fp32 sums' own error). A weight that is nothing to divide by (zero, tiny, huge,
+    not finite) leaves its own gradient right all the same, from h's two rounded factors: twice that."""
+    E, K, D, F = 4, 3, 512, 1024
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    x, g = rnd(tokens, D).bfloat16(), rnd(tokens, D).bfloat16()
+    w_up, w_down = (rnd(E, D, 2 * F) / math.sqrt(D)).bfloat16(), (rnd(E, F, D) / math.sqrt(F)).bfloat16()
+    ids = torch.topk(rnd(tokens, E), K, dim=-1).indices.int()
+    weights = rnd(tokens, K).sigmoid() + 0.1
+    special = torch.tensor([0.0, -0.0, 1e-30, -2.0**-33, 2.0**33, -1e30, math.inf, math.nan], device="cuda")
+    weights[-8:, 1] = special
+    weights[:8, 0] = torch.tensor([2.0**-32, -(2.0**-32), 2.0**32, -(2.0**32), 1e-6, -1e-6, -0.5, 3e4], device="cuda")
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=slice_size, transport="nvshmem", expert_compute="fused",
+                           stripe_width=stripe)
+    leaf = weights.clone().requires_grad_(True)
+    chunked_moe(x, ids, leaf, w_up, w_down, cfg).backward(g)
+    f = torch.arange(F, device="cuda")
+    gate = 2 * stripe * (f // stripe) + f % stripe
+    want = torch.zeros(tokens, K, device="cuda", dtype=torch.float64)
+    scale = torch.zeros_like(want)  # root of the sum of the squared terms: what unrelated relative errors of them add up to
+    for e in range(E):
+        t, k = (ids == e).nonzero(as_tuple=True)
+        h = x[t].double() @ w_up[e].double()
+        terms = (g[t].double() @ w_down[e].double().T) * torch.nn.functional.silu(h[:, gate]) * h[:, gate + stripe]
+        want[t, k], scale[t, k] = terms.sum(1), terms.square().sum(1).sqrt()
+    err = (leaf.grad.double() - want) / scale
+    odd = torch.zeros_like(err, dtype=torch.bool)
+    odd[-8:, 1] = True
+    assert torch.isfinite(leaf.grad).all()
+    rms = float(err[~odd].square().mean().sqrt())
+    assert rms <= 2.0**-8 / math.sqrt(3), rms
+    # one of 8 (or 16) rows: five times the root mean square of a sum of many unrelated errors
+    assert float(err[odd].abs().max()) <= 5 * 2 * 2.0**-8 / math.sqrt(3)
+    assert float(err[:8, 0].abs().max()) <= 5 * 2.0**-8 / math.sqrt(3)
+
+
 @pytest.mark.parametrize("training", [False, True], ids=["forward", "training"])
 @pytest.mark.parametrize("slice_size", [4096, 512], ids=["one slice", "several slices"])
 def test_passes_on_several_streams_follow_one_another(slice_size, training):
