@@ -154,6 +154,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("put", &cem::FusedRank::put)
       .def("compute_forward", &cem::FusedRank::compute_forward)
       .def("compute_backward", &cem::FusedRank::compute_backward)
+      .def("keep_rows", &cem::FusedRank::keep_rows)
       .def("forward_pass", &cem::FusedRank::forward_pass)
       .def("backward_pass", &cem::FusedRank::backward_pass)
       .def("finish_forward", &cem::FusedRank::finish_forward)

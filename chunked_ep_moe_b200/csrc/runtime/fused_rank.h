@@ -82,6 +82,9 @@ class FusedRank {
   void compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_up, torch::Tensor w_down);
   void compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_up, torch::Tensor w_down, torch::Tensor dw_up,
                         torch::Tensor dw_down);
+  // Behind begin_*: the pass keeps (forward) or finds (backward) h and w * act of its first `slices` slices in `h` [rows, 2F] and
+  // `act` [rows, F]. Lasts until the pass is finished.
+  void keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices);
   void finish_forward(torch::Tensor inv_order, torch::Tensor out);
   void finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights);
 
@@ -130,7 +133,6 @@ class FusedRank {
       if (std::uncaught_exceptions() > before) rank->quiesce();
     }
   };
-  void keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices);
   void release_kept();
   std::vector<torch::Tensor> allocate_kept(int64_t rows, const torch::TensorOptions& bf16) const;
   __nv_bfloat16* kept_h(int64_t j) const {

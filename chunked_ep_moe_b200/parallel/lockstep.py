@@ -46,8 +46,9 @@ class LockstepWorld:
         self.ranks = []
         self.arenas.close()
 
-    def forward(self, xs, ids, weights, w_ups, w_downs):
-        """Per-rank lists in, per-rank outputs and saved state out."""
+    def forward(self, xs, ids, weights, w_ups, w_downs, keep_slices: int = 0):
+        """Per-rank lists in, per-rank outputs and saved state out. The first `keep_slices` slices' activations are kept for
+        the backward, as a training pass with memory to spare does."""
         P, dev = self.world, xs[0].device
         n_exp = self.cfg.num_experts
         counts = torch.zeros(P, n_exp, dtype=torch.int32, device=dev)
@@ -68,6 +69,13 @@ class LockstepWorld:
         assert len(set(slices)) == 1, f"ranks disagree on the slice count: {slices}"
         n = slices[0]
         w_flats = [w.detach().float().reshape(-1).contiguous() for w in weights]
+        kept = []
+        if min(keep_slices, n) > 0:
+            rows = min(keep_slices, n) * self.cfg.slice_size
+            kept = [(torch.empty(rows, 2 * self.ffn, dtype=torch.bfloat16, device=dev),
+                     torch.empty(rows, self.ffn, dtype=torch.bfloat16, device=dev), min(keep_slices, n)) for _ in range(P)]
+            for rk, k in zip(self.ranks, kept):
+                rk.keep_rows(*k)
         for j in range(n):
             for r in range(P):
                 self.ranks[r].put(j, plans[r], orders[r], xs[r], None, w_flats[r])
@@ -80,12 +88,14 @@ class LockstepWorld:
             outs.append(out)
         for rk in self.ranks:
             rk.check_status()
-        return outs, (plans, orders, invs, w_flats, n)
+        return outs, (plans, orders, invs, w_flats, n, kept)
 
     def backward(self, xs, gs, w_ups, w_downs, saved):
-        plans, orders, invs, w_flats, _ = saved
+        plans, orders, invs, w_flats, _, kept = saved
         P, dev = self.world, xs[0].device
         slices = [self.ranks[r].begin_backward(plans[r]) for r in range(P)]
+        for rk, k in zip(self.ranks, kept):
+            rk.keep_rows(*k)
         n = slices[0]
         dw_ups = [torch.empty_like(w) for w in w_ups]
         dw_downs = [torch.empty_like(w) for w in w_downs]

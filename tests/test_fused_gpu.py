@@ -469,6 +469,71 @@ def test_kept_activations_give_the_same_bits(monkeypatch, tokens, stripe, wire):
     fused.release_workspaces()
 
 
+@pytest.mark.parametrize("wire", [None, "float8_e4m3fn"])
+@pytest.mark.parametrize("slices", [1, 2, 7])
+def test_some_slices_kept_and_some_recomputed_give_the_same_bits(slices, wire):
+    """One rank, two slices in flight: a backward that finds the first 0, 1, ... of its slices' activations and recomputes the
+    others (a pass that needed more slices than the one before, among several ranks)."""
+    from chunked_ep_moe_b200.ops import fused
+
+    E, K, D, F, S = 4, 2, 512, 256, 256
+    T = (slices * S - 37) // K
+    gen = torch.Generator(device="cuda").manual_seed(slices)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    x, g, w = rnd(T, D).bfloat16(), rnd(T, D).bfloat16(), rnd(T * K).sigmoid()
+    w_up, w_down = (rnd(E, D, 2 * F) / math.sqrt(D)).bfloat16(), (rnd(E, F, D) / math.sqrt(F)).bfloat16()
+    ids = torch.topk(rnd(T, E), K, dim=-1).indices.int()
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=S, transport="nvshmem", expert_compute="fused",
+                           stripe_width=64, comm_dtype=wire)
+    rank = fused.get_workspace(cfg, None, D, F, T * K).rank
+    dummy = torch.zeros(1, dtype=torch.int32, device="cuda")
+    plan = torch.empty(rank.plan_ints(), dtype=torch.int32, device="cuda")
+    order, inv = [torch.empty(T * K, dtype=torch.int32, device="cuda") for _ in range(2)]
+    h = torch.empty(T * K, 2 * F, dtype=torch.bfloat16, device="cuda")
+    act, out = torch.empty(T * K, F, dtype=torch.bfloat16, device="cuda"), torch.empty_like(x)
+    assert rank.begin_forward(ids, plan, order, inv, dummy, False) == slices
+    rank.keep_rows(h, act, slices)
+    rank.put(0, plan, order, x, None, w)
+    for j in range(slices):
+        if j + 1 < slices:
+            rank.put(j + 1, plan, order, x, None, w)
+        rank.compute_forward(j, plan, w_up, w_down)
+    rank.finish_forward(inv, out)
+    assert torch.equal(out, chunked_moe(x, ids, w.reshape(T, K), w_up, w_down, cfg))
+    want = rank.backward_pass(x, g, w, w_up, w_down, plan, order, inv, slices, [], 0)
+    for kept in range(1, slices + 1):
+        got = rank.backward_pass(x, g, w, w_up, w_down, plan, order, inv, slices, [h, act], kept)
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), kept
+    rank.check_status()
+
+
+@pytest.mark.parametrize("wire", [None, "float8_e4m3fn"])
+@pytest.mark.parametrize("world_size,skew,slice_size", [(2, "uniform", 64), (4, "all_one", 64), (4, "rank0", 256)])
+def test_lockstep_ranks_that_keep_some_slices_give_the_same_bits(world_size, skew, slice_size, wire):
+    """Several ranks: the SwiGLU' GEMM as the first consumer of a slice's rows (bf16 arrivals, fp8 expansion), and slices that
+    some ranks have no rows in."""
+    from chunked_ep_moe_b200.parallel.lockstep import LockstepWorld
+
+    T, E, K, D, F, stripe = 64, 8, 4, 256, 256, 64
+    x, ids, weights, w_up, w_down, g = moe_cases.setup(world_size, T, E, K, D, F, skew, seed=7)
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=slice_size, transport="nvshmem", expert_compute="fused",
+                           stripe_width=stripe, comm_dtype=wire)
+    bf = lambda t: t.cuda().to(torch.bfloat16).contiguous()
+    sh = lambda t: [moe_cases.shard(t, r, world_size) for r in range(world_size)]
+    xs, gs, ups, downs = [[bf(t) for t in sh(v)] for v in (x, g, w_up, w_down)]
+    idl, wl = [[t.cuda() for t in sh(v)] for v in (ids, weights)]
+    world = LockstepWorld(cfg, world_size, D, F, T)
+    results = []
+    for keep in (0, 1, 3, 1000):
+        outs, saved = world.forward(xs, idl, wl, ups, downs, keep_slices=keep)
+        grads = world.backward(xs, gs, ups, downs, saved)
+        torch.cuda.synchronize()
+        results.append([t.clone() for t in outs] + [t.clone() for group in grads for t in group])
+    world.close()
+    for r in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], r))
+
+
 def test_what_is_saved_under_hooks_does_not_depend_on_memory(monkeypatch):
     """Activation checkpointing compares the tensors saved by the forward with those of its recomputation, when more or less
     memory may be free: a layer large enough to keep activations saves the same ones whether it may keep any or not."""
