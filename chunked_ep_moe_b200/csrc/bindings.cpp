@@ -14,12 +14,9 @@ namespace {
 py::dict plan_layout_dict(int P, int L, int S, int max_slices) {
   const cem::PlanLayout y = cem::make_plan_layout(P, L, S, max_slices);
   py::dict d;
-  // "mtiles" and "ptiles" are one and the same table of GEMM row tiles (at most `tile_m` rows each).
-  for (const std::string kind : {"mtiles", "ptiles"}) {
-    d[("max_" + kind).c_str()] = y.max_tiles;
-    d[("num_" + kind).c_str()] = y.off_num_tiles;
-    d[kind.c_str()] = y.off_tiles;
-  }
+  d["max_tiles"] = y.max_tiles;
+  d["num_tiles"] = y.off_num_tiles;
+  d["tiles"] = y.off_tiles;
   d["max_gtiles"] = y.max_gtiles;
   d["send_start"] = y.off_send_start;
   d["seg_start"] = y.off_seg_start;
@@ -132,7 +129,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("gmm_swiglu", &cem::KernelRunner::gmm_swiglu, py::arg("x"), py::arg("w_up"), py::arg("act"),
            py::arg("h") = py::none())
       .def("gmm", &cem::KernelRunner::gmm)
-      .def("gmm_down_dw", &cem::KernelRunner::gmm_down_dw)
       .def("gmm_dswiglu", &cem::KernelRunner::gmm_dswiglu)
       .def("tgmm", &cem::KernelRunner::tgmm)
       .def("check_status", &cem::KernelRunner::check_status);
@@ -166,6 +162,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("set_pipeline_counters", &cem::FusedRank::set_pipeline_counters, py::arg("counters") = py::none())
       .def("act", &cem::FusedRank::act)
       .def("h", &cem::FusedRank::h)
-      .def("dh", &cem::FusedRank::dh)
-      .def("dy", &cem::FusedRank::dy);
+      .def("dh", &cem::FusedRank::dh);
 }

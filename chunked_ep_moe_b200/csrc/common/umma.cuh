@@ -110,36 +110,16 @@ __device__ __forceinline__ void tcgen05_fence_after_sync() {
 }
 
 // ---------------------------------------------------------------------------------------------
-// TMA: tiled 2-D load, global -> this CTA's shared memory, completion on an mbarrier
+// TMA stores and descriptors
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
-
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
-// ---------------------------------------------------------------------------------------------
-// Bulk stores: this CTA's shared memory -> global memory (local or a peer GPU's), tracked in the issuing thread's
-// bulk async-groups. Plain stores through the async proxy: no tensor map, no cluster delivery of any kind.
-// Both addresses 16-byte aligned, size a multiple of 16 bytes.
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void bulk_store(unsigned long long gdst, uint32_t smem_src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-               ::"l"(gdst), "r"(smem_src), "r"(bytes)
-               : "memory");
-}
-
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 
-// Waits until this thread's committed bulk stores have READ their shared-memory source (it may be overwritten).
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-
-// The same, but the most recently committed group may still be reading (double-buffered staging).
+// Waits until this thread's committed bulk stores have READ their shared-memory source (it may be overwritten), but for the
+// most recently committed group (double-buffered staging).
 __device__ __forceinline__ void bulk_wait_read_but_one() {
   asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
 }
@@ -154,22 +134,6 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t sm
 
 // Waits until this thread's committed bulk stores have completed (their writes are done).
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-// ---------------------------------------------------------------------------------------------
-// TMEM allocation (one warp, all 32 lanes)
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void tmem_alloc(uint32_t smem_result, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result), "r"(cols)
-               : "memory");
-}
-
-__device__ __forceinline__ void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
 
 // ---------------------------------------------------------------------------------------------
 // UMMA descriptors and issue
@@ -197,24 +161,6 @@ __host__ __device__ constexpr uint32_t make_instr_desc_bf16(int m, int n, bool a
          | ((b_mn_major ? 1u : 0u) << 16)          // B major
          | (static_cast<uint32_t>(n >> 3) << 17)   // N / 8
          | (static_cast<uint32_t>(m >> 4) << 24);  // M / 16
-}
-
-// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Arrives on `bar` once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -284,6 +230,7 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
+// TMEM of both CTAs (one warp of each, all 32 lanes).
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_result, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result), "r"(cols)
                : "memory");
@@ -437,11 +384,6 @@ __device__ __forceinline__ bool spin_until_reached(const uint32_t* p, uint32_t t
   }
   *seen = v;
   return true;
-}
-
-// Asks L2 for the line that holds `p` (no register, no wait).
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
 __device__ __forceinline__ int4 ld_nc_v4(const void* p) {

@@ -115,7 +115,6 @@ class FusedRank {
   torch::Tensor act() const { return act_[0]; }
   torch::Tensor h() const { return h_[0]; }
   torch::Tensor dh() const { return dh_[0]; }
-  torch::Tensor dy() const { return torch::empty({0}, act_[0].options()); }  // w * g is never materialised
 
  private:
   // Common start of a pass: counter targets on the device, what the pass will receive back (`pieces_per_row` of T*K rows).

@@ -47,14 +47,13 @@ KernelRunner KernelRunner::with_groups(torch::Tensor group_rows) const {
            group_rows.numel() == L_,
        "group_rows must be a contiguous CUDA int32 tensor of L elements");
   KernelRunner bound = *this;
-  bound.counts_ = group_rows;  // read by the plan kernel on this stream
   bound.plan_ = torch::empty({lay_.total}, group_rows.options());
   PlanKernelParams pp{};
   pp.lay = lay_;
   pp.me = 0;
   pp.plan = bound.plan_.data_ptr<int>();
-  pp.counts = bound.counts_.data_ptr<int>();
-  pp.my_counts = bound.counts_.data_ptr<int>();
+  pp.counts = group_rows.data_ptr<int>();  // (read on this stream)
+  pp.my_counts = group_rows.data_ptr<int>();
   pp.spin_limit = 1;
   pp.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
   launch_plan_build(pp, stream());
@@ -122,28 +121,6 @@ void KernelRunner::gmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out, 
     const CUtensorMap w = make_bf16_map_2d(rhs.data_ptr(), static_cast<uint64_t>(L_) * N, K, 128);
     launch_row_gemm(kModeDx, p, w, rows, num_sms_, stream());
   }
-}
-
-void KernelRunner::gmm_down_dw(torch::Tensor act, torch::Tensor w_down, torch::Tensor g, torch::Tensor row_w,
-                               torch::Tensor dy, torch::Tensor dwp) {
-  need_weights(w_down, L_, "w_down");
-  const int64_t F = w_down.size(1), D = w_down.size(2);
-  need(F % 64 == 0 && D % 256 == 0, "needs F % 64 == 0 and D % 256 == 0");
-  need_bf16(act, S_, F, "act");
-  need_bf16(g, S_, D, "g");
-  need_bf16(dy, S_, D, "dy");
-  need(row_w.is_cuda() && row_w.scalar_type() == torch::kFloat32 && row_w.is_contiguous() && row_w.numel() == S_,
-       "row_w must be a contiguous CUDA fp32 tensor of S elements");
-  need(dwp.is_cuda() && dwp.scalar_type() == torch::kFloat32 && dwp.is_contiguous() && dwp.dim() == 2 &&
-           dwp.size(0) == S_ && dwp.size(1) == D / kBlockN,
-       "dwp must be a contiguous CUDA fp32 [S, D/256] tensor");
-  // The grouped GEMM, then plain tensor ops (the layer itself forms neither y nor w * g, see FusedRank::compute_backward).
-  torch::Tensor y = torch::empty_like(g);
-  gmm(act, w_down, y, false);
-  const torch::Tensor live = (torch::arange(S_, counts_.options()) < counts_.sum()).unsqueeze(1);
-  const torch::Tensor gf = g.to(torch::kFloat32);
-  dy.copy_(torch::where(live, (row_w.unsqueeze(1) * gf).to(torch::kBFloat16), dy));
-  dwp.copy_(torch::where(live, (gf * y.to(torch::kFloat32)).view({S_, D / kBlockN, kBlockN}).sum(2), dwp));
 }
 
 void KernelRunner::gmm_dswiglu(torch::Tensor dy, torch::Tensor w_down, torch::Tensor h, torch::Tensor dh) {

@@ -32,9 +32,6 @@ class KernelRunner {
   void gmm_swiglu(torch::Tensor x, torch::Tensor w_up, torch::Tensor act, c10::optional<torch::Tensor> h);
   // out[S,N] = lhs[S,K] rhs[g]; rhs is [L,K,N], or [L,N,K] with transpose_rhs (no transpose is materialised)
   void gmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out, bool transpose_rhs);
-  // dy[S,D] = w * g and dwp[S, D/256] = partial sums of <g, act W_down> per 256 columns
-  void gmm_down_dw(torch::Tensor act, torch::Tensor w_down, torch::Tensor g, torch::Tensor row_w, torch::Tensor dy,
-                   torch::Tensor dwp);
   // dh[S,2F] = SwiGLU'(h) * (dy W_down^T), w_down [L,F,D]
   void gmm_dswiglu(torch::Tensor dy, torch::Tensor w_down, torch::Tensor h, torch::Tensor dh);
   // out[g][M,N] = lhs[rows_g]^T rhs[rows_g] (bf16), lhs [S,M], rhs [S,N]
@@ -46,7 +43,7 @@ class KernelRunner {
   GemmParams base() const;
   int L_, S_, stripe_, num_sms_;
   PlanLayout lay_;
-  torch::Tensor plan_, counts_, status_;
+  torch::Tensor plan_, status_;
 };
 
 }  // namespace cem

@@ -21,7 +21,7 @@ from .symm import LocalArenas
 
 class LockstepWorld:
     def __init__(self, cfg: ChunkedMoEConfig, world: int, hidden: int, ffn: int, tokens_per_rank: int,
-                 spin_limit: int = 1 << 16, cta_pairs: bool = True):
+                 spin_limit: int = 1 << 16):
         if cfg.num_experts % world:
             raise ValueError(f"num_experts={cfg.num_experts} is not divisible by world={world}")
         ext = _build.load()

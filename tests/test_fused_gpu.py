@@ -75,20 +75,9 @@ def test_single_rank_layer_matches_oracle(group_rows, slice_size, stripe):
     _check_single_rank_case(group_rows, slice_size, stripe)
 
 
-@pytest.mark.parametrize("switch", ["CEM_RET_BLOCKED", "CEM_RET_LSU"])
-def test_alternative_return_paths_match_oracle(monkeypatch, switch):
-    """The two measurement variants of the combine epilogues must not change the layer's results. `CEM_RET_BLOCKED=1`:
-    runs of rows stored into return buffers kept column tile by column tile, which `combine_reduce` then reads.
-    `CEM_RET_LSU=1`: staged rows written out with coalesced vector stores instead of bulk stores."""
-    from chunked_ep_moe_b200.ops import fused
-
-    fused.release_workspaces()  # the switches are read when a workspace's executor is created
-    monkeypatch.setenv(switch, "1")
-    try:
-        for group_rows, slice_size, stripe in CASES[:3]:
-            _check_single_rank_case(group_rows, slice_size, stripe, hidden=768)  # three column tiles
-    finally:
-        fused.release_workspaces()
+@pytest.mark.parametrize("group_rows,slice_size,stripe", CASES[:3])
+def test_three_column_tiles_match_oracle(group_rows, slice_size, stripe):
+    _check_single_rank_case(group_rows, slice_size, stripe, hidden=768)
 
 
 def _check_single_rank_case(group_rows, slice_size, stripe, hidden=256):
@@ -714,8 +703,7 @@ def test_fused_expert_compute_on_a_collective_transport():
     _close(ds.grad.cpu(), want["dw_down"], "dw_down")
 
 
-@pytest.mark.parametrize("cta_pairs", [True, False], ids=["pairs", "single"])
-def test_nan_poisoned_padding_does_not_leak(cta_pairs):
+def test_nan_poisoned_padding_does_not_leak():
     """Scratch and slice buffers full of NaN patterns: rows outside a group must never reach an output."""
     from chunked_ep_moe_b200 import _build
     from chunked_ep_moe_b200.parallel.lockstep import LockstepWorld
@@ -728,12 +716,12 @@ def test_nan_poisoned_padding_does_not_leak(cta_pairs):
     T = ids.shape[0]
     cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=S, transport="nvshmem", expert_compute="fused",
                            stripe_width=stripe)
-    world = LockstepWorld(cfg, 1, D, F, T, cta_pairs=cta_pairs)
+    world = LockstepWorld(cfg, 1, D, F, T)
     lay = ext.arena_layout(1, E, S, D, T * K, False)
     ext.arena_fill(world.arenas.bases[0] + lay["xbuf"], lay["xq"] - lay["xbuf"], 0xFF)  # x, g, w slice buffers
     ext.arena_fill(world.arenas.bases[0] + lay["ret"], lay["arrive"] - lay["ret"], 0xFF)
     rk = world.ranks[0]
-    for t in (rk.act(), rk.h(), rk.dh(), rk.dy()):
+    for t in (rk.act(), rk.h(), rk.dh()):
         t.fill_(float("nan"))
     bf = lambda t: t.cuda().to(torch.bfloat16)
     x, g = bf(torch.randn(T, D, generator=gen)), bf(torch.randn(T, D, generator=gen))
@@ -752,10 +740,9 @@ def test_nan_poisoned_padding_does_not_leak(cta_pairs):
     world.close()
 
 
-@pytest.mark.parametrize("cta_pairs", [True, False], ids=["pairs", "single"])
 @pytest.mark.parametrize("world_size,skew,slice_size", [(2, "uniform", 128), (4, "uniform", 64), (4, "all_one", 64),
                                                         (4, "rank0", 256), (8, "uniform", 2048)])
-def test_lockstep_multi_rank_matches_oracle(world_size, skew, slice_size, cta_pairs):
+def test_lockstep_multi_rank_matches_oracle(world_size, skew, slice_size):
     from chunked_ep_moe_b200.parallel.lockstep import LockstepWorld
 
     T, E, K, D, F, stripe = 48, 16, 4, 256, 256, 64
@@ -770,7 +757,7 @@ def test_lockstep_multi_rank_matches_oracle(world_size, skew, slice_size, cta_pa
     wl = [sh(weights, r).cuda() for r in range(world_size)]
     ups = [bf(sh(w_up, r)) for r in range(world_size)]
     downs = [bf(sh(w_down, r)) for r in range(world_size)]
-    world = LockstepWorld(cfg, world_size, D, F, T, cta_pairs=cta_pairs)
+    world = LockstepWorld(cfg, world_size, D, F, T)
     outs, saved = world.forward(xs, idl, wl, ups, downs)
     dxs, dws, dw_ups, dw_downs = world.backward(xs, gs, ups, downs, saved)
     torch.cuda.synchronize()
@@ -848,7 +835,7 @@ def test_buffers_and_wire_rows_do_not_depend_on_the_routing(skew):
     x, ids, weights, w_up, w_down, _ = moe_cases.setup(P, T, E, K, D, F, skew, seed=2)
     bf = lambda t: t.cuda().to(torch.bfloat16)
     sh = lambda t, r: moe_cases.shard(t, r, P)
-    world = LockstepWorld(cfg, P, D, F, T, cta_pairs=False)
+    world = LockstepWorld(cfg, P, D, F, T)
     # geometry alone fixes what a rank holds; the routing is not an argument of either size
     assert world.arenas.nbytes == ext.arena_bytes(P, E // P, S, D, T * K, False)
     torch.cuda.synchronize()

@@ -28,10 +28,10 @@ def _free_port():
         return s.getsockname()[1]
 
 
-def _worker(rank, world, port, out_dir, cases, pairs):
+def _worker(rank, world, port, out_dir, cases):
     import torch.distributed as dist
 
-    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port), NCCL_NVLS_ENABLE="0", CEM_CTA_PAIRS=pairs)
+    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port), NCCL_NVLS_ENABLE="0")
     torch.cuda.set_device(rank)
     dist.init_process_group("nccl", rank=rank, world_size=world, device_id=torch.device("cuda", rank))
     result = {"ok": True, "errors": {}}
@@ -77,30 +77,29 @@ def _worker(rank, world, port, out_dir, cases, pairs):
     dist.destroy_process_group()
 
 
-def _run(world, cases, pairs="0", worker=None):
+def _run(world, cases, worker=None):
     import torch.multiprocessing as mp
 
     with tempfile.TemporaryDirectory() as out_dir:
-        mp.spawn(worker or _worker, args=(world, _free_port(), out_dir, cases, pairs), nprocs=world, join=True)
+        mp.spawn(worker or _worker, args=(world, _free_port(), out_dir, cases), nprocs=world, join=True)
         return [torch.load(os.path.join(out_dir, f"{r}.pt"), weights_only=False) for r in range(world)]
 
 
 CASES = [("uniform", 128, None), ("all_one", 64, None), ("rank0", 256, None), ("uniform", 128, "float8_e4m3fn")]
 
 
-@pytest.mark.parametrize("pairs", ["0", "1"], ids=["single", "pairs"])
 @pytest.mark.parametrize("world", [2, 4, 8])
-def test_fused_layer_on_real_peers(world, pairs):
+def test_fused_layer_on_real_peers(world):
     if torch.cuda.device_count() < world:
         pytest.skip(f"needs {world} GPUs")
-    for rank, res in enumerate(_run(world, CASES, pairs)):
+    for rank, res in enumerate(_run(world, CASES)):
         assert res["ok"], f"rank {rank} failed:\n{res.get('trace')}"
         for key, (err, finite) in res["errors"].items():
             limit = 0.08 if key[0][2] is not None else TOL
             assert finite and err <= limit, f"rank {rank} {key}: err {err:.4f}"
 
 
-def _leaver_worker(rank, world, port, out_dir, cases, pairs):
+def _leaver_worker(rank, world, port, out_dir, cases):
     """Both ranks run step 0 of the fused layer to the end. Rank 1 then leaves (nothing of its own in flight, its
     device idle); rank 0 asks the heartbeat before launching step 1 and must be told who is missing."""
     import torch.distributed as dist

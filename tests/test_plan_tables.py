@@ -74,25 +74,16 @@ def _check_tables(P, L, S, tokens, top_k, skew, seed):
                 assert tab[lay["num_chunks"] + j] == chunks.sum()
             else:
                 assert tab[lay["num_chunks"] + j] == 0
-            # row tiles: cover each expert's rows of the slice exactly, in expert order, 128 rows at most
-            num_m = tab[lay["num_mtiles"] + j]
-            mt = tab[lay["mtiles"] + 4 * lay["max_mtiles"] * j:][: 4 * num_m].reshape(num_m, 4)
+            # row tiles: cover each expert's rows of the slice exactly, in expert order, at most `tile_m` rows each
+            num_t = tab[lay["num_tiles"] + j]
+            tt = tab[lay["tiles"] + 4 * lay["max_tiles"] * j:][: 4 * num_t].reshape(num_t, 4)
             starts = np.cumsum(groups) - groups
             covered = np.zeros(L, dtype=np.int64)
-            for e, row0, nrows, _ in mt:
-                assert 0 < nrows <= lay["tile_m"]
+            for e, row0, nrows, ncols in tt:
+                assert 0 < nrows <= lay["tile_m"] and ncols == -(-nrows // 32) * 32
                 assert row0 == starts[e] + covered[e]
                 covered[e] += nrows
             np.testing.assert_array_equal(covered, groups if j < ref.num_slices else 0 * groups)
-            # row-tile pairs (2-CTA GEMMs): same coverage in 256-row steps
-            num_p = tab[lay["num_ptiles"] + j]
-            pt = tab[lay["ptiles"] + 4 * lay["max_ptiles"] * j:][: 4 * num_p].reshape(num_p, 4)
-            covered_p = np.zeros(L, dtype=np.int64)
-            for e, row0, nrows, _ in pt:
-                assert 0 < nrows <= 2 * lay["tile_m"]
-                assert row0 == starts[e] + covered_p[e]
-                covered_p[e] += nrows
-            np.testing.assert_array_equal(covered_p, covered)
             # weight-gradient groups: one per expert present; first/final flags; empty experts once in slice 0
             num_g = tab[lay["num_gtiles"] + j]
             gt = tab[lay["gtiles"] + 4 * lay["max_gtiles"] * j:][: 4 * num_g].reshape(num_g, 4)
@@ -114,7 +105,7 @@ def _check_nothing_routed(tab, lay, P, L, max_slices):
     """Slice 0 finalises every expert's (empty) gradient, nothing else is in the tables."""
     assert tab[0] == 0 and tab[1] == 0
     for j in range(max_slices):
-        assert tab[lay["num_mtiles"] + j] == 0 and tab[lay["num_chunks"] + j] == 0
+        assert tab[lay["num_tiles"] + j] == 0 and tab[lay["num_chunks"] + j] == 0
         assert tab[lay["num_gtiles"] + j] == (L if j == 0 else 0)
     groups = tab[lay["gtiles"]: lay["gtiles"] + 4 * L].reshape(L, 4)
     np.testing.assert_array_equal(groups, [[l, 0, 0, 3] for l in range(L)])
@@ -172,13 +163,12 @@ def test_plan_kernel_matches_host_tables(P, L, S, tokens, top_k, skew):
     for me in sorted({0, P - 1}):
         host = ext.plan_build_host(counts, S, max_slices, me).numpy()
         dev = ext.plan_build_device(counts.cuda(), S, max_slices, me).cpu().numpy()
-        header_and_sums = lay["num_mtiles"]  # header + the per-segment and per-expert sums
+        header_and_sums = lay["num_tiles"]  # header + the per-segment and per-expert sums
         np.testing.assert_array_equal(dev[:header_and_sums], host[:header_and_sums])
-        for key in ("num_mtiles", "num_gtiles", "num_chunks", "num_ptiles"):
+        for key in ("num_tiles", "num_gtiles", "num_chunks"):
             np.testing.assert_array_equal(dev[lay[key]: lay[key] + max_slices], host[lay[key]: lay[key] + max_slices])
         for j in range(max_slices):
-            for key, cap, num in (("mtiles", lay["max_mtiles"], "num_mtiles"), ("gtiles", lay["max_gtiles"], "num_gtiles"),
-                                  ("ptiles", lay["max_ptiles"], "num_ptiles")):
+            for key, cap, num in (("tiles", lay["max_tiles"], "num_tiles"), ("gtiles", lay["max_gtiles"], "num_gtiles")):
                 used = 4 * host[lay[num] + j]
                 at = lay[key] + 4 * cap * j
                 np.testing.assert_array_equal(dev[at: at + used], host[at: at + used])
