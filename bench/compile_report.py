@@ -86,7 +86,7 @@ def ptxas_report() -> list:
 def work_report(world, experts, top_k, tokens, hidden, ffn, slice_size, fp8) -> dict:
     rows = tokens * top_k                      # token copies a rank sends = copies it receives under uniform routing
     slices = math.ceil(rows / slice_size)
-    flops = 18 * rows * hidden * ffn + 6 * rows * hidden * ffn  # fwd 6, remat 6, dgrad 6, wgrad 6 (x D x F per row)
+    flops = 18 * rows * hidden * ffn           # fwd 6, dgrad 6, wgrad 6 (x D x F per row; recomputation is not counted)
     wire_elem = 1 + 4 / 128 if fp8 else 2      # e4m3 + one fp32 scale per 128, or bf16
     remote = rows * (world - 1) / world
     dispatch = remote * hidden * wire_elem * 3  # x (fwd), x and g (bwd)
@@ -94,7 +94,7 @@ def work_report(world, experts, top_k, tokens, hidden, ffn, slice_size, fp8) -> 
     return {
         "rows per rank per pass": rows,
         "slices per pass (uniform routing)": slices,
-        "kernel launches per step": fused.expected_launches(slices, fp8),
+        "kernel launches per step": fused.expected_launches(slices, fp8 and world > 1),
         "GEMM TFLOP per rank per step": flops / 1e12,
         "NVLink GB out per rank per step": (dispatch + combine) / 1e9,
     }

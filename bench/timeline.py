@@ -107,7 +107,7 @@ def main():
     print("\nkernel                          launches   total ms    mean ms")
     for key, (n, total) in summary.items():
         print(f"{key:32s} {n:6d} {total:10.3f} {total / n:10.3f}")
-    flops = 24.0 * D * F * T * K
+    flops = 18.0 * D * F * T * K  # what the step cannot do without
     span /= args.steps
     print(f"\nstep span {span:.3f} ms   {T / (span / 1e3):.0f} tokens/s   {flops / (span / 1e3) / 1e12:.0f} TFLOP/s"
           + (f"   (mean of {args.steps} steps back to back)" if args.steps > 1 else ""))

@@ -24,8 +24,9 @@ def wire_bytes(rows_remote: int, hidden: int, comm_dtype: Optional[str], backwar
 
 
 def layer_flops(rows: int, hidden: int, ffn: int, backward: bool) -> float:
-    """FLOPs of the expert MLP on `rows` token copies: forward 6*D*F per row, backward (with remat) 18*D*F."""
-    return float(rows) * hidden * ffn * (18.0 if backward else 6.0)
+    """FLOPs the expert MLP cannot do without on `rows` token copies: forward 6*D*F per row, backward 12*D*F (what a backward
+    recomputes, at most 4*D*F, is not counted)."""
+    return float(rows) * hidden * ffn * (12.0 if backward else 6.0)
 
 
 def load_measured_peaks(path: Optional[str] = None) -> dict:

@@ -93,7 +93,7 @@ ptxas info    : Used 32 registers"""
     assert plan["total"] == sum(v for k, v in plan.items() if k != "total")
     assert plan["total"] < 16 * 2**30, "the DeepSeek-V3-size layer on 8 ranks fits in a fraction of 180 GB"
     work = compile_report.work_report(8, 256, 8, 8192, 7168, 2048, 8192, False)
-    assert abs(work["GEMM TFLOP per rank per step"] - 23.09) < 0.01
+    assert abs(work["GEMM TFLOP per rank per step"] - 17.32) < 0.01
     assert work["kernel launches per step"] == 104
 
 

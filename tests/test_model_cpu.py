@@ -92,7 +92,7 @@ def test_stats_helpers():
     assert wb["dispatch_bytes"] == 1000 * (7168 * 2 + 4) and wb["combine_bytes"] == 1000 * 7168 * 2
     wq = stats.wire_bytes(1000, 7168, "float8_e4m3fn", backward=True)
     assert wq["dispatch_bytes"] == 1000 * (2 * (7168 + 56 * 4) + 4)
-    assert stats.layer_flops(10, 4, 2, False) == 10 * 4 * 2 * 6
+    assert stats.layer_flops(10, 4, 2, False) == 10 * 4 * 2 * 6 and stats.layer_flops(10, 4, 2, True) == 10 * 4 * 2 * 12
     rl = stats.roofline_ms(23.09e12, 4.11e9, {"bf16_tflops_sustained": 1368.3, "bf16_tflops": 1629.7})
     assert abs(rl["compute_ms"] - 16.87) < 0.05 and rl["roofline_ms"] == rl["compute_ms"]
     hs = stats.header_stats([3, 20, 24, 5, 0, 16] + [0] * 10, 8)
