@@ -316,7 +316,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmParams p, const __grid_cons
     }
   } else if (warp == 1) {
     // ================================ MMA issuer (leader) / stage relay (peer) ==============
-    // As in the single-CTA kernel, the whole warp walks the k-blocks in step and one elected lane issues.
+    // The whole warp walks the k-blocks in step and one elected lane issues.
     constexpr uint32_t idesc = make_instr_desc_bf16(2 * kBlockM, kBlockN, true, true);
     constexpr uint32_t kDescStep = 2048u;  // bytes per 16-row k step inside a stage
     const uint32_t peer = static_cast<uint32_t>(rank ^ 1);

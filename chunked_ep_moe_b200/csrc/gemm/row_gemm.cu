@@ -14,7 +14,7 @@
 //                warp per SM sub-partition for a tile: with 16 k-blocks per tile one group could not keep up).
 //
 // Measured against the token-major kernels this one replaced (128 x 256 tiles on single CTAs below 768 rows per expert, 256 x
-// 256 on pairs above), same box: 490-510 cycles per k-block at D=7168, F=2048 in every mode (the tensor pipe's floor for the
+// 256 on pairs above), same box: 496-540 cycles per k-block at D=7168, F=2048 by mode (the tensor pipe's floor for the
 // mean width; 515-540 for the pairs, 610-700 for single CTAs), layer forward + backward with 256 rows per expert 7.86 -> 7.33
 // ms, Zipf routing in slices of 2048 rows 10.7 -> 9.1 ms, decode of 64 tokens (16 rows per expert) 776 -> 563 us, 2048 rows
 // per expert 21.4 -> 20.4 ms (there the 1000 W power cap sets the clock, so fewer padded rows are what counts).

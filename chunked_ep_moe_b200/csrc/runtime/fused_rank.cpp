@@ -27,13 +27,6 @@ constexpr int kExpandSms = 12;  // SMs the up-projection GEMM leaves to the fp8 
 // a second status block for `check_status`.
 constexpr int kHostSeq = kPlanHeaderInts + 8, kHostStatus = 32, kHostInts = 40;
 
-// Rows of a slice x D x F from which a training forward keeps h and w * act. Measured, forward + backward, keeping against
-// recomputing: 16384-row slices at D=1024, F=512 (2^33) 1026 against 1072 us, 7996 rows at D=2048, F=1024 (2^34) 503 against
-// 530 us; 1024-row slices at D=2048, F=1024 (2^31) 1133 against 1126 us (the GEMM it saves runs in the shadow of the next
-// put there), 1024 rows at D=F=512 204 us both ways (a kernel takes 8 us however little it does, and two allocations and a
-// slice's tensor maps cost the host what its launch does).
-constexpr int64_t kKeepWork = int64_t{1} << 32;
-
 struct NvtxRange {
   explicit NvtxRange(const char* name) { nvtxRangePushA(name); }
   NvtxRange(const char* name, int64_t j) {
@@ -826,8 +819,8 @@ void FusedRank::end_pass(int64_t n_slices) {
 // What a training forward keeps for its backward: h and w * act of its first `kept_slices_` slices (12 KB a row at F = 2048),
 // so that the backward starts from them instead of running the up-projection GEMM again (4 of its 16 D x F products per
 // row). Results do not change by it: the backward recomputes the same bits when it has to. Forward + backward, D=7168,
-// F=2048: 64 experts of 256 rows 7.10 -> 6.09 ms, Zipf routing in slices of 2048 rows 9.05 -> 7.80 ms, 32 experts of 1024
-// rows on the fp8 wire 12.0 -> 10.8 ms.
+// F=2048: 64 experts of 256 rows 7.10 -> 6.09 ms, Zipf routing in slices of 2048 rows 9.05 -> 7.67 ms, 32 experts of 1024
+// rows on the fp8 wire 12.0 -> 10.9 ms.
 void FusedRank::keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices) {
   expect(h.is_cuda() && h.is_contiguous() && h.scalar_type() == torch::kBFloat16 && h.dim() == 2 && h.size(1) == 2 * F_ &&
              act.is_cuda() && act.is_contiguous() && act.scalar_type() == torch::kBFloat16 && act.dim() == 2 &&

@@ -39,6 +39,13 @@ ArenaLayout make_arena_layout(int P, int L, int S, int D, int tk_cap, bool fp8);
 // Text of a recorded status block {code, kernel, mode, slice, detail, expected, seen, block} (what check_status raises).
 std::string format_status(const std::vector<int64_t>& status, int rank);
 
+// Rows of a slice x D x F from which a training forward keeps h and w * act. Measured, forward + backward, keeping against
+// recomputing: 16384-row slices at D=1024, F=512 (2^33) 1026 against 1072 us, 7996 rows at D=2048, F=1024 (2^34) 503 against
+// 530 us; 1024-row slices at D=2048, F=1024 (2^31) 1133 against 1126 us (the GEMM it saves runs in the shadow of the next
+// put there), 1024 rows at D=F=512 204 us both ways (a kernel takes 8 us however little it does, and two allocations and a
+// slice's tensor maps cost the host what its launch does).
+constexpr int64_t kKeepWork = int64_t{1} << 32;
+
 // Slices of a training forward that a rank among several keeps h and w * act of: those that its own stream reached in the pass
 // before (`stream_rows`), at most the `guess` it launches. Every rank loops as often as the fullest one, but a rank only has
 // memory reserved for about the rows that come to it; slices past them hold none, and one that does after all is recomputed.
@@ -59,14 +66,14 @@ class FusedRank {
   // Returns the number of slices (this synchronises the host with the plan kernel once).
   int64_t begin_forward(torch::Tensor expert_ids, torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order,
                         torch::Tensor counts, bool counts_prefilled);
-  // The same set-up without waiting for the device: the plan header and the status block are copied to pinned host
-  // memory behind the plan kernel and an event is recorded. Returns the slice count of this workspace's previous
+  // The same set-up without waiting for the device: the plan kernel stores the plan header and the status block to pinned
+  // host memory, their sequence number last. Returns the slice count of this workspace's previous
   // forward pass (-1 if there was none) as a GUESS; the caller may launch that many slices at once, then calls
   // `resolve_slices()` for the real count, launches what is still missing and reports what it launched with
   // `set_pass_slices()`. Slices past the real count find empty tables and do nothing, on every rank alike.
   int64_t begin_forward_async(torch::Tensor expert_ids, torch::Tensor plan, torch::Tensor order,
                               torch::Tensor inv_order, torch::Tensor counts, bool counts_prefilled);
-  // Waits for the header copy (not for the stream), raises a recorded kernel error, returns the real slice count.
+  // Polls for that sequence number (does not wait for the stream), raises a recorded kernel error, returns the real slice count.
   int64_t resolve_slices();
   void set_pass_slices(int64_t launched);
   // Microseconds a pipeline barrier inside a GEMM may take before the kernel gives up (default 20 s).

@@ -200,7 +200,8 @@ def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidd
         "expert weights (bf16)": weights,
         "expert weight gradients (bf16)": weights,
         "saved for backward (x, router weights, sort order, plan)": saved,
-        "kept for backward while memory allows (h, w * act; rows balanced over the ranks)": tk * 3 * F * 2,
+        "kept for backward while memory allows (h, w * act; rows balanced over the ranks)":
+            tk * 3 * F * 2 if min(tk, S) * D * F >= ext.keep_work else 0,
     }
     out["total"] = sum(out.values())
     return out

@@ -91,6 +91,9 @@ ptxas info    : Used 32 registers"""
                              slice_size=8192)
     assert plan["expert weights (bf16)"] == 32 * (7168 * 4096 + 2048 * 7168) * 2
     assert plan["total"] == sum(v for k, v in plan.items() if k != "total")
+    small = fused.memory_plan(world=1, experts=8, top_k=2, tokens_per_rank=192, hidden=256, ffn=256, slice_size=128)
+    kept = next(k for k in plan if k.startswith("kept"))
+    assert plan[kept] == 65536 * 3 * 2048 * 2 and small[kept] == 0  # a small slice's activations are never kept
     assert plan["total"] < 16 * 2**30, "the DeepSeek-V3-size layer on 8 ranks fits in a fraction of 180 GB"
     work = compile_report.work_report(8, 256, 8, 8192, 7168, 2048, 8192, False)
     assert abs(work["GEMM TFLOP per rank per step"] - 17.32) < 0.01
