@@ -30,6 +30,7 @@ _SOURCES = [
     "plan/expert_sort_noalloc.cu",
     "model/model_kernels.cu",
     "model/router_kernels.cu",
+    "model/embedding_kernels.cu",
     "model/model_ops.cpp",
 ]
 _lock = threading.Lock()

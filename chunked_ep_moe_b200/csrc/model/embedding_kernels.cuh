@@ -1,0 +1,17 @@
+// Gradient of an embedding table from the gradients of the rows that were looked up.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace cem {
+
+// A key is id * 2^14 + position.
+constexpr int kEmbedPosBits = 14, kEmbedMaxTokens = 1 << kEmbedPosBits, kEmbedMaxVocab = 1 << (32 - kEmbedPosBits);
+
+// dw[v] = sum of grad[i] over the positions i with ids[i] == v, in a fixed order, fp32 sums, rounded once; rows that no id names
+// become zero. `keys`: n words of scratch. n <= kEmbedMaxTokens, vocab <= kEmbedMaxVocab, cols % 8 == 0; bf16 grad and dw.
+void launch_embedding_bwd(const int64_t* ids, const void* grad, void* dw, uint32_t* keys, int n, int vocab, int cols,
+                          cudaStream_t stream);
+
+}  // namespace cem

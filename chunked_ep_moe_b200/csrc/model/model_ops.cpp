@@ -7,6 +7,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "embedding_kernels.cuh"
 #include "model_kernels.cuh"
 #include "router_kernels.cuh"
 
@@ -142,6 +143,20 @@ torch::Tensor dense_swiglu_bwd(torch::Tensor gu, torch::Tensor d_act) {
   launch_dense_swiglu(gu.data_ptr(), d_act.data_ptr(), d_gu.data_ptr(), static_cast<int>(gu.size(0)),
                       static_cast<int>(gu.size(1) / 2), true, stream());
   return d_gu;
+}
+
+torch::Tensor embedding_bwd(torch::Tensor ids, torch::Tensor grad, int64_t vocab) {
+  need(bf16_matrix(grad) && grad.size(1) % 8 == 0, "grad must be a contiguous CUDA bf16 [ids, cols % 8 == 0] matrix");
+  need(ids.is_cuda() && ids.scalar_type() == torch::kInt64 && ids.is_contiguous() && ids.numel() == grad.size(0),
+       "ids must be a contiguous CUDA int64 vector, one per row of grad");
+  need(ids.numel() <= kEmbedMaxTokens && vocab >= 1 && vocab <= kEmbedMaxVocab, "at most 16384 ids and 2^18 table rows");
+  const c10::cuda::CUDAGuard guard(grad.device());
+  if (reinterpret_cast<uintptr_t>(grad.data_ptr()) % 16 != 0) grad = grad.clone();  // (read 16 bytes at a time)
+  torch::Tensor dw = torch::empty({vocab, grad.size(1)}, grad.options());
+  torch::Tensor keys = torch::empty({ids.numel()}, grad.options().dtype(torch::kInt32));
+  launch_embedding_bwd(ids.data_ptr<int64_t>(), grad.data_ptr(), dw.data_ptr(), reinterpret_cast<uint32_t*>(keys.data_ptr()),
+                       static_cast<int>(ids.numel()), static_cast<int>(vocab), static_cast<int>(grad.size(1)), stream());
+  return dw;
 }
 
 std::vector<torch::Tensor> router_fwd(torch::Tensor logits, torch::Tensor bias, int64_t top_k, double scaling) {

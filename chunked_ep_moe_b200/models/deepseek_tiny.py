@@ -27,7 +27,7 @@ import torch.nn.functional as F
 
 from ..api import chunked_moe
 from ..config import ChunkedMoEConfig
-from .fused_ops import add_rms_norm, cross_entropy, dense_swiglu, rope_qkv, router_select
+from .fused_ops import add_rms_norm, cross_entropy, dense_swiglu, embedding, rope_qkv, router_select
 
 
 @dataclasses.dataclass
@@ -60,6 +60,11 @@ class DeepSeekTinyConfig:
         return ChunkedMoEConfig(num_experts=self.num_experts, top_k=self.top_k, slice_size=self.slice_size,
                                 transport=self.transport, expert_compute=self.expert_compute,
                                 comm_dtype=self.comm_dtype, stripe_width=self.stripe_width)
+
+
+class Embedding(nn.Embedding):
+    def forward(self, tokens):
+        return embedding(tokens, self.weight)
 
 
 class RMSNorm(nn.Module):
@@ -195,7 +200,7 @@ class DeepSeekTiny(nn.Module):
     def __init__(self, cfg: DeepSeekTinyConfig, group=None):
         super().__init__()
         self.cfg = cfg
-        self.embed = nn.Embedding(cfg.vocab_size, cfg.d_model)
+        self.embed = Embedding(cfg.vocab_size, cfg.d_model)
         self.blocks = nn.ModuleList([Block(cfg, i < cfg.first_dense, group) for i in range(cfg.n_layers)])
         self.norm = RMSNorm(cfg.d_model, cfg.norm_eps)
         self.lm_head = nn.Linear(cfg.d_model, cfg.vocab_size, bias=False)

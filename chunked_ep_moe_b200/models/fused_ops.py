@@ -1,5 +1,5 @@
 """Fused CUDA ops of the decoder around the MoE layers: residual add + RMSNorm, rotary embedding straight out of the
-qkv projection, the cross-entropy of bf16 logits, the sigmoid top-k router (everything after its logits GEMM) and the dense SwiGLU. Each is one kernel per direction (`csrc/model/`) instead of a
+qkv projection, the embedding table's gradient, the cross-entropy of bf16 logits, the sigmoid top-k router (everything after its logits GEMM) and the dense SwiGLU. Each is one kernel per direction (`csrc/model/`) instead of a
 chain of framework elementwise kernels, which took a third of a trainer step's device time. On CPU tensors (and for
 dtypes other than bf16) the same functions fall back to plain torch ops with identical semantics, so the model code
 has one path. The reference ships no model code; these serve `models/deepseek_tiny.py`.
@@ -84,6 +84,28 @@ def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> tuple[t
         return torch.view_as_real(xc * torch.complex(cos, sin)).flatten(-2).to(x.dtype)
 
     return rot(q), rot(k), v
+
+
+class _Embedding(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, tokens, weight):
+        ctx.save_for_backward(tokens)
+        ctx.vocab = weight.shape[0]
+        return F.embedding(tokens, weight)
+
+    @staticmethod
+    def backward(ctx, grad):
+        (tokens,) = ctx.saved_tensors
+        flat = grad.reshape(-1, grad.shape[-1]).contiguous()
+        return None, _ext().embedding_bwd(tokens.reshape(-1).contiguous().long(), flat, ctx.vocab)
+
+
+def embedding(tokens: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """`weight[tokens]`; the table's gradient by sorted ids, in fp32 and in a fixed order (up to 16384 tokens and 2^18 rows)."""
+    if (_fusable(weight) and tokens.is_cuda and 0 < tokens.numel() <= 1 << 14 and weight.shape[0] <= 1 << 18
+            and weight.shape[1] % 8 == 0):
+        return _Embedding.apply(tokens, weight)
+    return F.embedding(tokens, weight)
 
 
 class _CrossEntropy(torch.autograd.Function):

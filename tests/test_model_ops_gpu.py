@@ -157,3 +157,26 @@ def test_add_rms_norm_row_widths(rows, cols):
     for name, got, want in (("y", y, yr.detach()), ("dx", leaves[0].grad, sr.grad), ("dw", leaves[2].grad, wr.grad)):
         assert (got.double() - want).abs().le(want.abs() * 2.0**-8 + 1e-5 * want.abs().max()).all(), name
     assert torch.equal(leaves[0].grad, leaves[1].grad)
+
+
+@pytest.mark.parametrize("tokens,vocab,cols", [(1, 1, 8), (31, 7, 8), (33, 256, 264), (1025, 257, 256), (16384, 40, 264),
+                                               (16384, 1, 8), (500, 1 << 18, 8), (8191, 32000, 1032)])
+def test_embedding_gradient(tokens, vocab, cols):
+    """Rows with no, few and many pairs, one to three digits of the ids, ragged columns. fp32 sums of n terms (n 2^-24 of the sum
+    of their magnitudes) and one rounding to bf16 (2^-9 of the value; twice both allowed). The same bits every time."""
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    ids = torch.randint(0, vocab, (1, tokens), generator=gen, device="cuda")
+    ids[0, tokens // 2:] = ids[0, tokens // 2:] // 3  # unevenly
+    g = torch.randn(1, tokens, cols, generator=gen, device="cuda").bfloat16()
+    grads = []
+    for _ in range(2):
+        weight = torch.randn(vocab, cols, generator=gen, device="cuda").bfloat16().requires_grad_(True)
+        out = fused_ops.embedding(ids, weight)
+        assert torch.equal(out, F.embedding(ids, weight))
+        out.backward(g)
+        grads.append(weight.grad)
+    sums = lambda t: torch.zeros(vocab, cols, device="cuda", dtype=torch.float64).index_add_(0, ids[0], t)
+    want, size = sums(g[0].double()), sums(g[0].double().abs())
+    count = torch.bincount(ids[0], minlength=vocab)[:, None]
+    assert (grads[0].double() - want).abs().le(2.0**-8 * want.abs() + count * 2.0**-23 * size).all()
+    assert torch.equal(*grads)
