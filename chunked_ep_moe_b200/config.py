@@ -40,7 +40,9 @@ class ChunkedMoEConfig:
       top_k: experts per token K.
       slice_size: rows S of one dispatch slice. Every receiver's packed,
         expert-major stream is cut into S-row slices; all per-iteration
-        buffers are S rows whatever the routing imbalance.
+        buffers are S rows whatever the routing imbalance. (The fused path
+        on one rank exchanges nothing: it runs a pass as one slice where the
+        device has memory to spare.)
       transport / expert_compute: see module docstring.
       comm_dtype: None (rows travel in the compute dtype) or "float8_e4m3fn"
         (rows are quantised on put with one fp32 scale per 1x128 block and

@@ -30,6 +30,7 @@ py::dict plan_layout_dict(int P, int L, int S, int max_slices) {
   d["num_chunks"] = y.off_num_chunks;
   d["gtiles"] = y.off_gtiles;
   d["put"] = y.off_put;
+  d["tile_start"] = y.off_tile_start;
   d["total"] = y.total;
   d["tile_m"] = cem::kTileTokens;
   d["put_chunk_rows"] = cem::kPutChunkRows;
@@ -159,6 +160,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("finish_backward", &cem::FusedRank::finish_backward)
       .def("check_status", &cem::FusedRank::check_status)
       .def("plan_header", &cem::FusedRank::plan_header)
+      .def("set_whole_passes", &cem::FusedRank::set_whole_passes)
       .def("plan_ints", &cem::FusedRank::plan_ints)
       .def("launches", &cem::FusedRank::launches)
       .def("set_pipeline_counters", &cem::FusedRank::set_pipeline_counters, py::arg("counters") = py::none())

@@ -164,8 +164,9 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
   if (threadIdx.x == 0) s_abort = (p.status != nullptr && p.status->code != 0) ? 1 : 0;
   __syncthreads();
   if (s_abort) return;  // an earlier kernel of this pass already gave up
+  const bool whole = p.last_expert > 0;
   // Buffer reuse: sequence q overwrites what sequence q-2 used on every receiver.
-  if (p.seq >= 2 && threadIdx.x < p.lay.P) {
+  if (!whole && p.seq >= 2 && threadIdx.x < p.lay.P) {
     uint32_t seen = 0;
     if (!spin_until_reached(p.credit + threadIdx.x, p.seq - 1, p.spin_limit, &seen)) {
       report_status(p.status, kStatusCreditTimeout, kKernelPut, 0, static_cast<int>(p.seq), threadIdx.x, p.seq - 1, seen);
@@ -175,9 +176,13 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
   __syncthreads();
   if (s_abort) return;
 
-  const int num_chunks = p.plan[p.lay.off_num_chunks + p.slice];
   const int4* put = reinterpret_cast<const int4*>(p.plan + p.lay.off_put + 4 * n_seg * p.slice);
-  const int buf = static_cast<int>(p.seq & 1u);
+  int first_chunk = 0, num_chunks = p.plan[p.lay.off_num_chunks + p.slice];
+  if (whole) {
+    first_chunk = put[p.first_expert].w;
+    if (p.last_expert < n_seg) num_chunks = put[p.last_expert].w;
+  }
+  const int buf = whole ? 0 : static_cast<int>(p.seq & 1u);
   const int S = p.lay.S, D = p.hidden;
   const int warps_total = gridDim.x * (kPutThreads / 32);
   // Arrival releases are batched: a system-scope fence drains this warp's stores over NVLink, so one fence covers
@@ -191,7 +196,7 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
     if (lane < pending) release_count(pend_ptr, pend_cnt, p.lay.P);
     pending = 0;
   };
-  for (int c = blockIdx.x * (kPutThreads / 32) + warp; c < num_chunks; c += warps_total) {
+  for (int c = first_chunk + blockIdx.x * (kPutThreads / 32) + warp; c < num_chunks; c += warps_total) {
     const int seg = find_segment(put, n_seg, c, lane);
     const int4 e = put[seg];  // {send-order offset, rows, dest row, chunk prefix}
     const int r = seg / p.lay.L, l = seg - r * p.lay.L;
@@ -211,31 +216,41 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
                       static_cast<uint32_t>(token));
         token = -1;
       } else {
-        p.peer_w[r][drow + lane] = p.w_flat[flat];
+        float* w = whole ? p.whole_w : p.peer_w[r];
+        if (w != nullptr) w[drow + lane] = p.w_flat[flat];
       }
     }
     __syncwarp();
     if constexpr (WIRE == kWireBf16) {
 #pragma unroll 1
-      for (int what = 0; what < (p.g != nullptr ? 2 : 1); ++what)  // (one copy of the loop: it fills the registers)
-        copy_rows(what ? p.g : p.x, (what ? p.peer_g[r] : p.peer_x[r]) + drow * D, token, rows, D, lane);
+      for (int what = 0; what < 2; ++what) {  // (one copy of the loop: it fills the registers)
+        const __nv_bfloat16* from = what ? p.g : p.x;
+        if (from == nullptr) continue;
+        __nv_bfloat16* to = whole ? (what ? p.whole_g : p.whole_x) : (what ? p.peer_g[r] : p.peer_x[r]);
+        copy_rows(from, to + drow * D, token, rows, D, lane);
+      }
     } else {
       for (int rr = 0; rr < rows; ++rr) {
         const int t = __shfl_sync(0xffffffffu, token, rr);
         if (t < 0) continue;
-        const __nv_bfloat16* x = p.x + static_cast<size_t>(t) * D;
-        const __nv_bfloat16* g = p.g != nullptr ? p.g + static_cast<size_t>(t) * D : nullptr;
         const size_t to = drow + rr;
         if constexpr (WIRE == kWireFp8) {
+          const __nv_bfloat16* x = p.x + static_cast<size_t>(t) * D;
+          const __nv_bfloat16* g = p.g != nullptr ? p.g + static_cast<size_t>(t) * D : nullptr;
           put_row_fp8(x, p.peer_xq[r] + to * D, p.peer_xs[r] + to * (D >> 7), D, lane);
           if (g != nullptr) put_row_fp8(g, p.peer_gq[r] + to * D, p.peer_gs[r] + to * (D >> 7), D, lane);
         } else {
 #pragma unroll 1
-          for (int what = 0; what < (g != nullptr ? 2 : 1); ++what)
-            put_row_rounded(what ? g : x, (what ? p.peer_g[r] : p.peer_x[r]) + to * D, D, lane);
+          for (int what = 0; what < 2; ++what) {
+            const __nv_bfloat16* from = what ? p.g : p.x;
+            if (from == nullptr) continue;
+            __nv_bfloat16* dst = whole ? (what ? p.whole_g : p.whole_x) : (what ? p.peer_g[r] : p.peer_x[r]);
+            put_row_rounded(from + static_cast<size_t>(t) * D, dst + to * D, D, lane);
+          }
         }
       }
     }
+    if (whole) continue;
     if (lane == pending) {
       pend_ptr = p.peer_arrive[r] + p.me * p.lay.L + l;
       pend_cnt = static_cast<uint32_t>(rows);

@@ -31,6 +31,12 @@ struct PutParams {
   // fp8 wire (comm_dtype=float8_e4m3fn): rows travel as e4m3 + one fp32 scale per 128 columns. A rank on its own has no wire:
   // `round_fp8` stores the values that expansion would yield, as bf16.
   int round_fp8;
+  // A rank on its own that runs a pass as one slice (last > 0): rows of experts [first, last) go to matrices of the whole pass
+  // (those that are not null; x and g likewise), in stream order. No buffer to wait for, and nobody who counts arrivals.
+  int first_expert, last_expert;
+  __nv_bfloat16* whole_x;           // [T*K, D]
+  __nv_bfloat16* whole_g;
+  float* whole_w;                   // [T*K]
   uint8_t* const* peer_xq;          // [P] [2][S][D] e4m3, or null when rows travel in bf16
   uint8_t* const* peer_gq;
   float* const* peer_xs;            // [P] [2][S][D/128] scales

@@ -47,6 +47,9 @@ struct GemmParams {
   const int* plan;   // per-pass plan buffer (see plan_tables.cuh)
   PlanLayout lay;
   int slice;         // slice index inside the pass
+  // The tiles of experts [first, last) only; last = 0: of all. (Weight gradients: in the tables of a pass that is one slice, where
+  // every expert has a group.)
+  int first_expert, last_expert;
   int n_tiles;       // 256-column tiles of the weights (row-wise modes) or of the gradient (tgmm)
   int m_tiles;       // tgmm: M / 128 (row tiles of the weight gradient); unused otherwise
   int k_blocks;      // gmm modes: K / 64

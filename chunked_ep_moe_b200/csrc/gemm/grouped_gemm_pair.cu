@@ -43,7 +43,7 @@ __device__ __forceinline__ Tile decode_pair_tile(const GemmParams& p, int t, int
   Tile tl;
   const int per_group = (p.m_tiles / 2) * p.n_tiles;
   const int gi = t / per_group, rem = t - gi * per_group;
-  const int4 e = reinterpret_cast<const int4*>(p.plan + p.lay.off_gtiles + 4 * p.lay.max_gtiles * p.slice)[gi];
+  const int4 e = reinterpret_cast<const int4*>(p.plan + p.lay.off_gtiles + 4 * p.lay.max_gtiles * p.slice)[p.first_expert + gi];
   tl.g = e.x; tl.row0 = e.y; tl.nrows = e.z; tl.flags = e.w;
   const int mp = rem / p.n_tiles;
   tl.m = 2 * mp + rank; tl.n = rem - mp * p.n_tiles;
@@ -251,7 +251,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmParams p, const __grid_cons
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot_gen;
 
-  const int num_tiles = p.plan[p.lay.off_num_gtiles + p.slice] * (p.m_tiles / 2) * p.n_tiles;
+  const int groups = p.last_expert > 0 ? p.last_expert - p.first_expert : p.plan[p.lay.off_num_gtiles + p.slice];
+  const int num_tiles = groups * (p.m_tiles / 2) * p.n_tiles;
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
 
   if (warp == 0) {

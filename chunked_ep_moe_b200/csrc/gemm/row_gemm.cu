@@ -51,7 +51,7 @@ struct RowTile {
   int n;      // 256-column tile of the weights
 };
 
-__device__ __forceinline__ RowTile decode_row_tile(const GemmParams& p, int t, int num_entries) {
+__device__ __forceinline__ RowTile decode_row_tile(const GemmParams& p, int t, int first_entry, int num_entries) {
   RowTile tl;
   const int band_tiles = kRowBand * p.n_tiles;
   const int band = t / band_tiles, rem = t - band * band_tiles;
@@ -59,7 +59,7 @@ __device__ __forceinline__ RowTile decode_row_tile(const GemmParams& p, int t, i
   width = width > kRowBand ? kRowBand : width;
   tl.n = rem / width;
   const int ti = band * kRowBand + (rem - tl.n * width);
-  const int4 e = reinterpret_cast<const int4*>(p.plan + p.lay.off_tiles + 4 * p.lay.max_tiles * p.slice)[ti];
+  const int4 e = reinterpret_cast<const int4*>(p.plan + p.lay.off_tiles + 4 * p.lay.max_tiles * p.slice)[first_entry + ti];
   tl.g = e.x; tl.row0 = e.y; tl.nrows = e.z; tl.ncols = e.w;
   return tl;
 }
@@ -551,7 +551,16 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
   const uint32_t tmem_base = *tmem_slot_gen;
 
   const bool gave_up = *early_flag != 0;
-  const int num_entries = gave_up ? 0 : p.plan[p.lay.off_num_tiles + p.slice];
+  int first_entry = 0, num_entries = 0;
+  if (!gave_up) {
+    if (p.last_expert > 0) {
+      const int* start = p.plan + p.lay.off_tile_start + (p.lay.L + 1) * p.slice;
+      first_entry = start[p.first_expert];
+      num_entries = start[p.last_expert] - first_entry;
+    } else {
+      num_entries = p.plan[p.lay.off_num_tiles + p.slice];
+    }
+  }
   const int num_tiles = num_entries * p.n_tiles;
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
 
@@ -565,10 +574,10 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     bool dead = false;
     // The next tile is decoded one iteration ahead, so its plan-table load is in flight while this tile runs.
     RowTile nxt = {};
-    if (first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, num_entries);
+    if (first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, first_entry, num_entries);
     for (int t = first_tile; t < num_tiles && !dead && !*abort_flag; t += tile_step) {
       const RowTile tl = nxt;
-      if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, num_entries);
+      if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, first_entry, num_entries);
       if constexpr (MODE == kModeSwiglu || MODE == kModeDswiglu) {  // whichever reads a slice's dispatched rows first
         if ((p.arrive != nullptr || p.ready != nullptr) && tl.g != waited_expert) {
           if (!wait_expert_rows(p, MODE, tl.g, lane, abort_flag)) {
@@ -631,10 +640,10 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
       dead = true;
     };
     RowTile nxt = {};
-    if (leader && first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, num_entries);
+    if (leader && first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, first_entry, num_entries);
     for (int t = first_tile; leader && t < num_tiles && !dead && !*abort_flag; t += tile_step, ++tcount) {
       const RowTile tl = nxt;
-      if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, num_entries);
+      if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, first_entry, num_entries);
       const int as = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1u;
       const uint32_t tmem_d = tmem_base + as * kTileTokens;
@@ -696,10 +705,10 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     long long epi_wait = 0;
     if (!gave_up) zero_tail(p, (warp - 2) * 32 + lane);
     RowTile nxt = {};
-    if (first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, num_entries);
+    if (first_tile < num_tiles) nxt = decode_row_tile(p, first_tile, first_entry, num_entries);
     for (int t = first_tile; t < num_tiles; t += tile_step, ++tcount) {
       const RowTile tl = nxt;
-      if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, num_entries);
+      if (t + tile_step < num_tiles) nxt = decode_row_tile(p, t + tile_step, first_entry, num_entries);
       const int as = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1u;
       DswigluLoads first = {};  // (zeros: what rows past the tile are worked on with)

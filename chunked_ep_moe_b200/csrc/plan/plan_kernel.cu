@@ -1,6 +1,8 @@
 // Plan kernel (single CTA) and expert sort.
 #include "plan_kernel.cuh"
 
+#include <algorithm>
+
 #include "../common/pdl.cuh"
 #include "../common/umma.cuh"
 
@@ -97,6 +99,7 @@ __device__ void plan_phase_b_warps(int* plan, const PlanLayout& y, const int* se
   if (num_slices > y.max_slices) num_slices = y.max_slices;
   for (int j = warp; j < y.max_slices; j += nwarps) {
     int num_t = 0, num_g = 0, chunks = 0;
+    int* tile_start = plan + y.off_tile_start + (L + 1) * j;
     if (j < num_slices || j == 0) {
       const int lo = j * S, hi = lo + S;
       int* tt = plan + y.off_tiles + 4 * y.max_tiles * j;
@@ -115,6 +118,7 @@ __device__ void plan_phase_b_warps(int* plan, const PlanLayout& y, const int* se
         int tt_total, tg;
         const int et = num_t + warp_exclusive_scan(ct, lane, &tt_total);
         const int eg = num_g + warp_exclusive_scan(cg, lane, &tg);
+        if (l < L) tile_start[l] = et;
         for (int k = 0; k < ct; ++k) {
           const int at = plan_tile_begin(rows, ct, k), n = plan_tile_begin(rows, ct, k + 1) - at;
           reinterpret_cast<int4*>(tt)[et + k] = make_int4(l, first - lo + at, n, (n + kTileUnit - 1) / kTileUnit * kTileUnit);
@@ -144,6 +148,7 @@ __device__ void plan_phase_b_warps(int* plan, const PlanLayout& y, const int* se
       }
     }
     if (lane == 0) {
+      tile_start[L] = num_t;
       plan[y.off_num_tiles + j] = num_t;
       plan[y.off_num_gtiles + j] = num_g;
       plan[y.off_num_chunks + j] = chunks;
@@ -167,6 +172,50 @@ __device__ void publish_header(const PlanKernelParams& p) {
     __threadfence_system();
     st_release_sys(reinterpret_cast<uint32_t*>(p.host_out) + kPlanHeaderInts + 8, p.host_seq);
   }
+}
+
+// The tables from the traffic matrix, by one block. When the matrix and the per-segment sums fit into shared memory (always, at
+// real sizes) the block works from there and the per-slice tables are built a warp per slice; the arithmetic is `plan_phase_a/b`'s.
+__device__ void plan_tables_block(const PlanKernelParams& p, const int* counts, int* s_plan) {
+  const int P = p.lay.P, n = P * p.lay.L;
+  if (p.use_smem) {
+    const int L = p.lay.L;
+    int* s_counts = s_plan;
+    for (int i = threadIdx.x; i < P * n; i += blockDim.x) s_counts[i] = counts[i];
+    __syncthreads();
+    // scratch of the per-pass sums: rowsum [n], ebegin [n], prefix [P * n]; the same space holds phase B's inputs after
+    plan_phase_a_block(s_counts, p.plan, p.lay, p.me, s_counts + P * n, s_counts + P * n + n, s_counts + P * n + 2 * n);
+    __syncthreads();
+    int* s_seg_start = s_counts + P * n;
+    int* s_seg_size = s_seg_start + n;
+    int* s_send_start = s_seg_size + n;
+    int* s_expert_start = s_send_start + n;
+    int* s_expert_rows = s_expert_start + L;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      s_seg_start[i] = p.plan[p.lay.off_seg_start + i];
+      s_seg_size[i] = p.plan[p.lay.off_seg_size + i];
+      s_send_start[i] = p.plan[p.lay.off_send_start + i];
+    }
+    for (int l = threadIdx.x; l < L; l += blockDim.x) {
+      s_expert_start[l] = p.plan[p.lay.off_expert_start + l];
+      s_expert_rows[l] = p.plan[p.lay.off_expert_rows + l];
+    }
+    __syncthreads();
+    publish_header(p);
+    plan_phase_b_warps(p.plan, p.lay, s_seg_start, s_seg_size, s_send_start, s_expert_start, s_expert_rows);
+    return;
+  }
+  plan_phase_a(counts, p.plan, p.lay, p.me, threadIdx.x, blockDim.x);
+  __syncthreads();
+  publish_header(p);
+  plan_phase_b(p.plan, p.lay, threadIdx.x, blockDim.x);
+}
+
+// Shared memory of `plan_tables_block`: the matrix [P * n], then the larger of phase A's scratch (2 n + P * n) and phase B's inputs
+// (3 n + 2 L).
+size_t plan_smem_bytes(const PlanLayout& lay) {
+  const size_t P = static_cast<size_t>(lay.P), n = P * lay.L;
+  return sizeof(int) * (P * n + P * n + 2 * n + 2 * lay.L + n);
 }
 
 __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams p) {
@@ -203,40 +252,9 @@ __global__ void __launch_bounds__(256) plan_build_kernel(const PlanKernelParams 
     publish_header(p);
     return;
   }
-  // 3. tables. When the traffic matrix and the per-segment sums fit into shared memory (always, at real sizes) the block
-  // works from there and the per-slice tables are built a warp per slice; the arithmetic is `plan_phase_a/b`'s.
+  // 3. tables
   extern __shared__ int s_plan[];
-  if (p.use_smem) {
-    const int L = p.lay.L;
-    int* s_counts = s_plan;
-    for (int i = threadIdx.x; i < P * n; i += blockDim.x) s_counts[i] = p.counts[i];
-    __syncthreads();
-    // scratch of the per-pass sums: rowsum [n], ebegin [n], prefix [P * n]; the same space holds phase B's inputs after
-    plan_phase_a_block(s_counts, p.plan, p.lay, p.me, s_counts + P * n, s_counts + P * n + n, s_counts + P * n + 2 * n);
-    __syncthreads();
-    int* s_seg_start = s_counts + P * n;
-    int* s_seg_size = s_seg_start + n;
-    int* s_send_start = s_seg_size + n;
-    int* s_expert_start = s_send_start + n;
-    int* s_expert_rows = s_expert_start + L;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      s_seg_start[i] = p.plan[p.lay.off_seg_start + i];
-      s_seg_size[i] = p.plan[p.lay.off_seg_size + i];
-      s_send_start[i] = p.plan[p.lay.off_send_start + i];
-    }
-    for (int l = threadIdx.x; l < L; l += blockDim.x) {
-      s_expert_start[l] = p.plan[p.lay.off_expert_start + l];
-      s_expert_rows[l] = p.plan[p.lay.off_expert_rows + l];
-    }
-    __syncthreads();
-    publish_header(p);
-    plan_phase_b_warps(p.plan, p.lay, s_seg_start, s_seg_size, s_send_start, s_expert_start, s_expert_rows);
-    return;
-  }
-  plan_phase_a(p.counts, p.plan, p.lay, p.me, threadIdx.x, blockDim.x);
-  __syncthreads();
-  publish_header(p);
-  plan_phase_b(p.plan, p.lay, threadIdx.x, blockDim.x);
+  plan_tables_block(p, p.counts, s_plan);
 }
 
 // ---- expert sort: per-block histograms -> exclusive scan over (expert, block) -> stable scatter ----
@@ -341,11 +359,9 @@ __device__ __forceinline__ void sort_walk(const int (&e_of)[kSortItems], int bas
   }
 }
 
-__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* ids, int n, int num_experts,
-                                                                  const int* block_off, int* order, int* inv_order) {
-  extern __shared__ int s_slot[];  // [kSortWarps][num_experts]
-  release_successor();
-  wait_predecessor();
+// Block `blockIdx.x` of `blocks`; `s_slot`: [kSortWarps][num_experts].
+__device__ __forceinline__ void sort_scatter_block(const int* ids, int n, int num_experts, const int* block_off, int blocks,
+                                                   int* order, int* inv_order, int* s_slot) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int base = blockIdx.x * kSortThreads * kSortItems + warp * (kSortItems * 32);
   for (int i = threadIdx.x; i < kSortWarps * num_experts; i += blockDim.x) s_slot[i] = 0;
@@ -355,7 +371,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* i
   sort_count(ids, n, num_experts, base, lane, mine, e_of);
   __syncthreads();
   for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
-    int run = block_off[e * gridDim.x + blockIdx.x];
+    int run = block_off[e * blocks + blockIdx.x];
 #pragma unroll
     for (int w = 0; w < kSortWarps; ++w) {
       const int c = s_slot[w * num_experts + e];
@@ -365,6 +381,26 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* i
   }
   __syncthreads();
   sort_walk(e_of, base, lane, mine, order, inv_order);
+}
+
+__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* ids, int n, int num_experts,
+                                                                  const int* block_off, int* order, int* inv_order) {
+  extern __shared__ int s_slot[];
+  release_successor();
+  wait_predecessor();
+  sort_scatter_block(ids, n, num_experts, block_off, gridDim.x, order, inv_order, s_slot);
+}
+
+// The same for a pass of one rank that runs as one slice, and in one more block the plan's tables beside it: both need only what the
+// scan left, the slots and the counts. (Sort, plan and arrival targets are five kernels in a row otherwise.)
+__global__ void __launch_bounds__(kSortThreads) sort_scatter_plan_kernel(const PlanKernelParams p, const int* ids, int n,
+                                                                       const int* block_off, int* order, int* inv_order) {
+  extern __shared__ int s_mem[];
+  release_successor();
+  wait_predecessor();
+  const int blocks = gridDim.x - 1;
+  if (static_cast<int>(blockIdx.x) == blocks) plan_tables_block(p, p.my_counts, s_mem);
+  else sort_scatter_block(ids, n, p.lay.L, block_off, blocks, order, inv_order, s_mem);
 }
 
 __global__ void __launch_bounds__(kSortThreads) sort_scatter_serial_kernel(const int* ids, int n, int num_experts,
@@ -457,10 +493,7 @@ void launch_plan_small(const PlanKernelParams& p, const int* expert_ids, int n, 
 
 void launch_plan_build(const PlanKernelParams& p_in, cudaStream_t stream) {
   PlanKernelParams p = p_in;
-  const int n = p.lay.P * p.lay.L;
-  // the matrix [P * n], then the larger of phase A's scratch (2 n + P * n) and phase B's inputs (3 n + 2 L)
-  const size_t after = static_cast<size_t>(p.lay.P) * n + 2 * static_cast<size_t>(n) + 2 * p.lay.L + n;
-  const size_t smem = sizeof(int) * (static_cast<size_t>(p.lay.P) * n + after);
+  const size_t smem = plan_smem_bytes(p.lay);
   p.use_smem = smem <= 40 * 1024 ? 1 : 0;  // 256 experts on 8 ranks need 20 KB; anything larger takes the serial path
   launch_behind(plan_build_kernel, 1, 256, p.use_smem ? smem : 0, stream, p);
 }
@@ -473,6 +506,21 @@ void plan_build_host(const int* counts, int* plan, const PlanLayout& lay, int me
 size_t expert_sort_scratch_ints(int n, int num_experts) {
   const int blocks = (n + kSortThreads * kSortItems - 1) / (kSortThreads * kSortItems);
   return static_cast<size_t>(blocks > 0 ? blocks : 1) * num_experts;
+}
+
+void launch_sort_and_plan(const PlanKernelParams& p_in, const int* expert_ids, int n, int* order, int* inv_order, int* counts,
+                          int* scratch, cudaStream_t stream) {
+  PlanKernelParams p = p_in;
+  const int L = p.lay.L;
+  int blocks = (n + kSortThreads * kSortItems - 1) / (kSortThreads * kSortItems);
+  if (blocks < 1) blocks = 1;
+  p.use_smem = 1;
+  p.my_counts = counts;
+  // (28 KB and 32 KB at 1024 experts)
+  const size_t smem = std::max(plan_smem_bytes(p.lay), sizeof(int) * kSortWarps * static_cast<size_t>(L));
+  sort_hist_kernel<<<blocks, kSortThreads, L * sizeof(int), stream>>>(expert_ids, n, L, scratch, p.status);
+  launch_behind(sort_scan_kernel, 1, 256, 0, stream, scratch, L, blocks, counts);
+  launch_behind(sort_scatter_plan_kernel, blocks + 1, kSortThreads, smem, stream, p, expert_ids, n, scratch, order, inv_order);
 }
 
 void launch_expert_sort(const int* expert_ids, int n, int num_experts, int* order, int* inv_order, int* counts,

@@ -39,6 +39,11 @@ constexpr int kPlanSmallIds = 2048, kPlanSmallExperts = 512;
 void launch_plan_small(const PlanKernelParams& p, const int* expert_ids, int n, int* order, int* inv_order,
                        uint32_t* expected_total, uint32_t* pass_base, cudaStream_t stream);
 
+// The start of a pass of ONE rank that runs as one slice, whatever the number of ids (three kernels): the sort, the tables and the
+// header. At most 1024 experts. `counts` [L] and `scratch` (`expert_sort_scratch_ints`) are written.
+void launch_sort_and_plan(const PlanKernelParams& p, const int* expert_ids, int n, int* order, int* inv_order, int* counts,
+                          int* scratch, cudaStream_t stream);
+
 // Host restatement of the table build, for CPU tests of the shared arithmetic.
 void plan_build_host(const int* counts, int* plan, const PlanLayout& lay, int me);
 

@@ -21,6 +21,7 @@
 //                                                                                          expert, ncols = nrows up to 32
 //                 gtiles[j][max_gtiles]  {expert, row0, nrows, flags}                      weight-grad groups
 //                 put[j][P*L]            {send-order offset, rows, dest row, chunk prefix} my outgoing segments
+//                 tile_start[j][L+1]     first entry of `tiles[j]` that belongs to expert l or a later one
 #pragma once
 
 #include <stdint.h>
@@ -47,7 +48,7 @@ struct PlanLayout {
   int off_send_start, off_seg_start, off_seg_size, off_in_start, off_in_size, off_src_send_start;
   int off_expert_start, off_expert_rows;
   int off_num_tiles, off_num_gtiles, off_num_chunks;
-  int off_tiles, off_gtiles, off_put;
+  int off_tiles, off_gtiles, off_put, off_tile_start;
   int total;
 };
 
@@ -74,6 +75,7 @@ CEM_HD inline PlanLayout make_plan_layout(int P, int L, int S, int max_slices) {
   y.off_tiles = o; o += 4 * y.max_tiles * max_slices;
   y.off_gtiles = o; o += 4 * y.max_gtiles * max_slices;
   y.off_put = o; o += 4 * n * max_slices;
+  y.off_tile_start = o; o += plan_align4((L + 1) * max_slices);
   y.total = o;
   return y;
 }
@@ -162,6 +164,7 @@ CEM_HD inline void plan_phase_b(int* plan, const PlanLayout& y, int tid, int nth
   if (num_slices > y.max_slices) num_slices = y.max_slices;
   for (int j = tid; j < y.max_slices; j += nthreads) {
     int num_t = 0, num_g = 0, chunks = 0;
+    int* tile_start = plan + y.off_tile_start + (L + 1) * j;
     if (j < num_slices || j == 0) {  // (slice 0 also without rows: that is where empty experts' gradients are written)
       const int lo = j * S, hi = lo + S;
       int* tt = plan + y.off_tiles + 4 * y.max_tiles * j;
@@ -170,6 +173,7 @@ CEM_HD inline void plan_phase_b(int* plan, const PlanLayout& y, int tid, int nth
         const int es = plan[y.off_expert_start + l], er = plan[y.off_expert_rows + l];
         const int first = plan_clip(lo, es, es + er), last = plan_clip(hi, es, es + er);
         const int rows = last - first;
+        tile_start[l] = num_t;
         if (rows > 0) {
           const int tiles = plan_num_tiles(rows);
           for (int k = 0; k < tiles; ++k) {
@@ -205,6 +209,7 @@ CEM_HD inline void plan_phase_b(int* plan, const PlanLayout& y, int tid, int nth
         chunks += (last - first + kPutChunkRows - 1) / kPutChunkRows;
       }
     }
+    tile_start[L] = num_t;
     plan[y.off_num_tiles + j] = num_t;
     plan[y.off_num_gtiles + j] = num_g;
     plan[y.off_num_chunks + j] = chunks;

@@ -117,6 +117,7 @@ FusedRank::FusedRank(int P, int L, int me, int S, int D, int F, int K, int strip
   spin_limit_ = static_cast<uint32_t>(spin_limit);
   mbar_limit_ = 20u * 1000u * 1000u;  // microseconds: longer than any legitimate wait on another rank
   lay_ = make_plan_layout(P, L, S, max_slices);
+  whole_lay_ = make_plan_layout(P, L, std::max(8, (tk_cap + 7) / 8 * 8), 1);
   arena_lay_ = make_arena_layout(P, L, S, D, tk_cap, fp8);
   arena_ = reinterpret_cast<uint8_t*>(arena);
   cudaDeviceProp prop;
@@ -283,6 +284,7 @@ int64_t FusedRank::begin_forward_async(torch::Tensor expert_ids, torch::Tensor p
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
   expect_i32(plan, lay_.total, "plan");
   enter_pass();
+  header_whole_ = false;
   PlanKernelParams pp{};
   pp.lay = lay_;
   pp.me = me_;
@@ -840,12 +842,10 @@ void FusedRank::release_kept() {
 // Keeping pays once the GEMM that it saves is longer than a launch, and only while there is memory to spare: live tensors
 // and all of the process's arenas, these included, stay within half of the device, else (or when the allocation fails) the backward recomputes.
 // (What the caching allocator knows, not `cudaMemGetInfo`: that call takes 2 ms with a busy device.)
-std::vector<torch::Tensor> FusedRank::allocate_kept(int64_t rows, const torch::TensorOptions& bf16) const {
-  if (std::min<int64_t>(rows, S_) * D_ * F_ < kKeepWork || !keep_activations_) return {};
+std::vector<torch::Tensor> FusedRank::allocate_kept(int64_t rows, int64_t slice_rows, const torch::TensorOptions& bf16) const {
+  if (std::min<int64_t>(rows, slice_rows) * D_ * F_ < kKeepWork || !keep_activations_) return {};
   try {
-    const auto pool = c10::cuda::CUDACachingAllocator::getDeviceStats(bf16.device().index());
-    const size_t live = static_cast<size_t>(pool.allocated_bytes[0].current) + static_cast<size_t>(arenas_allocated());
-    if (live + static_cast<size_t>(rows) * 3 * F_ * 2 > device_bytes_ / 2) return {};
+    if (!within_half(static_cast<size_t>(rows) * 3 * F_ * 2, bf16.device().index())) return {};
     return {torch::empty({rows, 2 * F_}, bf16), torch::empty({rows, F_}, bf16)};
   } catch (const c10::Error&) {  // no memory, or an allocator that keeps no statistics
     return {};
@@ -904,7 +904,280 @@ void FusedRank::finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch
 }
 
 // ---------------------------------------------------------------------------------------------
-// whole passes
+// passes of a rank on its own, as one slice
+// ---------------------------------------------------------------------------------------------
+bool FusedRank::within_half(size_t bytes, int device) const {
+  const auto pool = c10::cuda::CUDACachingAllocator::getDeviceStats(device);
+  const size_t live = static_cast<size_t>(pool.allocated_bytes[0].current) + static_cast<size_t>(arenas_allocated());
+  return live + bytes <= device_bytes_ / 2;
+}
+
+// (Up to 2048 ids without autograd in one slice: the shorter pass of `plan_small_kernel`. Two or three slices of few rows: the
+// launches that `expected_launches` counts.)
+bool FusedRank::runs_whole(int64_t rows, bool training) const {
+  if (P_ != 1 || !whole_passes_ || !use_comm_stream_ || rows == 0) return false;
+  if (rows <= S_ ? !training && rows <= kPlanSmallIds : rows <= 3 * S_ && rows < kWholeRows) return false;
+  // x, act (and h, and in the backward g and dh), 2 bytes each
+  const size_t bytes = static_cast<size_t>(rows) * 2 * (training ? 2 * D_ + 5 * F_ : D_ + F_);
+  try {
+    return within_half(bytes, c10::cuda::current_device());
+  } catch (const c10::Error&) {  // an allocator that keeps no statistics
+    return false;
+  }
+}
+
+// Expert ranges in which a pass runs whose first GEMM is `columns` weight columns wide: at least four waves of that GEMM's tiles
+// each, so that what a range's put is hidden behind is longer than the tails that the range adds, and at most eight.
+int64_t FusedRank::whole_parts(int64_t rows, int64_t columns) const {
+  const int64_t tiles = (rows + 191) / 192 * (columns / kBlockN);
+  return std::max<int64_t>(1, std::min<int64_t>({8, L_, tiles / (4 * (num_sms_ / 2))}));
+}
+
+GemmParams FusedRank::range_params(const int* plan, int64_t first, int64_t last) const {
+  GemmParams p = base_params(plan, 0);
+  p.lay = whole_lay_;
+  p.first_expert = static_cast<int>(first);
+  p.last_expert = static_cast<int>(last);
+  return p;
+}
+
+// Runs `part(first expert, last expert, put stream, GEMM stream)` range by range: the puts one behind the other, the GEMMs in turn
+// on two streams (each fills the other's tail). The caller's stream then waits for all of them. One range: everything on the
+// caller's stream.
+template <typename Part>
+void FusedRank::run_parts(int64_t parts, Part&& part) {
+  cudaStream_t st = current_stream();
+  if (parts == 1) {
+    part(0, L_, st, st);
+    return;
+  }
+  cuda_check(cudaEventRecord(ev_pass_, st), "event record");
+  cuda_check(cudaStreamWaitEvent(comm_stream_, ev_pass_, 0), "wait pass event");
+  for (int64_t k = 0; k < parts; ++k) part(L_ * k / parts, L_ * (k + 1) / parts, comm_stream_, chain_[k & 1]);
+  for (int q = 0; q < 2; ++q) {
+    cuda_check(cudaEventRecord(ev_up_[q], chain_[q]), "event record");
+    cuda_check(cudaStreamWaitEvent(st, ev_up_[q], 0), "join chain stream");
+  }
+}
+
+void FusedRank::put_whole(const torch::Tensor& plan, const torch::Tensor& order, const torch::Tensor& x, const torch::Tensor* g,
+                          const torch::Tensor& w_flat, __nv_bfloat16* to_x, __nv_bfloat16* to_g, float* to_w, int64_t first,
+                          int64_t last, cudaStream_t st, bool behind) {
+  PutParams p{};
+  p.plan = plan.data_ptr<int>();
+  p.lay = whole_lay_;
+  p.top_k = K_;
+  p.hidden = D_;
+  p.order = order.data_ptr<int>();
+  p.x = to_x != nullptr ? reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()) : nullptr;
+  p.g = to_g != nullptr ? reinterpret_cast<const __nv_bfloat16*>(g->data_ptr()) : nullptr;
+  p.w_flat = w_flat.data_ptr<float>();
+  p.num_tokens = static_cast<int>(x.size(0));
+  p.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
+  p.round_fp8 = fp8_;
+  p.first_expert = static_cast<int>(first);
+  p.last_expert = static_cast<int>(last);
+  p.whole_x = to_x;
+  p.whole_g = to_g;
+  p.whole_w = to_w;
+  launch_dispatch_put(p, put_blocks_, st, behind);
+  ++launches_;
+}
+
+// `kept`: h and w * act, or nothing. `buffers`: x by rows, router weights by rows and, where nothing is kept, w * act.
+std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_whole(
+    torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
+    const std::vector<torch::Tensor>& kept, const std::vector<torch::Tensor>& buffers) {
+  cudaStream_t st = current_stream();
+  const int64_t tk = expert_ids.numel();
+  auto i32 = torch::TensorOptions().device(x.device()).dtype(torch::kInt32);
+  torch::Tensor plan = torch::empty({whole_lay_.total}, i32), order = torch::empty({tk}, i32),
+                inv_order = torch::empty({tk}, i32), out = torch::empty_like(x);
+  const torch::Tensor &rows_x = buffers[0], &rows_w = buffers[1], &act = kept.empty() ? buffers[2] : kept[1];
+  const QuiesceOnError guard{this};
+  expect_bf16_2d(x, D_, "x");
+  expect_weights(w_up, w_down, L_, D_, F_);
+  expect_i32(expert_ids, tk, "expert_ids");
+  expect(x.size(0) * K_ == tk && w_flat.is_cuda() && w_flat.scalar_type() == torch::kFloat32 && w_flat.is_contiguous() &&
+             w_flat.numel() == tk,
+         "router weights must be a contiguous CUDA fp32 tensor of T*K elements");
+  enter_pass();
+  header_whole_ = true;
+  cur_slices_ = 0;  // (no streams of slices to join)
+  {
+    NvtxRange range("chunked_moe/plan");
+    PlanKernelParams pp{};
+    pp.lay = whole_lay_;
+    pp.plan = plan.data_ptr<int>();
+    pp.spin_limit = spin_limit_;
+    pp.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
+    pp.host_out = host_header_;
+    pp.host_seq = ++host_seq_;
+    launch_sort_and_plan(pp, expert_ids.data_ptr<int>(), static_cast<int>(tk), order.data_ptr<int>(),
+                         inv_order.data_ptr<int>(), my_counts_.data_ptr<int>(), sort_scratch_.data_ptr<int>(), st);
+    launches_ += 3;
+  }
+  cur_rows_ = tk;
+  ret_target_ += static_cast<uint32_t>(tk) * static_cast<uint32_t>(D_ / kCombineCols);
+  const int* pl = plan.data_ptr<int>();
+  const int64_t parts = whole_parts(tk, 2 * F_);
+  inline_ = parts == 1;
+  const TokenMaps x_map = make_token_maps(rows_x.data_ptr(), tk, D_), act_map = make_token_maps(act.data_ptr(), tk, F_);
+  run_parts(parts, [&](int64_t first, int64_t last, cudaStream_t put_stream, cudaStream_t gemm_stream) {
+    NvtxRange range("chunked_moe/fwd experts from", first);
+    put_whole(plan, order, x, nullptr, w_flat, reinterpret_cast<__nv_bfloat16*>(rows_x.data_ptr()), nullptr,
+              rows_w.data_ptr<float>(), first, last, put_stream, inline_);
+    if (put_stream != gemm_stream) {
+      cuda_check(cudaEventRecord(ev_put_[0], put_stream), "event record");
+      cuda_check(cudaStreamWaitEvent(gemm_stream, ev_put_[0], 0), "wait put event");
+    }
+    {
+      GemmParams p = range_params(pl, first, last);
+      p.n_tiles = 2 * F_ / kBlockN;
+      p.k_blocks = D_ / kBlockK;
+      p.b_group_rows = D_;
+      p.row_w = rows_w.data_ptr<float>();
+      p.out0 = reinterpret_cast<__nv_bfloat16*>(act.data_ptr());
+      p.ld0 = F_;
+      p.out1 = kept.empty() ? nullptr : reinterpret_cast<__nv_bfloat16*>(kept[0].data_ptr());
+      p.ld1 = 2 * F_;
+      row_gemm(kModeSwiglu, p, up_map(w_up), x_map, gemm_stream);
+    }
+    GemmParams p = range_params(pl, first, last);
+    p.n_tiles = D_ / kBlockN;
+    p.k_blocks = F_ / kBlockK;
+    p.b_group_rows = F_;
+    p.peer_rows = table<__nv_bfloat16>(kTabRet);
+    p.peer_count = table<uint32_t>(kTabCount);
+    p.ld0 = D_;
+    row_gemm(kModeDownFwd, p, weight_map(w_down, 64, 2), act_map, gemm_stream);
+  });
+  {
+    NvtxRange range("chunked_moe/combine");
+    finish_forward(inv_order, out);
+  }
+  resolve_slices();  // raises what the pass's kernels had recorded by the time the plan was made
+  std::vector<torch::Tensor> result{out, plan, order, inv_order};
+  result.insert(result.end(), kept.begin(), kept.end());
+  return std::make_tuple(result, kWholePass, kept.empty() ? 0 : 1);
+}
+
+// `buffers`: x by rows, g by rows, router weights by rows, dh, d_weight shares and, where nothing was kept, h and w * act.
+void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up,
+                               torch::Tensor w_down, torch::Tensor plan, torch::Tensor order,
+                               const std::vector<torch::Tensor>& kept, const std::vector<torch::Tensor>& buffers,
+                               torch::Tensor dw_up, torch::Tensor dw_down) {
+  cudaStream_t st = current_stream();
+  const int64_t tk = order.numel();
+  expect_i32(plan, whole_lay_.total, "plan");
+  expect_bf16_2d(x, D_, "x");
+  expect_bf16_2d(g, D_, "g");
+  expect(g.size(0) == x.size(0) && x.size(0) * K_ == tk, "x and g rows do not match the pass");
+  expect_weights(w_up, w_down, L_, D_, F_);
+  expect_weights(dw_up, dw_down, L_, D_, F_);
+  enter_pass();
+  cur_slices_ = 0;
+  cur_rows_ = tk;
+  ret_target_ += static_cast<uint32_t>(tk) * static_cast<uint32_t>(D_ / kCombineCols + 1);
+  const bool keep = !kept.empty();
+  auto bf16 = [](const torch::Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); };
+  const torch::Tensor &rows_x = buffers[0], &rows_g = buffers[1], &rows_w = buffers[2], &dh = buffers[3], &dwp = buffers[4],
+                      &h = keep ? kept[0] : buffers[5], &act = keep ? kept[1] : buffers[6];
+  const int* pl = plan.data_ptr<int>();
+  const int dwp_tiles = F_ / 32;
+  const TokenMaps x_map = keep ? TokenMaps{} : make_token_maps(rows_x.data_ptr(), tk, D_);
+  const TokenMaps g_map = make_token_maps(rows_g.data_ptr(), tk, D_), dh_map = make_token_maps(dh.data_ptr(), tk, 2 * F_);
+  const CUtensorMap x_mn = make_bf16_map_chunked(rows_x.data_ptr(), tk, D_, 64, 2), g_mn = make_bf16_map_chunked(rows_g.data_ptr(), tk, D_, 64, 2),
+                    act_mn = make_bf16_map_chunked(act.data_ptr(), tk, F_, 64, 2), dh_mn = make_bf16_map_chunked(dh.data_ptr(), tk, 2 * F_, 64, 2);
+  // d_act = w * (g Wd^T) needs g's rows; x's, where nothing has to be recomputed from them, follow beside that GEMM.
+  const int64_t parts = whole_parts(tk, F_);
+  const bool x_later = keep && parts > 1;
+  run_parts(parts, [&](int64_t first, int64_t last, cudaStream_t put_stream, cudaStream_t gemm_stream) {
+    NvtxRange range("chunked_moe/bwd experts from", first);
+    put_whole(plan, order, x, &g, w_flat, x_later ? nullptr : bf16(rows_x), bf16(rows_g), rows_w.data_ptr<float>(), first, last,
+              put_stream, false);
+    if (put_stream != gemm_stream) {
+      cuda_check(cudaEventRecord(ev_put_[0], put_stream), "event record");
+      cuda_check(cudaStreamWaitEvent(gemm_stream, ev_put_[0], 0), "wait put event");
+    }
+    if (x_later) {
+      put_whole(plan, order, x, nullptr, w_flat, bf16(rows_x), nullptr, nullptr, first, last, put_stream, false);
+      cuda_check(cudaEventRecord(ev_put_[1], put_stream), "event record");
+    }
+    if (!keep) {
+      GemmParams p = range_params(pl, first, last);
+      p.n_tiles = 2 * F_ / kBlockN;
+      p.k_blocks = D_ / kBlockK;
+      p.b_group_rows = D_;
+      p.row_w = rows_w.data_ptr<float>();
+      p.out0 = bf16(act);
+      p.ld0 = F_;
+      p.out1 = bf16(h);
+      p.ld1 = 2 * F_;
+      row_gemm(kModeSwiglu, p, up_map(w_up), x_map, gemm_stream);
+    }
+    {  // acc = g Wd^T; dh = SwiGLU'(h) * (w * acc), d_weight shares <acc, w * act>
+      GemmParams p = range_params(pl, first, last);
+      p.n_tiles = F_ / kBlockN;
+      p.k_blocks = D_ / kBlockK;
+      p.b_group_rows = F_;
+      p.row_w = rows_w.data_ptr<float>();
+      p.in0 = bf16(h);
+      p.in1 = bf16(act);
+      p.ld1 = F_;
+      p.out0 = bf16(dh);
+      p.ld0 = 2 * F_;
+      p.dwp = dwp.data_ptr<float>();
+      p.dwp_tiles = dwp_tiles;
+      row_gemm(kModeDswiglu, p, weight_map(w_down, 128), g_map, gemm_stream);
+    }
+    cuda_check(cudaEventRecord(ev_ds_[0], gemm_stream), "event record");
+    cuda_check(cudaStreamWaitEvent(aux_stream_, ev_ds_[0], 0), "wait dswiglu event");
+    {  // dW_down[g] = (w act)^T g   (auxiliary stream)
+      GemmParams p = range_params(pl, first, last);
+      p.m_tiles = F_ / kBlockM;
+      p.n_tiles = D_ / kBlockN;
+      p.grad_out = bf16(dw_down);
+      weight_grad(p, act_mn, g_mn, weight_map(dw_down, 32), aux_stream_);
+    }
+    {  // dx = dh Wu^T
+      GemmParams p = range_params(pl, first, last);
+      p.n_tiles = D_ / kBlockN;
+      p.k_blocks = 2 * F_ / kBlockK;
+      p.b_group_rows = D_;
+      p.peer_rows = table<__nv_bfloat16>(kTabRet);
+      p.peer_count = table<uint32_t>(kTabCount);
+      p.ld0 = D_;
+      row_gemm(kModeDx, p, weight_map(w_up, 128), dh_map, gemm_stream);
+    }
+    if (x_later) cuda_check(cudaStreamWaitEvent(aux_stream_, ev_put_[1], 0), "wait put event");
+    if (last == L_) {  // d_weight of every row (this stream has waited for every range's shares)
+      ReturnDwParams r{};
+      r.plan = pl;
+      r.lay = whole_lay_;
+      r.dwp = dwp.data_ptr<float>();
+      r.row_w = rows_w.data_ptr<float>();
+      r.parts = dwp_tiles;
+      r.peer_dw = table<float>(kTabDw);
+      r.peer_count = table<uint32_t>(kTabCount);
+      r.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
+      launch_return_dw(r, aux_stream_);
+      ++launches_;
+    }
+    {  // dW_up[g] = x^T dh
+      GemmParams p = range_params(pl, first, last);
+      p.m_tiles = D_ / kBlockM;
+      p.n_tiles = 2 * F_ / kBlockN;
+      p.grad_out = bf16(dw_up);
+      weight_grad(p, x_mn, dh_mn, weight_map(dw_up, 32), aux_stream_);
+    }
+  });
+  cuda_check(cudaEventRecord(ev_tgu_[0], aux_stream_), "event record");
+  cuda_check(cudaStreamWaitEvent(st, ev_tgu_[0], 0), "join aux stream");
+}
+
+// ---------------------------------------------------------------------------------------------
+// passes as one call each
 // ---------------------------------------------------------------------------------------------
 std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass(
     torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
@@ -913,6 +1186,20 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
   release_kept();  // (of a pass that threw)
   short_pass_ = false;
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
+  // Under saved-tensor hooks a pass keeps nothing and runs slice by slice: whether it may do otherwise depends on the free memory,
+  // and its backward may get the plan of a recomputation.
+  const bool hooks = training && at::SavedTensorDefaultHooks::get_hooks().has_value();
+  if (!hooks && runs_whole(tk, training)) {
+    std::vector<torch::Tensor> kept, buffers;
+    if (training) kept = allocate_kept(tk, tk, x.options());
+    try {
+      buffers = {torch::empty({tk, D_}, x.options()), torch::empty({tk}, x.options().dtype(torch::kFloat32))};
+      if (kept.empty()) buffers.push_back(torch::empty({tk, F_}, x.options()));
+    } catch (const c10::Error&) {  // no memory for it after all
+      buffers.clear();
+    }
+    if (!buffers.empty()) return forward_whole(x, expert_ids, w_flat, w_up, w_down, kept, buffers);
+  }
   auto i32 = torch::TensorOptions().device(x.device()).dtype(torch::kInt32);
   // (The send order needs no initial values: an id the sort leaves out is recorded in the status block first, and with
   // that set every kernel that would read the order returns at once.)
@@ -950,9 +1237,9 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
   }
   if (known >= 0) guess = std::min<int64_t>(known, max_slices_);
   int64_t kept_slices = 0;
-  if (training && !at::SavedTensorDefaultHooks::get_hooks().has_value()) {
+  if (training && !hooks) {
     const int64_t slices = known >= 0 ? guess : slices_to_keep(guess, last_rows_, S_);  // the others are recomputed
-    if (slices > 0) kept = allocate_kept(known >= 0 ? tk : slices * S_, x.options());
+    if (slices > 0) kept = allocate_kept(known >= 0 ? tk : slices * S_, S_, x.options());
     if (!kept.empty()) {
       kept_slices = slices;
       keep_rows(kept[0], kept[1], kept_slices);
@@ -983,12 +1270,49 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
     const std::vector<torch::Tensor>& kept, int64_t kept_slices) {
   inline_ = short_pass_ = false;  // (also behind a forward that threw)
   release_kept();
-  if (kept.size() == 2) keep_rows(kept[0], kept[1], kept_slices);
-  // The slice count is the forward's: nothing is read back, the host never waits for the device here.
-  const int64_t n = begin_backward(plan, known_slices, order.numel());
+  const int64_t rows = order.numel();
   torch::Tensor dw_up = torch::empty_like(w_up), dw_down = torch::empty_like(w_down), dx = torch::empty_like(x);
   torch::Tensor d_weights = torch::empty({w_flat.numel()}, w_flat.options());
+  std::vector<torch::Tensor> buffers;
+  if (known_slices == kWholePass && whole_passes_) {
+    const auto f32 = x.options().dtype(torch::kFloat32);
+    try {
+      buffers = {torch::empty({rows, D_}, x.options()), torch::empty({rows, D_}, x.options()), torch::empty({rows}, f32),
+                 torch::empty({rows, 2 * F_}, x.options()), torch::empty({rows, F_ / 32}, f32)};
+      if (kept.size() != 2) {
+        buffers.push_back(torch::empty({rows, 2 * F_}, x.options()));
+        buffers.push_back(torch::empty({rows, F_}, x.options()));
+      }
+    } catch (const c10::Error&) {  // no memory for it: slice by slice
+      buffers.clear();
+    }
+  }
   const QuiesceOnError guard{this};
+  if (!buffers.empty()) {
+    backward_whole(x, g, w_flat, w_up, w_down, plan, order, kept, buffers, dw_up, dw_down);
+    finish_backward(inv_order, dx, d_weights);
+    return std::make_tuple(dx, d_weights, dw_up, dw_down);
+  }
+  if (known_slices == kWholePass) {
+    // The workspace's slices after all, with tables made of the row counts in the forward's.
+    torch::Tensor sliced = torch::empty({lay_.total}, plan.options());
+    PlanKernelParams pp{};
+    pp.lay = lay_;
+    pp.me = me_;
+    pp.plan = sliced.data_ptr<int>();
+    pp.counts = plan.data_ptr<int>() + whole_lay_.off_in_size;
+    pp.my_counts = pp.counts;
+    pp.spin_limit = spin_limit_;
+    pp.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
+    launch_plan_build(pp, current_stream());
+    ++launches_;
+    plan = sliced;
+    known_slices = (rows + S_ - 1) / S_;
+    if (kept.size() == 2) kept_slices = known_slices;
+  }
+  if (kept.size() == 2) keep_rows(kept[0], kept[1], kept_slices);
+  // The slice count is the forward's: nothing is read back, the host never waits for the device here.
+  const int64_t n = begin_backward(plan, known_slices, rows);
   if (n > 0) {
     put(0, plan, order, x, g, w_flat);
   } else {

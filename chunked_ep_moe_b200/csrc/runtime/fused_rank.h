@@ -53,6 +53,11 @@ inline int64_t slices_to_keep(int64_t guess, int64_t stream_rows, int64_t slice_
   return std::min<int64_t>(guess, (stream_rows + slice_rows - 1) / slice_rows);
 }
 
+// What a forward that ran as one slice (`FusedRank::runs_whole`) gives as its slice count.
+constexpr int64_t kWholePass = -1;
+// Two or three slices of fewer rows run as slices.
+constexpr int64_t kWholeRows = 16384;
+
 class FusedRank {
  public:
   FusedRank(int P, int L, int me, int S, int D, int F, int K, int stripe, int tk_cap, int max_slices, int num_sms,
@@ -111,8 +116,15 @@ class FusedRank {
 
   // Reads the status block (synchronises); throws std::runtime_error describing the first recorded error.
   void check_status();
-  std::vector<int64_t> plan_header() const { return std::vector<int64_t>(host_header_, host_header_ + 16); }
+  std::vector<int64_t> plan_header() const {
+    std::vector<int64_t> header(host_header_, host_header_ + 16);
+    if (header_whole_) header[0] = (header[2] + S_ - 1) / S_;  // in slices of the configured size
+    return header;
+  }
   int64_t plan_ints() const { return lay_.total; }
+  // Whether passes of a rank on its own may run as one slice (default). Off: slice by slice, also the backward of a forward that
+  // ran as one.
+  void set_whole_passes(bool on) { whole_passes_ = on; }
   int64_t launches() const { return launches_; }
   // Turns the GEMM kernels' pipeline counters on: `counters` is a zeroed int64 CUDA tensor [6 modes, num_sms, 8]
   // (slots: ProfSlot in gemm/grouped_gemm.cuh) that every later GEMM launch adds to. An undefined tensor turns
@@ -140,7 +152,7 @@ class FusedRank {
     }
   };
   void release_kept();
-  std::vector<torch::Tensor> allocate_kept(int64_t rows, const torch::TensorOptions& bf16) const;
+  std::vector<torch::Tensor> allocate_kept(int64_t rows, int64_t slice_rows, const torch::TensorOptions& bf16) const;
   __nv_bfloat16* kept_h(int64_t j) const {
     return reinterpret_cast<__nv_bfloat16*>(kept_h_.data_ptr()) + static_cast<size_t>(j) * S_ * 2 * F_;
   }
@@ -152,6 +164,31 @@ class FusedRank {
   // rank the put kernel stores the expanded values at once (32 experts of 1024 rows,
   // D=7168, F=2048, forward + backward: 11.1 -> 9.06 ms).
   bool expands() const { return fp8_ && P_ > 1; }
+  // Slices are what ranks exchange. A rank on its own exchanges nothing, so its passes run as ONE slice, in ranges of whole experts
+  // (`whole_parts`): no tail of a GEMM per slice (1024 rows at F=1024 are 0.2-0.8 waves of tiles), no fp32 carry of the experts that
+  // straddle slices (176 MB written and read per boundary at D=7168, F=2048), no put that waits for a buffer. Rows are still put
+  // into expert order, range by range, each beside the GEMMs of the range before: only the first is waited for; and a range's
+  // GEMMs follow one another, so that what one writes the next finds in L2. (The whole pass GEMM by GEMM, with ranges for the first one only: 15.72
+  // ms at 32 experts x 2048 rows, D=7168, F=2048, where slices of 8192 rows took 15.63; range by range 15.41 against 16.04.)
+  // Forward + backward, slices -> one slice: 8 x 1024 rows at D=2048, F=1024 0.955 -> 0.430 ms, Zipf routing in 12 slices of 2048
+  // rows at D=7168 7.50 -> 6.21, 3 x 16384 rows at D=1024, F=512 0.887 -> 0.832, 4 x 8192 rows on the fp8 wire 8.84 -> 8.47, 64
+  // experts of 256 rows 5.64 -> 5.60; forward alone of 4 x 8192 rows 2.78 -> 2.71. The buffers are the pass's own, from the caching
+  // allocator, while live tensors and arenas stay within half of the device; otherwise the pass runs slice by slice.
+  bool runs_whole(int64_t rows, bool training) const;
+  bool within_half(size_t bytes, int device) const;
+  int64_t whole_parts(int64_t rows, int64_t columns) const;
+  GemmParams range_params(const int* plan, int64_t first, int64_t last) const;
+  template <typename Part>
+  void run_parts(int64_t parts, Part&& part);
+  std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> forward_whole(
+      torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
+      const std::vector<torch::Tensor>& kept, const std::vector<torch::Tensor>& buffers);
+  void backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
+                      torch::Tensor plan, torch::Tensor order, const std::vector<torch::Tensor>& kept,
+                      const std::vector<torch::Tensor>& buffers, torch::Tensor dw_up, torch::Tensor dw_down);
+  void put_whole(const torch::Tensor& plan, const torch::Tensor& order, const torch::Tensor& x, const torch::Tensor* g,
+                 const torch::Tensor& w_flat, __nv_bfloat16* to_x, __nv_bfloat16* to_g, float* to_w, int64_t first, int64_t last,
+                 cudaStream_t st, bool behind);
   bool overlapped() const { return use_comm_stream_ && !inline_; }
   void join_streams(bool backward);
   GemmParams base_params(const int* plan, int j) const;
@@ -169,6 +206,9 @@ class FusedRank {
   bool fp8_, use_comm_stream_;
   uint32_t spin_limit_, mbar_limit_;
   PlanLayout lay_;
+  PlanLayout whole_lay_{};      // one slice of tk_cap rows
+  bool whole_passes_ = true;
+  bool header_whole_ = false;   // the forward that filled the header ran as one slice
   ArenaLayout arena_lay_;
   uint8_t* arena_;
   std::vector<uint8_t*> peers_;

@@ -15,7 +15,10 @@ reached the host. Compared with the reference's loop
   * the backward starts from `h` and `w * act` where the forward could keep them (large slices, memory to spare,
     `CEM_KEEP_ACTIVATIONS=0` never) and recomputes them, slice by slice, where it could not: the same bits either way;
   * weight gradients are written once per expert in bf16; only the (at most one) expert that
-    straddles a slice boundary carries an fp32 partial to the next slice.
+    straddles a slice boundary carries an fp32 partial to the next slice;
+  * a rank on its own exchanges nothing, so its passes run as ONE slice, in up to eight ranges of experts, as long as their
+    buffers fit beside what is live in half of the device's memory (`FusedRank::runs_whole`); slice by slice otherwise, under
+    saved-tensor hooks, and in passes of two or three slices of fewer than 16384 rows.
 
 Everything else the backward needs are the inputs and the integer plan (tables, send order, its inverse).
 """
@@ -169,8 +172,10 @@ def expected_launches(num_slices: int, fp8: bool = False, kept_slices: int = 0) 
     Forward: sort (3) + plan build + pass begin + per slice (put, swiglu, down+combine, slice done) + combine reduce.
     Backward: pass begin + per slice (put, swiglu+h, dswiglu, dW_down, d_weight return, dx+combine, dW_up, slice done)
     + combine reduce. `fp8`: among several ranks the fp8 wire adds one expansion kernel per slice and pass (a rank on its own
-    launches none: pass False). A slice whose activations the forward kept needs no swiglu+h in the backward. A forward of one
-    rank and one slice without autograd launches fewer: 9 kernels (no slice done), or 5 up to 2048 ids and 512 experts.
+    launches none: pass False). A slice whose activations the forward kept needs no swiglu+h in the backward. A pass of a
+    rank on its own that runs as one slice launches fewer: sort and plan (3), per range of experts (put, swiglu, down+combine),
+    combine reduce; backward per range (put, put of x, dswiglu, dW_down, dx+combine, dW_up), d_weight return, combine reduce. A
+    forward of one slice, up to 2048 ids and 512 experts, without autograd: 5.
     """
     per_slice = 12 + (2 if fp8 else 0)
     return 8 + per_slice * num_slices - kept_slices
@@ -203,6 +208,8 @@ def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidd
         "kept for backward while memory allows (h, w * act; rows balanced over the ranks)":
             tk * 3 * F * 2 if min(tk, S) * D * F >= ext.keep_work else 0,
     }
+    if world == 1:
+        out["during a pass that runs as one slice, while memory allows (x, g, dh by rows)"] = tk * (2 * D + 2 * F) * 2
     out["total"] = sum(out.values())
     return out
 

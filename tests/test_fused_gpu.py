@@ -854,3 +854,57 @@ def test_buffers_and_wire_rows_do_not_depend_on_the_routing(skew):
     torch.cuda.synchronize()
     assert torch.cuda.memory_allocated() <= before + (1 << 20), "a pass must not grow what the ranks hold"
     world.close()
+
+
+@pytest.mark.parametrize("keep", ["1", "0"], ids=["kept", "recomputed"])
+@pytest.mark.parametrize("tokens,hidden,ffn,slice_size,wire", [(14501, 256, 2048, 1024, None), (131, 512, 256, 32, None),
+                                                               (700, 512, 1024, 4096, None), (333, 768, 256, 64, "float8_e4m3fn")])
+def test_one_rank_passes_as_one_slice_equal_slices(monkeypatch, tokens, hidden, ffn, slice_size, wire, keep):
+    """A pass of a rank on its own that runs as one slice against the same pass slice by slice: several expert ranges per pass, one
+    range, one slice of rows, the fp8 wire; an expert without rows and one with most of them. A row's results do not depend on
+    where it is: equal bits. A weight gradient is an fp32 sum in another order, rounded to bf16 once: at most a unit in the last
+    place (2^-7 of the value) apart, in the root mean square less than half of one. A backward that runs slice by slice behind a
+    forward that did not gives the slices' bits."""
+    from chunked_ep_moe_b200.ops import fused
+
+    E, K = 5, 2
+    monkeypatch.setenv("CEM_KEEP_ACTIVATIONS", keep)
+    fused.release_workspaces()
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    x, g, w = rnd(tokens, hidden).bfloat16(), rnd(tokens, hidden).bfloat16(), rnd(tokens, K).sigmoid()
+    w_up = (rnd(E, hidden, 2 * ffn) / math.sqrt(hidden)).bfloat16()
+    w_down = (rnd(E, ffn, hidden) / math.sqrt(ffn)).bfloat16()
+    logits = rnd(tokens, E)
+    logits[:, 1] -= 100.0
+    logits[:, 3] += 2.0
+    ids = torch.topk(logits, K, dim=-1).indices.int()
+    cfg = ChunkedMoEConfig(num_experts=E, top_k=K, slice_size=slice_size, transport="nvshmem", expert_compute="fused",
+                           stripe_width=64, comm_dtype=wire)
+    rank = fused.get_workspace(cfg, None, hidden, ffn, tokens * K).rank
+
+    def one(forward, backward):
+        leaves = [t.clone().requires_grad_(True) for t in (x, w, w_up, w_down)]
+        rank.set_whole_passes(forward)
+        out = chunked_moe(leaves[0], ids, *leaves[1:], cfg)
+        rank.set_whole_passes(backward)
+        before = fused.launches()
+        out.backward(g)
+        return [out.detach()] + [t.grad for t in leaves], fused.launches() - before
+
+    slices, launched = one(False, False)
+    for _ in range(2):  # counters and buffers carry over from pass to pass
+        whole, fewer = one(True, True)
+        assert fewer < launched
+        for name, a, b in zip(("out", "dx", "dweights"), whole, slices):
+            assert torch.equal(a, b), name
+        for name, a, b in zip(("dw_up", "dw_down"), whole[3:], slices[3:]):
+            assert torch.linalg.vector_norm(a.float() - b.float()) <= 2.0**-8 * torch.linalg.vector_norm(b.float()), name
+            assert torch.count_nonzero(a[1]) == 0, name
+        mixed, _ = one(True, False)
+        assert all(torch.equal(a, b) for a, b in zip(mixed, slices))
+    with torch.no_grad():
+        rank.set_whole_passes(True)
+        assert torch.equal(chunked_moe(x, ids, w, w_up, w_down, cfg), slices[0])
+    rank.check_status()
+    fused.release_workspaces()

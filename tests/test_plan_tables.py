@@ -175,3 +175,25 @@ def test_plan_kernel_matches_host_tables(P, L, S, tokens, top_k, skew):
             if j < host[0]:
                 at = lay["put"] + 4 * n * j
                 np.testing.assert_array_equal(dev[at: at + 4 * n], host[at: at + 4 * n])
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("P,L,S,tokens,top_k,skew", [(1, 5, 4096, 700, 2, "empty"), (1, 40, 64, 300, 3, "uniform"), (2, 33, 512, 300, 2, "all_one"),
+                                                     (8, 128, 64, 16, 2, "uniform")])
+def test_tile_starts_point_at_each_experts_first_tile(device, P, L, S, tokens, top_k, skew):
+    """`tile_start[l]` is the first row tile of expert l or a later one, `tile_start[L]` their number (8 x 128 experts: the serial
+    tables on the device too)."""
+    ext = _build.load()
+    _, _, counts = _counts(P, L, tokens, top_k, skew, seed=L)
+    max_slices = P * tokens * top_k // S + 2
+    lay = ext.plan_layout(P, L, S, max_slices)
+    build = ext.plan_build_host if device == "cpu" else ext.plan_build_device
+    tab = build(counts.to(torch.int32).contiguous().to(device), S, max_slices, P - 1).cpu().numpy()
+    for j in range(max_slices):
+        num = tab[lay["num_tiles"] + j]
+        experts = tab[lay["tiles"] + 4 * lay["max_tiles"] * j:][: 4 * num: 4]
+        got = tab[lay["tile_start"] + (L + 1) * j:][: L + 1]
+        if j < tab[0] or j == 0:
+            np.testing.assert_array_equal(got, np.searchsorted(experts, np.arange(L + 1)))
+        else:
+            assert got[L] == 0
