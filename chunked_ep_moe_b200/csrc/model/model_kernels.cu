@@ -201,9 +201,8 @@ __global__ void __launch_bounds__(256) norm_dw_kernel(const float* partial, int 
 // qkv [B, S, 3, H, hd] -> q, k (rotated) and v as contiguous [B, H, S, hd]. cos/sin: [S, hd/2] fp32.
 // `inverse`: rotate by -theta and write back into the qkv layout (the backward).
 template <bool kBackward>
-__global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* qkv, __nv_bfloat16* q, __nv_bfloat16* k,
-                                                       __nv_bfloat16* v, const float* cos_t, const float* sin_t,
-                                                       int B, int S, int H, int hd) {
+__global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* qkv, HeadMatrix q, HeadMatrix k, HeadMatrix v,
+                                                       const float* cos_t, const float* sin_t, int B, int S, int H, int hd) {
   const int units = hd >> 3;  // 8 values = 4 rotation pairs per unit
   const size_t total = static_cast<size_t>(B) * S * H * units;
   for (size_t idx = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; idx < total;
@@ -214,7 +213,9 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* qkv, __nv_
     const int s = static_cast<int>(rest % S);
     const int b = static_cast<int>(rest / S);
     const size_t in_base = ((static_cast<size_t>(b) * S + s) * 3 * H + h) * hd + static_cast<size_t>(u) * 8;
-    const size_t out_base = ((static_cast<size_t>(b) * H + h) * S + s) * hd + static_cast<size_t>(u) * 8;
+    auto at = [&](const HeadMatrix& m) {
+      return reinterpret_cast<int4*>(static_cast<__nv_bfloat16*>(m.data) + b * m.batch + h * m.head + s * m.row + u * 8);
+    };
     const float4 c = *reinterpret_cast<const float4*>(cos_t + static_cast<size_t>(s) * (hd >> 1) + u * 4);
     const float4 sn = *reinterpret_cast<const float4*>(sin_t + static_cast<size_t>(s) * (hd >> 1) + u * 4);
     const float cs[4] = {c.x, c.y, c.z, c.w};
@@ -222,9 +223,9 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* qkv, __nv_
                          kBackward ? -sn.w : sn.w};
 #pragma unroll
     for (int part = 0; part < 2; ++part) {  // q then k
-      __nv_bfloat16* rot = part == 0 ? q : k;
+      int4* rot = at(part == 0 ? q : k);
       const size_t in_off = in_base + static_cast<size_t>(part) * H * hd;
-      const int4 raw = kBackward ? *reinterpret_cast<const int4*>(rot + out_base)
+      const int4 raw = kBackward ? *rot
                                  : *reinterpret_cast<const int4*>(qkv + in_off);
       const uint32_t wds[4] = {(uint32_t)raw.x, (uint32_t)raw.y, (uint32_t)raw.z, (uint32_t)raw.w};
       uint32_t o[4];
@@ -235,11 +236,11 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* qkv, __nv_
       }
       const int4 res = make_int4(o[0], o[1], o[2], o[3]);
       if (kBackward) *reinterpret_cast<int4*>(qkv + in_off) = res;
-      else *reinterpret_cast<int4*>(rot + out_base) = res;
+      else *rot = res;
     }
     const size_t v_off = in_base + static_cast<size_t>(2) * H * hd;
-    if (kBackward) *reinterpret_cast<int4*>(qkv + v_off) = *reinterpret_cast<const int4*>(v + out_base);
-    else *reinterpret_cast<int4*>(v + out_base) = *reinterpret_cast<const int4*>(qkv + v_off);
+    if (kBackward) *reinterpret_cast<int4*>(qkv + v_off) = *at(v);
+    else *at(v) = *reinterpret_cast<const int4*>(qkv + v_off);
   }
 }
 
@@ -418,20 +419,16 @@ void launch_add_rms_norm_bwd(const void* dy, const void* ds_in, const void* s, c
   norm_dw_kernel<<<(cols + 31) / 32, 256, 0, stream>>>(dw_partial, grid, cols, static_cast<__nv_bfloat16*>(dw));
 }
 
-void launch_rope_qkv(void* qkv, void* q, void* k, void* v, const float* cos_t, const float* sin_t, int B, int S, int H,
+void launch_rope_qkv(void* qkv, HeadMatrix q, HeadMatrix k, HeadMatrix v, const float* cos_t, const float* sin_t, int B, int S, int H,
                      int hd, bool backward, cudaStream_t stream) {
   const size_t total = static_cast<size_t>(B) * S * H * (hd >> 3);
   int grid = static_cast<int>((total + 255) / 256);
   if (grid > 148 * 16) grid = 148 * 16;
   if (grid < 1) grid = 1;
   if (backward)
-    rope_qkv_kernel<true><<<grid, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q),
-                                                    static_cast<__nv_bfloat16*>(k), static_cast<__nv_bfloat16*>(v),
-                                                    cos_t, sin_t, B, S, H, hd);
+    rope_qkv_kernel<true><<<grid, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(qkv), q, k, v, cos_t, sin_t, B, S, H, hd);
   else
-    rope_qkv_kernel<false><<<grid, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q),
-                                                     static_cast<__nv_bfloat16*>(k), static_cast<__nv_bfloat16*>(v),
-                                                     cos_t, sin_t, B, S, H, hd);
+    rope_qkv_kernel<false><<<grid, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(qkv), q, k, v, cos_t, sin_t, B, S, H, hd);
 }
 
 void launch_cross_entropy_fwd(const void* logits, const int64_t* targets, float* loss, float* lse, int rows, int cols,

@@ -14,10 +14,15 @@ void launch_add_rms_norm_fwd(const void* x, const void* delta, const void* w, vo
 int add_rms_norm_bwd_blocks(int rows);
 void launch_add_rms_norm_bwd(const void* dy, const void* ds_in, const void* s, const void* w, const float* rstd,
                              void* ds_out, float* dw_partial, void* dw, int rows, int cols, cudaStream_t stream);
-// Forward: qkv [B,S,3,H,hd] -> q, k rotated, v copied, each contiguous [B,H,S,hd]. Backward: the three gradients in
+// A [B, H, S, hd] tensor of any layout whose heads' rows are contiguous: strides in elements, multiples of 8; 16-byte aligned.
+struct HeadMatrix {
+  void* data;
+  int64_t batch, head, row;
+};
+// Forward: qkv [B,S,3,H,hd] -> q, k rotated, v copied, each [B,H,S,hd]. Backward: the three gradients in
 // [B,H,S,hd] -> d_qkv in the qkv layout (q and k rotated back). cos/sin: [S, hd/2] fp32; hd a multiple of 8.
-void launch_rope_qkv(void* qkv, void* q, void* k, void* v, const float* cos_t, const float* sin_t, int B, int S, int H,
-                     int hd, bool backward, cudaStream_t stream);
+void launch_rope_qkv(void* qkv, HeadMatrix q, HeadMatrix k, HeadMatrix v, const float* cos_t, const float* sin_t, int B,
+                     int S, int H, int hd, bool backward, cudaStream_t stream);
 // bf16 logits [rows, cols] (cols a multiple of 8), int64 targets; per-row loss and log-sum-exp in fp32.
 void launch_cross_entropy_fwd(const void* logits, const int64_t* targets, float* loss, float* lse, int rows, int cols,
                               cudaStream_t stream);

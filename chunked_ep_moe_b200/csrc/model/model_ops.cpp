@@ -25,6 +25,8 @@ bool bf16_matrix(const torch::Tensor& t) {
 
 cudaStream_t stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
+HeadMatrix head_matrix(const torch::Tensor& t) { return {t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)}; }
+
 }  // namespace
 
 std::vector<torch::Tensor> add_rms_norm_fwd(torch::Tensor x, c10::optional<torch::Tensor> delta, torch::Tensor weight,
@@ -76,8 +78,11 @@ std::vector<torch::Tensor> rope_qkv_fwd(torch::Tensor qkv, torch::Tensor cos_t, 
            sin_t.scalar_type() == torch::kFloat32,
        "cos / sin must be contiguous CUDA fp32 [>= S, hd/2] tables");
   const c10::cuda::CUDAGuard guard(qkv.device());
-  torch::Tensor q = torch::empty({B, H, S, hd}, qkv.options()), k = torch::empty_like(q), v = torch::empty_like(q);
-  launch_rope_qkv(qkv.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), cos_t.data_ptr<float>(),
+  // [B, H, S, hd] in the order of [B, S, H, hd]: the attention gives its output in its operands' order, and the projection behind
+  // it then finds its rows without a copy (24 us per layer at 8192 tokens x 1024).
+  auto heads = [&]() { return torch::empty({B, S, H, hd}, qkv.options()).transpose(1, 2); };
+  torch::Tensor q = heads(), k = heads(), v = heads();
+  launch_rope_qkv(qkv.data_ptr(), head_matrix(q), head_matrix(k), head_matrix(v), cos_t.data_ptr<float>(),
                   sin_t.data_ptr<float>(), static_cast<int>(B), static_cast<int>(S), static_cast<int>(H),
                   static_cast<int>(hd), false, stream());
   return {q, k, v};
@@ -85,14 +90,18 @@ std::vector<torch::Tensor> rope_qkv_fwd(torch::Tensor qkv, torch::Tensor cos_t, 
 
 torch::Tensor rope_qkv_bwd(torch::Tensor dq, torch::Tensor dk, torch::Tensor dv, torch::Tensor cos_t,
                            torch::Tensor sin_t) {
-  need(dq.is_cuda() && dq.scalar_type() == torch::kBFloat16 && dq.dim() == 4 && dq.is_contiguous() &&
-           dk.sizes() == dq.sizes() && dv.sizes() == dq.sizes() && dk.is_contiguous() && dv.is_contiguous() &&
-           dk.scalar_type() == torch::kBFloat16 && dv.scalar_type() == torch::kBFloat16,
-       "dq, dk, dv must be contiguous CUDA bf16 [B, H, S, hd] tensors");
+  need(dq.is_cuda() && dq.scalar_type() == torch::kBFloat16 && dq.dim() == 4 && dk.sizes() == dq.sizes() &&
+           dv.sizes() == dq.sizes() && dk.is_cuda() && dv.is_cuda() && dk.scalar_type() == torch::kBFloat16 &&
+           dv.scalar_type() == torch::kBFloat16 && dq.size(3) % 8 == 0,
+       "dq, dk, dv must be CUDA bf16 [B, H, S, hd] tensors, hd % 8 == 0");
   const int64_t B = dq.size(0), H = dq.size(1), S = dq.size(2), hd = dq.size(3);
   const c10::cuda::CUDAGuard guard(dq.device());
   torch::Tensor dqkv = torch::empty({B, S, 3, H, hd}, dq.options());
-  launch_rope_qkv(dqkv.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cos_t.data_ptr<float>(),
+  for (torch::Tensor* t : {&dq, &dk, &dv})  // any layout that the kernel can read 16 bytes at a time
+    if (t->stride(3) != 1 || t->stride(0) % 8 != 0 || t->stride(1) % 8 != 0 || t->stride(2) % 8 != 0 ||
+        reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0)
+      *t = t->clone(at::MemoryFormat::Contiguous);
+  launch_rope_qkv(dqkv.data_ptr(), head_matrix(dq), head_matrix(dk), head_matrix(dv), cos_t.data_ptr<float>(),
                   sin_t.data_ptr<float>(), static_cast<int>(B), static_cast<int>(S), static_cast<int>(H),
                   static_cast<int>(hd), true, stream());
   return dqkv;
@@ -157,6 +166,16 @@ torch::Tensor embedding_bwd(torch::Tensor ids, torch::Tensor grad, int64_t vocab
   launch_embedding_bwd(ids.data_ptr<int64_t>(), grad.data_ptr(), dw.data_ptr(), reinterpret_cast<uint32_t*>(keys.data_ptr()),
                        static_cast<int>(ids.numel()), static_cast<int>(vocab), static_cast<int>(grad.size(1)), stream());
   return dw;
+}
+
+torch::Tensor split_bf16(torch::Tensor x) {
+  need(x.is_cuda() && x.scalar_type() == torch::kFloat32 && x.dim() == 2 && x.is_contiguous() && x.size(1) % 2 == 0 &&
+           reinterpret_cast<uintptr_t>(x.data_ptr()) % 8 == 0,
+       "x must be a contiguous CUDA fp32 matrix with an even number of columns, 8-byte aligned");
+  const c10::cuda::CUDAGuard guard(x.device());
+  torch::Tensor parts = torch::empty({x.size(0), 3 * x.size(1)}, x.options().dtype(torch::kBFloat16));
+  launch_split_bf16(x.data_ptr<float>(), parts.data_ptr(), x.size(0), static_cast<int>(x.size(1)), stream());
+  return parts;
 }
 
 std::vector<torch::Tensor> router_fwd(torch::Tensor logits, torch::Tensor bias, int64_t top_k, double scaling) {

@@ -27,7 +27,7 @@ import torch.nn.functional as F
 
 from ..api import chunked_moe
 from ..config import ChunkedMoEConfig
-from .fused_ops import add_rms_norm, cross_entropy, dense_swiglu, embedding, rope_qkv, router_select
+from .fused_ops import add_rms_norm, cross_entropy, dense_swiglu, embedding, rope_qkv, router_logits, router_select
 
 
 @dataclasses.dataclass
@@ -135,7 +135,7 @@ class Router(nn.Module):
 
     def forward(self, x):
         cfg = self.cfg
-        logits = F.linear(x.float(), self.weight.float())  # [T, E] fp32
+        logits = router_logits(x, self.weight)  # [T, E] fp32
         ids, weights, counts, score_sums = router_select(logits, self.routed_bias, cfg.top_k, cfg.routed_scaling)
         with torch.no_grad():
             self.load_counts += counts

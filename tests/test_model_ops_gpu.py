@@ -180,3 +180,45 @@ def test_embedding_gradient(tokens, vocab, cols):
     count = torch.bincount(ids[0], minlength=vocab)[:, None]
     assert (grads[0].double() - want).abs().le(2.0**-8 * want.abs() + count * 2.0**-23 * size).all()
     assert torch.equal(*grads)
+
+
+@pytest.mark.parametrize("tokens,experts,dim", [(1, 8, 64), (333, 64, 256), (8192, 64, 1024), (257, 32, 520)])
+def test_router_logits(tokens, experts, dim):
+    """The logits are the fp32 GEMM's. Both gradients against 64 bits: one rounding to bf16 (2^-9 of the value, 2^-8 of it allowed) and
+    fp32 sums (2^-20 of the sum of the terms' magnitudes), with gradients of the logits over seven orders of magnitude; and no
+    further from 64 bits than the library's fp32 GEMMs behind the same rounding."""
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, dim, generator=gen, device="cuda").bfloat16().requires_grad_(True)
+    w = (0.05 * torch.randn(experts, dim, generator=gen, device="cuda")).bfloat16().requires_grad_(True)
+    g = torch.randn(tokens, experts, generator=gen, device="cuda") * torch.logspace(-6, 1, experts, device="cuda")
+    logits = fused_ops.router_logits(x, w)
+    logits.backward(g)
+    xf, wf = x.detach().float(), w.detach().float()
+    assert logits.dtype == torch.float32 and torch.equal(logits.detach(), F.linear(xf, wf))
+    xd, wd, gd = xf.double(), wf.double(), g.double()
+    for name, got, want, lib, size in (("dx", x.grad, gd @ wd, g @ wf, gd.abs() @ wd.abs()),
+                                       ("dw", w.grad, gd.T @ xd, g.T @ xf, gd.abs().T @ xd.abs())):
+        err, lib_err = (got.double() - want).abs(), (lib.bfloat16().double() - want).abs()
+        assert err.le(2.0**-8 * want.abs() + 2.0**-20 * size).all(), name
+        assert torch.linalg.vector_norm(err) <= 1.01 * torch.linalg.vector_norm(lib_err), name
+
+
+@pytest.mark.parametrize("layout", ["heads first", "rows first", "odd"])
+def test_rope_gradients_of_any_layout(layout):
+    """Gradients in the attention's [B, H, S, hd] order, in the projection's [B, S, H, hd] order, and with strides that 16-byte
+    accesses cannot take: the same bits."""
+    B, S, H, hd = 2, 33, 3, 64
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    qkv = torch.randn(B, S, 3, H, hd, device="cuda", generator=gen).bfloat16()
+    ang = torch.rand(S, hd // 2, device="cuda", generator=gen)
+    g = [torch.randn(B, H, S, hd, device="cuda", generator=gen).bfloat16() for _ in range(3)]
+    relaid = {"heads first": lambda t: t, "rows first": lambda t: t.transpose(1, 2).contiguous().transpose(1, 2),
+              "odd": lambda t: F.pad(t, (1, 2))[..., 1:-2]}[layout]
+    grads = []
+    for gi in (g, [relaid(t) for t in g]):
+        leaf = qkv.clone().requires_grad_(True)
+        outs = fused_ops.rope_qkv(leaf, ang.cos(), ang.sin())
+        assert all(o.shape == (B, H, S, hd) for o in outs)
+        torch.autograd.backward(outs, gi)
+        grads.append(leaf.grad)
+    assert torch.equal(*grads)
