@@ -24,6 +24,8 @@
 
 #include <cuda_fp8.h>
 
+#include <algorithm>
+
 #include "../common/pdl.cuh"
 #include "../common/umma.cuh"
 
@@ -164,9 +166,8 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
   if (threadIdx.x == 0) s_abort = (p.status != nullptr && p.status->code != 0) ? 1 : 0;
   __syncthreads();
   if (s_abort) return;  // an earlier kernel of this pass already gave up
-  const bool whole = p.last_expert > 0;
   // Buffer reuse: sequence q overwrites what sequence q-2 used on every receiver.
-  if (!whole && p.seq >= 2 && threadIdx.x < p.lay.P) {
+  if (p.seq >= 2 && threadIdx.x < p.lay.P) {
     uint32_t seen = 0;
     if (!spin_until_reached(p.credit + threadIdx.x, p.seq - 1, p.spin_limit, &seen)) {
       report_status(p.status, kStatusCreditTimeout, kKernelPut, 0, static_cast<int>(p.seq), threadIdx.x, p.seq - 1, seen);
@@ -177,12 +178,8 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
   if (s_abort) return;
 
   const int4* put = reinterpret_cast<const int4*>(p.plan + p.lay.off_put + 4 * n_seg * p.slice);
-  int first_chunk = 0, num_chunks = p.plan[p.lay.off_num_chunks + p.slice];
-  if (whole) {
-    first_chunk = put[p.first_expert].w;
-    if (p.last_expert < n_seg) num_chunks = put[p.last_expert].w;
-  }
-  const int buf = whole ? 0 : static_cast<int>(p.seq & 1u);
+  const int num_chunks = p.plan[p.lay.off_num_chunks + p.slice];
+  const int buf = static_cast<int>(p.seq & 1u);
   const int S = p.lay.S, D = p.hidden;
   const int warps_total = gridDim.x * (kPutThreads / 32);
   // Arrival releases are batched: a system-scope fence drains this warp's stores over NVLink, so one fence covers
@@ -196,7 +193,7 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
     if (lane < pending) release_count(pend_ptr, pend_cnt, p.lay.P);
     pending = 0;
   };
-  for (int c = first_chunk + blockIdx.x * (kPutThreads / 32) + warp; c < num_chunks; c += warps_total) {
+  for (int c = blockIdx.x * (kPutThreads / 32) + warp; c < num_chunks; c += warps_total) {
     const int seg = find_segment(put, n_seg, c, lane);
     const int4 e = put[seg];  // {send-order offset, rows, dest row, chunk prefix}
     const int r = seg / p.lay.L, l = seg - r * p.lay.L;
@@ -216,8 +213,7 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
                       static_cast<uint32_t>(token));
         token = -1;
       } else {
-        float* w = whole ? p.whole_w : p.peer_w[r];
-        if (w != nullptr) w[drow + lane] = p.w_flat[flat];
+        p.peer_w[r][drow + lane] = p.w_flat[flat];
       }
     }
     __syncwarp();
@@ -226,8 +222,7 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
       for (int what = 0; what < 2; ++what) {  // (one copy of the loop: it fills the registers)
         const __nv_bfloat16* from = what ? p.g : p.x;
         if (from == nullptr) continue;
-        __nv_bfloat16* to = whole ? (what ? p.whole_g : p.whole_x) : (what ? p.peer_g[r] : p.peer_x[r]);
-        copy_rows(from, to + drow * D, token, rows, D, lane);
+        copy_rows(from, (what ? p.peer_g[r] : p.peer_x[r]) + drow * D, token, rows, D, lane);
       }
     } else {
       for (int rr = 0; rr < rows; ++rr) {
@@ -244,13 +239,11 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
           for (int what = 0; what < 2; ++what) {
             const __nv_bfloat16* from = what ? p.g : p.x;
             if (from == nullptr) continue;
-            __nv_bfloat16* dst = whole ? (what ? p.whole_g : p.whole_x) : (what ? p.peer_g[r] : p.peer_x[r]);
-            put_row_rounded(from + static_cast<size_t>(t) * D, dst + to * D, D, lane);
+            put_row_rounded(from + static_cast<size_t>(t) * D, (what ? p.peer_g[r] : p.peer_x[r]) + to * D, D, lane);
           }
         }
       }
     }
-    if (whole) continue;
     if (lane == pending) {
       pend_ptr = p.peer_arrive[r] + p.me * p.lay.L + l;
       pend_cnt = static_cast<uint32_t>(rows);
@@ -258,6 +251,80 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
     if (++pending == kPendingSignals) flush();
   }
   flush();
+}
+
+// The put of a rank on its own is a plain scatter: its stream is in send order, so `inv_order` says where a token's rows are. A warp
+// takes up to 256 16-byte units of one token's row, all of them in flight together, and stores them to each of the token's rows: x
+// is read (and rounded for the fp8 wire) once a token and range instead of once a copy, and no copy waits for a search of the segments
+// and a send-order entry first, which is what bounded the dispatch put here (1.9 TB/s of stores from 128 blocks). Bound by its stores:
+// 8192 tokens x 6 copies at D=1024 x 34 us (of x alone, 100 MB) and 41 us (x and g; 85 by the dispatch put), 2048 x 8 at D=7168 103 us
+// (x and g, 470 MB; 247), first range of 4096 x 8 rounded tokens at D=7168 33 us (116). Forward + backward at those sizes: 797 -> 732
+// us, 5.64 -> 5.12 ms, 8.70 -> 8.39 ms; 1999 x 4 at D=2048 443 -> 431 us. Beside GEMMs (ranges) it keeps to the dispatch put's 128 blocks.
+constexpr int kWholeAhead = 8;
+
+template <bool ROUND>
+__global__ void __launch_bounds__(kPutThreads, 4) whole_put_kernel(const WholePutParams p) {
+  __shared__ int s_abort;
+  release_successor();
+  wait_predecessor();
+  if (threadIdx.x == 0) s_abort = (p.status != nullptr && p.status->code != 0) ? 1 : 0;
+  __syncthreads();
+  if (s_abort) return;  // an earlier kernel of this pass already gave up
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int all = p.plan[1], L = p.lay.L;
+  const int* expert_start = p.plan + p.lay.off_expert_start;
+  const int begin = p.first_expert > 0 ? expert_start[p.first_expert] : 0;
+  const int end = p.last_expert < L ? expert_start[p.last_expert] : all;
+  const int units = p.hidden >> 3;  // of a row, a multiple of 32
+  const int parts = (units + 32 * kWholeAhead - 1) / (32 * kWholeAhead);
+  const int tasks = p.num_tokens * parts;
+  for (int task = blockIdx.x * (kPutThreads / 32) + warp; task < tasks; task += gridDim.x * (kPutThreads / 32)) {
+    const int t = task / parts, part = task - t * parts;
+    const int u0 = part * 32 * kWholeAhead + lane;
+    for (int k0 = 0; k0 < p.top_k; k0 += 32) {
+      int row = -1;  // of copy k0 + lane
+      if (k0 + lane < p.top_k) {
+        const int flat = t * p.top_k + k0 + lane, at = p.inv_order[flat];
+        // Index check: a row outside the stream is recorded and skipped, never written.
+        if (at < 0 || at >= all) {
+          report_status(p.status, kStatusBadIndex, kKernelPut, 0, 0, flat, static_cast<uint32_t>(all), static_cast<uint32_t>(at));
+        } else if (at >= begin && at < end) {
+          row = at;
+          if (part == 0 && p.rows_w != nullptr) p.rows_w[row] = p.w_flat[flat];
+        }
+      }
+      const unsigned copies = __ballot_sync(0xffffffffu, row >= 0);
+      if (copies == 0) continue;
+#pragma unroll 1
+      for (int what = 0; what < 2; ++what) {
+        const __nv_bfloat16* from = what ? p.g : p.x;
+        if (from == nullptr) continue;
+        const int4* s = reinterpret_cast<const int4*>(from + static_cast<size_t>(t) * p.hidden) + u0;
+        int4* d = reinterpret_cast<int4*>(what ? p.rows_g : p.rows_x) + u0;
+        int4 v[kWholeAhead];
+#pragma unroll
+        for (int i = 0; i < kWholeAhead; ++i)
+          if (u0 + 32 * i < units) v[i] = ld_nc_v4(s + 32 * i);
+        if constexpr (ROUND) {
+#pragma unroll
+          for (int i = 0; i < kWholeAhead; ++i) {
+            if (u0 + 32 * i < units) {  // (the same in all lanes)
+              float scale;
+              const uint2 q = quantise_e4m3(v[i], &scale);
+              v[i] = expand_e4m3(q, scale);
+            }
+          }
+        }
+        for (unsigned left = copies; left != 0; left &= left - 1) {
+          const int r = __shfl_sync(0xffffffffu, row, __ffs(left) - 1);
+          int4* to = d + static_cast<size_t>(r) * units;
+#pragma unroll
+          for (int i = 0; i < kWholeAhead; ++i)
+            if (u0 + 32 * i < units) to[32 * i] = v[i];
+        }
+      }
+    }
+  }
 }
 
 __global__ void slice_done_kernel(uint32_t* const* peer_credit, int num_ranks, int me, uint32_t seq) {
@@ -423,6 +490,13 @@ void launch_dispatch_put(const PutParams& p, int grid, cudaStream_t stream, bool
   if (p.peer_xq != nullptr) launch_maybe_behind(behind, dispatch_put_kernel<kWireFp8>, grid, kPutThreads, 0, stream, p);
   else if (p.round_fp8) launch_maybe_behind(behind, dispatch_put_kernel<kWireRounded>, grid, kPutThreads, 0, stream, p);
   else launch_maybe_behind(behind, dispatch_put_kernel<kWireBf16>, grid, kPutThreads, 0, stream, p);
+}
+
+void launch_whole_put(const WholePutParams& p, int grid, cudaStream_t stream, bool behind) {
+  const int parts = (p.hidden / 8 + 32 * kWholeAhead - 1) / (32 * kWholeAhead);
+  grid = std::max(1, std::min(grid, (p.num_tokens * parts + kPutThreads / 32 - 1) / (kPutThreads / 32)));
+  if (p.round_fp8) launch_maybe_behind(behind, whole_put_kernel<true>, grid, kPutThreads, 0, stream, p);
+  else launch_maybe_behind(behind, whole_put_kernel<false>, grid, kPutThreads, 0, stream, p);
 }
 
 void launch_slice_done(uint32_t* const* peer_credit, int num_ranks, int me, uint32_t seq, cudaStream_t stream) {

@@ -31,12 +31,6 @@ struct PutParams {
   // fp8 wire (comm_dtype=float8_e4m3fn): rows travel as e4m3 + one fp32 scale per 128 columns. A rank on its own has no wire:
   // `round_fp8` stores the values that expansion would yield, as bf16.
   int round_fp8;
-  // A rank on its own that runs a pass as one slice (last > 0): rows of experts [first, last) go to matrices of the whole pass
-  // (those that are not null; x and g likewise), in stream order. No buffer to wait for, and nobody who counts arrivals.
-  int first_expert, last_expert;
-  __nv_bfloat16* whole_x;           // [T*K, D]
-  __nv_bfloat16* whole_g;
-  float* whole_w;                   // [T*K]
   uint8_t* const* peer_xq;          // [P] [2][S][D] e4m3, or null when rows travel in bf16
   uint8_t* const* peer_gq;
   float* const* peer_xs;            // [P] [2][S][D/128] scales
@@ -45,6 +39,26 @@ struct PutParams {
 
 // `behind`: may become resident in its predecessor's tail (see `launch_row_gemm`).
 void launch_dispatch_put(const PutParams& p, int grid, cudaStream_t stream, bool behind = false);
+
+// A rank on its own that runs a pass as one slice: the copies of every token for experts [first, last) go to the matrices of the whole
+// pass, in stream order, which here is the sorted order. No buffer to wait for, and nobody who counts arrivals.
+struct WholePutParams {
+  const int* plan;
+  PlanLayout lay;
+  int first_expert, last_expert;
+  int top_k, hidden, num_tokens;
+  const int* inv_order;       // [T*K] row of each flat assignment t*K+k
+  const float* w_flat;        // [T*K] router weights
+  const __nv_bfloat16* x;     // [T, D], or null
+  const __nv_bfloat16* g;     // [T, D], or null
+  __nv_bfloat16* rows_x;      // [T*K, D]
+  __nv_bfloat16* rows_g;
+  float* rows_w;              // [T*K], or null
+  int round_fp8;              // as in `PutParams`
+  StatusBlock* status;
+};
+
+void launch_whole_put(const WholePutParams& p, int grid, cudaStream_t stream, bool behind = false);
 
 // Tells every sender that this rank has finished reading the slice buffers of sequence `seq`.
 void launch_slice_done(uint32_t* const* peer_credit, int num_ranks, int me, uint32_t seq, cudaStream_t stream);

@@ -22,6 +22,7 @@ namespace cem {
 
 namespace {
 
+constexpr int kPutAloneBlocks = 592;  // of a put that has the device to itself: four blocks on each SM
 constexpr int kExpandSms = 12;  // SMs the up-projection GEMM leaves to the fp8 expansion kernel
 // Pinned words: 16 of the plan header, 8 of the status block and their sequence number (written by the plan kernel), then
 // a second status block for `check_status`.
@@ -956,27 +957,28 @@ void FusedRank::run_parts(int64_t parts, Part&& part) {
   }
 }
 
-void FusedRank::put_whole(const torch::Tensor& plan, const torch::Tensor& order, const torch::Tensor& x, const torch::Tensor* g,
+// `beside`: GEMMs run at the same time.
+void FusedRank::put_whole(const torch::Tensor& plan, const torch::Tensor& inv_order, const torch::Tensor& x, const torch::Tensor* g,
                           const torch::Tensor& w_flat, __nv_bfloat16* to_x, __nv_bfloat16* to_g, float* to_w, int64_t first,
-                          int64_t last, cudaStream_t st, bool behind) {
-  PutParams p{};
+                          int64_t last, cudaStream_t st, bool behind, bool beside) {
+  WholePutParams p{};
   p.plan = plan.data_ptr<int>();
   p.lay = whole_lay_;
-  p.top_k = K_;
-  p.hidden = D_;
-  p.order = order.data_ptr<int>();
-  p.x = to_x != nullptr ? reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()) : nullptr;
-  p.g = to_g != nullptr ? reinterpret_cast<const __nv_bfloat16*>(g->data_ptr()) : nullptr;
-  p.w_flat = w_flat.data_ptr<float>();
-  p.num_tokens = static_cast<int>(x.size(0));
-  p.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
-  p.round_fp8 = fp8_;
   p.first_expert = static_cast<int>(first);
   p.last_expert = static_cast<int>(last);
-  p.whole_x = to_x;
-  p.whole_g = to_g;
-  p.whole_w = to_w;
-  launch_dispatch_put(p, put_blocks_, st, behind);
+  p.top_k = K_;
+  p.hidden = D_;
+  p.num_tokens = static_cast<int>(x.size(0));
+  p.inv_order = inv_order.data_ptr<int>();
+  p.w_flat = w_flat.data_ptr<float>();
+  p.x = to_x != nullptr ? reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()) : nullptr;
+  p.g = to_g != nullptr ? reinterpret_cast<const __nv_bfloat16*>(g->data_ptr()) : nullptr;
+  p.rows_x = to_x;
+  p.rows_g = to_g;
+  p.rows_w = to_w;
+  p.round_fp8 = fp8_;
+  p.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
+  launch_whole_put(p, beside ? put_blocks_ : kPutAloneBlocks, st, behind);
   ++launches_;
 }
 
@@ -1021,8 +1023,8 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_whol
   const TokenMaps x_map = make_token_maps(rows_x.data_ptr(), tk, D_), act_map = make_token_maps(act.data_ptr(), tk, F_);
   run_parts(parts, [&](int64_t first, int64_t last, cudaStream_t put_stream, cudaStream_t gemm_stream) {
     NvtxRange range("chunked_moe/fwd experts from", first);
-    put_whole(plan, order, x, nullptr, w_flat, reinterpret_cast<__nv_bfloat16*>(rows_x.data_ptr()), nullptr,
-              rows_w.data_ptr<float>(), first, last, put_stream, inline_);
+    put_whole(plan, inv_order, x, nullptr, w_flat, reinterpret_cast<__nv_bfloat16*>(rows_x.data_ptr()), nullptr,
+              rows_w.data_ptr<float>(), first, last, put_stream, inline_, first > 0);
     if (put_stream != gemm_stream) {
       cuda_check(cudaEventRecord(ev_put_[0], put_stream), "event record");
       cuda_check(cudaStreamWaitEvent(gemm_stream, ev_put_[0], 0), "wait put event");
@@ -1060,11 +1062,11 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_whol
 
 // `buffers`: x by rows, g by rows, router weights by rows, dh, d_weight shares and, where nothing was kept, h and w * act.
 void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up,
-                               torch::Tensor w_down, torch::Tensor plan, torch::Tensor order,
+                               torch::Tensor w_down, torch::Tensor plan, torch::Tensor inv_order,
                                const std::vector<torch::Tensor>& kept, const std::vector<torch::Tensor>& buffers,
                                torch::Tensor dw_up, torch::Tensor dw_down) {
   cudaStream_t st = current_stream();
-  const int64_t tk = order.numel();
+  const int64_t tk = inv_order.numel();
   expect_i32(plan, whole_lay_.total, "plan");
   expect_bf16_2d(x, D_, "x");
   expect_bf16_2d(g, D_, "g");
@@ -1090,14 +1092,14 @@ void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w
   const bool x_later = keep && parts > 1;
   run_parts(parts, [&](int64_t first, int64_t last, cudaStream_t put_stream, cudaStream_t gemm_stream) {
     NvtxRange range("chunked_moe/bwd experts from", first);
-    put_whole(plan, order, x, &g, w_flat, x_later ? nullptr : bf16(rows_x), bf16(rows_g), rows_w.data_ptr<float>(), first, last,
-              put_stream, false);
+    put_whole(plan, inv_order, x, &g, w_flat, x_later ? nullptr : bf16(rows_x), bf16(rows_g), rows_w.data_ptr<float>(), first, last,
+              put_stream, false, first > 0);
     if (put_stream != gemm_stream) {
       cuda_check(cudaEventRecord(ev_put_[0], put_stream), "event record");
       cuda_check(cudaStreamWaitEvent(gemm_stream, ev_put_[0], 0), "wait put event");
     }
     if (x_later) {
-      put_whole(plan, order, x, nullptr, w_flat, bf16(rows_x), nullptr, nullptr, first, last, put_stream, false);
+      put_whole(plan, inv_order, x, nullptr, w_flat, bf16(rows_x), nullptr, nullptr, first, last, put_stream, false, true);
       cuda_check(cudaEventRecord(ev_put_[1], put_stream), "event record");
     }
     if (!keep) {
@@ -1293,7 +1295,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
   }
   const QuiesceOnError guard{this};
   if (!buffers.empty()) {
-    backward_whole(x, g, w_flat, w_up, w_down, plan, order, kept, buffers, dw_up, dw_down);
+    backward_whole(x, g, w_flat, w_up, w_down, plan, inv_order, kept, buffers, dw_up, dw_down);
     finish_backward(inv_order, dx, d_weights);
     return std::make_tuple(dx, d_weights, dw_up, dw_down);
   }

@@ -202,11 +202,11 @@ class FusedRank {
       torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
       const std::vector<torch::Tensor>& kept, const std::vector<torch::Tensor>& buffers, bool training);
   void backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
-                      torch::Tensor plan, torch::Tensor order, const std::vector<torch::Tensor>& kept,
+                      torch::Tensor plan, torch::Tensor inv_order, const std::vector<torch::Tensor>& kept,
                       const std::vector<torch::Tensor>& buffers, torch::Tensor dw_up, torch::Tensor dw_down);
-  void put_whole(const torch::Tensor& plan, const torch::Tensor& order, const torch::Tensor& x, const torch::Tensor* g,
+  void put_whole(const torch::Tensor& plan, const torch::Tensor& inv_order, const torch::Tensor& x, const torch::Tensor* g,
                  const torch::Tensor& w_flat, __nv_bfloat16* to_x, __nv_bfloat16* to_g, float* to_w, int64_t first, int64_t last,
-                 cudaStream_t st, bool behind);
+                 cudaStream_t st, bool behind, bool beside);
   bool overlapped() const { return use_comm_stream_ && !inline_; }
   void join_streams(bool backward);
   GemmParams base_params(const int* plan, int j) const;
