@@ -353,6 +353,8 @@ __global__ void pass_begin_kernel(const int* plan, PlanLayout lay, uint32_t* exp
 // segments of that expert. (The up-projection gradient's GEMM follows on the same stream; this is a few us beside the
 // chain's GEMMs, where summing inside the dX epilogue kept one column tile's warps busy with strided reads.)
 __global__ void __launch_bounds__(256) return_dw_kernel(const ReturnDwParams p) {
+  release_successor();
+  wait_predecessor();
   if (p.status != nullptr && p.status->code != 0) return;  // an earlier kernel of this pass already gave up
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * blockDim.x + threadIdx.x, at = p.slice * p.lay.S + row;  // slice row, stream row
@@ -508,8 +510,8 @@ void launch_pass_begin(const int* plan, PlanLayout lay, uint32_t* expected_total
   launch_behind(pass_begin_kernel, 1, 256, 0, stream, plan, lay, expected_total, pass_base, ready_total, ready_base);
 }
 
-void launch_return_dw(const ReturnDwParams& p, cudaStream_t stream) {
-  return_dw_kernel<<<(p.lay.S + 255) / 256, 256, 0, stream>>>(p);
+void launch_return_dw(const ReturnDwParams& p, cudaStream_t stream, bool behind) {
+  launch_maybe_behind(behind, return_dw_kernel, (p.lay.S + 255) / 256, 256, 0, stream, p);
 }
 
 void launch_combine_reduce(const CombineParams& p, cudaStream_t stream, bool behind) {

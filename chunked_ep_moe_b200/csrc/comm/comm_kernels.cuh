@@ -83,7 +83,7 @@ struct ReturnDwParams {
   StatusBlock* status;
 };
 
-void launch_return_dw(const ReturnDwParams& p, cudaStream_t stream);
+void launch_return_dw(const ReturnDwParams& p, cudaStream_t stream, bool behind = false);
 
 struct CombineParams {
   const __nv_bfloat16* rows;  // [T*K, D] returned rows in send order

@@ -101,14 +101,16 @@ struct alignas(64) TokenMaps {
 // its predecessor's tail (programmatic dependent launch). Only where nothing else wants the SMs meanwhile: a waiting CTA holds
 // one, which two slices in flight would miss, and which a kernel that the PREDECESSOR waits for (the expansion of the fp8
 // wire, a put to this rank) may need. So: one rank, one stream (one-slice forwards: one token 46.3 -> 43.1 us, 64 tokens at
-// D=7168 497 -> 487 us, 2000 tokens at D=2048 153 -> 147 us; a kernel-level forward + backward gained nothing, 248 against 251).
+// D=7168 497 -> 487 us, 2000 tokens at D=2048 153 -> 147 us; a kernel-level forward + backward gained nothing, 248 against 251 and, with
+// the weight gradients too, 251 against 254). And in one-range backwards, on the caller's stream and the auxiliary one, whose kernels
+// wait for nothing that comes behind them: see `FusedRank::backward_whole`.
 void launch_row_gemm(int mode, const GemmParams& p, const CUtensorMap& map_a, const TokenMaps& maps_b, int grid,
                      cudaStream_t stream, bool behind = false);
 
 // Weight gradients (kModeTgmm). `map_a`, `map_b`: chunked descriptions with boxes of 64 rows x 2 chunks; `map_c`: the bf16
 // gradient [L*M, N] with boxes of 32 rows x 64 columns (tiled stores).
 void launch_weight_grad(const GemmParams& p, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                        const CUtensorMap& map_c, int grid, cudaStream_t stream);
+                        const CUtensorMap& map_c, int grid, cudaStream_t stream, bool behind = false);
 
 int row_gemm_smem_bytes();    // dynamic shared memory of a row-wise GEMM CTA
 extern int g_pair_grid_used;  // grid of the last GEMM launch, for diagnostics

@@ -13,6 +13,7 @@
 //
 // The pair splits the dense feature dimension, so it costs no token padding. Every wait is bounded; a CTA that gives up
 // records a status and unwinds, and its partner then runs into its own limits.
+#include "../common/pdl.cuh"
 #include "gemm_common.cuh"
 
 namespace cem {
@@ -215,14 +216,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmParams p, const __grid_cons
                                         smem_base - smem_u32(smem_raw));
     return;
   }
-  // An earlier kernel of this pass already gave up: both CTAs of the pair leave together (the leader decides).
-  if (threadIdx.x == 0 && leader) {
-    const uint32_t v = (p.status != nullptr && p.status->code != 0) ? 1u : 0u;
-    *early_flag = static_cast<int>(v);
-    st_shared_cluster_u32(map_to_cta(bar_base + kSlotOff + 8, 1), v);
-  }
-  cluster_sync_all();
-  if (*early_flag) return;
+  release_successor();
+  cluster_sync_all();  // both CTAs run
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPairStages; ++s) {
@@ -245,13 +240,22 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmParams p, const __grid_cons
     tmem_alloc_pair(tmem_slot, 512);
     tmem_relinquish_pair();
   }
+  // Launched behind its predecessor, the kernel has come this far in that one's tail; global memory from here on.
+  wait_predecessor();
+  // An earlier kernel of this pass already gave up: neither CTA of the pair does anything (the leader decides).
+  if (threadIdx.x == 0 && leader) {
+    const uint32_t v = (p.status != nullptr && p.status->code != 0) ? 1u : 0u;
+    *early_flag = static_cast<int>(v);
+    st_shared_cluster_u32(map_to_cta(bar_base + kSlotOff + 8, 1), v);
+  }
   tcgen05_fence_before_sync();
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers exist before anyone signals across the pair
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot_gen;
 
-  const int groups = p.last_expert > 0 ? p.last_expert - p.first_expert : p.plan[p.lay.off_num_gtiles + p.slice];
+  int groups = 0;
+  if (*early_flag == 0) groups = p.last_expert > 0 ? p.last_expert - p.first_expert : p.plan[p.lay.off_num_gtiles + p.slice];
   const int num_tiles = groups * (p.m_tiles / 2) * p.n_tiles;
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
 
@@ -481,12 +485,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmParams p, const __grid_cons
 int g_pair_grid_used = 0;  // last pair grid size, for diagnostics
 
 void launch_weight_grad(const GemmParams& p, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                        const CUtensorMap& map_c, int grid, cudaStream_t stream) {
+                        const CUtensorMap& map_c, int grid, cudaStream_t stream, bool behind) {
   static const int resident = resident_pair_grid(grouped_gemm_pair_kernel, kPairThreads, kPairSmemBytes);
   grid &= ~1;  // whole pairs only
   const int g = grid < resident ? grid : resident;
   g_pair_grid_used = g;
-  grouped_gemm_pair_kernel<<<g, kPairThreads, kPairSmemBytes, stream>>>(p, map_a, map_b, map_c);
+  launch_maybe_behind(behind, grouped_gemm_pair_kernel, g, kPairThreads, kPairSmemBytes, stream, p, map_a, map_b, map_c);
 }
 
 }  // namespace cem

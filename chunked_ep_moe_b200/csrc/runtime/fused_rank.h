@@ -118,7 +118,9 @@ class FusedRank {
   // `act` [rows, F]. Lasts until the pass is finished.
   void keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices);
   void finish_forward(torch::Tensor inv_order, torch::Tensor out);
-  void finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights);
+  void finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights) {
+    reduce_backward(inv_order, dx, d_weights, nullptr);
+  }
 
   // The two passes as one call each (what `chunked_moe` runs). Forward: ([out, plan, order, inv_order] and, when a
   // `training` pass keeps them, [h, w * act]; slice count; slices kept); it throws a recorded kernel error. Nothing is kept
@@ -160,6 +162,8 @@ class FusedRank {
   void begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row,
                   bool targets_set = false);
   void enter_pass();
+  // `after`: an event that the caller's stream waits for behind the pass's last kernel, or null.
+  void reduce_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights, cudaEvent_t after);
   void end_pass(int64_t n_slices);
   void wait_header();
   void quiesce() const;
