@@ -116,6 +116,14 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// Asynchronous 16-byte copy global -> this CTA's shared memory by the thread itself (past L1; both addresses 16-byte aligned).
+__device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
+}
+
+// Waits until all of this thread's copies have landed.
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 
 // Waits until this thread's committed bulk stores have READ their shared-memory source (it may be overwritten), but for the
@@ -397,6 +405,49 @@ __device__ __forceinline__ int4 ld_nc_v4(const void* p) {
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
+}
+
+// Two fp32 values in one register pair: Blackwell's FMUL2 / FADD2 / FFMA2, rounded like the scalar instructions.
+struct f32x2 {
+  unsigned long long v;
+};
+
+__device__ __forceinline__ f32x2 make_f32x2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+
+__device__ __forceinline__ void split_f32x2(f32x2 x, float* a, float* b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(x.v));
+}
+
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+__device__ __forceinline__ f32x2 bf16x2_to_f32x2(uint32_t v) {
+  return make_f32x2(__uint_as_float(v << 16), __uint_as_float(v & 0xFFFF0000u));
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(f32x2 x) {
+  float a, b;
+  split_f32x2(x, &a, &b);
+  return pack_bf16(a, b);
 }
 
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }

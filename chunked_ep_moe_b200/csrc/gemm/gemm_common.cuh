@@ -61,11 +61,29 @@ __device__ __forceinline__ bool wait_expert_rows(const GemmParams& p, int mode, 
   return ok;
 }
 
-// Sigmoid with the approximate divide (`__fdividef`: a reciprocal and a multiply, 2 ulp). The IEEE division the plain
-// `/` compiles to is a subroutine of a dozen instructions, and in the SwiGLU epilogues it was most of the work per
-// element; the results are rounded to bf16 right after, which has 16 bits less precision than the error made here.
-__device__ __forceinline__ float sigmoid_f(float g) { return __fdividef(1.0f, 1.0f + __expf(-g)); }
+// Sigmoid from the approximate exponential and reciprocal (2 ulp). The IEEE division the plain `/` compiles to is a subroutine of a
+// dozen instructions, and in the SwiGLU epilogues it was most of the work per element; the results are rounded to bf16 right after,
+// which has 16 bits less precision than the error made here. The forms that flush subnormals: neither 1 + 2^-127 nor the reciprocal
+// of 2^127 differs by them in a sigmoid that is rounded to bf16, and the others cost eight more instructions an element.
+constexpr float kMinusLog2e = -1.4426950408889634f;
+__device__ __forceinline__ float exp2_approx(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float reciprocal_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sigmoid_f(float g) { return reciprocal_approx(1.0f + exp2_approx(g * kMinusLog2e)); }
 __device__ __forceinline__ float silu_f(float g) { return g * sigmoid_f(g); }
+__device__ __forceinline__ f32x2 sigmoid_f(f32x2 g) {
+  float a, b;
+  split_f32x2(mul2(g, make_f32x2(kMinusLog2e, kMinusLog2e)), &a, &b);
+  split_f32x2(add2(make_f32x2(1.0f, 1.0f), make_f32x2(exp2_approx(a), exp2_approx(b))), &a, &b);
+  return make_f32x2(reciprocal_approx(a), reciprocal_approx(b));
+}
 
 
 // Largest persistent grid whose clusters of two are all resident at once (sets the kernel's shared-memory limit first). A

@@ -33,14 +33,17 @@ namespace cem {
 
 namespace {
 
-constexpr int kRowStages = 6;
+// Stages of the operand ring. SwiGLU' gives one up for two buffers of h for each epilogue warp.
+template <int MODE>
+constexpr int kRowStagesOf = MODE == kModeDswiglu ? 5 : 6;
 constexpr int kRowStageBytesA = kBlockM * kBlockK * 2;  // this CTA's 128 weight columns
 constexpr int kRowStageBytesB = (kTileTokens / 2) * kBlockK * 2;  // up to 128 rows
 constexpr int kRowStageBytes = kRowStageBytesA + kRowStageBytesB;
 constexpr int kRowBand = 4;                             // token tiles swept together over the weight columns
 constexpr int kRowThreads = 64 + 8 * 32;
 constexpr int kGroupStaging = 16384;                    // per epilogue group
-constexpr int kRowSmemBytes = kSmemAlignSlack + kRowStages * kRowStageBytes + 2 * kGroupStaging + kSmemTailBytes;
+constexpr int kRowSmemBytes = kSmemAlignSlack + 6 * kRowStageBytes + 2 * kGroupStaging + kSmemTailBytes;
+static_assert(5 * kRowStageBytes + 8 * 8192 <= 6 * kRowStageBytes + 2 * kGroupStaging, "SwiGLU' has no room for its buffers");
 static_assert(kRowSmemBytes + 1024 + 1024 + 16 <= 233472, "no room for a second, small CTA on the SM");
 
 struct RowTile {
@@ -146,7 +149,7 @@ __device__ __forceinline__ void flush_rows(uint32_t buf, int gt, uint8_t* out, s
 
 struct GroupCtx {
   int h, q, lane, gt, rank;
-  uint32_t staging;  // this group's staging buffer
+  uint32_t staging;  // this group's staging buffer (SwiGLU': this warp's)
 };
 
 template <typename Release>
@@ -291,169 +294,175 @@ __device__ __forceinline__ void combine_epilogue(const GemmParams& p, const RowT
   if (c.h >= chunks) release();
 }
 
-// SwiGLU': 128 columns of d_act and the 256 striped columns of h / dh that belong to them (512 bytes of a row). The
-// group brings a chunk of h into its staging buffer (the next chunk's loads are in flight meanwhile), every warp turns
-// its own gate and up columns into gradients in place, the group writes the chunk out as dh.
+// SwiGLU': 128 columns of d_act and the 256 striped columns of h / dh that belong to them. A warp's 32 columns of d_act need 32 gate
+// and 32 up columns of h and nothing of what the other warps have, so every warp brings its own two 64-byte pieces of a chunk's
+// rows into its own staging, turns gate and up into gradients in place and writes them out as dh: no group barrier anywhere, and two
+// elements an instruction (f32x2). With short contractions this epilogue is what bounds the GEMM: 1029 cycles per k-block at D=1024, F=512
+// (16 k-blocks a tile), where the group moving whole 512-byte rows through six barriers a chunk, an element at a time, took 1363
+// (75,000 instructions a scheduler and launch, now 44,000). Forward + backward, with the launches of one-range backwards: 8192 x 6
+// rows there 698 -> 667 us, 1999 x 4 at D=2048 411 -> 393 us, the expert kernels on 4001 rows 250 -> 246.5 us.
 //
 // d_weight = <acc, act> is summed against the stored w * act and divided by w where the shares are added up
 // (`weight_divides`): one rounding of act away from exact. Against the act that h gives, two rounded factors, it is 8 % further
 // from 64 bits than a GEMM on the rounded act is (0.00253 against 0.00235 at D=7168, F=2048; this way 0.00167). A chunk of
-// w * act passes through the buffer that h goes into next, at two more group barriers.
+// w * act passes through the buffer that the next chunk's h goes into.
 //
-// Nothing of this depends on the accumulator: the first chunk is staged while the tile's MMAs run. (The router weights are not
-// asked for before the accumulator is there: in a backward that starts with this GEMM they arrive with the rows it waits for.)
-struct DswigluLoads {
-  int4 h[8];    // this thread's 16-byte pieces of the chunk's 512-byte rows of h
-  int4 act[4];  // and of the 256-byte rows of w * act
+// What a chunk needs is asked for a whole chunk earlier, across tiles: h by asynchronous copies into the one of the warp's two buffers that
+// the chunk before is not in, w * act and the router weight into registers. (Asked for half a chunk ahead and the weight when
+// needed, a chunk took 5000 cycles, most of them waiting for L2 in turn; now 3700.)
+struct DswigluNext {
+  int4 act[4];  // row 8 i + lane / 4: a 16-byte piece of the 64 bytes of w * act
+  float w;      // router weight of row `lane`
 };
 
-// A chunk's loads; rows past the tile keep what the registers hold.
-__device__ __forceinline__ void load_dswiglu(const GemmParams& p, const RowTile& tl, const GroupCtx& c, int ch, DswigluLoads* v) {
-  const int row0 = tl.row0 + ch * 32, nvalid = tl.nrows - ch * 32, col = tl.n * kBlockN + c.rank * kBlockM;
-  const uint8_t* h = reinterpret_cast<const uint8_t*>(p.in0 + static_cast<size_t>(row0) * p.ld0 + 2 * col) + c.lane * 16;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int row = c.q + 4 * i;
-    if (row < nvalid) v->h[i] = *reinterpret_cast<const int4*>(h + static_cast<size_t>(row) * p.ld0 * 2);
-  }
-  if (p.dwp != nullptr) {
-    const __nv_bfloat16* act = p.in1 + static_cast<size_t>(row0) * p.ld1 + col + (c.gt & 15) * 8;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = (c.gt >> 4) + 8 * i;
-      if (row < nvalid) v->act[i] = *reinterpret_cast<const int4*>(act + static_cast<size_t>(row) * p.ld1);
-    }
-  }
+// First of the warp's 32 gate columns among the CTA's 256 striped ones; the up columns are `stripe` further.
+__device__ __forceinline__ int gate_column(const GemmParams& p, int q) { return 2 * p.stripe * (q * 32 / p.stripe) + q * 32 % p.stripe; }
+
+// A chunk: its first row, how many of its 32 rows there are (none: no chunk) and its column tile.
+struct Chunk {
+  int row0, rows, n;
+};
+
+__device__ __forceinline__ Chunk chunk_of(const RowTile& tl, int ch) { return {tl.row0 + ch * 32, tl.nrows - ch * 32, tl.n}; }
+
+// This lane's 16-byte piece of the warp's columns of h and dh.
+__device__ __forceinline__ int dswiglu_column(const GemmParams& p, int n, const GroupCtx& c) {
+  return 2 * (n * kBlockN + c.rank * kBlockM) + gate_column(p, c.q) + (c.lane & 4 ? p.stripe : 0) + (c.lane & 3) * 8;
 }
 
-// Loaded pieces of a chunk -> h in the group's buffer, w * act in the accumulator's fragment layout (m[j][s]: columns
-// 8 s + lane / 4, rows 8 j + 2 (lane & 3) + e).
-__device__ __forceinline__ void stage_dswiglu(const GemmParams& p, const GroupCtx& c, const DswigluLoads& v, uint32_t (&m)[4][4]) {
-  group_sync(c.h);  // the previous chunk has left the buffer
-  if (p.dwp != nullptr) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      st_shared_v4(staged<256>(c.staging, (c.gt >> 4) + 8 * i, c.gt & 15), v.act[i].x, v.act[i].y, v.act[i].z, v.act[i].w);
-    group_sync(c.h);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) ldmatrix_x4_trans(staged<256>(c.staging, 8 * j + (c.lane & 7), c.q * 4 + (c.lane >> 3)), m[j]);
-    group_sync(c.h);  // every warp has read it: h goes over it
-  }
+// 16-byte piece `piece` of row `row` in the warp's staging: h (128 bytes a row) and w * act (64 bytes, two rows side by side).
+__device__ __forceinline__ uint32_t staged_h(uint32_t buf, int row, int piece) { return buf + row * 128 + ((piece ^ (row & 7)) << 4); }
+__device__ __forceinline__ uint32_t staged_act(uint32_t buf, int row, int piece) {
+  return buf + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4);
+}
+
+// Router weight of row `lane` of a chunk (read past L1: the line may also hold weights of rows that had not arrived when another tile
+// read it).
+__device__ __forceinline__ float dswiglu_weight(const GemmParams& p, const GroupCtx& c, const Chunk& at) {
+  return p.row_w != nullptr && c.lane < at.rows ? __ldcg(p.row_w + at.row0 + c.lane) : 1.0f;
+}
+
+// This lane's 16-byte piece of the chunk's row lane / 8.
+__device__ __forceinline__ size_t dswiglu_offset(const GemmParams& p, const GroupCtx& c, const Chunk& at) {
+  return static_cast<size_t>(at.row0 + (c.lane >> 3)) * p.ld0 + dswiglu_column(p, at.n, c);
+}
+
+// Asks for a chunk: its h, w * act and weights. Rows past the tile keep what is there: they are worked on and thrown away.
+__device__ __forceinline__ void fetch_dswiglu(const GemmParams& p, const GroupCtx& c, const Chunk& at, uint32_t buf, bool weights,
+                                              DswigluNext* v) {
+  const __nv_bfloat16* h = p.in0 + dswiglu_offset(p, c, at);
 #pragma unroll
   for (int i = 0; i < 8; ++i)
-    st_shared_v4(staged<512>(c.staging, c.q + 4 * i, c.lane), v.h[i].x, v.h[i].y, v.h[i].z, v.h[i].w);
-  group_sync(c.h);
+    if ((c.lane >> 3) + 4 * i < at.rows) cp_async_16(staged_h(buf, (c.lane >> 3) + 4 * i, c.lane & 7), h + static_cast<size_t>(4 * i) * p.ld0);
+  if (p.dwp != nullptr) {
+    const __nv_bfloat16* act =
+        p.in1 + static_cast<size_t>(at.row0 + (c.lane >> 2)) * p.ld1 + at.n * kBlockN + c.rank * kBlockM + c.q * 32 + (c.lane & 3) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if ((c.lane >> 2) + 8 * i < at.rows) v->act[i] = *reinterpret_cast<const int4*>(act + static_cast<size_t>(8 * i) * p.ld1);
+  }
+  if (weights) v->w = dswiglu_weight(p, c, at);
 }
 
-// `v`, `m`: the first chunk's, staged.
-template <typename Release>
-__device__ __forceinline__ void dswiglu_epilogue(const GemmParams& p, const RowTile& tl, uint32_t tacc,
-                                                 const GroupCtx& c, DswigluLoads& v, uint32_t (&m)[4][4],
-                                                 Release&& release) {
-  const int chunks = (tl.nrows + 31) >> 5;
-  const int col = 2 * (tl.n * kBlockN + c.rank * kBlockM);  // first striped column
-  const int f = c.q * 32 + (c.lane >> 3) * 8;               // column (of 128) whose 16-byte piece this lane addresses
-  const int gpiece = (2 * p.stripe * (f / p.stripe) + f % p.stripe) >> 3, upiece = gpiece + (p.stripe >> 3);
-  const size_t ld_bytes = static_cast<size_t>(p.ld0) * 2;
-  for (int ch = c.h; ch < chunks; ch += 2) {
-    const int row0 = tl.row0 + ch * 32, nvalid = tl.nrows - ch * 32;
-    float w[8];  // this thread's rows' router weights (past L1 and ahead of time, as in the up-projection)
+// w * act of the chunk at hand from `v` into the accumulator's fragment layout (m[j][s]: columns 8 s + lane / 4, rows
+// 8 j + 2 (lane & 3) + e), by way of a buffer that is free.
+__device__ __forceinline__ void turn_act(const GroupCtx& c, uint32_t buf, const DswigluNext& v, uint32_t (&m)[4][4]) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int t = 8 * (i >> 1) + 2 * (c.lane & 3) + (i & 1);
-      w[i] = p.row_w != nullptr && t < nvalid ? __ldcg(p.row_w + row0 + t) : 1.0f;
+  for (int i = 0; i < 4; ++i)
+    st_shared_v4(staged_act(buf, (c.lane >> 2) + 8 * i, c.lane & 3), v.act[i].x, v.act[i].y, v.act[i].z, v.act[i].w);
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) ldmatrix_x4_trans(staged_act(buf, 8 * j + (c.lane & 7), c.lane >> 3), m[j]);
+  __syncwarp();  // every lane has read it: the next chunk's h goes over it
+}
+
+// A chunk's d_weight shares. `r`: the accumulator; `m`: w * act (in fragments); `odd`: rows whose weight is nothing to divide by, their
+// sum is <acc, act> with act from h in `buf` (`h_landed` waits for it).
+template <typename Landed>
+__device__ __forceinline__ void dswiglu_shares(const GemmParams& p, const uint32_t (&r)[32], const GroupCtx& c, const Chunk& at,
+                                               uint32_t buf, const uint32_t (&m)[4][4], uint32_t odd, Landed&& h_landed) {
+  float part[8];  // <acc, w * act> over this thread's columns, rows 8 j + 2 (lane & 3) + e
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    f32x2 sum = make_f32x2(0.0f, 0.0f);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
+      sum = fma2(make_f32x2(__uint_as_float(r[b]), __uint_as_float(r[b + 1])), bf16x2_to_f32x2(m[j][s]), sum);
     }
-    if (ch != c.h) stage_dswiglu(p, c, v, m);
-    uint32_t r[32];
-    load_fragment(tacc + ch * 32, r);
-    if (ch + 2 >= chunks) release();
-    float part[8];      // <acc, w * act> over this thread's columns, rows 8 j + 2 (lane & 3) + e
-    if (p.dwp != nullptr) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        part[2 * j] = part[2 * j + 1] = 0.0f;
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
-          part[2 * j] += __uint_as_float(r[b]) * bf16_lo(m[j][s]);
-          part[2 * j + 1] += __uint_as_float(r[b + 1]) * bf16_hi(m[j][s]);
-        }
-      }
-      uint32_t odd = 0;  // bit 2 j + e: the row's weight is nothing to divide by, its sum is <acc, act> with act from h
-#pragma unroll
-      for (int i = 0; i < 8; ++i) odd |= weight_divides(w[i]) ? 0u : 1u << i;
-      if (__any_sync(0xffffffffu, odd != 0)) {  // (rare: not in the loop below)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t g[4], u[4];
-          ldmatrix_x4_trans(staged<512>(c.staging, 8 * j + (c.lane & 7), gpiece), g);
-          ldmatrix_x4_trans(staged<512>(c.staging, 8 * j + (c.lane & 7), upiece), u);
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            float sum = 0.0f;
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-              sum += __uint_as_float(r[(s >> 1) * 16 + j * 4 + (s & 1) * 2 + e]) *
-                     (silu_f(e ? bf16_hi(g[s]) : bf16_lo(g[s])) * (e ? bf16_hi(u[s]) : bf16_lo(u[s])));
-            if ((odd >> (2 * j + e)) & 1u) part[2 * j + e] = sum;
-          }
-        }
-        __syncwarp();
-      }
-    }
-    if (ch + 2 < chunks) load_dswiglu(p, tl, c, ch + 2, &v);
+    split_f32x2(sum, &part[2 * j], &part[2 * j + 1]);
+  }
+  if (odd != 0) {  // (rare)
+    h_landed();
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const uint32_t ga = staged<512>(c.staging, 8 * j + (c.lane & 7), gpiece);
-      const uint32_t ua = staged<512>(c.staging, 8 * j + (c.lane & 7), upiece);
       uint32_t g[4], u[4];
-      ldmatrix_x4_trans(ga, g);
-      ldmatrix_x4_trans(ua, u);
+      ldmatrix_x4_trans(staged_h(buf, 8 * j + (c.lane & 7), c.lane >> 3), g);
+      ldmatrix_x4_trans(staged_h(buf, 8 * j + (c.lane & 7), 4 + (c.lane >> 3)), u);
 #pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
-        const float a[2] = {__uint_as_float(r[b]), __uint_as_float(r[b + 1])};
-        // d_act is rounded to bf16 first, as the unfused reference stores it.
-        const uint32_t db = pack_bf16(w[2 * j] * a[0], w[2 * j + 1] * a[1]);
-        float dg[2], du[2];
+      for (int e = 0; e < 2; ++e) {
+        float sum = 0.0f;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float d = e ? bf16_hi(db) : bf16_lo(db);
-          const float gt = e ? bf16_hi(g[s]) : bf16_lo(g[s]);
-          const float up = e ? bf16_hi(u[s]) : bf16_lo(u[s]);
-          const float sig = sigmoid_f(gt);
-          const float sl = gt * sig;
-          dg[e] = d * up * (sig + sl * (1.0f - sig));
-          du[e] = d * sl;
-        }
-        g[s] = pack_bf16(dg[0], dg[1]);
-        u[s] = pack_bf16(du[0], du[1]);
-      }
-      __syncwarp();  // all lanes' ldmatrix reads of these rows are done (they cross lanes) before the rows are overwritten
-      stmatrix_x4_trans(ga, g);
-      stmatrix_x4_trans(ua, u);
-    }
-    if (p.dwp != nullptr) {
-      // Sum over the 8 lanes that hold the same rows, then one partial per (row, 32 columns).
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-#pragma unroll
-        for (int o = 4; o <= 16; o <<= 1) part[k] += __shfl_xor_sync(0xffffffffu, part[k], o);
-      }
-      if (c.lane < 4) {
-        float* out = p.dwp + static_cast<size_t>(row0) * p.dwp_tiles + (tl.n * 2 + c.rank) * 4 + c.q;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int t = 8 * (k >> 1) + 2 * c.lane + (k & 1);
-          if (t < nvalid) out[static_cast<size_t>(t) * p.dwp_tiles] = part[k];
-        }
+        for (int s = 0; s < 4; ++s)
+          sum += __uint_as_float(r[(s >> 1) * 16 + j * 4 + (s & 1) * 2 + e]) *
+                 (silu_f(e ? bf16_hi(g[s]) : bf16_lo(g[s])) * (e ? bf16_hi(u[s]) : bf16_lo(u[s])));
+        if ((odd >> (8 * j + 2 * (c.lane & 3) + e)) & 1u) part[2 * j + e] = sum;
       }
     }
-    group_sync(c.h);
-    flush_rows<512>(c.staging, c.gt, reinterpret_cast<uint8_t*>(p.out0 + static_cast<size_t>(row0) * p.ld0 + col),
-                    ld_bytes, nvalid);
+    __syncwarp();
   }
-  if (c.h >= chunks) release();
+  // Sum over the 8 lanes that hold the same rows, halving the rows a lane keeps at each step: then lane l has row
+  // 8 (k / 2) + 2 (l & 3) + k % 2, k = l / 4, of one partial per (row, 32 columns).
+#pragma unroll
+  for (int step = 0; step < 3; ++step) {
+    const int o = 4 << step;
+    const bool upper = (c.lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < 8; k += 2 << step) {
+      const float keep = upper ? part[k + (1 << step)] : part[k], give = upper ? part[k] : part[k + (1 << step)];
+      part[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  const int k = c.lane >> 2, t = 8 * (k >> 1) + 2 * (c.lane & 3) + (k & 1);
+  if (t < at.rows) p.dwp[static_cast<size_t>(at.row0 + t) * p.dwp_tiles + (at.n * 2 + c.rank) * 4 + c.q] = part[0];
+}
+
+// A chunk's dh. `buf`: its h, from here on dh; `wl`: the router weight of row `lane`. (Writing eight rows out and asking for eight of the
+// next chunk's while the next eight are worked on is slower: 1107 against 1029 cycles per k-block at D=1024, F=512.)
+__device__ __forceinline__ void dswiglu_chunk(const GemmParams& p, const uint32_t (&r)[32], const GroupCtx& c, const Chunk& at,
+                                              uint32_t buf, float wl) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t ga = staged_h(buf, 8 * j + (c.lane & 7), c.lane >> 3);
+    const uint32_t ua = staged_h(buf, 8 * j + (c.lane & 7), 4 + (c.lane >> 3));
+    const f32x2 w = make_f32x2(__shfl_sync(0xffffffffu, wl, 8 * j + 2 * (c.lane & 3)),
+                               __shfl_sync(0xffffffffu, wl, 8 * j + 2 * (c.lane & 3) + 1));
+    uint32_t g[4], u[4];
+    ldmatrix_x4_trans(ga, g);
+    ldmatrix_x4_trans(ua, u);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int b = (s >> 1) * 16 + j * 4 + (s & 1) * 2;
+      // d_act is rounded to bf16 first, as the unfused reference stores it.
+      const f32x2 d = bf16x2_to_f32x2(pack_bf16(mul2(w, make_f32x2(__uint_as_float(r[b]), __uint_as_float(r[b + 1])))));
+      const f32x2 gate = bf16x2_to_f32x2(g[s]), up = bf16x2_to_f32x2(u[s]);
+      const f32x2 sig = sigmoid_f(gate), sl = mul2(gate, sig);
+      const f32x2 rest = fma2(sig, make_f32x2(-1.0f, -1.0f), make_f32x2(1.0f, 1.0f));  // 1 - sig, rounded like the subtraction
+      g[s] = pack_bf16(mul2(mul2(d, up), fma2(sl, rest, sig)));
+      u[s] = pack_bf16(mul2(d, sl));
+    }
+    __syncwarp();  // all lanes' ldmatrix reads of these rows are done (they cross lanes) before the rows are overwritten
+    stmatrix_x4_trans(ga, g);
+    stmatrix_x4_trans(ua, u);
+  }
+  __syncwarp();
+  __nv_bfloat16* out = p.out0 + dswiglu_offset(p, c, at);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int4 o = ld_shared_v4(staged_h(buf, (c.lane >> 3) + 4 * i, c.lane & 7));
+    if ((c.lane >> 3) + 4 * i < at.rows) *reinterpret_cast<int4*>(out + static_cast<size_t>(4 * i) * p.ld0) = o;
+  }
+  __syncwarp();  // the chunk has left the buffer
 }
 
 // Zeroes an output's rows past the groups' last one, a row per CTA and turn, by the epilogue warps while the first tile is
@@ -476,12 +485,14 @@ __global__ void __cluster_dims__(2, 1, 1) __maxnreg__(152)
 row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap map_a,
                 const __grid_constant__ TokenMaps maps_b) {
   using Traits = RowTraits<MODE>;
+  constexpr int kRowStages = kRowStagesOf<MODE>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t staging_base = smem_base + kRowStages * kRowStageBytes;
   uint8_t* staging_gen = smem_gen + kRowStages * kRowStageBytes;
-  const uint32_t bar_base = staging_base + 2 * kGroupStaging;
+  constexpr int kBarriers = 6 * kRowStageBytes + 2 * kGroupStaging;  // offset, behind ring and staging
+  const uint32_t bar_base = smem_base + kBarriers;
   // barriers: full[6], empty[6], acc_full[2], acc_empty[2], drain; then tmem slot, abort flag, early flag, first entry
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (kRowStages + s); };
@@ -491,7 +502,7 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
   constexpr int kSlotOff = 8 * (2 * kRowStages + 5);
   static_assert(kSlotOff + 16 <= kSmemTailBytes, "barrier area too small");
   const uint32_t tmem_slot = bar_base + kSlotOff;
-  uint8_t* tail_gen = staging_gen + 2 * kGroupStaging;
+  uint8_t* tail_gen = smem_gen + kBarriers;
   volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(tail_gen + kSlotOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail_gen + kSlotOff + 4);
   volatile int* early_flag = reinterpret_cast<volatile int*>(tail_gen + kSlotOff + 8);
@@ -705,20 +716,25 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
     c.gt = c.q * 32 + lane;
     c.rank = rank;
     c.staging = staging_base + c.h * kGroupStaging;
+    if constexpr (MODE == kModeDswiglu) c.staging = staging_base + (c.h * 4 + c.q) * 8192;  // two buffers for each warp
     const uint32_t leader_acc_empty0 = map_to_cta(acc_empty_bar(0), 0);
     // Combine modes: the row table sits behind the 8 KB that a chunk is staged in.
     uint32_t* s_dst = reinterpret_cast<uint32_t*>(staging_gen + c.h * kGroupStaging + 8192);
-    uint32_t tcount = 0, returned = 0;
-    long long epi_wait = 0;
+    uint32_t turn = 0, returned = 0;  // turn: accumulator buffer in bit 0, its phase in bit 1
     if (!gave_up) zero_tail(p, (warp - 2) * 32 + lane);
+    // SwiGLU': the next chunk, whether it has been asked for and the buffer it is in.
+    DswigluNext ahead = {};
+    bool fetched = false;
+    uint32_t cur = 0;
+    // Where this GEMM is the one that waits for a slice's rows, a tile's weights are there once its accumulator is.
+    const bool arrives = p.arrive != nullptr || p.ready != nullptr;
     RowTile nxt = {};
     if (first_tile < num_tiles) nxt = decode_row_tile<RANGED>(p, first_tile, first_entry, num_entries);
-    for (int t = first_tile; t < num_tiles; t += tile_step, ++tcount) {
+    for (int t = first_tile; t < num_tiles; t += tile_step, turn = (turn + 1) & 3u) {
       const RowTile tl = nxt;
       if (t + tile_step < num_tiles) nxt = decode_row_tile<RANGED>(p, t + tile_step, first_entry, num_entries);
-      const int as = tcount & 1;
-      const uint32_t aph = (tcount >> 1) & 1u;
-      DswigluLoads first = {};  // (zeros: what rows past the tile are worked on with)
+      const int as = turn & 1;
+      const uint32_t aph = turn >> 1;
       if constexpr (Traits::kCombine) {
         // Where the rows of this group's chunks go (thread = row), worked out while the accumulator is being made.
         group_sync(c.h);  // the previous tile's table has been used up
@@ -732,20 +748,19 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
           if (lane == s) returned += cnt;
         }
       }
-      uint32_t first_act[4][4] = {};
       if constexpr (MODE == kModeDswiglu) {
-        load_dswiglu(p, tl, c, c.h, &first);
-        stage_dswiglu(p, c, first, first_act);
+        if (!fetched && c.h * 32 < tl.nrows) fetch_dswiglu(p, c, chunk_of(tl, c.h), c.staging + cur * 4096, !arrives, &ahead);
+        fetched = false;
       }
       const long long w0 = counting ? clock64() : 0;
       const bool reached_acc = mbar_wait(acc_full_bar(as), aph, p.mbar_limit, abort_flag);
-      if (counting) epi_wait += clock64() - w0;
+      if (counting && warp == 2 && lane == 0) prof_add(kProfEpiWait, clock64() - w0);
       if (!reached_acc && lane == 0) {
         report_status(p.status, kStatusMbarTimeout, kKernelGemm, MODE, t, 1500 + as, 0, 0);
         raise_abort();
       }
-      // One decision for the whole group: nobody may be left alone at a group barrier.
-      if (!group_vote(c.h, reached_acc)) break;
+      // One decision for the whole group: nobody may be left alone at a group barrier. (SwiGLU' has none.)
+      if (MODE == kModeDswiglu ? !__all_sync(0xffffffffu, reached_acc) : !group_vote(c.h, reached_acc)) break;
       tcgen05_fence_after_sync();
       const uint32_t tacc = tmem_base + (static_cast<uint32_t>(c.q * 32) << 16) + as * kTileTokens;
       auto release = [&]() {  // this warp has read its last accumulator value
@@ -754,10 +769,34 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
         if (lane == 0) mbar_arrive_cluster(leader_acc_empty0 + 8u * as);
       };
       if constexpr (MODE == kModeSwiglu) swiglu_epilogue(p, tl, tacc, c, release);
-      else if constexpr (MODE == kModeDswiglu) dswiglu_epilogue(p, tl, tacc, c, first, first_act, release);
+      else if constexpr (MODE == kModeDswiglu) {
+        const int chunks = (tl.nrows + 31) >> 5;
+        for (int ch = c.h; ch < chunks; ch += 2) {
+          const uint32_t buf = c.staging + cur * 4096, other = c.staging + (cur ^ 1) * 4096;
+          const bool last = ch + 2 >= chunks;
+          const Chunk at = chunk_of(tl, ch);
+          auto h_landed = [&]() { cp_async_wait_all(); __syncwarp(); };
+          const float wl = arrives && ch == c.h ? dswiglu_weight(p, c, at) : ahead.w;
+          const uint32_t odd = __ballot_sync(0xffffffffu, !weight_divides(wl));
+          uint32_t m[4][4], r[32];
+          if (p.dwp != nullptr) turn_act(c, other, ahead, m);
+          load_fragment(tacc + ch * 32, r);
+          if (last) release();
+          if (p.dwp != nullptr) dswiglu_shares(p, r, c, at, buf, m, odd, h_landed);
+          // (Behind the last use of what the chunk before asked for: a load that shares its scoreboard would be waited for with it.)
+          Chunk next = chunk_of(last ? nxt : tl, last ? c.h : ch + 2);
+          if (last && t + tile_step >= num_tiles) next.rows = 0;
+          fetched = next.rows > 0;
+          h_landed();
+          if (fetched) fetch_dswiglu(p, c, next, other, !last || !arrives, &ahead);
+          dswiglu_chunk(p, r, c, at, buf, wl);
+          cur ^= 1;
+        }
+        if (c.h >= chunks) release();
+      }
       else combine_epilogue(p, tl, tacc, c, s_dst, release);
     }
-    if (counting && warp == 2 && lane == 0) prof_add(kProfEpiWait, epi_wait);
+    if constexpr (MODE == kModeDswiglu) cp_async_wait_all();  // (on the way out of an error: no exit while a copy may still land)
     if constexpr (Traits::kCombine) {
       // The group's stores are all issued before any of its warps releases its counts (also on the unwind path).
       group_sync(c.h);
