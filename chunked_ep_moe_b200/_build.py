@@ -24,6 +24,7 @@ _SOURCES = [
     "runtime/fused_rank.cpp",
     "runtime/kernel_runner.cpp",
     "gemm/row_gemm.cu",
+    "gemm/gather_gemm.cu",
     "gemm/grouped_gemm_pair.cu",
     "comm/comm_kernels.cu",
     "plan/plan_kernel.cu",

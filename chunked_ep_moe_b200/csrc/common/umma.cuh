@@ -121,6 +121,11 @@ __device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void* src) 
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
 }
 
+// One arrival (of the barrier's count) on a barrier of this CTA once every copy that this thread has issued so far has landed.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 // Waits until all of this thread's copies have landed.
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 

@@ -77,6 +77,9 @@ struct GemmParams {
                               // 32 columns [S, dwp_tiles], or null
   int dwp_tiles;
   int ld0, ld1;
+  // --- gathered rows (`launch_gather_swiglu`): row r of the slice is row tokens[r] of `gather` --------------------------------
+  const __nv_bfloat16* gather;  // [tokens, 64 k_blocks]
+  const int* tokens;
   // --- combine targets (down_fwd, dx) --------------------------------------------------------
   __nv_bfloat16* const* peer_rows;   // [P] base of each source rank's [T*K, ld] return buffer; null: rows go to out0
   uint32_t* const* peer_count;       // [P] each source rank's returned-row counter; null: nobody waits for the rows
@@ -106,6 +109,9 @@ struct alignas(64) TokenMaps {
 // wait for nothing that comes behind them: see `FusedRank::backward_whole`.
 void launch_row_gemm(int mode, const GemmParams& p, const CUtensorMap& map_a, const TokenMaps& maps_b, int grid,
                      cudaStream_t stream, bool behind = false);
+
+// kModeSwiglu on all experts' rows, gathered: no map of them.
+void launch_gather_swiglu(const GemmParams& p, const CUtensorMap& map_a, int grid, cudaStream_t stream, bool behind = false);
 
 // Weight gradients (kModeTgmm). `map_a`, `map_b`: chunked descriptions with boxes of 64 rows x 2 chunks; `map_c`: the bf16
 // gradient [L*M, N] with boxes of 32 rows x 64 columns (tiled stores).

@@ -337,7 +337,7 @@ __device__ __forceinline__ void sort_count(const int* ids, int n, int num_expert
 
 // The same ids, 32 at a time and in order, to their output slots.
 __device__ __forceinline__ void sort_walk(const int (&e_of)[kSortItems], int base, int lane, int* mine, int* order,
-                                          int* inv_order) {
+                                          int* inv_order, const RowTable& rows = {}) {
 #pragma unroll
   for (int g = 0; g < kSortItems; ++g) {
     const int e = e_of[g];
@@ -354,6 +354,10 @@ __device__ __forceinline__ void sort_walk(const int (&e_of)[kSortItems], int bas
       const int idx = base + g * 32 + lane;
       order[slot] = idx;
       inv_order[idx] = slot;
+      if (rows.tokens != nullptr) {
+        rows.tokens[slot] = idx / rows.top_k;
+        rows.weights[slot] = rows.w_flat[idx];
+      }
     }
     __syncwarp();  // the next group's leaders see this group's slot updates
   }
@@ -435,7 +439,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_serial_kernel(const
 // went from 61 to 46 us, a 64-token decode at D=7168 from 509 to 493 us.
 __global__ void __launch_bounds__(kSortThreads) plan_small_kernel(const PlanKernelParams p, const int* ids, int n, int* order,
                                                                   int* inv_order, uint32_t* expected_total,
-                                                                  uint32_t* pass_base) {
+                                                                  uint32_t* pass_base, const RowTable rows) {
   extern __shared__ int s_small[];
   release_successor();
   const int L = p.lay.L, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -473,22 +477,25 @@ __global__ void __launch_bounds__(kSortThreads) plan_small_kernel(const PlanKern
       s_slot[w * L + e] = run;
       run += c;
     }
-    const uint32_t total = expected_total[e];
-    pass_base[e] = total;
-    expected_total[e] = total + static_cast<uint32_t>(s_counts[e]);
+    if (expected_total != nullptr) {
+      const uint32_t total = expected_total[e];
+      pass_base[e] = total;
+      expected_total[e] = total + static_cast<uint32_t>(s_counts[e]);
+    }
   }
   __syncthreads();
   publish_header(p);
-  sort_walk(e_of, base, lane, mine, order, inv_order);
+  sort_walk(e_of, base, lane, mine, order, inv_order, rows);
   plan_phase_b_warps(p.plan, p.lay, send_start, s_counts, send_start, send_start, s_counts);
 }
 
 }  // namespace
 
 void launch_plan_small(const PlanKernelParams& p, const int* expert_ids, int n, int* order, int* inv_order,
-                       uint32_t* expected_total, uint32_t* pass_base, cudaStream_t stream) {
+                       uint32_t* expected_total, uint32_t* pass_base, const RowTable& rows, cudaStream_t stream) {
   const size_t smem = sizeof(int) * (4 + kSortWarps) * static_cast<size_t>(p.lay.L);
-  plan_small_kernel<<<1, kSortThreads, smem, stream>>>(p, expert_ids, n, order, inv_order, expected_total, pass_base);
+  plan_small_kernel<<<1, kSortThreads, smem, stream>>>(p, expert_ids, n, order, inv_order, expected_total, pass_base,
+                                                     rows);
 }
 
 void launch_plan_build(const PlanKernelParams& p_in, cudaStream_t stream) {

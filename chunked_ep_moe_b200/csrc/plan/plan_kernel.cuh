@@ -32,12 +32,21 @@ struct PlanKernelParams {
 // prefix sums + per-slice argument builders (src/chunked_moe/plan.py:77-163).
 void launch_plan_build(const PlanKernelParams& p, cudaStream_t stream);
 
+// What a GEMM that gathers its rows (gemm/row_gemm.cuh) knows about them, by sorted position: the token and the router weight.
+struct RowTable {
+  int* tokens = nullptr;           // [T*K], or null: no table
+  float* weights = nullptr;        // [T*K]
+  const float* w_flat = nullptr;   // [T*K] router weights by flat index
+  int top_k = 1;
+};
+
 // Everything that starts a pass of ONE rank with few ids, as one kernel: the stable sort (order, inv_order), the tables, header
-// and status to the host, and the arrival targets (`expected_total`, `pass_base`: as in `launch_pass_begin`). `p.counts`,
+// and status to the host, and the arrival targets (`expected_total`, `pass_base`: as in `launch_pass_begin`; null where rows are
+// gathered by `rows` and none arrive). `p.counts`,
 // `p.my_counts` and the exchange's fields are not used. At most kPlanSmallIds ids and kPlanSmallExperts experts.
 constexpr int kPlanSmallIds = 2048, kPlanSmallExperts = 512;
 void launch_plan_small(const PlanKernelParams& p, const int* expert_ids, int n, int* order, int* inv_order,
-                       uint32_t* expected_total, uint32_t* pass_base, cudaStream_t stream);
+                       uint32_t* expected_total, uint32_t* pass_base, const RowTable& rows, cudaStream_t stream);
 
 // The start of a pass of ONE rank that runs as one slice, whatever the number of ids (three kernels): the sort, the tables and the
 // header. At most 1024 experts. `counts` [L] and `scratch` (`expert_sort_scratch_ints`) are written.

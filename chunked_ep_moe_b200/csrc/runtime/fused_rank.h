@@ -198,6 +198,11 @@ class FusedRank {
   // routing in 12 slices of 2048 rows at D=7168 7.50 -> 6.21, 3 x 16384 rows at D=1024, F=512 0.895 -> 0.792. The buffers are the
   // pass's own, from the caching allocator, while live tensors and arenas stay within half of the device; otherwise slice by slice.
   bool runs_whole(int64_t rows, bool training) const;
+  bool runs_brief(int64_t tokens, int64_t rows, bool training) const;
+  void expect_pass(const torch::Tensor& x, const torch::Tensor& expert_ids, const torch::Tensor& w_flat, const torch::Tensor& w_up,
+                   const torch::Tensor& w_down) const;
+  std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> forward_brief(torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat,
+                                                                         torch::Tensor w_up, torch::Tensor w_down);
   bool within_half(size_t bytes) const;
   GemmParams range_params(const int* plan, int64_t first, int64_t last) const;
   template <typename Part>
@@ -243,6 +248,7 @@ class FusedRank {
   bool keep_activations_ = true;  // CEM_KEEP_ACTIVATIONS=0: always recompute (least memory)
   torch::Tensor carry_up_, carry_down_, pass_base_, expected_total_, status_, tables_,
       sort_scratch_, my_counts_;
+  torch::Tensor brief_tokens_;  // tokens by row of a pass that `runs_brief`
   torch::Tensor ready_, ready_base_, ready_total_;  // fp8 wire: per-expert "rows expanded" counter, its base, its target
   // device pointer tables, rows of `tables_`
   enum Table { kTabX, kTabG, kTabW, kTabXq, kTabGq, kTabXs, kTabGs, kTabArrive, kTabRet, kTabDw, kTabCount,
