@@ -80,6 +80,10 @@ struct GemmParams {
   // --- gathered rows (`launch_gather_swiglu`): row r of the slice is row tokens[r] of `gather` --------------------------------
   const __nv_bfloat16* gather;  // [tokens, 64 k_blocks]
   const int* tokens;
+  // `launch_few_swiglu`: [num_ids] expert ids and router weights by flat index t * top_k + k, in place of `tokens` and `row_w`
+  const int* ids;
+  const float* w_flat;
+  int num_ids, top_k;
   // --- combine targets (down_fwd, dx) --------------------------------------------------------
   __nv_bfloat16* const* peer_rows;   // [P] base of each source rank's [T*K, ld] return buffer; null: rows go to out0
   uint32_t* const* peer_count;       // [P] each source rank's returned-row counter; null: nobody waits for the rows
@@ -112,6 +116,18 @@ void launch_row_gemm(int mode, const GemmParams& p, const CUtensorMap& map_a, co
 
 // kModeSwiglu on all experts' rows, gathered: no map of them.
 void launch_gather_swiglu(const GemmParams& p, const CUtensorMap& map_a, int grid, cudaStream_t stream, bool behind = false);
+
+// The same as the first kernel of a pass of at most 32 expert ids, without a plan: what the kernels behind it need of one goes to `plan`.
+struct FewPlan {
+  int* plan;          // tiles and their number, header, in_start, in_size and src_send_start of experts with rows; nothing else
+  int* order;         // [num_ids]
+  int* inv_order;
+  int32_t* host_out;  // as in `PlanKernelParams`
+  uint32_t host_seq;
+};
+constexpr int kFewIds = 32;
+void launch_few_swiglu(const GemmParams& p, const CUtensorMap& map_a, const FewPlan& plan, int grid, cudaStream_t stream,
+                       bool behind = false);
 
 // Weight gradients (kModeTgmm). `map_a`, `map_b`: chunked descriptions with boxes of 64 rows x 2 chunks; `map_c`: the bf16
 // gradient [L*M, N] with boxes of 32 rows x 64 columns (tiled stores).

@@ -11,7 +11,7 @@ template <int MODE, bool RANGED>
 __global__ void __cluster_dims__(2, 1, 1) __maxnreg__(152)
 row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap map_a,
                 const __grid_constant__ TokenMaps maps_b) {
-  row_gemm_body<MODE, RANGED, false>(p, map_a, &maps_b);
+  row_gemm_body<MODE, RANGED, kRowsMapped>(p, map_a, &maps_b);
 }
 
 }  // namespace

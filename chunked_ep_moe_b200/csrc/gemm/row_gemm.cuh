@@ -56,11 +56,23 @@ struct RowTile {
   int n;      // 256-column tile of the weights
 };
 
+// Where a GEMM's token rows come from: a matrix in expert order (tensor maps); `p.gather`, by a table of tokens; or the same for at
+// most 32 expert ids, which every CTA sorts for itself.
+enum RowSource : int { kRowsMapped, kRowsGathered, kRowsFew };
+
+// What a CTA keeps of few ids, in shared memory behind the barriers.
+struct FewRows {
+  int4 tiles[32];     // as in the plan's tables: one tile per expert that has rows
+  int tokens[32];     // by row
+  float weights[32];
+};
+
 // `RANGED`: the tiles of a range of experts. A variant of its own, with the range's first entry in shared memory: as a register of every
 // warp it made the SwiGLU' GEMM spill, and passes without ranges up to 1.4 % slower (620 rows of 107 experts at D=1792, F=512, forward
 // 134.1 -> 135.2 us; the expert kernels on 6086 rows of 9 experts at D=256, F=1024 127.7 -> 129.5).
 template <bool RANGED>
-__device__ __forceinline__ RowTile decode_row_tile(const GemmParams& p, int t, volatile const int* first_entry, int num_entries) {
+__device__ __forceinline__ RowTile decode_row_tile(const GemmParams& p, int t, volatile const int* first_entry, int num_entries,
+                                                   const FewRows* few = nullptr) {
   RowTile tl;
   const int band_tiles = kRowBand * p.n_tiles;
   const int band = t / band_tiles, rem = t - band * band_tiles;
@@ -69,7 +81,8 @@ __device__ __forceinline__ RowTile decode_row_tile(const GemmParams& p, int t, v
   tl.n = rem / width;
   const int ti = band * kRowBand + (rem - tl.n * width);
   const int first = RANGED ? *first_entry : 0;
-  const int4 e = reinterpret_cast<const int4*>(p.plan + p.lay.off_tiles + 4 * p.lay.max_tiles * p.slice)[first + ti];
+  const int4 e = few != nullptr ? few->tiles[ti]
+                                : reinterpret_cast<const int4*>(p.plan + p.lay.off_tiles + 4 * p.lay.max_tiles * p.slice)[first + ti];
   tl.g = e.x; tl.row0 = e.y; tl.nrows = e.z; tl.ncols = e.w;
   return tl;
 }
@@ -80,7 +93,7 @@ struct RowTraits {
   static constexpr bool kCombine = (MODE == kModeDownFwd || MODE == kModeDx);
 };
 
-template <int MODE, bool GATHER>
+template <int MODE, RowSource SRC>
 __device__ __forceinline__ void issue_row_kblock(const GemmParams& p, const RowTile& tl, int kb, int rank,
                                                  const CUtensorMap* map_a, const CUtensorMap* map_b, uint32_t sa,
                                                  uint32_t bar) {
@@ -96,7 +109,7 @@ __device__ __forceinline__ void issue_row_kblock(const GemmParams& p, const RowT
   } else {
     tma_load_2d_pair(sa, map_a, bar, kb * kBlockK, tl.g * p.b_group_rows + tl.n * kBlockN + rank * kBlockM);
   }
-  if constexpr (!GATHER) tma_load_2d_pair(sa + kRowStageBytesA, map_b, bar, kb * kBlockK, tl.row0 + rank * (tl.ncols >> 1));
+  if constexpr (SRC == kRowsMapped) tma_load_2d_pair(sa + kRowStageBytesA, map_b, bar, kb * kBlockK, tl.row0 + rank * (tl.ncols >> 1));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -116,8 +129,8 @@ constexpr int kGatherWarps = 2;
 template <int MODE, bool RANGED, typename RaiseAbort>
 __device__ __forceinline__ void gather_rows(const GemmParams& p, int warp, int lane, int rank, uint32_t smem_base, uint32_t empty0,
                                             uint32_t gathered0, int first_tile, int tile_step, int num_tiles,
-                                            volatile const int* first_entry, int num_entries, volatile int* abort_flag,
-                                            RaiseAbort&& raise_abort) {
+                                            volatile const int* first_entry, int num_entries, const FewRows* few,
+                                            volatile int* abort_flag, RaiseAbort&& raise_abort) {
   constexpr int kRows = kTileTokens / 16;
   const int piece = lane & 7, row = 4 * warp + (lane >> 3);  // (row < 8)
   const uint32_t dst0 = smem_base + kRowStageBytesA + row * 128 + ((piece ^ row) << 4);
@@ -125,13 +138,15 @@ __device__ __forceinline__ void gather_rows(const GemmParams& p, int warp, int l
   uint32_t ps = 0, pph = 0;
   bool dead = false;
   for (int t = first_tile; t < num_tiles && !dead && !*abort_flag; t += tile_step) {
-    const RowTile tl = decode_row_tile<RANGED>(p, t, first_entry, num_entries);
+    const RowTile tl = decode_row_tile<RANGED>(p, t, first_entry, num_entries, few);
     const int half = tl.ncols >> 1;
     uint32_t at[kRows];  // bytes from p.gather; ~0: past the tile
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
       const int r = rank * half + 8 * i + row;
-      at[i] = 8 * i < half && r < tl.nrows ? static_cast<uint32_t>(p.tokens[tl.row0 + r]) * pitch + piece * 16 : ~0u;
+      at[i] = ~0u;
+      if (8 * i < half && r < tl.nrows)
+        at[i] = static_cast<uint32_t>(few != nullptr ? few->tokens[tl.row0 + r] : p.tokens[tl.row0 + r]) * pitch + piece * 16;
     }
     const uint8_t* src = reinterpret_cast<const uint8_t*>(p.gather);
     for (int kb = 0; kb < p.k_blocks; ++kb, src += kBlockK * 2) {
@@ -154,6 +169,64 @@ __device__ __forceinline__ void gather_rows(const GemmParams& p, int warp, int l
     }
   }
   cp_async_wait_all();  // no exit while a copy may still land
+}
+
+// Few ids: one warp, a lane an id, sorts them stably by expert. Ids outside the experts have no row. Returns the number of tiles.
+__device__ __forceinline__ int sort_few(const GemmParams& p, int lane, int* expert, int* row, int* first_row, int* count) {
+  const int e = lane < p.num_ids ? p.ids[lane] : -1;
+  const bool good = e >= 0 && e < p.lay.L;
+  const unsigned peers = __match_any_sync(0xffffffffu, good ? e : -1);
+  const bool first = good && __ffs(peers) - 1 == lane;
+  const int key = good ? e : 0x7fffffff;
+  int before = 0, tiles_before = 0;
+#pragma unroll
+  for (int l = 0; l < 32; ++l) {
+    const int other = __shfl_sync(0xffffffffu, first ? key | static_cast<int>(0x80000000u) : key, l);
+    if ((other & 0x7fffffff) < key) {
+      ++before;
+      tiles_before += other < 0 ? 1 : 0;
+    }
+  }
+  *expert = good ? e : -1;
+  *first_row = before;
+  *row = before + __popc(peers & ((1u << lane) - 1u));
+  *count = first ? __popc(peers) : 0;
+  // (lanes of one expert agree on tiles_before; it is the first one's that counts)
+  *count |= tiles_before << 8;
+  return __popc(__ballot_sync(0xffffffffu, first));
+}
+
+// The same for everybody behind this kernel: the tables that the down-projection and the sum read, header and status for the host.
+__device__ __forceinline__ void publish_few(const GemmParams& p, const FewPlan& out, int lane) {
+  int e, row, first_row, count;
+  const int tiles = sort_few(p, lane, &e, &row, &first_row, &count);
+  const int rows = __popc(__ballot_sync(0xffffffffu, e >= 0));
+  if (lane < p.num_ids && e < 0)
+    report_status(p.status, kStatusBadIndex, kKernelPlan, 1, 0, lane, static_cast<uint32_t>(p.lay.L), static_cast<uint32_t>(p.ids[lane]));
+  if (e >= 0) {
+    out.order[row] = lane;
+    out.inv_order[lane] = row;
+    const int n = count & 0xff;
+    if (n > 0) {
+      reinterpret_cast<int4*>(out.plan + p.lay.off_tiles)[count >> 8] = make_int4(e, first_row, n, kTileUnit);
+      out.plan[p.lay.off_in_start + e] = first_row;
+      out.plan[p.lay.off_in_size + e] = n;
+      out.plan[p.lay.off_src_send_start + e] = first_row;
+    }
+  }
+  if (lane == 0) out.plan[p.lay.off_num_tiles] = tiles;
+  // header: slices, rows of the stream (mine, the fullest), rows for other ranks, too many slices, token copies
+  int word = lane == 0 ? 1 : lane == 1 || lane == 2 || lane == 5 ? rows : 0;
+  if (lane < kPlanHeaderInts) out.plan[lane] = word;
+  __syncwarp();
+  if (lane >= kPlanHeaderInts && lane < kPlanHeaderInts + 8)
+    word = p.status != nullptr ? __ldcg(reinterpret_cast<const int*>(p.status) + lane - kPlanHeaderInts) : 0;
+  if (lane < kPlanHeaderInts + 8) out.host_out[lane] = word;
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence_system();
+    st_release_sys(reinterpret_cast<uint32_t*>(out.host_out) + kPlanHeaderInts + 8, out.host_seq);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -213,7 +286,7 @@ struct GroupCtx {
 
 template <typename Release>
 __device__ __forceinline__ void swiglu_epilogue(const GemmParams& p, const RowTile& tl, uint32_t tacc,
-                                                const GroupCtx& c, Release&& release) {
+                                                const GroupCtx& c, const FewRows* few, Release&& release) {
   const int chunks = (tl.nrows + 31) >> 5;
   // Lanes 0-63 of the accumulator are gate columns and 64-127 the up columns that belong to them (stripes of 32: both
   // kinds alternate every 32 lanes), so a gate warp and its partner exchange half of a chunk through shared memory
@@ -233,11 +306,11 @@ __device__ __forceinline__ void swiglu_epilogue(const GemmParams& p, const RowTi
     // Router weights of this thread's four rows, asked for before anything else: they come from L2 (read past L1: the line
     // may also hold weights of rows that had not arrived when another tile read it).
     float w[4] = {1.0f, 1.0f, 1.0f, 1.0f};
-    if (p.row_w != nullptr) {
+    if (few != nullptr || p.row_w != nullptr) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int t = (is_gate ? 0 : 16) + 8 * (i >> 1) + 2 * (c.lane & 3) + (i & 1);
-        if (t < nvalid) w[i] = __ldcg(p.row_w + row0 + t);
+        if (t < nvalid) w[i] = few != nullptr ? few->weights[row0 + t] : __ldcg(p.row_w + row0 + t);
       }
     }
     uint32_t r[32];
@@ -537,9 +610,11 @@ __device__ __forceinline__ void zero_tail(const GemmParams& p, int thread) {
   }
 }
 
-// The kernels' common body (`maps_b`: null with gathered rows).
-template <int MODE, bool RANGED, bool GATHER>
-__device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtensorMap& map_a, const TokenMaps* maps_b) {
+// The kernels' common body (`maps_b`: null with gathered rows; `plan`: with few ids).
+template <int MODE, bool RANGED, RowSource SRC>
+__device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtensorMap& map_a, const TokenMaps* maps_b,
+                                              const FewPlan* plan = nullptr) {
+  constexpr bool GATHER = SRC != kRowsMapped;
   using Traits = RowTraits<MODE>;
   constexpr int kRowStages = kRowStagesOf<MODE>;
   extern __shared__ uint8_t smem_raw[];
@@ -589,7 +664,8 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
                                         smem_base - smem_u32(smem_raw));
     return;
   }
-  release_successor();
+  // (Few ids: the successor writes nothing before this kernel's own predecessor has ended.)
+  if constexpr (SRC != kRowsFew) release_successor();
   cluster_sync_all();  // both CTAs run
 
   if (threadIdx.x == 0) {
@@ -616,6 +692,22 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
   }
   // Launched behind its predecessor, the kernel has come this far in that one's tail; global memory from here on.
   wait_predecessor();
+  FewRows* few = nullptr;
+  if constexpr (SRC == kRowsFew) {
+    static_assert(kSlotOff + 16 + 8 * kRowStages <= kSmemTailBytes && kSmemTailBytes % 16 == 0, "no place for the few rows");
+    release_successor();
+    few = reinterpret_cast<FewRows*>(tail_gen + kSmemTailBytes);
+    if (warp == 0) {
+      int e, row, first_row, count;
+      const int tiles = sort_few(p, lane, &e, &row, &first_row, &count);
+      if (e >= 0) {
+        few->tokens[row] = lane / p.top_k;
+        few->weights[row] = p.w_flat[lane];
+        if ((count & 0xff) > 0) few->tiles[count >> 8] = make_int4(e, first_row, count & 0xff, kTileUnit);
+      }
+      if (lane == 0) *first_entry = tiles;  // (read back behind the barrier below)
+    }
+  }
   // An earlier kernel of this pass already gave up: neither CTA of the pair does anything (the leader decides).
   if (threadIdx.x == 0 && leader) {
     const uint32_t v = (p.status != nullptr && p.status->code != 0) ? 1u : 0u;
@@ -636,6 +728,8 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
       const int first = start[p.first_expert];
       num_entries = start[p.last_expert] - first;
       *first_entry = first;  // (the same from every thread; each reads back what it has written itself)
+    } else if constexpr (SRC == kRowsFew) {
+      num_entries = *first_entry;
     } else {
       num_entries = p.plan[p.lay.off_num_tiles + p.slice];
     }
@@ -653,10 +747,10 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
     bool dead = false;
     // The next tile is decoded one iteration ahead, so its plan-table load is in flight while this tile runs.
     RowTile nxt = {};
-    if (first_tile < num_tiles) nxt = decode_row_tile<RANGED>(p, first_tile, first_entry, num_entries);
+    if (first_tile < num_tiles) nxt = decode_row_tile<RANGED>(p, first_tile, first_entry, num_entries, few);
     for (int t = first_tile; t < num_tiles && !dead && !*abort_flag; t += tile_step) {
       const RowTile tl = nxt;
-      if (t + tile_step < num_tiles) nxt = decode_row_tile<RANGED>(p, t + tile_step, first_entry, num_entries);
+      if (t + tile_step < num_tiles) nxt = decode_row_tile<RANGED>(p, t + tile_step, first_entry, num_entries, few);
       if constexpr (!GATHER && (MODE == kModeSwiglu || MODE == kModeDswiglu)) {  // whichever reads a slice's dispatched rows first
         if ((p.arrive != nullptr || p.ready != nullptr) && tl.g != waited_expert) {
           if (!wait_expert_rows(p, MODE, tl.g, lane, abort_flag)) {
@@ -683,7 +777,7 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
         if (elect_one()) {
           const uint32_t fb = map_to_cta(full_bar(ps), 0);
           mbar_expect_tx_cluster(fb, bytes);
-          issue_row_kblock<MODE, GATHER>(p, tl, kb, rank, &map_a, map_b, smem_base + ps * kRowStageBytes, fb);
+          issue_row_kblock<MODE, SRC>(p, tl, kb, rank, &map_a, map_b, smem_base + ps * kRowStageBytes, fb);
         }
         ++it;
         if (++ps == kRowStages) { ps = 0; pph ^= 1u; }
@@ -719,10 +813,10 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
       dead = true;
     };
     RowTile nxt = {};
-    if (leader && first_tile < num_tiles) nxt = decode_row_tile<RANGED>(p, first_tile, first_entry, num_entries);
+    if (leader && first_tile < num_tiles) nxt = decode_row_tile<RANGED>(p, first_tile, first_entry, num_entries, few);
     for (int t = first_tile; leader && t < num_tiles && !dead && !*abort_flag; t += tile_step, ++tcount) {
       const RowTile tl = nxt;
-      if (t + tile_step < num_tiles) nxt = decode_row_tile<RANGED>(p, t + tile_step, first_entry, num_entries);
+      if (t + tile_step < num_tiles) nxt = decode_row_tile<RANGED>(p, t + tile_step, first_entry, num_entries, few);
       const int as = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1u;
       const uint32_t tmem_d = tmem_base + as * kTileTokens;
@@ -785,7 +879,7 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
   } else if (GATHER && warp >= kRowThreads / 32) {
     // ================================ gathered rows (both CTAs) =============================
     gather_rows<MODE, RANGED>(p, warp - kRowThreads / 32, lane, rank, smem_base, empty_bar(0), gathered_bar(0), first_tile, tile_step,
-                              num_tiles, first_entry, num_entries, abort_flag, raise_abort);
+                              num_tiles, first_entry, num_entries, few, abort_flag, raise_abort);
   } else {
     // ================================ epilogue (both CTAs) ==================================
     GroupCtx c;
@@ -801,6 +895,10 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
     uint32_t* s_dst = reinterpret_cast<uint32_t*>(staging_gen + c.h * kGroupStaging + 8192);
     uint32_t turn = 0, returned = 0;  // turn: accumulator buffer in bit 0, its phase in bit 1
     if (!gave_up) zero_tail(p, (warp - 2) * 32 + lane);
+    // (The last CTA is the last to get a tile. Also when an earlier kernel gave up: the host waits for it.)
+    if constexpr (SRC == kRowsFew) {
+      if (warp == 9 && blockIdx.x == gridDim.x - 1) publish_few(p, *plan, lane);
+    }
     // SwiGLU': the next chunk, whether it has been asked for and the buffer it is in.
     DswigluNext ahead = {};
     bool fetched = false;
@@ -808,10 +906,10 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
     // Where this GEMM is the one that waits for a slice's rows, a tile's weights are there once its accumulator is.
     const bool arrives = p.arrive != nullptr || p.ready != nullptr;
     RowTile nxt = {};
-    if (first_tile < num_tiles) nxt = decode_row_tile<RANGED>(p, first_tile, first_entry, num_entries);
+    if (first_tile < num_tiles) nxt = decode_row_tile<RANGED>(p, first_tile, first_entry, num_entries, few);
     for (int t = first_tile; t < num_tiles; t += tile_step, turn = (turn + 1) & 3u) {
       const RowTile tl = nxt;
-      if (t + tile_step < num_tiles) nxt = decode_row_tile<RANGED>(p, t + tile_step, first_entry, num_entries);
+      if (t + tile_step < num_tiles) nxt = decode_row_tile<RANGED>(p, t + tile_step, first_entry, num_entries, few);
       const int as = turn & 1;
       const uint32_t aph = turn >> 1;
       if constexpr (Traits::kCombine) {
@@ -847,7 +945,7 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(leader_acc_empty0 + 8u * as);
       };
-      if constexpr (MODE == kModeSwiglu) swiglu_epilogue(p, tl, tacc, c, release);
+      if constexpr (MODE == kModeSwiglu) swiglu_epilogue(p, tl, tacc, c, few, release);
       else if constexpr (MODE == kModeDswiglu) {
         const int chunks = (tl.nrows + 31) >> 5;
         for (int ch = c.h; ch < chunks; ch += 2) {

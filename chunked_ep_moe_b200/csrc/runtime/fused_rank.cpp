@@ -1193,7 +1193,7 @@ void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w
 }
 
 // A forward of few tokens without autograd, on the caller's stream: plan, up-projection with its rows gathered, down-projection, sum of the
-// K rows a token. No put, no buffer of a slice and no arrival is involved. 64 tokens at D=7168 477 -> 462 us, one token 45 -> 41.5 us (the put
+// K rows a token. No put, no buffer of a slice and no arrival is involved, and up to 32 ids no plan kernel (`launch_few_swiglu`). 64 tokens at D=7168 477 -> 462 us, one token 45 -> 41.5 us (the put
 // between was a launch and 5 us of latency). Up to 96 tokens the gather keeps up with the tensor cores, whatever the routing (gemm/row_gemm.cuh).
 bool FusedRank::runs_brief(int64_t tokens, int64_t rows, bool training) const {
   return P_ == 1 && use_comm_stream_ && !training && !fp8_ && tokens > 0 && tokens <= kBriefTokens && rows <= S_ &&
@@ -1214,12 +1214,14 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brie
   header_whole_ = true;
   cur_slices_ = 0;
   inline_ = true;
+  const bool few = tk <= kFewIds;
   RowTable rows;
   rows.tokens = brief_tokens_.data_ptr<int>();
   rows.weights = reinterpret_cast<float*>(arena_ + arena_lay_.wbuf);
   rows.w_flat = w_flat.data_ptr<float>();
   rows.top_k = K_;
-  {
+  ++host_seq_;
+  if (!few) {
     NvtxRange range("chunked_moe/plan");
     PlanKernelParams pp{};
     pp.lay = whole_lay_;
@@ -1227,7 +1229,7 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brie
     pp.spin_limit = spin_limit_;
     pp.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
     pp.host_out = host_header_;
-    pp.host_seq = ++host_seq_;
+    pp.host_seq = host_seq_;
     launch_plan_small(pp, expert_ids.data_ptr<int>(), static_cast<int>(tk), order.data_ptr<int>(), inv_order.data_ptr<int>(), nullptr,
                       nullptr, rows, st);
     ++launches_;
@@ -1245,7 +1247,16 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brie
     p.gather = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr());
     p.tokens = rows.tokens;
     count_pipeline(kModeSwiglu, &p);
-    launch_gather_swiglu(p, up_map(w_up), std::max(2, num_sms_), st, /*behind=*/true);
+    if (few) {
+      p.ids = expert_ids.data_ptr<int>();
+      p.w_flat = rows.w_flat;
+      p.num_ids = static_cast<int>(tk);
+      p.top_k = K_;
+      const FewPlan made{plan.data_ptr<int>(), order.data_ptr<int>(), inv_order.data_ptr<int>(), host_header_, host_seq_};
+      launch_few_swiglu(p, up_map(w_up), made, std::max(2, num_sms_), st, /*behind=*/true);
+    } else {
+      launch_gather_swiglu(p, up_map(w_up), std::max(2, num_sms_), st, /*behind=*/true);
+    }
     ++launches_;
   }
   {

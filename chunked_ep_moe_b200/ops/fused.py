@@ -185,7 +185,8 @@ def expected_launches_alone(rows: int, experts: int, hidden: int, ffn: int, kept
 
     Forward: sort and plan (3) + per range of experts (put, swiglu, down+combine) + combine reduce. Backward: per range (put,
     dswiglu, dW_down, dx+combine, dW_up, and swiglu+h or, beside the first GEMM of several kept ranges, a put of x) + d_weight
-    return + combine reduce. (A forward of one slice, up to 2048 ids and 512 experts, without autograd: 5, up to 96 tokens 4.)
+    return + combine reduce. (A forward of one slice, up to 2048 ids and 512 experts, without autograd: 5, up to 96 tokens 4,
+    up to 32 ids 3.)
     """
     forward, backward = [_build.load().whole_ranges(rows, experts, hidden, ffn, True, b) for b in (False, True)]
     return 4 + 3 * forward + 2 + (5 if kept and backward == 1 else 6) * backward
