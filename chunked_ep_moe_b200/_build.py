@@ -22,6 +22,7 @@ _SOURCES = [
     "bindings.cpp",
     "runtime/tensor_map.cpp",
     "runtime/fused_rank.cpp",
+    "runtime/layer_node.cpp",
     "runtime/kernel_runner.cpp",
     "gemm/row_gemm.cu",
     "gemm/gather_gemm.cu",
@@ -115,7 +116,7 @@ def build(verbose: bool = False, force: bool = False):
 
 def load():
     """Returns the extension, building it first when needed. Raises if it cannot be had."""
-    return build()
+    return _module if _module is not None else build()
 
 
 def is_built() -> bool:

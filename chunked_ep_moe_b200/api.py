@@ -64,7 +64,8 @@ def _check_inputs(x, expert_ids, weights, w_up, w_down, cfg: ChunkedMoEConfig, g
     if x.dim() != 2:
         raise ValueError(f"x must be [T, D], got {tuple(x.shape)}")
     t, d = x.shape
-    if tuple(expert_ids.shape) != (t, cfg.top_k) or tuple(weights.shape) != (t, cfg.top_k):
+    routed = (t, cfg.top_k)
+    if expert_ids.shape != routed or weights.shape != routed:
         raise ValueError(f"expert_ids/router_weights must be [T={t}, K={cfg.top_k}], got "
                          f"{tuple(expert_ids.shape)} and {tuple(weights.shape)}")
     world = dist.get_world_size(group) if (dist.is_available() and dist.is_initialized()) else 1
@@ -74,7 +75,7 @@ def _check_inputs(x, expert_ids, weights, w_up, w_down, cfg: ChunkedMoEConfig, g
     if w_up.dim() != 3 or w_up.shape[0] != local or w_up.shape[1] != d or w_up.shape[2] % 2:
         raise ValueError(f"w_up must be [L={local}, D={d}, 2F], got {tuple(w_up.shape)}")
     ffn = w_up.shape[2] // 2
-    if tuple(w_down.shape) != (local, ffn, d):
+    if w_down.shape != (local, ffn, d):
         raise ValueError(f"w_down must be [L={local}, F={ffn}, D={d}], got {tuple(w_down.shape)}")
     if ffn % cfg.stripe_width:
         raise ValueError(f"F={ffn} is not a multiple of stripe_width={cfg.stripe_width}")

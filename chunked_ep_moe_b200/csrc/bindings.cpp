@@ -7,6 +7,7 @@
 #include "plan/plan_kernel.cuh"
 #include "model/model_ops.h"
 #include "runtime/fused_rank.h"
+#include "runtime/layer_node.h"
 #include "runtime/kernel_runner.h"
 
 namespace {
@@ -136,7 +137,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("gmm_dswiglu", &cem::KernelRunner::gmm_dswiglu)
       .def("tgmm", &cem::KernelRunner::tgmm)
       .def("check_status", &cem::KernelRunner::check_status);
-  py::class_<cem::FusedRank>(m, "FusedRank")
+  // Passes run without the interpreter's lock: those of a rank have one of their own, which a backward on the engine's thread may hold.
+  m.def("chunked_moe_layer", &cem::chunked_moe_layer, py::call_guard<py::gil_scoped_release>(),
+        "(rank, x, expert_ids, router_weights, w_up, w_down) -> the layer's output, differentiable");
+  py::class_<cem::FusedRank, std::shared_ptr<cem::FusedRank>>(m, "FusedRank")
       .def(py::init<int, int, int, int, int, int, int, int, int, int, int, bool, int64_t, std::vector<int64_t>, bool,
                     int64_t, int>(),
            py::arg("P"), py::arg("L"), py::arg("me"), py::arg("S"), py::arg("D"), py::arg("F"), py::arg("K"),
@@ -155,11 +159,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("compute_forward", &cem::FusedRank::compute_forward)
       .def("compute_backward", &cem::FusedRank::compute_backward)
       .def("keep_rows", &cem::FusedRank::keep_rows)
-      .def("forward_pass", &cem::FusedRank::forward_pass)
-      .def("backward_pass", &cem::FusedRank::backward_pass)
+      .def("forward_pass", &cem::FusedRank::forward_pass, py::call_guard<py::gil_scoped_release>())
+      .def("backward_pass", &cem::FusedRank::backward_pass, py::call_guard<py::gil_scoped_release>())
       .def("finish_forward", &cem::FusedRank::finish_forward)
       .def("finish_backward", &cem::FusedRank::finish_backward)
-      .def("check_status", &cem::FusedRank::check_status)
+      .def("check_status", &cem::FusedRank::check_status, py::call_guard<py::gil_scoped_release>())
+      .def("release", &cem::FusedRank::release, py::call_guard<py::gil_scoped_release>())
       .def("plan_header", &cem::FusedRank::plan_header)
       .def("set_whole_passes", &cem::FusedRank::set_whole_passes)
       .def("plan_ints", &cem::FusedRank::plan_ints)

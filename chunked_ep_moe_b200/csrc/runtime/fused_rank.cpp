@@ -239,6 +239,7 @@ FusedRank::~FusedRank() {
 }
 
 void FusedRank::check_status() {
+  const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
   cudaStream_t st = current_stream();
   cuda_check(cudaMemcpyAsync(host_header_ + kHostStatus, status_.data_ptr(), 8 * sizeof(int32_t),
                              cudaMemcpyDeviceToHost, st),
@@ -1283,6 +1284,7 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brie
 std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass(
     torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
     bool training) {
+  const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
   const int64_t tk = expert_ids.numel();
   release_kept();  // (of a pass that threw)
   short_pass_ = false;
@@ -1370,6 +1372,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
     torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
     torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
     const std::vector<torch::Tensor>& kept, int64_t kept_slices) {
+  const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
   inline_ = short_pass_ = false;  // (also behind a forward that threw)
   release_kept();
   const int64_t rows = order.numel();

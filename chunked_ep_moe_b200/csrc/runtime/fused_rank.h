@@ -16,7 +16,9 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <map>
+#include <mutex>
 #include <algorithm>
 #include <exception>
 #include <string>
@@ -135,6 +137,13 @@ class FusedRank {
       torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
       torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
       const std::vector<torch::Tensor>& kept, int64_t kept_slices);
+
+  // The arena is about to go: a backward that still comes is refused.
+  void release() {
+    const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);  // (not in the middle of a backward on another thread)
+    released_ = true;
+  }
+  bool released() const { return released_; }
 
   // Reads the status block (synchronises); throws std::runtime_error describing the first recorded error.
   void check_status();
@@ -260,6 +269,10 @@ class FusedRank {
   CUtensorMap map_x_mn_[2], map_g_mn_[2], map_act_mn_[2], map_dh_mn_[2];
   std::map<std::tuple<const void*, uint32_t, int64_t, int64_t>, CUtensorMap> weight_maps_;
 
+  // One pass (as one call) or status check at a time: a forward on the caller's thread and a backward on the autograd engine's share all
+  // of the above and the counters below.
+  std::recursive_mutex pass_mutex_;
+  std::atomic<bool> released_{false};
   cudaStream_t comm_stream_ = nullptr, aux_stream_ = nullptr, chain_[2] = {};
   cudaStream_t expand_stream_ = nullptr;  // fp8 wire: the expansion kernels run here, beside the GEMM chains
   cudaEvent_t ev_expand_[4] = {};  // expansion of slice j (mod 4) has finished

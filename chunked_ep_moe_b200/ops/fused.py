@@ -137,6 +137,8 @@ def release_workspaces() -> None:
     """Frees every workspace, cached or replaced (collective when a process group is involved). A pass whose backward
     has not run yet must not be kept across this call: its backward raises."""
     for ws in list(_workspaces.values()) + _retired:
+        if ws.rank is not None:
+            ws.rank.release()
         ws.rank = None
         ws.arena.close()
     _workspaces.clear()
@@ -258,34 +260,6 @@ def _require(cond: bool, msg: str) -> None:
         raise ValueError("chunked_moe fused path: " + msg)
 
 
-class _ChunkedMoEFused(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, expert_ids, weights, w_up, w_down, cfg, group, training):
-        tokens, hidden = x.shape
-        ffn = w_down.shape[1]
-        ws = get_workspace(cfg, group, hidden, ffn, tokens * cfg.top_k)
-        ids32 = expert_ids.to(torch.int32).contiguous()
-        w_flat = weights.detach().float().reshape(-1).contiguous()
-        xc, w_up_c, w_down_c = x.detach().contiguous(), w_up.detach().contiguous(), w_down.detach().contiguous()
-        (out, *saved), n, kept_slices = ws.rank.forward_pass(xc, ids32, w_flat, w_up_c, w_down_c, training)
-        ctx.save_for_backward(xc, weights, w_up_c, w_down_c, *saved)
-        ctx.ws, ctx.num_slices, ctx.kept_slices = ws, n, kept_slices
-        ctx.mark_non_differentiable(expert_ids)
-        return out
-
-    @staticmethod
-    def backward(ctx, g_out):
-        x, weights, w_up, w_down, plan, order, inv_order, *kept = ctx.saved_tensors
-        rank = ctx.ws.rank
-        if rank is None or ctx.ws.arena.local == 0:
-            raise RuntimeError("chunked_moe fused path: the workspace of this pass was released before its backward")
-        g = g_out.to(x.dtype).contiguous()
-        w_flat = weights.detach().float().reshape(-1).contiguous()
-        dx, d_weights, dw_up, dw_down = rank.backward_pass(x, g, w_flat, w_up, w_down, plan, order, inv_order,
-                                                           ctx.num_slices, kept, ctx.kept_slices)
-        return dx, None, d_weights.reshape(weights.shape).to(weights.dtype), dw_up, dw_down, None, None, None
-
-
 def unsupported_reason(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor,
                        cfg: ChunkedMoEConfig) -> Optional[str]:
     """Why these tensors cannot run on the fused kernels (shape or dtype), or None. The caller may then fall back to
@@ -315,5 +289,6 @@ def chunked_moe_fused(x: torch.Tensor, expert_ids: torch.Tensor, weights: torch.
     _require(cfg.stripe_width in (32, 64, 128), "needs stripe_width in {32, 64, 128}")
     _require(cfg.slice_size % 8 == 0, "needs slice_size % 8 == 0")
     _require(cfg.accum_dtype == "float32", "weight gradients are accumulated in float32 (accum_dtype)")
-    training = torch.is_grad_enabled() and any(t.requires_grad for t in (x, weights, w_up, w_down))
-    return _ChunkedMoEFused.apply(x, expert_ids, weights, w_up, w_down, cfg, group, training)
+    tokens, hidden = x.shape
+    ws = get_workspace(cfg, group, hidden, w_down.shape[1], tokens * cfg.top_k)
+    return _build.load().chunked_moe_layer(ws.rank, x, expert_ids, weights, w_up, w_down)
