@@ -114,6 +114,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.attr("gemm_smem_bytes") = cem::row_gemm_smem_bytes();
   m.def("pair_grid_used", []() { return cem::g_pair_grid_used; }, "grid of the last GEMM launch");
   m.attr("keep_work") = cem::kKeepWork;
+  m.attr("plan_small") = py::make_tuple(cem::kPlanSmallIds, cem::kPlanSmallExperts);
   m.def("wait_probe", &wait_probe, "bounded-wait self test kernel");
   m.def("format_status", &cem::format_status, "text of a recorded status block");
   m.def("add_rms_norm_fwd", &cem::add_rms_norm_fwd, "s = x + delta, y = RMSNorm(s) * w -> (s, y, rstd)");

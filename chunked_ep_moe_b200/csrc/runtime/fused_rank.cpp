@@ -1022,9 +1022,16 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_whol
     pp.status = reinterpret_cast<StatusBlock*>(status_.data_ptr());
     pp.host_out = host_header_;
     pp.host_seq = ++host_seq_;
-    launch_sort_and_plan(pp, expert_ids.data_ptr<int>(), static_cast<int>(tk), order.data_ptr<int>(),
-                         inv_order.data_ptr<int>(), my_counts_.data_ptr<int>(), sort_scratch_.data_ptr<int>(), st);
-    launches_ += 3;
+    if (tk <= kPlanSmallIds && L_ <= kPlanSmallExperts) {
+      // (Sort and tables as one kernel: 192 x 2 ids, forward + backward 162 -> 156 us, the host's wait for the header among them.)
+      launch_plan_small(pp, expert_ids.data_ptr<int>(), static_cast<int>(tk), order.data_ptr<int>(), inv_order.data_ptr<int>(), nullptr,
+                        nullptr, RowTable{}, st);
+      ++launches_;
+    } else {
+      launch_sort_and_plan(pp, expert_ids.data_ptr<int>(), static_cast<int>(tk), order.data_ptr<int>(),
+                           inv_order.data_ptr<int>(), my_counts_.data_ptr<int>(), sort_scratch_.data_ptr<int>(), st);
+      launches_ += 3;
+    }
   }
   cur_rows_ = tk;
   ret_target_ += static_cast<uint32_t>(tk) * static_cast<uint32_t>(D_ / kCombineCols);

@@ -185,13 +185,15 @@ def expected_launches(num_slices: int, fp8: bool = False, kept_slices: int = 0) 
 def expected_launches_alone(rows: int, experts: int, hidden: int, ffn: int, kept: bool) -> int:
     """Kernels one forward+backward launches on a rank on its own that runs it as one slice; `kept`: h and w * act stay.
 
-    Forward: sort and plan (3) + per range of experts (put, swiglu, down+combine) + combine reduce. Backward: per range (put,
-    dswiglu, dW_down, dx+combine, dW_up, and swiglu+h or, beside the first GEMM of several kept ranges, a put of x) + d_weight
-    return + combine reduce. (A forward of one slice, up to 2048 ids and 512 experts, without autograd: 5, up to 96 tokens 4,
+    Forward: sort and plan (3, or 1 up to 2048 ids and 512 experts) + per range of experts (put, swiglu, down+combine) + combine
+    reduce. Backward: per range (put, dswiglu, dW_down, dx+combine, dW_up, and swiglu+h or, beside the first GEMM of several kept
+    ranges, a put of x) + d_weight return + combine reduce. (A forward of one slice, up to 2048 ids and 512 experts, without autograd: 5, up to 96 tokens 4,
     up to 32 ids 3.)
     """
-    forward, backward = [_build.load().whole_ranges(rows, experts, hidden, ffn, True, b) for b in (False, True)]
-    return 4 + 3 * forward + 2 + (5 if kept and backward == 1 else 6) * backward
+    ext = _build.load()
+    forward, backward = [ext.whole_ranges(rows, experts, hidden, ffn, True, b) for b in (False, True)]
+    plan = 1 if rows <= ext.plan_small[0] and experts <= ext.plan_small[1] else 3
+    return plan + 1 + 3 * forward + 2 + (5 if kept and backward == 1 else 6) * backward
 
 
 def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidden: int, ffn: int, slice_size: int,
