@@ -51,6 +51,8 @@ struct GemmParams {
   // every expert has a group.)
   int first_expert, last_expert;
   int n_tiles;       // 256-column tiles of the weights (row-wise modes) or of the gradient (tgmm)
+  int unit_cols, row_units;  // tgmm: column tiles that a pair takes together of experts of few rows, and how many such units a row of
+                             // tiles has (set by the launcher)
   int m_tiles;       // tgmm: M / 128 (row tiles of the weight gradient); unused otherwise
   int k_blocks;      // gmm modes: K / 64
   int b_group_rows;  // rows one expert occupies in the flattened 2-D weight tensor map
@@ -130,10 +132,11 @@ void launch_few_swiglu(const GemmParams& p, const CUtensorMap& map_a, const FewP
                        bool behind = false);
 
 // Weight gradients (kModeTgmm). `map_a`, `map_b`: chunked descriptions with boxes of 64 rows x 2 chunks; `map_c`: the bf16
-// gradient [L*M, N] with boxes of 32 rows x 64 columns (tiled stores).
-void launch_weight_grad(const GemmParams& p, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                        const CUtensorMap& map_c, int grid, cudaStream_t stream, bool behind = false);
+// gradient [L*M, N] with boxes of 32 rows x 64 columns (tiled stores). `rows`: of the slice, or what it can hold.
+void launch_weight_grad(const GemmParams& p, const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c, int grid,
+                        int64_t rows, cudaStream_t stream, bool behind = false);
 
+int weight_grad_unit_cols(int rows_of_tiles, int n_tiles, int pairs);  // (the launcher's choice of `unit_cols`)
 int row_gemm_smem_bytes();    // dynamic shared memory of a row-wise GEMM CTA
 extern int g_pair_grid_used;  // grid of the last GEMM launch, for diagnostics
 

@@ -598,7 +598,8 @@ void FusedRank::weight_grad(const GemmParams& p0, const CUtensorMap& a, const CU
                             cudaStream_t st) {
   GemmParams p = p0;
   count_pipeline(kModeTgmm, &p);
-  launch_weight_grad(p, a, b, out, std::max(2, num_sms_), st, inline_);
+  // (Slice by slice the rows are cut as they come: how many an expert has of them is anything up to a slice.)
+  launch_weight_grad(p, a, b, out, std::max(2, num_sms_), p0.lay.S == whole_lay_.S ? cur_rows_ : S_, st, inline_);
   ++launches_;
 }
 

@@ -161,7 +161,7 @@ void KernelRunner::tgmm(torch::Tensor lhs, torch::Tensor rhs, torch::Tensor out)
   const CUtensorMap a = make_bf16_map_chunked(lhs.data_ptr(), S_, M, 64, 2);
   const CUtensorMap b = make_bf16_map_chunked(rhs.data_ptr(), S_, N, 64, 2);
   const CUtensorMap c = make_bf16_map_2d(out.data_ptr(), static_cast<uint64_t>(L_) * M, N, 32);
-  launch_weight_grad(p, a, b, c, num_sms_, stream());
+  launch_weight_grad(p, a, b, c, num_sms_, S_, stream());
 }
 
 void KernelRunner::check_status() {
