@@ -913,11 +913,11 @@ void FusedRank::reduce_backward(torch::Tensor inv_order, torch::Tensor dx, torch
 // ---------------------------------------------------------------------------------------------
 // passes of a rank on its own, as one slice
 // ---------------------------------------------------------------------------------------------
-bool FusedRank::within_half(size_t bytes) const {
+bool FusedRank::within_half(size_t bytes, int share) const {
   try {
     const auto pool = c10::cuda::CUDACachingAllocator::getDeviceStats(c10::cuda::current_device());
     const size_t live = static_cast<size_t>(pool.allocated_bytes[0].current) + static_cast<size_t>(arenas_allocated());
-    return live + bytes <= device_bytes_ / 2;
+    return live + bytes <= device_bytes_ / share;
   } catch (const c10::Error&) {  // an allocator that keeps no statistics
     return false;
   }
@@ -1076,6 +1076,10 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_whol
   resolve_slices();  // raises what the pass's kernels had recorded by the time the plan was made
   std::vector<torch::Tensor> result{out, plan, order, inv_order};
   result.insert(result.end(), kept.begin(), kept.end());
+  // x by rows stays for the backward of a pass of one range as well, while what lives stays within a quarter of the device (activations,
+  // which save a GEMM, come first: they have the half). Its put then moves g alone: forward + backward of 8192 x 6 rows at D=1024 711 -> 693
+  // us, 1999 x 4 at D=2048 410 -> 400 us, 2048 x 8 at D=7168 5.67 -> 5.60 ms.
+  if (training && parts == 1 && keep_activations_ && within_half(0, 4)) result.push_back(rows_x);
   return std::make_tuple(result, kWholePass, kept.empty() ? 0 : 1);
 }
 
@@ -1087,8 +1091,8 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_whol
 // wire 8.39 -> 8.11 ms, Zipf routing 6.20 -> 6.14, many small or very large experts unchanged (power: what runs side by side draws more).
 void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up,
                                torch::Tensor w_down, torch::Tensor plan, torch::Tensor inv_order,
-                               const std::vector<torch::Tensor>& kept, const std::vector<torch::Tensor>& buffers,
-                               torch::Tensor dw_up, torch::Tensor dw_down) {
+                               const std::vector<torch::Tensor>& kept, const torch::Tensor& kept_x,
+                               const std::vector<torch::Tensor>& buffers, torch::Tensor dw_up, torch::Tensor dw_down) {
   cudaStream_t st = current_stream();
   const int64_t tk = inv_order.numel();
   expect_i32(plan, whole_lay_.total, "plan");
@@ -1103,7 +1107,7 @@ void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w
   ret_target_ += static_cast<uint32_t>(tk) * static_cast<uint32_t>(D_ / kCombineCols + 1);
   const bool keep = !kept.empty();
   auto bf16 = [](const torch::Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); };
-  const torch::Tensor &rows_x = buffers[0], &rows_g = buffers[1], &rows_w = buffers[2], &dh = buffers[3], &dwp = buffers[4],
+  const torch::Tensor &rows_x = kept_x.defined() ? kept_x : buffers[0], &rows_g = buffers[1], &rows_w = buffers[2], &dh = buffers[3], &dwp = buffers[4],
                       &h = keep ? kept[0] : buffers[5], &act = keep ? kept[1] : buffers[6];
   const int* pl = plan.data_ptr<int>();
   const int dwp_tiles = F_ / 32;
@@ -1113,11 +1117,11 @@ void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w
                     act_mn = make_bf16_map_chunked(act.data_ptr(), tk, F_, 64, 2), dh_mn = make_bf16_map_chunked(dh.data_ptr(), tk, 2 * F_, 64, 2);
   // d_act = w * (g Wd^T) needs g's rows; x's, where nothing has to be recomputed from them, follow beside that GEMM.
   const int64_t parts = whole_ranges(tk, L_, D_, F_, /*training=*/true, /*backward=*/true);
-  const bool x_later = keep && parts > 1;
+  const bool x_later = keep && parts > 1 && !kept_x.defined();
   inline_ = parts == 1;
   run_parts(parts, [&](int64_t first, int64_t last, cudaStream_t put_stream, cudaStream_t gemm_stream) {
     NvtxRange range("chunked_moe/bwd experts from", first);
-    put_whole(plan, inv_order, x, &g, w_flat, x_later ? nullptr : bf16(rows_x), bf16(rows_g), rows_w.data_ptr<float>(), first, last,
+    put_whole(plan, inv_order, x, &g, w_flat, x_later || kept_x.defined() ? nullptr : bf16(rows_x), bf16(rows_g), rows_w.data_ptr<float>(), first, last,
               put_stream, inline_, first > 0);
     if (put_stream != gemm_stream) {
       cuda_check(cudaEventRecord(ev_put_[0], put_stream), "event record");
@@ -1379,11 +1383,17 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
 std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank::backward_pass(
     torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
     torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
-    const std::vector<torch::Tensor>& kept, int64_t kept_slices) {
+    const std::vector<torch::Tensor>& saved, int64_t kept_slices) {
   const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
   inline_ = short_pass_ = false;  // (also behind a forward that threw)
   release_kept();
   const int64_t rows = order.numel();
+  // Saved: h and w * act, x by rows, both or neither.
+  const std::vector<torch::Tensor> kept(saved.begin(), saved.size() >= 2 ? saved.begin() + 2 : saved.begin());
+  const torch::Tensor kept_x = saved.size() % 2 == 1 ? saved.back() : torch::Tensor();
+  expect(!kept_x.defined() || (kept_x.is_cuda() && kept_x.is_contiguous() && kept_x.scalar_type() == torch::kBFloat16 &&
+                               kept_x.dim() == 2 && kept_x.size(0) == rows && kept_x.size(1) == D_),
+         "x by rows must be a contiguous CUDA bf16 [T*K, D] matrix");
   torch::Tensor dw_up = torch::empty_like(w_up), dw_down = torch::empty_like(w_down), dx = torch::empty_like(x);
   torch::Tensor d_weights = torch::empty({w_flat.numel()}, w_flat.options());
   std::vector<torch::Tensor> buffers;
@@ -1393,7 +1403,8 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
       within_half(static_cast<size_t>(rows) * (2 * (2 * D_ + 2 * F_ + (kept.size() == 2 ? 0 : 3 * F_)) + F_ / 8 + 4))) {
     const auto f32 = x.options().dtype(torch::kFloat32);
     try {
-      buffers = {torch::empty({rows, D_}, x.options()), torch::empty({rows, D_}, x.options()), torch::empty({rows}, f32),
+      buffers = {kept_x.defined() ? torch::Tensor() : torch::empty({rows, D_}, x.options()),
+                 torch::empty({rows, D_}, x.options()), torch::empty({rows}, f32),
                  torch::empty({rows, 2 * F_}, x.options()), torch::empty({rows, F_ / 32}, f32)};
       if (kept.size() != 2) {
         buffers.push_back(torch::empty({rows, 2 * F_}, x.options()));
@@ -1405,7 +1416,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
   }
   const QuiesceOnError guard{this};
   if (!buffers.empty()) {
-    backward_whole(x, g, w_flat, w_up, w_down, plan, inv_order, kept, buffers, dw_up, dw_down);
+    backward_whole(x, g, w_flat, w_up, w_down, plan, inv_order, kept, kept_x, buffers, dw_up, dw_down);
     // (dx and d_weight need nothing of the weight gradients, which are still running on the auxiliary stream)
     reduce_backward(inv_order, dx, d_weights, ev_tgu_[0]);
     return std::make_tuple(dx, d_weights, dw_up, dw_down);

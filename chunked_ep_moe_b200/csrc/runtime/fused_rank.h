@@ -212,7 +212,7 @@ class FusedRank {
                    const torch::Tensor& w_down) const;
   std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> forward_brief(torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat,
                                                                          torch::Tensor w_up, torch::Tensor w_down);
-  bool within_half(size_t bytes) const;
+  bool within_half(size_t bytes, int share = 2) const;  // (or another share of the device)
   GemmParams range_params(const int* plan, int64_t first, int64_t last) const;
   template <typename Part>
   void run_parts(int64_t parts, Part&& part);
@@ -220,7 +220,7 @@ class FusedRank {
       torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
       const std::vector<torch::Tensor>& kept, const std::vector<torch::Tensor>& buffers, bool training);
   void backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
-                      torch::Tensor plan, torch::Tensor inv_order, const std::vector<torch::Tensor>& kept,
+                      torch::Tensor plan, torch::Tensor inv_order, const std::vector<torch::Tensor>& kept, const torch::Tensor& kept_x,
                       const std::vector<torch::Tensor>& buffers, torch::Tensor dw_up, torch::Tensor dw_down);
   void put_whole(const torch::Tensor& plan, const torch::Tensor& inv_order, const torch::Tensor& x, const torch::Tensor* g,
                  const torch::Tensor& w_flat, __nv_bfloat16* to_x, __nv_bfloat16* to_g, float* to_w, int64_t first, int64_t last,

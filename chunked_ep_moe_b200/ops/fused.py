@@ -225,7 +225,8 @@ def memory_plan(world: int, experts: int, top_k: int, tokens_per_rank: int, hidd
             tk * 3 * F * 2 if (tk if alone else min(tk, S)) * D * F >= ext.keep_work else 0,
     }
     if alone:
-        out["during a pass that runs as one slice, while memory allows (x, g, dh by rows)"] = tk * (2 * D + 2 * F) * 2
+        out["during a pass that runs as one slice, while memory allows (x, g, dh by rows; x up to the backward, while a quarter of the "
+            "device allows)"] = tk * (2 * D + 2 * F) * 2
     out["total"] = sum(out.values())
     return out
 
