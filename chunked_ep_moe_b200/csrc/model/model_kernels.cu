@@ -7,7 +7,10 @@
 
 #include <cuda_bf16.h>
 
+#include <cfloat>
 #include <type_traits>
+
+#include "../common/umma.cuh"
 
 namespace cem {
 
@@ -244,29 +247,58 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* qkv, HeadM
   }
 }
 
+// e^x without the cases that `__expf` has for subnormals: a term below 2^-126 is nothing beside the largest, which is 1.
+__device__ __forceinline__ float exp_term(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // Cross-entropy of bf16 logits, one CTA per row: loss[row] = logsumexp(row) - row[target]; lse is kept for the backward.
+// Bound by the read of the logits as long as enough of it is in flight and the exponentials are all that a value costs beside two or three
+// other instructions: four 16-byte loads a thread, one rescaling of the sum for their 32 values, subtraction, scaling and sum two values an
+// instruction, the maximum on pairs of bf16. 8192 x 32000: 112 us with one load and one rescaling at a time, 103 us with four, 92 us like this
+// (5.2e8 bytes: 82 us at the measured copy rate).
 __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const __nv_bfloat16* logits, const int64_t* targets,
                                                                 float* loss, float* lse_out, int cols) {
+  constexpr int kAhead = 4;
+  constexpr float kLog2e = 1.4426950408889634f;
   __shared__ float s_m[8], s_s[8];
   const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int4* lr = reinterpret_cast<const int4*>(logits + static_cast<size_t>(row) * cols);
   const int units = cols >> 3;
-  float m = -INFINITY, sum = 0.0f;  // online softmax: sum of exp(v - m)
-  for (int u = threadIdx.x; u < units; u += blockDim.x) {
-    const int4 raw = lr[u];
-    const uint32_t wds[4] = {(uint32_t)raw.x, (uint32_t)raw.y, (uint32_t)raw.z, (uint32_t)raw.w};
-    float vals[8];
+  const f32x2 log2e = make_f32x2(kLog2e, kLog2e);
+  float m = -FLT_MAX, sum = 0.0f;  // online softmax: sum of exp(v - m); finite, so that a batch of -inf adds nothing
+  for (int u0 = threadIdx.x; u0 < units; u0 += kAhead * 256) {
+    int4 raw[kAhead];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) { vals[2 * e] = bf_lo(wds[e]); vals[2 * e + 1] = bf_hi(wds[e]); }
-    float mx = vals[0];
+    for (int k = 0; k < kAhead; ++k)  // (past the end the first once more: no larger a maximum, and left out of the sum)
+      raw[k] = lr[u0 + k * 256 < units ? u0 + k * 256 : u0];
+    __nv_bfloat162 top = *reinterpret_cast<const __nv_bfloat162*>(&raw[0].x);
 #pragma unroll
-    for (int e = 1; e < 8; ++e) mx = fmaxf(mx, vals[e]);
-    const float nm = fmaxf(m, mx);
-    float add = 0.0f;
+    for (int k = 0; k < kAhead; ++k) {
+      const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw[k]);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) add += __expf(vals[e] - nm);
-    sum = sum * __expf(m - nm) + add;
-    m = nm;
+      for (int e = 0; e < 4; ++e) top = __hmax2(top, pairs[e]);
+    }
+    const float mx = fmaxf(m, fmaxf(__low2float(top), __high2float(top)));
+    const f32x2 less = make_f32x2(-mx, -mx);
+    f32x2 add = make_f32x2(sum * exp_term((m - mx) * kLog2e), 0.0f);
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      if (u0 + k * 256 >= units) break;
+      const uint32_t wds[4] = {(uint32_t)raw[k].x, (uint32_t)raw[k].y, (uint32_t)raw[k].z, (uint32_t)raw[k].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float lo, hi;
+        split_f32x2(mul2(add2(make_f32x2(bf_lo(wds[e]), bf_hi(wds[e])), less), log2e), &lo, &hi);
+        add = add2(add, make_f32x2(exp_term(lo), exp_term(hi)));
+      }
+    }
+    float even, odd;
+    split_f32x2(add, &even, &odd);
+    sum = even + odd;
+    m = mx;
   }
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {

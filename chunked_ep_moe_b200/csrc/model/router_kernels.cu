@@ -8,6 +8,8 @@
 // fixed order (per warp over its rows, per block over its warps, then over blocks by the caller).
 #include "router_kernels.cuh"
 
+#include <cstdint>
+
 #include <math_constants.h>
 
 namespace cem {
@@ -23,6 +25,14 @@ __device__ __forceinline__ float warp_sum_f(float v) {
   return v;
 }
 
+// Unsigned integers in the order of floats (none of them NaN; both zeros the same).
+__device__ __forceinline__ uint32_t ordered_bits(float v) {
+  const uint32_t u = __float_as_uint(v + 0.0f);
+  return u ^ ((u >> 31) != 0 ? 0xffffffffu : 0x80000000u);
+}
+
+// What bounds it is a token's selection, one warp reduction after the other (as integers: one instruction each; ten shuffles and their
+// comparisons a choice before), and was the counts' atomics, one a choice to two lines of memory: 8192 tokens, top-6 of 64, 28 -> 8 us.
 template <int V>
 __global__ void __launch_bounds__(kRouterWarps * 32)
 router_fwd_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int* __restrict__ ids,
@@ -30,13 +40,18 @@ router_fwd_kernel(const float* __restrict__ logits, const float* __restrict__ bi
                   int top_k, float scaling) {
   constexpr int E = V * 32;
   __shared__ float s_acc[kRouterWarps][E];
+  __shared__ int s_counts[E];
+  for (int e = threadIdx.x; e < E; e += blockDim.x) s_counts[e] = 0;
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gw = blockIdx.x * kRouterWarps + warp, nw = gridDim.x * kRouterWarps;
   float b[V], acc[V];
+  int chosen[V];  // tokens of this warp that go to the lane's experts
 #pragma unroll
   for (int v = 0; v < V; ++v) {
     b[v] = bias[v * 32 + lane];
     acc[v] = 0.0f;
+    chosen[v] = 0;
   }
   for (int t = gw; t < T; t += nw) {
     float s[V], key[V];
@@ -62,21 +77,16 @@ router_fwd_kernel(const float* __restrict__ logits, const float* __restrict__ bi
           best_e = v * 32 + lane;
         }
       }
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, d);
-        const int oe = __shfl_xor_sync(0xffffffffu, best_e, d);
-        if (ob > best || (ob == best && oe < best_e)) {
-          best = ob;
-          best_e = oe;
-        }
-      }
+      // The largest key of all lanes, and of the lanes that have it the lowest expert.
+      const uint32_t ordered = ordered_bits(best), top = __reduce_max_sync(0xffffffffu, ordered);
+      best_e = __reduce_min_sync(0xffffffffu, ordered == top ? best_e : E);
       float sc = 0.0f;
 #pragma unroll
       for (int v = 0; v < V; ++v) {
         if (best_e == v * 32 + lane) {
           sc = s[v];
           key[v] = -CUDART_INF_F;
+          ++chosen[v];
         }
       }
       sc = __shfl_sync(0xffffffffu, sc, best_e & 31);
@@ -89,17 +99,20 @@ router_fwd_kernel(const float* __restrict__ logits, const float* __restrict__ bi
     if (lane < top_k) {
       ids[static_cast<size_t>(t) * top_k + lane] = my_id;
       weights[static_cast<size_t>(t) * top_k + lane] = my_score / fmaxf(chosen_sum, 1e-20f) * scaling;
-      atomicAdd(counts + my_id, 1);
     }
   }
 #pragma unroll
-  for (int v = 0; v < V; ++v) s_acc[warp][v * 32 + lane] = acc[v];
+  for (int v = 0; v < V; ++v) {
+    s_acc[warp][v * 32 + lane] = acc[v];
+    atomicAdd(s_counts + v * 32 + lane, chosen[v]);
+  }
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     float sum = 0.0f;
 #pragma unroll
     for (int w = 0; w < kRouterWarps; ++w) sum += s_acc[w][e];
     prob_partial[static_cast<size_t>(blockIdx.x) * E + e] = sum;
+    if (s_counts[e] > 0) atomicAdd(counts + e, s_counts[e]);
   }
 }
 

@@ -84,6 +84,46 @@ def test_cross_entropy(rows, cols):
     _close(logits.grad, ref.grad, "dlogits", 1e-2)
 
 
+@pytest.mark.parametrize("cols", [8, 2040, 2048, 2056, 8184, 8192, 8200, 10248])
+def test_cross_entropy_row_widths(cols):
+    """A thread's loads of a row full, partly and just filled; rows that begin with masked logits, have one in sight, have an infinity or a
+    NaN. The log-sum-exp is fp32 sums of positive terms: 2^-24 for each of the at most 8 + 13 additions and 4 roundings on a term's way,
+    and of the result."""
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    logits = (4 * torch.randn(9, cols, device="cuda", generator=gen)).bfloat16()
+    logits[0, : cols - 1] = -float("inf")
+    logits[1, : cols // 2] = -float("inf")
+    logits[2, cols // 2] = float("nan")
+    logits[3, cols // 2] = float("inf")
+    logits[4] = -1e30
+    targets = torch.full((9,), cols - 1, device="cuda")
+    loss, lse = fused_ops._ext().cross_entropy_fwd(logits, targets)
+    want = torch.logsumexp(logits.double(), 1)
+    assert torch.isnan(lse[2]) and not torch.isfinite(loss[3])
+    rest = [0, 1, 4, 5, 6, 7, 8]
+    assert ((lse.double() - want).abs() <= (64 + want.abs()) * 2.0**-24)[rest].all()
+    torch.testing.assert_close(loss[rest], (want - logits[:, -1].double())[rest].float(), rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("tokens,experts,top_k", [(1, 32, 32), (700, 64, 6), (5000, 256, 8)])
+def test_router_select_of_equal_and_negative_scores(tokens, experts, top_k):
+    """Ties go to the lower expert, zeros of either sign are equal, and the order holds below zero; the counts are those of the ids."""
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    logits = torch.randint(-2, 3, (tokens, experts), generator=gen, device="cuda").float()
+    bias = torch.randint(-3, 1, (experts,), generator=gen, device="cuda").float()
+    logits[0] = float("-inf")  # scores of 0
+    bias[::2], bias[1::3] = 0.0, -0.0
+    ids, _, counts, _ = fused_ops.router_select(logits, bias, top_k, 1.0)
+    keys = 1.0 / (1.0 + torch.exp(-logits)) + bias
+    order = torch.sort(keys, dim=1, descending=True, stable=True).indices[:, :top_k]
+    picked, best = torch.gather(keys, 1, ids.long()), torch.gather(keys, 1, order)
+    assert torch.equal(ids[0].long(), order[0])
+    # (exp and the kernel's differ in the last bits, so that sums which are equal in one may not be in the other)
+    assert (picked - best).abs().max() <= 1e-6
+    assert (torch.sort(ids.long(), dim=1).values.diff(dim=1) > 0).all()
+    assert torch.equal(counts.long(), torch.bincount(ids.long().reshape(-1), minlength=experts))
+
+
 @pytest.mark.parametrize("tokens,experts,top_k", [(1000, 64, 6), (8192, 256, 8), (7, 32, 1), (333, 96, 5)])
 def test_router_select(tokens, experts, top_k):
     """Selection, weights, load counts, score sums and the gradient w.r.t. the logits against fp64 torch ops."""
