@@ -18,9 +18,11 @@ row_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CU
 
 int row_gemm_smem_bytes() { return kRowSmemBytes; }
 
-void launch_row_gemm(int mode, const GemmParams& p, const CUtensorMap& map_a, const TokenMaps& maps_b, int grid,
+void launch_row_gemm(int mode, const GemmParams& params, const CUtensorMap& map_a, const TokenMaps& maps_b, int grid,
                      cudaStream_t stream, bool behind) {
   grid &= ~1;  // whole pairs only
+  GemmParams p = params;
+  if (p.last_expert == 0 && p.n_tiles * p.k_blocks >= kByExpert) p.last_expert = p.lay.L;  // all experts, their tiles by expert
 #define CEM_LAUNCH_ROW(M, RANGED)                                                                                        \
   {                                                                                                                      \
     static const int resident = resident_pair_grid(row_gemm_kernel<M, RANGED>, kRowThreads, kRowSmemBytes);              \

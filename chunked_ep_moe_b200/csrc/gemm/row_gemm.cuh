@@ -41,7 +41,9 @@ constexpr int kRowStagesOf = MODE == kModeDswiglu ? 5 : 6;
 constexpr int kRowStageBytesA = kBlockM * kBlockK * 2;  // this CTA's 128 weight columns
 constexpr int kRowStageBytesB = (kTileTokens / 2) * kBlockK * 2;  // up to 128 rows
 constexpr int kRowStageBytes = kRowStageBytesA + kRowStageBytesB;
-constexpr int kRowBand = 4;                             // token tiles swept together over the weight columns
+constexpr int kRowBand = 4;                             // token tiles swept together over the weight columns, in short launches
+constexpr int kRowBandMax = 12;                         // and of one expert in long ones
+constexpr int kByExpert = 512;                          // 256 x 64 pieces of an expert's weights (32 KB) from which this pays: 16 MB
 constexpr int kRowThreads = 64 + 8 * 32;
 constexpr int kGroupStaging = 16384;                    // per epilogue group
 constexpr int kRowSmemBytes = kSmemAlignSlack + 6 * kRowStageBytes + 2 * kGroupStaging + kSmemTailBytes;
@@ -70,19 +72,44 @@ struct FewRows {
 // `RANGED`: the tiles of a range of experts. A variant of its own, with the range's first entry in shared memory: as a register of every
 // warp it made the SwiGLU' GEMM spill, and passes without ranges up to 1.4 % slower (620 rows of 107 experts at D=1792, F=512, forward
 // 134.1 -> 135.2 us; the expert kernels on 6086 rows of 9 experts at D=256, F=1024 127.7 -> 129.5).
+//
+// The order of the tiles decides how often weights and rows come from DRAM or from the other die's L2, and under the power cap that is
+// time: 32 experts x 2048 rows, D=7168, F=2048, the up-projection runs at 1177 TFLOP/s and, with every load from a few lines in the nearest
+// L2, at 1413. So an expert's tiles go over its weight columns together, up to `kRowBandMax` at a time, and its weights are read once; by
+// fours, wherever experts end, the bands of one expert find them gone (an expert's are 59 and 29 MB; a die's L2 holds 63, of both dies'
+// lines). DRAM reads at 8 experts: up-projection 1289 -> 1075 MB, dX 893 -> 631, down-projection 307 -> 302. Forward + backward of
+// 8192 x 8 rows of 32 experts 1.033 and 1.031 times as fast, 4096 x 8 rows (fp8 put) 1.02, Zipf routing in slices of 2048 rows 1.02, 256 rows
+// per expert 1.00 to 1.02. At most 8 or 6 at a time: 1.019 and 1.000. (Cache hints gave nothing, weights as evict-first took 5 %.)
+// The way to a tile is two dependent loads longer: in launches of few or cheap tiles 1 us of 50, and what an expert's bands share is still
+// in L2 there. So by fours below 16 MB of weights an expert (`kByExpert`: the launcher then takes the variant without ranges) and below
+// four tiles a pair.
 template <bool RANGED>
 __device__ __forceinline__ RowTile decode_row_tile(const GemmParams& p, int t, volatile const int* first_entry, int num_entries,
                                                    const FewRows* few = nullptr) {
   RowTile tl;
-  const int band_tiles = kRowBand * p.n_tiles;
-  const int band = t / band_tiles, rem = t - band * band_tiles;
-  int width = num_entries - band * kRowBand;
-  width = width > kRowBand ? kRowBand : width;
-  tl.n = rem / width;
-  const int ti = band * kRowBand + (rem - tl.n * width);
   const int first = RANGED ? *first_entry : 0;
-  const int4 e = few != nullptr ? few->tiles[ti]
-                                : reinterpret_cast<const int4*>(p.plan + p.lay.off_tiles + 4 * p.lay.max_tiles * p.slice)[first + ti];
+  const int4* tiles = reinterpret_cast<const int4*>(p.plan + p.lay.off_tiles + 4 * p.lay.max_tiles * p.slice) + first;
+  int ti;
+  if (RANGED && p.n_tiles * p.k_blocks >= kByExpert && num_entries * p.n_tiles >= 4 * static_cast<int>(gridDim.x >> 1)) {
+    // (every expert's tiles take the places of its entries, times the weight columns)
+    const int* start = p.plan + p.lay.off_tile_start + (p.lay.L + 1) * p.slice + tiles[t / p.n_tiles].x;
+    const int begin = start[0] - first, count = start[1] - first - begin;
+    const int bands = (count + kRowBandMax - 1) / kRowBandMax, most = (count + bands - 1) / bands;
+    int rem = t - begin * p.n_tiles;
+    const int in_band = rem / (most * p.n_tiles) * most;
+    rem -= in_band * p.n_tiles;
+    const int width = min(most, count - in_band);
+    tl.n = rem / width;
+    ti = begin + in_band + (rem - tl.n * width);
+  } else {
+    const int band_tiles = kRowBand * p.n_tiles;
+    const int band = t / band_tiles, rem = t - band * band_tiles;
+    int width = num_entries - band * kRowBand;
+    width = width > kRowBand ? kRowBand : width;
+    tl.n = rem / width;
+    ti = band * kRowBand + (rem - tl.n * width);
+  }
+  const int4 e = few != nullptr ? few->tiles[ti] : tiles[ti];
   tl.g = e.x; tl.row0 = e.y; tl.nrows = e.z; tl.ncols = e.w;
   return tl;
 }
@@ -209,12 +236,17 @@ __device__ __forceinline__ void publish_few(const GemmParams& p, const FewPlan& 
     const int n = count & 0xff;
     if (n > 0) {
       reinterpret_cast<int4*>(out.plan + p.lay.off_tiles)[count >> 8] = make_int4(e, first_row, n, kTileUnit);
+      out.plan[p.lay.off_tile_start + e] = count >> 8;
+      out.plan[p.lay.off_tile_start + e + 1] = (count >> 8) + 1;  // (what the next expert writes, if it has a tile)
       out.plan[p.lay.off_in_start + e] = first_row;
       out.plan[p.lay.off_in_size + e] = n;
       out.plan[p.lay.off_src_send_start + e] = first_row;
     }
   }
-  if (lane == 0) out.plan[p.lay.off_num_tiles] = tiles;
+  if (lane == 0) {
+    out.plan[p.lay.off_num_tiles] = tiles;
+    out.plan[p.lay.off_tile_start + p.lay.L] = tiles;
+  }
   // header: slices, rows of the stream (mine, the fullest), rows for other ranks, too many slices, token copies
   int word = lane == 0 ? 1 : lane == 1 || lane == 2 || lane == 5 ? rows : 0;
   if (lane < kPlanHeaderInts) out.plan[lane] = word;
@@ -725,7 +757,7 @@ __device__ __forceinline__ void row_gemm_body(const GemmParams& p, const CUtenso
   if (!gave_up) {
     if constexpr (RANGED) {
       const int* start = p.plan + p.lay.off_tile_start + (p.lay.L + 1) * p.slice;
-      const int first = start[p.first_expert];
+      const int first = p.first_expert > 0 ? start[p.first_expert] : 0;  // (past the last slice only start[L] is written)
       num_entries = start[p.last_expert] - first;
       *first_entry = first;  // (the same from every thread; each reads back what it has written itself)
     } else if constexpr (SRC == kRowsFew) {

@@ -182,3 +182,34 @@ def test_weight_gradients_of_many_small_experts():
             # rounded once to bf16: 2^-9 of the value; the fp32 sums of up to 700 products differ by far less
             assert torch.linalg.vector_norm(out[g].float() - want) <= 2.0**-8 * torch.linalg.vector_norm(want), g
     fx.check_status()
+
+
+def test_tiles_in_the_order_of_their_experts():
+    """Large weights: an expert's tiles (none, 1, 2, 12, 13, 25) go over its weight columns together, at most 12 at a time. Every mode has the
+    bits of calls on pieces of one expert's rows that are too short for that order."""
+    D, F, stripe = 4096, 2048, 64
+    groups = [0, 1, 3072, 3073, 0, 6400, 31, 257]
+    S, L = sum(groups) + 6, len(groups)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x, dy = [torch.randn(S, D, generator=gen, device="cuda").bfloat16() for _ in range(2)]
+    w_up = (0.02 * torch.randn(L, D, 2 * F, generator=gen, device="cuda")).bfloat16()
+    w_down = (0.02 * torch.randn(L, F, D, generator=gen, device="cuda")).bfloat16()
+
+    def every_mode(x, dy, w_up, w_down, groups):
+        act, h = fx.gmm_swiglu(x, w_up, groups, stripe=stripe, return_h=True)
+        return [act, h, fx.gmm(act, w_down, groups, stripe=stripe), fx.gmm(h, w_up, groups, transpose_rhs=True, stripe=stripe),
+                fx.gmm_dswiglu(dy, w_down, h, groups, stripe=stripe)]
+
+    whole = every_mode(x, dy, w_up, w_down, groups)
+    assert all(torch.count_nonzero(t[sum(groups):]) == 0 for t in whole)
+    at = 0
+    for g, n in enumerate(groups):
+        for begin in range(0, n, 1024):
+            rows = min(1024, n - begin)
+            piece = slice(at + begin, at + begin + rows)
+            xs, dys = [torch.nn.functional.pad(t[piece], (0, 0, 0, -rows % 8)) for t in (x, dy)]
+            alone = every_mode(xs, dys, w_up[g:g + 1], w_down[g:g + 1], [rows])
+            for name, a, b in zip(("act", "h", "y", "dx", "dh"), whole, alone):
+                assert torch.equal(a[piece], b[:rows]), (name, g, begin)
+        at += n
+    fx.check_status()
