@@ -18,7 +18,8 @@ reached the host. Compared with the reference's loop
     straddles a slice boundary carries an fp32 partial to the next slice;
   * a rank on its own exchanges nothing, so its passes run as ONE slice, in up to eight ranges of experts, as long as their
     buffers fit beside what is live in half of the device's memory (`FusedRank::runs_whole`); slice by slice otherwise, with
-    `always_slice` and under saved-tensor hooks.
+    `always_slice` and under saved-tensor hooks. Passes of one range also keep x in expert order, as long as live tensors stay within a
+    quarter of the device; forwards of few tokens gather their rows in the up-projection (`FusedRank::runs_brief`).
 
 Everything else the backward needs are the inputs and the integer plan (tables, send order, its inverse).
 """
