@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* qkv, HeadM
   }
 }
 
-// e^x without the cases that `__expf` has for subnormals: a term below 2^-126 is nothing beside the largest, which is 1.
-__device__ __forceinline__ float exp_term(float x) {
+// 2^x, subnormal results flushed to zero: a term below 2^-126 is nothing beside the largest, which is 1.
+__device__ __forceinline__ float exp2_term(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const __nv_bfloa
     }
     const float mx = fmaxf(m, fmaxf(__low2float(top), __high2float(top)));
     const f32x2 less = make_f32x2(-mx, -mx);
-    f32x2 add = make_f32x2(sum * exp_term((m - mx) * kLog2e), 0.0f);
+    f32x2 add = make_f32x2(sum * exp2_term((m - mx) * kLog2e), 0.0f);
 #pragma unroll
     for (int k = 0; k < kAhead; ++k) {
       if (u0 + k * 256 >= units) break;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const __nv_bfloa
       for (int e = 0; e < 4; ++e) {
         float lo, hi;
         split_f32x2(mul2(add2(make_f32x2(bf_lo(wds[e]), bf_hi(wds[e])), less), log2e), &lo, &hi);
-        add = add2(add, make_f32x2(exp_term(lo), exp_term(hi)));
+        add = add2(add, make_f32x2(exp2_term(lo), exp2_term(hi)));
       }
     }
     float even, odd;
