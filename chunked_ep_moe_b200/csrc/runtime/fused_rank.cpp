@@ -123,9 +123,8 @@ FusedRank::FusedRank(int P, int L, int me, int S, int D, int F, int K, int strip
   arena_lay_ = make_arena_layout(P, L, S, D, tk_cap, fp8);
   arena_ = reinterpret_cast<uint8_t*>(arena);
   cudaDeviceProp prop;
-  int device = 0;
-  cuda_check(cudaGetDevice(&device), "device");
-  cuda_check(cudaGetDeviceProperties(&prop, device), "device properties");
+  cuda_check(cudaGetDevice(&device_), "device");
+  cuda_check(cudaGetDeviceProperties(&prop, device_), "device properties");
   device_bytes_ = prop.totalGlobalMem;
   if (const char* v = std::getenv("CEM_KEEP_ACTIVATIONS")) keep_activations_ = std::atoi(v) != 0;
   for (int64_t p : peer_arenas) peers_.push_back(reinterpret_cast<uint8_t*>(p));
@@ -238,6 +237,17 @@ FusedRank::~FusedRank() {
   if (host_header_) cudaFreeHost(host_header_);
 }
 
+void FusedRank::release() {
+  const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
+  released_ = true;
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_));
+  cudaDeviceSynchronize();  // (an error of the device is raised by whoever frees the arena)
+}
+
+void FusedRank::expect_arena(const char* what) const {
+  expect(!released_, std::string("chunked_moe fused path: the workspace of this pass was released before its ") + what);
+}
+
 void FusedRank::check_status() {
   const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
   cudaStream_t st = current_stream();
@@ -269,6 +279,7 @@ std::string format_status(const std::vector<int64_t>& s, int rank) {
 
 void FusedRank::sort_only(torch::Tensor expert_ids, torch::Tensor order, torch::Tensor inv_order,
                           torch::Tensor my_counts) {
+  expect_arena("step");
   const int64_t tk = expert_ids.numel();
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
   expect_i32(expert_ids, tk, "expert_ids");
@@ -283,6 +294,7 @@ void FusedRank::sort_only(torch::Tensor expert_ids, torch::Tensor order, torch::
 
 int64_t FusedRank::begin_forward_async(torch::Tensor expert_ids, torch::Tensor plan, torch::Tensor order,
                                        torch::Tensor inv_order, torch::Tensor counts, bool counts_prefilled) {
+  expect_arena("step");
   cudaStream_t st = current_stream();
   const int64_t tk = expert_ids.numel();
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
@@ -410,6 +422,7 @@ int64_t FusedRank::begin_forward(torch::Tensor expert_ids, torch::Tensor plan, t
 
 
 int64_t FusedRank::begin_backward(torch::Tensor plan, int64_t known_slices, int64_t known_rows) {
+  expect_arena("step");
   cudaStream_t st = current_stream();
   expect_i32(plan, lay_.total, "plan");
   enter_pass();
@@ -461,6 +474,7 @@ void FusedRank::begin_pass(const torch::Tensor& plan, int64_t slices, int64_t ro
 
 void FusedRank::put(int64_t j, torch::Tensor plan, torch::Tensor order, torch::Tensor x,
                     c10::optional<torch::Tensor> g, torch::Tensor w_flat) {
+  expect_arena("step");
   expect(j >= 0 && j < cur_slices_, "slice index out of range");
   expect_bf16_2d(x, D_, "x");
   if (g.has_value()) expect_bf16_2d(*g, D_, "g");
@@ -620,6 +634,7 @@ void expect_weights(const torch::Tensor& w_up, const torch::Tensor& w_down, int 
 // later one's CTAs start as the earlier one's CTAs finish, i.e. every kernel fills the idle tail of the previous
 // (independent) one instead of waiting for it. Scratch reuse and the carry chain are ordered by events.
 void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_up, torch::Tensor w_down) {
+  expect_arena("step");
   expect(j >= 0 && j < cur_slices_, "slice index out of range");
   expect_weights(w_up, w_down, L_, D_, F_);
   const bool async = overlapped();
@@ -679,6 +694,7 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
 
 void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_up, torch::Tensor w_down,
                                  torch::Tensor dw_up, torch::Tensor dw_down) {
+  expect_arena("step");
   expect(j >= 0 && j < cur_slices_, "slice index out of range");
   expect_weights(w_up, w_down, L_, D_, F_);
   expect_weights(dw_up, dw_down, L_, D_, F_);
@@ -858,6 +874,7 @@ std::vector<torch::Tensor> FusedRank::allocate_kept(int64_t rows, int64_t slice_
 }
 
 void FusedRank::finish_forward(torch::Tensor inv_order, torch::Tensor out) {
+  expect_arena("step");
   expect_bf16_2d(out, D_, "out");
   expect(out.size(0) * K_ == cur_rows_, "out rows do not match the pass");
   expect_i32(inv_order, cur_rows_, "inv_order");
@@ -883,6 +900,7 @@ void FusedRank::finish_forward(torch::Tensor inv_order, torch::Tensor out) {
 }
 
 void FusedRank::reduce_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights, cudaEvent_t after) {
+  expect_arena("step");
   expect_bf16_2d(dx, D_, "dx");
   expect(dx.size(0) * K_ == cur_rows_, "dx rows do not match the pass");
   expect(d_weights.is_cuda() && d_weights.scalar_type() == torch::kFloat32 && d_weights.is_contiguous() &&
@@ -1297,6 +1315,7 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
     torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
     bool training) {
   const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
+  expect_arena("forward");
   const int64_t tk = expert_ids.numel();
   release_kept();  // (of a pass that threw)
   short_pass_ = false;
@@ -1385,6 +1404,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
     torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
     const std::vector<torch::Tensor>& saved, int64_t kept_slices) {
   const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
+  expect_arena("backward");
   inline_ = short_pass_ = false;  // (also behind a forward that threw)
   release_kept();
   const int64_t rows = order.numel();

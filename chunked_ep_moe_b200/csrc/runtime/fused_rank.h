@@ -16,7 +16,6 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <map>
 #include <mutex>
 #include <algorithm>
@@ -138,12 +137,9 @@ class FusedRank {
       torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
       const std::vector<torch::Tensor>& kept, int64_t kept_slices);
 
-  // The arena is about to go: a backward that still comes is refused.
-  void release() {
-    const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);  // (not in the middle of a backward on another thread)
-    released_ = true;
-  }
-  bool released() const { return released_; }
+  // The arena is about to go. Waits for the pass under way on another thread and for the device; whatever comes later is refused
+  // behind the same lock, before it launches anything.
+  void release();
 
   // Reads the status block (synchronises); throws std::runtime_error describing the first recorded error.
   void check_status();
@@ -171,6 +167,7 @@ class FusedRank {
   void begin_pass(const torch::Tensor& plan, int64_t slices, int64_t rows, int pieces_per_row,
                   bool targets_set = false);
   void enter_pass();
+  void expect_arena(const char* what) const;
   // `after`: an event that the caller's stream waits for behind the pass's last kernel, or null.
   void reduce_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights, cudaEvent_t after);
   void end_pass(int64_t n_slices);
@@ -253,6 +250,7 @@ class FusedRank {
   torch::Tensor act_[2], h_[2], dh_[2], dwp_[2];
   torch::Tensor kept_h_, kept_act_;  // of the current pass: [rows, 2F], [rows, F] of its first kept_slices_ slices
   int64_t kept_slices_ = 0;
+  int device_ = 0;
   size_t device_bytes_ = 0;
   bool keep_activations_ = true;  // CEM_KEEP_ACTIVATIONS=0: always recompute (least memory)
   torch::Tensor carry_up_, carry_down_, pass_base_, expected_total_, status_, tables_,
@@ -272,7 +270,7 @@ class FusedRank {
   // One pass (as one call) or status check at a time: a forward on the caller's thread and a backward on the autograd engine's share all
   // of the above and the counters below.
   std::recursive_mutex pass_mutex_;
-  std::atomic<bool> released_{false};
+  bool released_ = false;
   cudaStream_t comm_stream_ = nullptr, aux_stream_ = nullptr, chain_[2] = {};
   cudaStream_t expand_stream_ = nullptr;  // fp8 wire: the expansion kernels run here, beside the GEMM chains
   cudaEvent_t ev_expand_[4] = {};  // expansion of slice j (mod 4) has finished

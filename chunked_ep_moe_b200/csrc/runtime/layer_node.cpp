@@ -40,8 +40,6 @@ struct Layer : public torch::autograd::Function<Layer> {
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const auto saved = ctx->get_saved_variables();  // (hooks run here, before anything is locked)
     const std::shared_ptr<FusedRank> rank = static_cast<Held*>(ctx->saved_data["rank"].toCapsule().get())->rank;
-    if (rank->released())
-      throw std::runtime_error("chunked_moe fused path: the workspace of this pass was released before its backward");
     const torch::Tensor &x = saved[0], &weights = saved[1];
     const torch::Tensor g = grads[0].to(x.scalar_type()).contiguous();
     const std::vector<torch::Tensor> kept(saved.begin() + 7, saved.end());
@@ -57,6 +55,8 @@ struct Layer : public torch::autograd::Function<Layer> {
 
 torch::Tensor chunked_moe_layer(std::shared_ptr<FusedRank> rank, const torch::Tensor& x, const torch::Tensor& expert_ids,
                                 const torch::Tensor& weights, const torch::Tensor& w_up, const torch::Tensor& w_down) {
+  // (Released between the caller's look-up and this call; what is released later is refused by the pass.)
+  if (rank == nullptr) throw std::runtime_error("chunked_moe fused path: the workspace was released before the forward");
   bool training = false;
   if (at::GradMode::is_enabled())
     training = x.requires_grad() || weights.requires_grad() || w_up.requires_grad() || w_down.requires_grad();
