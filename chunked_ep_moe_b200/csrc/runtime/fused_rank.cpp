@@ -53,9 +53,15 @@ inline cudaStream_t current_stream() { return at::cuda::getCurrentCUDAStream().s
     if (!(cond)) throw std::runtime_error(msg);      \
   } while (0)
 
+// What kernels read and write 16 bytes at a time begins at an address of 16 bytes (a contiguous view may begin anywhere).
+void expect_at_16(const torch::Tensor& t, const char* name) {
+  expect(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, std::string(name) + " must be at an address of 16 bytes");
+}
+
 void expect_bf16_2d(const torch::Tensor& t, int64_t cols, const char* name) {
   expect(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 2 && t.size(1) == cols && t.is_contiguous(),
          std::string(name) + " must be a contiguous CUDA bf16 matrix with " + std::to_string(cols) + " columns");
+  expect_at_16(t, name);
 }
 
 void expect_i32(const torch::Tensor& t, int64_t min_numel, const char* name) {
@@ -299,6 +305,7 @@ int64_t FusedRank::begin_forward_async(torch::Tensor expert_ids, torch::Tensor p
   const int64_t tk = expert_ids.numel();
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
   expect_i32(plan, lay_.total, "plan");
+  expect_at_16(plan, "plan");
   enter_pass();
   header_whole_ = false;
   PlanKernelParams pp{};
@@ -425,6 +432,7 @@ int64_t FusedRank::begin_backward(torch::Tensor plan, int64_t known_slices, int6
   expect_arena("step");
   cudaStream_t st = current_stream();
   expect_i32(plan, lay_.total, "plan");
+  expect_at_16(plan, "plan");
   enter_pass();
   if (known_slices >= 0 && known_rows >= 0) {
     // The caller kept what the forward of this plan read back: no device-to-host copy, no synchronisation, so the
@@ -849,6 +857,8 @@ void FusedRank::keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices) {
              act.is_cuda() && act.is_contiguous() && act.scalar_type() == torch::kBFloat16 && act.dim() == 2 &&
              act.size(1) == F_ && act.size(0) == h.size(0) && act.size(0) > (slices - 1) * S_,
          "kept activations must be contiguous CUDA bf16 [rows, 2F] and [rows, F] matrices that reach into every slice");
+  expect_at_16(h, "kept h");
+  expect_at_16(act, "kept w * act");
   kept_h_ = h;
   kept_act_ = act;
   kept_slices_ = slices;
@@ -1028,7 +1038,6 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_whol
                 inv_order = torch::empty({tk}, i32), out = torch::empty_like(x);
   const torch::Tensor &rows_x = buffers[0], &rows_w = buffers[1], &act = kept.empty() ? buffers[2] : kept[1];
   const QuiesceOnError guard{this};
-  expect_pass(x, expert_ids, w_flat, w_up, w_down);
   enter_pass();
   header_whole_ = true;
   cur_slices_ = 0;  // (no streams of slices to join)
@@ -1113,12 +1122,11 @@ void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w
                                const std::vector<torch::Tensor>& buffers, torch::Tensor dw_up, torch::Tensor dw_down) {
   cudaStream_t st = current_stream();
   const int64_t tk = inv_order.numel();
-  expect_i32(plan, whole_lay_.total, "plan");
-  expect_bf16_2d(x, D_, "x");
-  expect_bf16_2d(g, D_, "g");
-  expect(g.size(0) == x.size(0) && x.size(0) * K_ == tk, "x and g rows do not match the pass");
-  expect_weights(w_up, w_down, L_, D_, F_);
-  expect_weights(dw_up, dw_down, L_, D_, F_);
+  if (!kept.empty()) {
+    expect_bf16_2d(kept[0], 2 * F_, "kept h");
+    expect_bf16_2d(kept[1], F_, "kept w * act");
+    expect(kept[0].size(0) == tk && kept[1].size(0) == tk, "kept rows do not match the pass");
+  }
   enter_pass();
   cur_slices_ = 0;
   cur_rows_ = tk;
@@ -1240,7 +1248,6 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brie
   torch::Tensor plan = torch::empty({whole_lay_.total}, i32), order = torch::empty({tk}, i32),
                 inv_order = torch::empty({tk}, i32), out = torch::empty_like(x);
   const QuiesceOnError guard{this};
-  expect_pass(x, expert_ids, w_flat, w_up, w_down);
   enter_pass();
   header_whole_ = true;
   cur_slices_ = 0;
@@ -1320,7 +1327,8 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
   release_kept();  // (of a pass that threw)
   short_pass_ = false;
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
-  if (runs_brief(x.dim() == 2 ? x.size(0) : 0, tk, training)) return forward_brief(x, expert_ids, w_flat, w_up, w_down);
+  expect_pass(x, expert_ids, w_flat, w_up, w_down);
+  if (runs_brief(x.size(0), tk, training)) return forward_brief(x, expert_ids, w_flat, w_up, w_down);
   // Under saved-tensor hooks a pass keeps nothing and runs slice by slice: whether it may do otherwise depends on the free memory,
   // and its backward may get the plan of a recomputation.
   const bool hooks = training && at::SavedTensorDefaultHooks::get_hooks().has_value();
@@ -1408,6 +1416,13 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
   inline_ = short_pass_ = false;  // (also behind a forward that threw)
   release_kept();
   const int64_t rows = order.numel();
+  expect_bf16_2d(x, D_, "x");
+  expect_bf16_2d(g, D_, "g");
+  expect(g.size(0) == x.size(0) && x.size(0) * K_ == rows, "x and g rows do not match the pass");
+  expect_weights(w_up, w_down, L_, D_, F_);
+  expect_i32(inv_order, rows, "inv_order");
+  expect_i32(plan, known_slices == kWholePass ? whole_lay_.total : lay_.total, "plan");
+  expect_at_16(plan, "plan");
   // Saved: h and w * act, x by rows, both or neither.
   const std::vector<torch::Tensor> kept(saved.begin(), saved.size() >= 2 ? saved.begin() + 2 : saved.begin());
   const torch::Tensor kept_x = saved.size() % 2 == 1 ? saved.back() : torch::Tensor();

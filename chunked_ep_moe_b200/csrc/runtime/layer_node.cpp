@@ -1,5 +1,6 @@
 #include "layer_node.h"
 
+#include <cstdint>
 #include <stdexcept>
 
 namespace cem {
@@ -11,6 +12,13 @@ struct Held : torch::CustomClassHolder {
   explicit Held(std::shared_ptr<FusedRank> r) : rank(std::move(r)) {}
   std::shared_ptr<FusedRank> rank;
 };
+
+// Contiguous, and at an address of 16 bytes: what a pass reads 16 bytes at a time without a tensor map, which would refuse others. A
+// contiguous view may begin anywhere.
+torch::Tensor aligned(const torch::Tensor& t) {
+  const torch::Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 ? c : c.clone();
+}
 
 // In C++ because the host is what bounds small passes: a node written in Python, its checks and conversions took 145 of 215 us a step
 // of forward + backward of 192 tokens at D=F=256, and 22 of 46 us a one-token forward, during which the device idles: the forward ends
@@ -24,7 +32,7 @@ struct Layer : public torch::autograd::Function<Layer> {
                                const torch::Tensor& weights, const torch::Tensor& w_up, const torch::Tensor& w_down,
                                const std::shared_ptr<FusedRank>& rank, bool training) {
     const torch::Tensor ids = expert_ids.to(torch::kInt32).contiguous(), w_flat = router_weights(weights);
-    const torch::Tensor xc = x.detach().contiguous(), up = w_up.detach().contiguous(), down = w_down.detach().contiguous();
+    const torch::Tensor xc = aligned(x.detach()), up = w_up.detach().contiguous(), down = w_down.detach().contiguous();
     auto [made, slices, kept_slices] = rank->forward_pass(xc, ids, w_flat, up, down, training);
     if (training) {
       torch::autograd::variable_list saved{xc, weights, up, down};
@@ -40,11 +48,12 @@ struct Layer : public torch::autograd::Function<Layer> {
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const auto saved = ctx->get_saved_variables();  // (hooks run here, before anything is locked)
     const std::shared_ptr<FusedRank> rank = static_cast<Held*>(ctx->saved_data["rank"].toCapsule().get())->rank;
-    const torch::Tensor &x = saved[0], &weights = saved[1];
-    const torch::Tensor g = grads[0].to(x.scalar_type()).contiguous();
+    // (x and the plan's tables too: hooks may have put them elsewhere)
+    const torch::Tensor x = aligned(saved[0]), plan = aligned(saved[4]), &weights = saved[1];
+    const torch::Tensor g = aligned(grads[0].to(x.scalar_type()));
     const std::vector<torch::Tensor> kept(saved.begin() + 7, saved.end());
     auto [dx, d_weights, dw_up, dw_down] =
-        rank->backward_pass(x, g, router_weights(weights), saved[2], saved[3], saved[4], saved[5], saved[6],
+        rank->backward_pass(x, g, router_weights(weights), saved[2], saved[3], plan, saved[5], saved[6],
                             ctx->saved_data["slices"].toInt(), kept, ctx->saved_data["kept_slices"].toInt());
     return {dx, torch::Tensor(), d_weights.reshape(weights.sizes()).to(weights.scalar_type()), dw_up, dw_down, torch::Tensor(),
             torch::Tensor()};

@@ -213,3 +213,17 @@ def test_tiles_in_the_order_of_their_experts():
                 assert torch.equal(a[piece], b[:rows]), (name, g, begin)
         at += n
     fx.check_status()
+
+
+def test_kernels_refuse_rows_at_odd_addresses():
+    """h and w * act are read 16 bytes at a time beside the tensor maps, which refuse other addresses of the operands."""
+    S, D, F = 64, 256, 256
+    bf = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    shifted = lambda t: torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t)
+    x, h, w_up, w_down = bf(S, D), bf(S, 2 * F), bf(2, D, 2 * F), bf(2, F, D)
+    for call in (lambda: fx.gmm_dswiglu(x, w_down, shifted(h), [30, 34], stripe=64),
+                 lambda: fx.gmm_dswiglu(shifted(x), w_down, h, [30, 34], stripe=64),
+                 lambda: fx.gmm_swiglu(shifted(x), w_up, [30, 34], stripe=64), lambda: fx.gmm(shifted(x), w_up, [30, 34])):
+        with pytest.raises(RuntimeError, match="16 bytes|16-byte"):
+            call()
+    fx.check_status()
