@@ -112,7 +112,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("arena_layout", &arena_layout_dict, "byte offsets inside one rank's symmetric arena");
   m.def("arena_read_i32", &cem::arena_read_i32, "device synchronise + copy int32 values of an arena to the host");
   m.attr("gemm_smem_bytes") = cem::row_gemm_smem_bytes();
-  m.def("pair_grid_used", []() { return cem::g_pair_grid_used; }, "grid of the last GEMM launch");
+  m.def("pair_grid_used", []() { return cem::g_pair_grid_used.load(); }, "grid of the last GEMM launch");
   m.attr("keep_work") = cem::kKeepWork;
   m.attr("plan_small") = py::make_tuple(cem::kPlanSmallIds, cem::kPlanSmallExperts);
   m.def("wait_probe", &wait_probe, "bounded-wait self test kernel");
@@ -138,8 +138,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("gmm_dswiglu", &cem::KernelRunner::gmm_dswiglu)
       .def("tgmm", &cem::KernelRunner::tgmm)
       .def("check_status", &cem::KernelRunner::check_status);
-  // Passes run without the interpreter's lock: those of a rank have one of their own, which a backward on the engine's thread may hold.
-  m.def("chunked_moe_layer", &cem::chunked_moe_layer, py::call_guard<py::gil_scoped_release>(),
+  // Whatever may wait for a rank's lock does so without the interpreter's: a pass on another thread holds the one and may need the other.
+  using NoGil = py::call_guard<py::gil_scoped_release>;
+  m.def("chunked_moe_layer", &cem::chunked_moe_layer, NoGil(),
         "(rank, x, expert_ids, router_weights, w_up, w_down) -> the layer's output, differentiable");
   py::class_<cem::FusedRank, std::shared_ptr<cem::FusedRank>>(m, "FusedRank")
       .def(py::init<int, int, int, int, int, int, int, int, int, int, int, bool, int64_t, std::vector<int64_t>, bool,
@@ -148,29 +149,29 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            py::arg("stripe"), py::arg("tk_cap"), py::arg("max_slices"), py::arg("num_sms"), py::arg("fp8"),
            py::arg("arena"), py::arg("peer_arenas"), py::arg("use_comm_stream"), py::arg("spin_limit"),
            py::arg("put_blocks"))
-      .def("begin_forward", &cem::FusedRank::begin_forward)
-      .def("begin_forward_async", &cem::FusedRank::begin_forward_async)
-      .def("resolve_slices", &cem::FusedRank::resolve_slices)
-      .def("set_pass_slices", &cem::FusedRank::set_pass_slices)
-      .def("set_mbar_limit_us", &cem::FusedRank::set_mbar_limit_us)
-      .def("sort_only", &cem::FusedRank::sort_only)
-      .def("begin_backward", &cem::FusedRank::begin_backward, py::arg("plan"), py::arg("known_slices") = -1,
+      .def("begin_forward", &cem::FusedRank::begin_forward, NoGil())
+      .def("begin_forward_async", &cem::FusedRank::begin_forward_async, NoGil())
+      .def("resolve_slices", &cem::FusedRank::resolve_slices, NoGil())
+      .def("set_pass_slices", &cem::FusedRank::set_pass_slices, NoGil())
+      .def("set_mbar_limit_us", &cem::FusedRank::set_mbar_limit_us, NoGil())
+      .def("sort_only", &cem::FusedRank::sort_only, NoGil())
+      .def("begin_backward", &cem::FusedRank::begin_backward, NoGil(), py::arg("plan"), py::arg("known_slices") = -1,
            py::arg("known_rows") = -1)
-      .def("put", &cem::FusedRank::put)
-      .def("compute_forward", &cem::FusedRank::compute_forward)
-      .def("compute_backward", &cem::FusedRank::compute_backward)
-      .def("keep_rows", &cem::FusedRank::keep_rows)
-      .def("forward_pass", &cem::FusedRank::forward_pass, py::call_guard<py::gil_scoped_release>())
-      .def("backward_pass", &cem::FusedRank::backward_pass, py::call_guard<py::gil_scoped_release>())
-      .def("finish_forward", &cem::FusedRank::finish_forward)
-      .def("finish_backward", &cem::FusedRank::finish_backward)
-      .def("check_status", &cem::FusedRank::check_status, py::call_guard<py::gil_scoped_release>())
-      .def("release", &cem::FusedRank::release, py::call_guard<py::gil_scoped_release>())
-      .def("plan_header", &cem::FusedRank::plan_header)
-      .def("set_whole_passes", &cem::FusedRank::set_whole_passes)
+      .def("put", &cem::FusedRank::put, NoGil())
+      .def("compute_forward", &cem::FusedRank::compute_forward, NoGil())
+      .def("compute_backward", &cem::FusedRank::compute_backward, NoGil())
+      .def("keep_rows", &cem::FusedRank::keep_rows, NoGil())
+      .def("forward_pass", &cem::FusedRank::forward_pass, NoGil())
+      .def("backward_pass", &cem::FusedRank::backward_pass, NoGil())
+      .def("finish_forward", &cem::FusedRank::finish_forward, NoGil())
+      .def("finish_backward", &cem::FusedRank::finish_backward, NoGil())
+      .def("check_status", &cem::FusedRank::check_status, NoGil())
+      .def("release", &cem::FusedRank::release, NoGil())
+      .def("plan_header", &cem::FusedRank::plan_header, NoGil())
+      .def("set_whole_passes", &cem::FusedRank::set_whole_passes, NoGil())
       .def("plan_ints", &cem::FusedRank::plan_ints)
-      .def("launches", &cem::FusedRank::launches)
-      .def("set_pipeline_counters", &cem::FusedRank::set_pipeline_counters, py::arg("counters") = py::none())
+      .def("launches", &cem::FusedRank::launches, NoGil())
+      .def("set_pipeline_counters", &cem::FusedRank::set_pipeline_counters, NoGil(), py::arg("counters") = py::none())
       .def("act", &cem::FusedRank::act)
       .def("h", &cem::FusedRank::h)
       .def("dh", &cem::FusedRank::dh);

@@ -5,6 +5,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../common/status.cuh"
 #include "../plan/plan_tables.cuh"
 
@@ -138,6 +140,6 @@ void launch_weight_grad(const GemmParams& p, const CUtensorMap& map_a, const CUt
 
 int weight_grad_unit_cols(int rows_of_tiles, int n_tiles, int pairs);  // (the launcher's choice of `unit_cols`)
 int row_gemm_smem_bytes();    // dynamic shared memory of a row-wise GEMM CTA
-extern int g_pair_grid_used;  // grid of the last GEMM launch, for diagnostics
+extern std::atomic<int> g_pair_grid_used;  // grid of the last GEMM launch, for diagnostics (passes of several workspaces store it)
 
 }  // namespace cem

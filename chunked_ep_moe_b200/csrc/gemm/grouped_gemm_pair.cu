@@ -659,7 +659,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmParams p, const __grid_cons
 
 }  // namespace
 
-int g_pair_grid_used = 0;  // last pair grid size, for diagnostics
+std::atomic<int> g_pair_grid_used{0};
 
 // Column tiles along which a pair keeps its panel: all of a row, or fewer where the last turn of longer units would leave more pairs
 // idle than the loads saved are worth. A tile crosses the port in 2048 cycles of stores and, at 256 rows, 576 of B and 576 of A / the

@@ -244,7 +244,7 @@ FusedRank::~FusedRank() {
 }
 
 void FusedRank::release() {
-  const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
+  const Turn turn(pass_mutex_);
   released_ = true;
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_));
   cudaDeviceSynchronize();  // (an error of the device is raised by whoever frees the arena)
@@ -255,7 +255,7 @@ void FusedRank::expect_arena(const char* what) const {
 }
 
 void FusedRank::check_status() {
-  const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
+  const Turn turn(pass_mutex_);
   cudaStream_t st = current_stream();
   cuda_check(cudaMemcpyAsync(host_header_ + kHostStatus, status_.data_ptr(), 8 * sizeof(int32_t),
                              cudaMemcpyDeviceToHost, st),
@@ -285,6 +285,7 @@ std::string format_status(const std::vector<int64_t>& s, int rank) {
 
 void FusedRank::sort_only(torch::Tensor expert_ids, torch::Tensor order, torch::Tensor inv_order,
                           torch::Tensor my_counts) {
+  const Turn turn(pass_mutex_);
   expect_arena("step");
   const int64_t tk = expert_ids.numel();
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
@@ -300,6 +301,7 @@ void FusedRank::sort_only(torch::Tensor expert_ids, torch::Tensor order, torch::
 
 int64_t FusedRank::begin_forward_async(torch::Tensor expert_ids, torch::Tensor plan, torch::Tensor order,
                                        torch::Tensor inv_order, torch::Tensor counts, bool counts_prefilled) {
+  const Turn turn(pass_mutex_);
   expect_arena("step");
   cudaStream_t st = current_stream();
   const int64_t tk = expert_ids.numel();
@@ -390,6 +392,7 @@ void FusedRank::quiesce() const {
 }
 
 int64_t FusedRank::resolve_slices() {
+  const Turn turn(pass_mutex_);
   wait_header();
   std::string message;
   const int32_t* st = host_header_ + 16;
@@ -410,17 +413,20 @@ int64_t FusedRank::resolve_slices() {
 }
 
 void FusedRank::set_pass_slices(int64_t launched) {
+  const Turn turn(pass_mutex_);
   expect(launched >= 0 && launched <= max_slices_, "slice count exceeds the workspace");
   cur_slices_ = launched;
 }
 
 void FusedRank::set_mbar_limit_us(int64_t us) {
+  const Turn turn(pass_mutex_);
   expect(us > 0 && us <= 600ll * 1000 * 1000, "barrier limit must be between 1 us and 600 s");
   mbar_limit_ = static_cast<uint32_t>(us);
 }
 
 int64_t FusedRank::begin_forward(torch::Tensor expert_ids, torch::Tensor plan, torch::Tensor order,
                                  torch::Tensor inv_order, torch::Tensor counts, bool counts_prefilled) {
+  const Turn turn(pass_mutex_);
   begin_forward_async(expert_ids, plan, order, inv_order, counts, counts_prefilled);
   const int64_t n = resolve_slices();
   set_pass_slices(n);
@@ -429,6 +435,7 @@ int64_t FusedRank::begin_forward(torch::Tensor expert_ids, torch::Tensor plan, t
 
 
 int64_t FusedRank::begin_backward(torch::Tensor plan, int64_t known_slices, int64_t known_rows) {
+  const Turn turn(pass_mutex_);
   expect_arena("step");
   cudaStream_t st = current_stream();
   expect_i32(plan, lay_.total, "plan");
@@ -482,6 +489,7 @@ void FusedRank::begin_pass(const torch::Tensor& plan, int64_t slices, int64_t ro
 
 void FusedRank::put(int64_t j, torch::Tensor plan, torch::Tensor order, torch::Tensor x,
                     c10::optional<torch::Tensor> g, torch::Tensor w_flat) {
+  const Turn turn(pass_mutex_);
   expect_arena("step");
   expect(j >= 0 && j < cur_slices_, "slice index out of range");
   expect_bf16_2d(x, D_, "x");
@@ -591,6 +599,9 @@ void FusedRank::dequant(const int* plan, int j, int b, bool with_g, cudaStream_t
 }
 
 void FusedRank::set_pipeline_counters(c10::optional<torch::Tensor> counters) {
+  const Turn turn(pass_mutex_);
+  if (passed_) cuda_check(cudaEventSynchronize(ev_end_), "wait for the last pass");
+  quiesce();  // (and for whatever has filled the new counters)
   if (!counters.has_value()) {
     prof_ = torch::Tensor();
     return;
@@ -642,6 +653,7 @@ void expect_weights(const torch::Tensor& w_up, const torch::Tensor& w_down, int 
 // later one's CTAs start as the earlier one's CTAs finish, i.e. every kernel fills the idle tail of the previous
 // (independent) one instead of waiting for it. Scratch reuse and the carry chain are ordered by events.
 void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_up, torch::Tensor w_down) {
+  const Turn turn(pass_mutex_);
   expect_arena("step");
   expect(j >= 0 && j < cur_slices_, "slice index out of range");
   expect_weights(w_up, w_down, L_, D_, F_);
@@ -702,6 +714,7 @@ void FusedRank::compute_forward(int64_t j, torch::Tensor plan, torch::Tensor w_u
 
 void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_up, torch::Tensor w_down,
                                  torch::Tensor dw_up, torch::Tensor dw_down) {
+  const Turn turn(pass_mutex_);
   expect_arena("step");
   expect(j >= 0 && j < cur_slices_, "slice index out of range");
   expect_weights(w_up, w_down, L_, D_, F_);
@@ -853,6 +866,7 @@ void FusedRank::end_pass(int64_t n_slices) {
 // F=2048: 64 experts of 256 rows 7.10 -> 6.09 ms, Zipf routing in slices of 2048 rows 9.05 -> 7.67 ms, 32 experts of 1024
 // rows on the fp8 wire 12.0 -> 10.9 ms.
 void FusedRank::keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices) {
+  const Turn turn(pass_mutex_);
   expect(h.is_cuda() && h.is_contiguous() && h.scalar_type() == torch::kBFloat16 && h.dim() == 2 && h.size(1) == 2 * F_ &&
              act.is_cuda() && act.is_contiguous() && act.scalar_type() == torch::kBFloat16 && act.dim() == 2 &&
              act.size(1) == F_ && act.size(0) == h.size(0) && act.size(0) > (slices - 1) * S_,
@@ -884,6 +898,7 @@ std::vector<torch::Tensor> FusedRank::allocate_kept(int64_t rows, int64_t slice_
 }
 
 void FusedRank::finish_forward(torch::Tensor inv_order, torch::Tensor out) {
+  const Turn turn(pass_mutex_);
   expect_arena("step");
   expect_bf16_2d(out, D_, "out");
   expect(out.size(0) * K_ == cur_rows_, "out rows do not match the pass");
@@ -1321,7 +1336,7 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brie
 std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass(
     torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
     bool training) {
-  const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
+  const Turn turn(pass_mutex_);
   expect_arena("forward");
   const int64_t tk = expert_ids.numel();
   release_kept();  // (of a pass that threw)
@@ -1411,7 +1426,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
     torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
     torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
     const std::vector<torch::Tensor>& saved, int64_t kept_slices) {
-  const std::lock_guard<std::recursive_mutex> lock(pass_mutex_);
+  const Turn turn(pass_mutex_);
   expect_arena("backward");
   inline_ = short_pass_ = false;  // (also behind a forward that threw)
   release_kept();

@@ -80,6 +80,8 @@ inline int64_t whole_ranges(int64_t rows, int64_t L, int64_t D, int64_t F, bool 
 }
 
 class FusedRank {
+  using Turn = std::lock_guard<std::recursive_mutex>;
+
  public:
   FusedRank(int P, int L, int me, int S, int D, int F, int K, int stripe, int tk_cap, int max_slices, int num_sms,
             bool fp8, int64_t arena, std::vector<int64_t> peer_arenas, bool use_comm_stream, int64_t spin_limit,
@@ -120,6 +122,7 @@ class FusedRank {
   void keep_rows(torch::Tensor h, torch::Tensor act, int64_t slices);
   void finish_forward(torch::Tensor inv_order, torch::Tensor out);
   void finish_backward(torch::Tensor inv_order, torch::Tensor dx, torch::Tensor d_weights) {
+    const Turn turn(pass_mutex_);
     reduce_backward(inv_order, dx, d_weights, nullptr);
   }
 
@@ -144,6 +147,7 @@ class FusedRank {
   // Reads the status block (synchronises); throws std::runtime_error describing the first recorded error.
   void check_status();
   std::vector<int64_t> plan_header() const {
+    const Turn turn(pass_mutex_);
     std::vector<int64_t> header(host_header_, host_header_ + 16);
     if (header_whole_) header[0] = (header[2] + S_ - 1) / S_;  // in slices of the configured size
     return header;
@@ -151,11 +155,18 @@ class FusedRank {
   int64_t plan_ints() const { return lay_.total; }
   // Whether passes of a rank on its own may run as one slice (default). Off: slice by slice, also the backward of a forward that
   // ran as one.
-  void set_whole_passes(bool on) { whole_passes_ = on; }
-  int64_t launches() const { return launches_; }
+  void set_whole_passes(bool on) {
+    const Turn turn(pass_mutex_);
+    whole_passes_ = on;
+  }
+  int64_t launches() const {
+    const Turn turn(pass_mutex_);
+    return launches_;
+  }
   // Turns the GEMM kernels' pipeline counters on: `counters` is a zeroed int64 CUDA tensor [6 modes, num_sms, 8]
   // (slots: ProfSlot in gemm/grouped_gemm.cuh) that every later GEMM launch adds to. An undefined tensor turns
-  // them off again. Diagnostics only: the counting costs a few clock reads per k-block.
+  // them off again. Waits for the last pass, whose kernels still add to the counters before. Diagnostics only: the counting costs a
+  // few clock reads per k-block.
   void set_pipeline_counters(c10::optional<torch::Tensor> counters);
   // Debug views of the local scratch (tests compare them with the torch reference).
   torch::Tensor act() const { return act_[0]; }
@@ -267,9 +278,9 @@ class FusedRank {
   CUtensorMap map_x_mn_[2], map_g_mn_[2], map_act_mn_[2], map_dh_mn_[2];
   std::map<std::tuple<const void*, uint32_t, int64_t, int64_t>, CUtensorMap> weight_maps_;
 
-  // One pass (as one call) or status check at a time: a forward on the caller's thread and a backward on the autograd engine's share all
-  // of the above and the counters below.
-  std::recursive_mutex pass_mutex_;
+  // One public call at a time: a forward on the caller's thread, a backward on the autograd engine's and whoever asks for a header or a
+  // count share all of the above and the counters below, and none of them holds the interpreter's lock meanwhile.
+  mutable std::recursive_mutex pass_mutex_;
   bool released_ = false;
   cudaStream_t comm_stream_ = nullptr, aux_stream_ = nullptr, chain_[2] = {};
   cudaStream_t expand_stream_ = nullptr;  // fp8 wire: the expansion kernels run here, beside the GEMM chains
