@@ -172,7 +172,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("plan_ints", &cem::FusedRank::plan_ints)
       .def("launches", &cem::FusedRank::launches, NoGil())
       .def("set_pipeline_counters", &cem::FusedRank::set_pipeline_counters, NoGil(), py::arg("counters") = py::none())
-      .def("act", &cem::FusedRank::act)
-      .def("h", &cem::FusedRank::h)
-      .def("dh", &cem::FusedRank::dh);
+      .def("act", &cem::FusedRank::act, NoGil())
+      .def("h", &cem::FusedRank::h, NoGil())
+      .def("dh", &cem::FusedRank::dh, NoGil());
 }

@@ -248,6 +248,11 @@ void FusedRank::release() {
   released_ = true;
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_));
   cudaDeviceSynchronize();  // (an error of the device is raised by whoever frees the arena)
+  // Nodes of graphs that are still alive hold the rank, but they have no use for its scratch any more.
+  for (auto* scratch : {&act_, &h_, &dh_, &dwp_})
+    for (torch::Tensor& t : *scratch) t = torch::Tensor();
+  carry_up_ = carry_down_ = sort_scratch_ = prof_ = torch::Tensor();
+  release_kept();
 }
 
 void FusedRank::expect_arena(const char* what) const {

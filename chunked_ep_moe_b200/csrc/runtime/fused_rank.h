@@ -141,7 +141,7 @@ class FusedRank {
       const std::vector<torch::Tensor>& kept, int64_t kept_slices);
 
   // The arena is about to go. Waits for the pass under way on another thread and for the device; whatever comes later is refused
-  // behind the same lock, before it launches anything.
+  // behind the same lock, before it launches anything. Gives the scratch back.
   void release();
 
   // Reads the status block (synchronises); throws std::runtime_error describing the first recorded error.
@@ -169,9 +169,18 @@ class FusedRank {
   // few clock reads per k-block.
   void set_pipeline_counters(c10::optional<torch::Tensor> counters);
   // Debug views of the local scratch (tests compare them with the torch reference).
-  torch::Tensor act() const { return act_[0]; }
-  torch::Tensor h() const { return h_[0]; }
-  torch::Tensor dh() const { return dh_[0]; }
+  torch::Tensor act() const {
+    const Turn turn(pass_mutex_);
+    return act_[0];
+  }
+  torch::Tensor h() const {
+    const Turn turn(pass_mutex_);
+    return h_[0];
+  }
+  torch::Tensor dh() const {
+    const Turn turn(pass_mutex_);
+    return dh_[0];
+  }
 
  private:
   // Common start of a pass: counter targets on the device, what the pass will receive back (`pieces_per_row` of T*K rows).
