@@ -161,7 +161,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("compute_forward", &cem::FusedRank::compute_forward, NoGil())
       .def("compute_backward", &cem::FusedRank::compute_backward, NoGil())
       .def("keep_rows", &cem::FusedRank::keep_rows, NoGil())
-      .def("forward_pass", &cem::FusedRank::forward_pass, NoGil())
+      .def("forward_pass", &cem::FusedRank::forward_pass, NoGil(), py::arg("x"), py::arg("expert_ids"), py::arg("w_flat"),
+           py::arg("w_up"), py::arg("w_down"), py::arg("training"), py::arg("plan_wanted") = true)
       .def("backward_pass", &cem::FusedRank::backward_pass, NoGil())
       .def("finish_forward", &cem::FusedRank::finish_forward, NoGil())
       .def("finish_backward", &cem::FusedRank::finish_backward, NoGil())

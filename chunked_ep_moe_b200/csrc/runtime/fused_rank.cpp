@@ -1252,7 +1252,8 @@ void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w
 }
 
 // A forward of few tokens without autograd, on the caller's stream: plan, up-projection with its rows gathered, down-projection, sum of the
-// K rows a token. No put, no buffer of a slice and no arrival is involved, and up to 32 ids no plan kernel (`launch_few_swiglu`). 64 tokens at D=7168 477 -> 462 us, one token 45 -> 41.5 us (the put
+// K rows a token. No put, no buffer of a slice and no arrival is involved, and up to 32 ids no plan kernel (`launch_few_swiglu`) where
+// nobody wants the plan: what that kernel leaves of one is enough for the two behind it, not for a backward. 64 tokens at D=7168 477 -> 462 us, one token 45 -> 41.5 us (the put
 // between was a launch and 5 us of latency). Up to 96 tokens the gather keeps up with the tensor cores, whatever the routing (gemm/row_gemm.cuh).
 bool FusedRank::runs_brief(int64_t tokens, int64_t rows, bool training) const {
   return P_ == 1 && use_comm_stream_ && !training && !fp8_ && tokens > 0 && tokens <= kBriefTokens && rows <= S_ &&
@@ -1261,7 +1262,8 @@ bool FusedRank::runs_brief(int64_t tokens, int64_t rows, bool training) const {
 
 std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brief(torch::Tensor x, torch::Tensor expert_ids,
                                                                                   torch::Tensor w_flat, torch::Tensor w_up,
-                                                                                  torch::Tensor w_down) {
+                                                                                  torch::Tensor w_down,
+                                                                                  bool plan_wanted) {
   cudaStream_t st = current_stream();
   const int64_t tk = expert_ids.numel();
   auto i32 = torch::TensorOptions().device(x.device()).dtype(torch::kInt32);
@@ -1272,7 +1274,7 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brie
   header_whole_ = true;
   cur_slices_ = 0;
   inline_ = true;
-  const bool few = tk <= kFewIds;
+  const bool few = tk <= kFewIds && !plan_wanted;
   RowTable rows;
   rows.tokens = brief_tokens_.data_ptr<int>();
   rows.weights = reinterpret_cast<float*>(arena_ + arena_lay_.wbuf);
@@ -1331,8 +1333,9 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brie
     NvtxRange range("chunked_moe/combine");
     finish_forward(inv_order, out);
   }
-  const int64_t n = resolve_slices();
-  return std::make_tuple(std::vector<torch::Tensor>{out, plan, order, inv_order}, n, 0);
+  resolve_slices();
+  if (few) return std::make_tuple(std::vector<torch::Tensor>{out}, kWholePass, 0);
+  return std::make_tuple(std::vector<torch::Tensor>{out, plan, order, inv_order}, kWholePass, 0);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1340,7 +1343,7 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_brie
 // ---------------------------------------------------------------------------------------------
 std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass(
     torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
-    bool training) {
+    bool training, bool plan_wanted) {
   const Turn turn(pass_mutex_);
   expect_arena("forward");
   const int64_t tk = expert_ids.numel();
@@ -1348,7 +1351,7 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_pass
   short_pass_ = false;
   expect(tk <= tk_cap_, "T*K exceeds the workspace capacity");
   expect_pass(x, expert_ids, w_flat, w_up, w_down);
-  if (runs_brief(x.size(0), tk, training)) return forward_brief(x, expert_ids, w_flat, w_up, w_down);
+  if (runs_brief(x.size(0), tk, training)) return forward_brief(x, expert_ids, w_flat, w_up, w_down, plan_wanted);
   // Under saved-tensor hooks a pass keeps nothing and runs slice by slice: whether it may do otherwise depends on the free memory,
   // and its backward may get the plan of a recomputation.
   const bool hooks = training && at::SavedTensorDefaultHooks::get_hooks().has_value();

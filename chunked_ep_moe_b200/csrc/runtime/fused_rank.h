@@ -131,10 +131,10 @@ class FusedRank {
   // under saved-tensor hooks: what is saved may then not depend on how much memory is free (activation checkpointing wants
   // the same tensors from the recomputation) and may be on its way to the host. Backward:
   // (dx, d_weights, dw_up, dw_down). Tensors are contiguous CUDA tensors of the workspace's geometry: x, g [T, D] bf16,
-  // expert_ids [T, K] int32, w_flat [T*K] fp32.
+  // expert_ids [T, K] int32, w_flat [T*K] fp32. A forward whose plan is not wanted (no backward follows) may give `out` alone.
   std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> forward_pass(
       torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
-      bool training);
+      bool training, bool plan_wanted = true);
   std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> backward_pass(
       torch::Tensor x, torch::Tensor g, torch::Tensor w_flat, torch::Tensor w_up, torch::Tensor w_down,
       torch::Tensor plan, torch::Tensor order, torch::Tensor inv_order, int64_t known_slices,
@@ -228,7 +228,7 @@ class FusedRank {
   void expect_pass(const torch::Tensor& x, const torch::Tensor& expert_ids, const torch::Tensor& w_flat, const torch::Tensor& w_up,
                    const torch::Tensor& w_down) const;
   std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> forward_brief(torch::Tensor x, torch::Tensor expert_ids, torch::Tensor w_flat,
-                                                                         torch::Tensor w_up, torch::Tensor w_down);
+                                                                         torch::Tensor w_up, torch::Tensor w_down, bool plan_wanted);
   bool within_half(size_t bytes, int share = 2) const;  // (or another share of the device)
   GemmParams range_params(const int* plan, int64_t first, int64_t last) const;
   template <typename Part>

@@ -33,7 +33,7 @@ struct Layer : public torch::autograd::Function<Layer> {
                                const std::shared_ptr<FusedRank>& rank, bool training) {
     const torch::Tensor ids = expert_ids.to(torch::kInt32).contiguous(), w_flat = router_weights(weights);
     const torch::Tensor xc = aligned(x.detach()), up = w_up.detach().contiguous(), down = w_down.detach().contiguous();
-    auto [made, slices, kept_slices] = rank->forward_pass(xc, ids, w_flat, up, down, training);
+    auto [made, slices, kept_slices] = rank->forward_pass(xc, ids, w_flat, up, down, training, /*plan_wanted=*/training);
     if (training) {
       torch::autograd::variable_list saved{xc, weights, up, down};
       saved.insert(saved.end(), made.begin() + 1, made.end());
