@@ -1256,7 +1256,7 @@ void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w
 // nobody wants the plan: what that kernel leaves of one is enough for the two behind it, not for a backward. 64 tokens at D=7168 477 -> 462 us, one token 45 -> 41.5 us (the put
 // between was a launch and 5 us of latency). Up to 96 tokens the gather keeps up with the tensor cores, whatever the routing (gemm/row_gemm.cuh).
 bool FusedRank::runs_brief(int64_t tokens, int64_t rows, bool training) const {
-  return P_ == 1 && use_comm_stream_ && !training && !fp8_ && tokens > 0 && tokens <= kBriefTokens && rows <= S_ &&
+  return P_ == 1 && whole_passes_ && use_comm_stream_ && !training && !fp8_ && tokens > 0 && tokens <= kBriefTokens && rows <= S_ &&
          rows <= kPlanSmallIds && L_ <= kPlanSmallExperts;
 }
 
