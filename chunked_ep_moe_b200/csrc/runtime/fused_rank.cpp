@@ -1455,10 +1455,10 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> FusedRank
   torch::Tensor dw_up = torch::empty_like(w_up), dw_down = torch::empty_like(w_down), dx = torch::empty_like(x);
   torch::Tensor d_weights = torch::empty({w_flat.numel()}, w_flat.options());
   std::vector<torch::Tensor> buffers;
-  // (x, g, dh by rows, router weights and d_weight shares; h and w * act unless they were kept. What lives by now is not what lived
-  // when the forward decided: a model's later layers have saved theirs.)
-  if (known_slices == kWholePass && whole_passes_ &&
-      within_half(static_cast<size_t>(rows) * (2 * (2 * D_ + 2 * F_ + (kept.size() == 2 ? 0 : 3 * F_)) + F_ / 8 + 4))) {
+  // (g, dh by rows, router weights and d_weight shares; x, h and w * act unless they were kept and live already. What lives by now is not
+  // what lived when the forward decided: a model's later layers have saved theirs.)
+  const int64_t columns = (kept_x.defined() ? 1 : 2) * D_ + (kept.size() == 2 ? 2 : 5) * F_;
+  if (known_slices == kWholePass && whole_passes_ && within_half(static_cast<size_t>(rows) * (2 * columns + F_ / 8 + 4))) {
     const auto f32 = x.options().dtype(torch::kFloat32);
     try {
       buffers = {kept_x.defined() ? torch::Tensor() : torch::empty({rows, D_}, x.options()),
