@@ -7,6 +7,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "../common/aligned.h"
 #include "embedding_kernels.cuh"
 #include "model_kernels.cuh"
 #include "router_kernels.cuh"
@@ -17,6 +18,12 @@ namespace {
 
 void need(bool cond, const char* msg) {
   if (!cond) throw std::runtime_error(std::string("model ops: ") + msg);
+}
+
+// Operands that the kernels read 16 bytes at a time.
+template <typename... Tensors>
+void align(Tensors&... tensors) {
+  ((tensors = aligned(tensors)), ...);
 }
 
 bool bf16_matrix(const torch::Tensor& t) {
@@ -38,6 +45,8 @@ std::vector<torch::Tensor> add_rms_norm_fwd(torch::Tensor x, c10::optional<torch
        "weight must be a contiguous CUDA bf16 vector of `cols` elements");
   if (delta.has_value()) need(bf16_matrix(*delta) && delta->sizes() == x.sizes(), "delta must match x");
   const c10::cuda::CUDAGuard guard(x.device());
+  align(x, weight);
+  if (delta.has_value()) align(*delta);
   torch::Tensor s = delta.has_value() ? torch::empty_like(x) : x;
   torch::Tensor y = torch::empty_like(x);
   torch::Tensor rstd = torch::empty({rows}, x.options().dtype(torch::kFloat32));
@@ -57,6 +66,8 @@ std::vector<torch::Tensor> add_rms_norm_bwd(torch::Tensor dy, c10::optional<torc
   need(weight.is_cuda() && weight.scalar_type() == torch::kBFloat16 && weight.is_contiguous() && weight.numel() == cols,
        "weight must be a contiguous CUDA bf16 vector of `cols` elements");
   const c10::cuda::CUDAGuard guard(s.device());
+  align(dy, s, weight);
+  if (ds_in.has_value()) align(*ds_in);
   torch::Tensor ds = torch::empty_like(s);
   const int blocks = add_rms_norm_bwd_blocks(static_cast<int>(rows));
   torch::Tensor partial = torch::empty({blocks, cols}, s.options().dtype(torch::kFloat32));
@@ -78,6 +89,7 @@ std::vector<torch::Tensor> rope_qkv_fwd(torch::Tensor qkv, torch::Tensor cos_t, 
            sin_t.scalar_type() == torch::kFloat32,
        "cos / sin must be contiguous CUDA fp32 [>= S, hd/2] tables");
   const c10::cuda::CUDAGuard guard(qkv.device());
+  align(qkv, cos_t, sin_t);
   // [B, H, S, hd] in the order of [B, S, H, hd]: the attention gives its output in its operands' order, and the projection behind
   // it then finds its rows without a copy (24 us per layer at 8192 tokens x 1024).
   auto heads = [&]() { return torch::empty({B, S, H, hd}, qkv.options()).transpose(1, 2); };
@@ -96,10 +108,11 @@ torch::Tensor rope_qkv_bwd(torch::Tensor dq, torch::Tensor dk, torch::Tensor dv,
        "dq, dk, dv must be CUDA bf16 [B, H, S, hd] tensors, hd % 8 == 0");
   const int64_t B = dq.size(0), H = dq.size(1), S = dq.size(2), hd = dq.size(3);
   const c10::cuda::CUDAGuard guard(dq.device());
+  align(cos_t, sin_t);
   torch::Tensor dqkv = torch::empty({B, S, 3, H, hd}, dq.options());
   for (torch::Tensor* t : {&dq, &dk, &dv})  // any layout that the kernel can read 16 bytes at a time
     if (t->stride(3) != 1 || t->stride(0) % 8 != 0 || t->stride(1) % 8 != 0 || t->stride(2) % 8 != 0 ||
-        reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0)
+        !at_16_bytes(*t))
       *t = t->clone(at::MemoryFormat::Contiguous);
   launch_rope_qkv(dqkv.data_ptr(), head_matrix(dq), head_matrix(dk), head_matrix(dv), cos_t.data_ptr<float>(),
                   sin_t.data_ptr<float>(), static_cast<int>(B), static_cast<int>(S), static_cast<int>(H),
@@ -113,6 +126,7 @@ std::vector<torch::Tensor> cross_entropy_fwd(torch::Tensor logits, torch::Tensor
            targets.numel() == logits.size(0),
        "targets must be a contiguous CUDA int64 vector of `rows` elements");
   const c10::cuda::CUDAGuard guard(logits.device());
+  align(logits);
   torch::Tensor loss = torch::empty({logits.size(0)}, logits.options().dtype(torch::kFloat32));
   torch::Tensor lse = torch::empty_like(loss);
   launch_cross_entropy_fwd(logits.data_ptr(), targets.data_ptr<int64_t>(), loss.data_ptr<float>(),
@@ -127,6 +141,7 @@ torch::Tensor cross_entropy_bwd(torch::Tensor logits, torch::Tensor targets, tor
   need(grad_scale.is_cuda() && grad_scale.scalar_type() == torch::kFloat32 && grad_scale.numel() == 1,
        "grad_scale must be a CUDA fp32 scalar");
   const c10::cuda::CUDAGuard guard(logits.device());
+  align(logits);
   torch::Tensor dlogits = torch::empty_like(logits);
   launch_cross_entropy_bwd(logits.data_ptr(), targets.data_ptr<int64_t>(), lse.data_ptr<float>(),
                            grad_scale.data_ptr<float>(), dlogits.data_ptr(), static_cast<int>(logits.size(0)),
@@ -137,6 +152,7 @@ torch::Tensor cross_entropy_bwd(torch::Tensor logits, torch::Tensor targets, tor
 torch::Tensor dense_swiglu_fwd(torch::Tensor gu) {
   need(bf16_matrix(gu) && gu.size(1) % 16 == 0, "gu must be a contiguous CUDA bf16 [rows, 2*ffn] matrix, ffn % 8 == 0");
   const c10::cuda::CUDAGuard guard(gu.device());
+  align(gu);
   torch::Tensor act = torch::empty({gu.size(0), gu.size(1) / 2}, gu.options());
   launch_dense_swiglu(gu.data_ptr(), nullptr, act.data_ptr(), static_cast<int>(gu.size(0)),
                       static_cast<int>(gu.size(1) / 2), false, stream());
@@ -148,6 +164,7 @@ torch::Tensor dense_swiglu_bwd(torch::Tensor gu, torch::Tensor d_act) {
   need(bf16_matrix(d_act) && d_act.size(0) == gu.size(0) && d_act.size(1) * 2 == gu.size(1),
        "d_act must be a contiguous CUDA bf16 [rows, ffn] matrix");
   const c10::cuda::CUDAGuard guard(gu.device());
+  align(gu, d_act);
   torch::Tensor d_gu = torch::empty_like(gu);
   launch_dense_swiglu(gu.data_ptr(), d_act.data_ptr(), d_gu.data_ptr(), static_cast<int>(gu.size(0)),
                       static_cast<int>(gu.size(1) / 2), true, stream());
@@ -159,7 +176,7 @@ namespace {
 // ids int64, grad bf16 [ids, cols], both contiguous; cols % 8 == 0.
 torch::Tensor embedding_bwd(const torch::Tensor& ids, torch::Tensor grad, int64_t vocab, int64_t cols) {
   const c10::cuda::CUDAGuard guard(grad.device());
-  if (reinterpret_cast<uintptr_t>(grad.data_ptr()) % 16 != 0) grad = grad.clone();  // (read 16 bytes at a time)
+  align(grad);
   torch::Tensor dw = torch::empty({vocab, cols}, grad.options());
   torch::Tensor keys = torch::empty({embedding_scratch_words(static_cast<int>(ids.numel()))}, grad.options().dtype(torch::kInt32));
   launch_embedding_bwd(ids.data_ptr<int64_t>(), grad.data_ptr(), dw.data_ptr(), reinterpret_cast<uint32_t*>(keys.data_ptr()),

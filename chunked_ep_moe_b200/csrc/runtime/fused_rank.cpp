@@ -16,6 +16,7 @@
 #include <mutex>
 #include <stdexcept>
 
+#include "../common/aligned.h"
 #include "tensor_map.h"
 
 namespace cem {
@@ -53,9 +54,8 @@ inline cudaStream_t current_stream() { return at::cuda::getCurrentCUDAStream().s
     if (!(cond)) throw std::runtime_error(msg);      \
   } while (0)
 
-// What kernels read and write 16 bytes at a time begins at an address of 16 bytes (a contiguous view may begin anywhere).
 void expect_at_16(const torch::Tensor& t, const char* name) {
-  expect(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, std::string(name) + " must be at an address of 16 bytes");
+  expect(at_16_bytes(t), std::string(name) + " must be at an address of 16 bytes");
 }
 
 void expect_bf16_2d(const torch::Tensor& t, int64_t cols, const char* name) {

@@ -3,10 +3,10 @@
 #include <ATen/cuda/CUDAContext.h>
 
 #include <algorithm>
-#include <cstdint>
 #include <stdexcept>
 #include <string>
 
+#include "../common/aligned.h"
 #include "fused_rank.h"
 #include "tensor_map.h"
 
@@ -23,7 +23,7 @@ void need_bf16(const torch::Tensor& t, int64_t rows, int64_t cols, const char* n
            t.size(1) == cols,
        std::string(name) + " must be a contiguous CUDA bf16 [" + std::to_string(rows) + ", " + std::to_string(cols) +
            "] matrix");
-  need(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, std::string(name) + " must be at an address of 16 bytes");
+  need(at_16_bytes(t), std::string(name) + " must be at an address of 16 bytes");
 }
 
 void need_weights(const torch::Tensor& w, int64_t L, const char* name) {

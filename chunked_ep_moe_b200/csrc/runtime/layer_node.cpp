@@ -1,7 +1,8 @@
 #include "layer_node.h"
 
-#include <cstdint>
 #include <stdexcept>
+
+#include "../common/aligned.h"
 
 namespace cem {
 
@@ -12,13 +13,6 @@ struct Held : torch::CustomClassHolder {
   explicit Held(std::shared_ptr<FusedRank> r) : rank(std::move(r)) {}
   std::shared_ptr<FusedRank> rank;
 };
-
-// Contiguous, and at an address of 16 bytes: what a pass reads 16 bytes at a time without a tensor map, which would refuse others. A
-// contiguous view may begin anywhere.
-torch::Tensor aligned(const torch::Tensor& t) {
-  const torch::Tensor c = t.contiguous();
-  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 ? c : c.clone();
-}
 
 // In C++ because the host is what bounds small passes: a node written in Python, its checks and conversions took 145 of 215 us a step
 // of forward + backward of 192 tokens at D=F=256, and 22 of 46 us a one-token forward, during which the device idles: the forward ends

@@ -351,3 +351,38 @@ def test_rope_gradients_of_any_layout(layout):
         torch.autograd.backward(outs, gi)
         grads.append(leaf.grad)
     assert torch.equal(*grads)
+
+
+def test_operands_at_any_address():
+    """The kernels read 16 bytes at a time; a contiguous view may begin anywhere. Bits of the aligned operands, forward and backward."""
+    gen = torch.Generator(device="cuda").manual_seed(31)
+    bf = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()
+
+    def shifted(t):
+        view = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t)
+        assert view.is_contiguous() and view.data_ptr() % 16
+        return view
+
+    angles = torch.rand(24, 8, device="cuda", generator=gen)
+    targets = torch.randint(0, 264, (33,), device="cuda", generator=gen)
+    tokens = torch.randint(0, 50, (70,), device="cuda", generator=gen)
+    ops = {
+        "norm": (lambda x, w: fused_ops.add_rms_norm(x, None, w, 1e-6), bf(33, 264), bf(264)),
+        "add norm": (lambda x, d, w: fused_ops.add_rms_norm(x, d, w, 1e-6), bf(33, 264), bf(33, 264), bf(264)),
+        "rope": (lambda qkv, c, s: fused_ops.rope_qkv(qkv, c.detach(), s.detach()), bf(2, 24, 3, 2, 16), angles.cos(), angles.sin()),
+        "cross-entropy": (lambda x: fused_ops.cross_entropy(x, targets), bf(33, 264)),
+        "swiglu": (lambda x: fused_ops.dense_swiglu(x), bf(33, 528)),
+        "embedding": (lambda w: fused_ops.embedding(tokens, w), bf(50, 264)),
+        "router": (lambda x, b: fused_ops.router_select(x, b.detach(), 4, 1.5)[1:4:2], bf(33, 64).float(), bf(64).float()),
+    }
+    for name, (op, *args) in ops.items():
+        results, grads = [], None
+        for moved in (lambda t: t.clone(), shifted):
+            leaves = [moved(t).requires_grad_(True) for t in args]
+            out = op(*leaves)
+            out = out if isinstance(out, (tuple, list)) else (out,)
+            grads = grads or [torch.randn(t.shape, device="cuda", generator=gen).to(t.dtype) for t in out]
+            torch.autograd.backward(out, [moved(t) for t in grads])
+            results.append([t.detach() for t in out] + [t.grad for t in leaves if t.grad is not None])
+        assert len(results[0]) == len(results[1]) > 1, name
+        assert all(torch.equal(a, b) for a, b in zip(*results)), name
