@@ -26,8 +26,10 @@ Everything else the backward needs are the inputs and the integer plan (tables, 
 
 from __future__ import annotations
 
+import contextlib
 import math
 import os
+import threading
 from typing import Optional
 
 import torch
@@ -42,6 +44,7 @@ _PUT_BLOCKS = 128  # measured: 128 blocks finish a put soonest and disturb the G
 
 _workspaces: dict = {}
 _retired: list = []  # workspaces replaced by `reserve()`; passes in flight may still hold them
+_making: dict = {}  # a lock for every geometry and group whose workspace is being made or replaced
 
 #: Pass as `group` to run the fused kernels on this rank alone (a 1-rank expert-parallel world), whatever
 #: process groups exist. Used by `ops.fused_expert` to serve `expert_compute="fused"` on collective transports.
@@ -88,6 +91,21 @@ def _workspace_key(cfg: ChunkedMoEConfig, group, hidden: int, ffn: int):
             cfg.always_slice, hidden, ffn, torch.cuda.current_device())
 
 
+@contextlib.contextmanager
+def _alone_with(key):
+    """One thread at a time makes or replaces a geometry's workspace. (No lock for all of them: making one is collective, and the threads
+    of two ranks may come to two groups in different orders.)"""
+    while True:
+        lock = _making.setdefault(key, threading.Lock())
+        with lock:
+            if _making.get(key) is lock:  # (else whoever was waited for has taken it away)
+                try:
+                    yield
+                finally:
+                    del _making[key]  # the key holds a process group
+                return
+
+
 def get_workspace(cfg: ChunkedMoEConfig, group, hidden: int, ffn: int, tokens_times_k: int) -> FusedWorkspace:
     """The cached workspace for this geometry and group; the first call creates it (collectively).
 
@@ -99,16 +117,18 @@ def get_workspace(cfg: ChunkedMoEConfig, group, hidden: int, ffn: int, tokens_ti
     key = _workspace_key(cfg, group, hidden, ffn)
     ws = _workspaces.get(key)
     if ws is None:
-        ws = FusedWorkspace(cfg, group, hidden, ffn, tokens_times_k)
-        _workspaces[key] = ws
-    elif ws.tk_cap < tokens_times_k and ws.world == 1:
-        ws = reserve(cfg, group, hidden, ffn, tokens_times_k)  # nobody to agree with: make room right away
-    elif ws.tk_cap < tokens_times_k:
-        raise RuntimeError(
-            f"chunked_moe fused path: this call has {tokens_times_k} token copies but the workspace of this geometry "
-            f"was created for {ws.tk_cap}. Capacity is agreed between the ranks when the workspace is created; call "
-            f"ops.fused.reserve(cfg, group, hidden, ffn, tokens_times_k) on every rank first.")
-    return ws
+        with _alone_with(key):
+            ws = _workspaces.get(key)  # (another thread's by now?)
+            if ws is None:
+                ws = _workspaces[key] = FusedWorkspace(cfg, group, hidden, ffn, tokens_times_k)
+    if ws.tk_cap >= tokens_times_k:
+        return ws
+    if ws.world == 1:
+        return reserve(cfg, group, hidden, ffn, tokens_times_k)  # nobody to agree with: make room right away
+    raise RuntimeError(
+        f"chunked_moe fused path: this call has {tokens_times_k} token copies but the workspace of this geometry "
+        f"was created for {ws.tk_cap}. Capacity is agreed between the ranks when the workspace is created; call "
+        f"ops.fused.reserve(cfg, group, hidden, ffn, tokens_times_k) on every rank first.")
 
 
 def reserve(cfg: ChunkedMoEConfig, group, hidden: int, ffn: int, tokens_times_k: int) -> FusedWorkspace:
@@ -118,40 +138,44 @@ def reserve(cfg: ChunkedMoEConfig, group, hidden: int, ffn: int, tokens_times_k:
     they started with, and the old workspace is only released by `release_workspaces()`.
     """
     key = _workspace_key(cfg, group, hidden, ffn)
-    ws = _workspaces.get(key)
-    need = tokens_times_k
-    if dist.is_available() and dist.is_initialized() and group is not SOLO and dist.get_world_size(group) > 1:
-        t = torch.tensor([need, ws.tk_cap if ws is not None else 0], device="cuda", dtype=torch.int64)
-        dist.all_reduce(t, op=dist.ReduceOp.MAX, group=group)
-        need, have = int(t[0]), int(t[1])
-    else:
-        have = ws.tk_cap if ws is not None else 0
-    if ws is None or have < need:  # every rank takes the same branch: both numbers are maxima over the ranks
-        if ws is not None:
-            _retired.append(ws)
-        ws = FusedWorkspace(cfg, group, hidden, ffn, need)
-        _workspaces[key] = ws
-    return ws
+    with _alone_with(key):
+        ws = _workspaces.get(key)
+        need = tokens_times_k
+        if dist.is_available() and dist.is_initialized() and group is not SOLO and dist.get_world_size(group) > 1:
+            t = torch.tensor([need, ws.tk_cap if ws is not None else 0], device="cuda", dtype=torch.int64)
+            dist.all_reduce(t, op=dist.ReduceOp.MAX, group=group)
+            need, have = int(t[0]), int(t[1])
+        else:
+            have = ws.tk_cap if ws is not None else 0
+        if ws is None or have < need:  # every rank takes the same branch: both numbers are maxima over the ranks
+            if ws is not None:
+                _retired.append(ws)
+            ws = _workspaces[key] = FusedWorkspace(cfg, group, hidden, ffn, need)
+        return ws
 
 
 def release_workspaces() -> None:
     """Frees every workspace, cached or replaced (collective when a process group is involved). A pass whose backward
     has not run yet must not be kept across this call: its backward raises."""
-    for ws in list(_workspaces.values()) + _retired:
+    going = [ws for ws in (_workspaces.pop(key, None) for key in list(_workspaces)) if ws is not None]
+    while _retired:
+        going.append(_retired.pop(0))
+    for ws in going:  # (what another thread makes meanwhile stays, for its next call)
         if ws.rank is not None:
             ws.rank.release()
         ws.rank = None
         ws.arena.close()
-    _workspaces.clear()
-    _retired.clear()
+
+
+def _ranks() -> list:
+    return [rank for rank in (ws.rank for ws in list(_workspaces.values())) if rank is not None]
 
 
 def last_plan_stats(cfg: ChunkedMoEConfig) -> list:
     """Load statistics of the most recent pass of every cached workspace (rows, slices, padding, remote rows)."""
     from ..utils.stats import header_stats
 
-    return [header_stats(list(ws.rank.plan_header()), cfg.slice_size) for ws in _workspaces.values()
-            if ws.rank is not None]
+    return [header_stats(list(rank.plan_header()), cfg.slice_size) for rank in _ranks()]
 
 
 def check_status() -> None:
@@ -160,14 +184,13 @@ def check_status() -> None:
     The forward checks on its own (it has to read the slice count back anyway); the backward does not synchronise,
     so a training loop calls this once per step, before the optimizer consumes the gradients.
     """
-    for ws in _workspaces.values():
-        if ws.rank is not None:
-            ws.rank.check_status()
+    for rank in _ranks():
+        rank.check_status()
 
 
 def launches() -> int:
     """Kernels launched so far by every cached workspace of this process."""
-    return sum(int(ws.rank.launches()) for ws in _workspaces.values() if ws.rank is not None)
+    return sum(int(rank.launches()) for rank in _ranks())
 
 
 def expected_launches(num_slices: int, fp8: bool = False, kept_slices: int = 0) -> int:
@@ -246,15 +269,13 @@ def pipeline_counters(enable: bool = True) -> list:
     kernels really ran at. Diagnostics: counting costs a few clock reads per k-block.
     """
     out = []
-    for ws in _workspaces.values():
-        if ws.rank is None:
-            continue
+    for rank in _ranks():
         if not enable:
-            ws.rank.set_pipeline_counters(None)
+            rank.set_pipeline_counters(None)
             continue
         t = torch.zeros(6, max(148, torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count),
                         len(PIPELINE_COUNTER_SLOTS), dtype=torch.int64, device="cuda")
-        ws.rank.set_pipeline_counters(t)
+        rank.set_pipeline_counters(t)
         out.append(t)
     return out
 
