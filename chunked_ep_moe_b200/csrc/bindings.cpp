@@ -121,7 +121,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add_rms_norm_bwd", &cem::add_rms_norm_bwd, "-> (ds, dweight)");
   m.def("rope_qkv_fwd", &cem::rope_qkv_fwd, "qkv [B,S,3,H,hd] -> rotated q, k and v as [B,H,S,hd]");
   m.def("rope_qkv_bwd", &cem::rope_qkv_bwd, "gradients of q, k, v -> gradient of qkv");
-  m.def("whole_ranges", &cem::whole_ranges, "(rows, experts, D, F, training, backward) -> ranges in which a rank on its own runs a pass as one slice");
+  m.def("whole_ranges", &cem::whole_ranges,
+        "(rows, experts, D, F, training, backward) -> ranges in which a rank on its own runs a pass as one slice");
   m.def("embedding", &cem::embedding, "(ids, bf16 table) -> its rows, differentiable");
   m.def("cross_entropy_fwd", &cem::cross_entropy_fwd, "bf16 logits -> (loss per row, log-sum-exp per row)");
   m.def("cross_entropy_bwd", &cem::cross_entropy_bwd, "-> bf16 gradient of the logits");

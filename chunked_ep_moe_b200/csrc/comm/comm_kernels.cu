@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(kPutThreads, 4) dispatch_put_kernel(const PutP
 // is read (and rounded for the fp8 wire) once a token and range instead of once a copy, and no copy waits for a search of the segments
 // and a send-order entry first, which is what bounded the dispatch put here (1.9 TB/s of stores from 128 blocks). Bound by its stores:
 // 8192 tokens x 6 copies at D=1024 x 34 us (of x alone, 100 MB) and 41 us (x and g; 85 by the dispatch put), 2048 x 8 at D=7168 103 us
-// (x and g, 470 MB; 247), first range of 4096 x 8 rounded tokens at D=7168 33 us (116). Forward + backward at those sizes: 797 -> 732
-// us, 5.64 -> 5.12 ms, 8.70 -> 8.39 ms; 1999 x 4 at D=2048 443 -> 431 us. Beside GEMMs (ranges) it keeps to the dispatch put's 128 blocks.
+// (x and g, 470 MB; 247), first range of 4096 x 8 rounded tokens at D=7168 33 us (116). Forward + backward at those sizes, dispatch put
+// and this one in turn on one GPU: 790 -> 721 us, 5.49 -> 5.43 ms, 8.47 -> 8.19 ms; 1999 x 4 at D=2048 429 -> 418 us. Beside GEMMs (ranges) it keeps to the dispatch put's 128 blocks.
 constexpr int kWholeAhead = 8;
 
 template <bool ROUND>

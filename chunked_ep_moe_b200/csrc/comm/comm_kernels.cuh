@@ -70,7 +70,8 @@ void launch_pass_begin(const int* plan, PlanLayout lay, uint32_t* expected_total
                        uint32_t* ready_total, uint32_t* ready_base, cudaStream_t stream);
 
 // Backward: adds up each slice row's shares of the router weight's gradient (written per column tile by the SwiGLU'
-// GEMM), takes the weight itself out of the sum and stores it to the row's source rank, then counts the rows there like any other returned piece.
+// GEMM), takes the weight itself out of the sum and stores it to the row's source rank, then counts the rows there like any
+// other returned piece.
 struct ReturnDwParams {
   const int* plan;
   PlanLayout lay;

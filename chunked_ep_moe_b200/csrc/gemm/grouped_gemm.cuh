@@ -123,7 +123,8 @@ void launch_gather_swiglu(const GemmParams& p, const CUtensorMap& map_a, int gri
 
 // The same as the first kernel of a pass of at most 32 expert ids, without a plan: what the kernels behind it need of one goes to `plan`.
 struct FewPlan {
-  int* plan;          // tiles and their number, header, in_start, in_size and src_send_start of experts with rows; nothing else
+  int* plan;          // header, tiles and their number, the last entry of tile_start, and of experts with rows tile_start (their own
+                      // and the next expert's), in_start, in_size and src_send_start; nothing else
   int* order;         // [num_ids]
   int* inv_order;
   int32_t* host_out;  // as in `PlanKernelParams`

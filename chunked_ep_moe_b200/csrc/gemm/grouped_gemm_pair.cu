@@ -35,7 +35,7 @@ static_assert(kPairSmemBytes + 1024 + 1024 + 16 <= 233472, "no room for a second
 // Experts of few rows: the A operand of a row of output tiles (an expert's rows x this CTA's 128 columns, up to five k-blocks) stays in
 // shared memory while the pair walks `p.unit_cols` tiles along that row, and a k-block loads 16 KB instead of 32. Their tiles are a few
 // k-blocks of MMA work for 64 KB of output, and the port that both have to cross is what bounds them. 256 rows of 64 experts at D=7168,
-// F=2048: 880 -> 785 cycles per k-block, forward + backward 5.78 -> 5.56 ms (5.65 -> 5.42 on another GPU); of 256 experts 22.05 -> 21.32.
+// F=2048: 880 -> 785 cycles per k-block, forward + backward (with the registers below) 5.61 -> 5.35 ms; of 256 experts 22.05 -> 21.32.
 constexpr int kResidentBlocks = 5;                        // 16 KB slots of the panel; the ring's other seven hold B
 constexpr int kResidentRing = 2 * kPairStages - kResidentBlocks;
 
@@ -65,8 +65,8 @@ __device__ __forceinline__ void tile_unit(const GemmParams& p, int t, int rank, 
   u->resident = false;
 }
 
-// Walks a pair's units, `step` apart in the order group, row of tiles, columns; a whole warp, which holds 32 groups at a time (one after the
-// other, each an access to L2, they took longer than the tiles of small experts).
+// Walks a pair's units, `step` apart in the order group, row of tiles, columns; a whole warp, which holds 32 groups at a time (one after
+// the other, each an access to L2, they took longer than the tiles of small experts).
 struct UnitWalk {
   int unit, window, base;  // next unit; first of the groups at hand and its first unit
   int4 e;                  // this lane's group
@@ -247,8 +247,9 @@ __device__ __forceinline__ void tgmm_epilogue(const GemmParams& p, const Unit& t
   }
 }
 
-// 192 registers per thread (at 168 the epilogue spills: 4001 rows of 16 experts at D=2048, F=1024 257.5 -> 253.8 us): two warps of 192 leave room in a quarter of the SM for two of the copy CTAs' 64 (the dispatch put, the
-// fp8 expansion), which have to become resident BESIDE this kernel for the overlap to happen.
+// 192 registers per thread (at 168 the epilogue spills: expert kernels on 4001 rows of 16 experts at D=2048, F=1024 257.5 -> 253.8 us): two
+// warps of 192 leave room in a quarter of the SM for two of the copy CTAs' 64 (the dispatch put, the fp8 expansion), which have to become
+// resident BESIDE this kernel for the overlap to happen.
 template <bool PANEL>
 __global__ void __cluster_dims__(2, 1, 1) __maxnreg__(192)
 grouped_gemm_pair_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap map_a,
@@ -358,7 +359,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmParams p, const __grid_cons
     // ================================ TMA producer (both CTAs) ==============================
     // The whole warp walks the k-blocks in step; one elected lane issues the copies.
     uint32_t it = 0, rit = 0, panels = 0;  // uses of the six stages, of the ring beside a panel, of the panel
-    uint32_t own_used = 0, own_parity = 0;  // per stage (bits 6 on: the ring): this CTA's own full barrier has been used / parity of its next use
+    // per stage (bits 6 on: the ring): this CTA's own full barrier has been used / parity of its next use
+    uint32_t own_used = 0, own_parity = 0;
     long long empty_wait = 0;
     uint32_t ps = 0, pph = 0, rs = 0, rph = 0;
     bool dead = false, was_resident = false;

@@ -78,7 +78,7 @@ struct FewRows {
 // L2, at 1413. So an expert's tiles go over its weight columns together, up to `kRowBandMax` at a time, and its weights are read once; by
 // fours, wherever experts end, the bands of one expert find them gone (an expert's are 59 and 29 MB; a die's L2 holds 63, of both dies'
 // lines). DRAM reads at 8 experts: up-projection 1289 -> 1075 MB, dX 893 -> 631, down-projection 307 -> 302. Forward + backward of
-// 8192 x 8 rows of 32 experts 1.033 and 1.031 times as fast, 4096 x 8 rows (fp8 put) 1.02, Zipf routing in slices of 2048 rows 1.02, 256 rows
+// 8192 x 8 rows of 32 experts 1.033 and 1.031 times as fast, 4096 x 8 rows (fp8 put) 1.02, Zipf routing of 2999 x 8 rows 1.02, 256 rows
 // per expert 1.00 to 1.02. At most 8 or 6 at a time: 1.019 and 1.000. (Cache hints gave nothing, weights as evict-first took 5 %.)
 // The way to a tile is two dependent loads longer: in launches of few or cheap tiles 1 us of 50, and what an expert's bands share is still
 // in L2 there. So by fours below 16 MB of weights an expert (`kByExpert`: the launcher then takes the variant without ranges) and below
@@ -517,7 +517,8 @@ __device__ __forceinline__ void fetch_dswiglu(const GemmParams& p, const GroupCt
   const __nv_bfloat16* h = p.in0 + dswiglu_offset(p, c, at);
 #pragma unroll
   for (int i = 0; i < 8; ++i)
-    if ((c.lane >> 3) + 4 * i < at.rows) cp_async_16(staged_h(buf, (c.lane >> 3) + 4 * i, c.lane & 7), h + static_cast<size_t>(4 * i) * p.ld0);
+    if ((c.lane >> 3) + 4 * i < at.rows)
+      cp_async_16(staged_h(buf, (c.lane >> 3) + 4 * i, c.lane & 7), h + static_cast<size_t>(4 * i) * p.ld0);
   if (p.dwp != nullptr) {
     const __nv_bfloat16* act =
         p.in1 + static_cast<size_t>(at.row0 + (c.lane >> 2)) * p.ld1 + at.n * kBlockN + c.rank * kBlockM + c.q * 32 + (c.lane & 3) * 8;

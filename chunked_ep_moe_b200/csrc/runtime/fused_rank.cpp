@@ -751,8 +751,8 @@ void FusedRank::compute_backward(int64_t j, torch::Tensor plan, torch::Tensor w_
     p->ready = expands() ? reinterpret_cast<const uint32_t*>(ready_.data_ptr()) : nullptr;
     p->ready_base = reinterpret_cast<const uint32_t*>(ready_base_.data_ptr());
   };
-  // Unless the forward kept them: h and w * act again. y is not recomputed: d_weight = <g, act Wd> = <g Wd^T, act> is a by-product of the next GEMM, so
-  // the down-projection GEMM that used to form <g, y> and w * g here (8 % of a step's FLOPs, 230 us per 8192-row slice at
+  // Unless the forward kept them: h and w * act again. y is not recomputed: d_weight = <g, act Wd> = <g Wd^T, act> is a
+  // by-product of the next GEMM, so the down-projection GEMM that used to form <g, y> and w * g here (8 % of a step's FLOPs, 230 us per 8192-row slice at
   // D=7168, F=2048) and the w * g matrix are gone: 23.1 -> 21.4 ms per forward + backward at 32 experts, 65,536 rows.
   if (!keep) {
     GemmParams p = base_params(pl, static_cast<int>(j));
@@ -890,7 +890,8 @@ void FusedRank::release_kept() {
 }
 
 // Keeping pays once the GEMM that it saves is longer than a launch, and only while there is memory to spare: live tensors
-// and all of the process's arenas, these included, stay within half of the device, else (or when the allocation fails) the backward recomputes.
+// and all of the process's arenas, these included, stay within half of the device, else (or when the allocation fails) the
+// backward recomputes.
 // (What the caching allocator knows, not `cudaMemGetInfo`: that call takes 2 ms with a busy device.)
 std::vector<torch::Tensor> FusedRank::allocate_kept(int64_t rows, int64_t slice_rows, const torch::TensorOptions& bf16) const {
   if (std::min<int64_t>(rows, slice_rows) * D_ * F_ < kKeepWork || !keep_activations_) return {};
@@ -1123,9 +1124,9 @@ std::tuple<std::vector<torch::Tensor>, int64_t, int64_t> FusedRank::forward_whol
   resolve_slices();  // raises what the pass's kernels had recorded by the time the plan was made
   std::vector<torch::Tensor> result{out, plan, order, inv_order};
   result.insert(result.end(), kept.begin(), kept.end());
-  // x by rows stays for the backward of a pass of one range as well, while what lives stays within a quarter of the device (activations,
-  // which save a GEMM, come first: they have the half). Its put then moves g alone: forward + backward of 8192 x 6 rows at D=1024 711 -> 693
-  // us, 1999 x 4 at D=2048 410 -> 400 us, 2048 x 8 at D=7168 5.67 -> 5.60 ms.
+  // x by rows stays for the backward of a pass of one range as well, while what lives stays within a quarter of the device
+  // (activations, which save a GEMM, come first: they have the half). Its put then moves g alone: forward + backward of 8192 x 6
+  // rows at D=1024 711 -> 693 us, 1999 x 4 at D=2048 410 -> 400 us, 2048 x 8 at D=7168 5.67 -> 5.60 ms.
   if (training && parts == 1 && keep_activations_ && within_half(0, 4)) result.push_back(rows_x);
   return std::make_tuple(result, kWholePass, kept.empty() ? 0 : 1);
 }
@@ -1153,22 +1154,24 @@ void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w
   ret_target_ += static_cast<uint32_t>(tk) * static_cast<uint32_t>(D_ / kCombineCols + 1);
   const bool keep = !kept.empty();
   auto bf16 = [](const torch::Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); };
-  const torch::Tensor &rows_x = kept_x.defined() ? kept_x : buffers[0], &rows_g = buffers[1], &rows_w = buffers[2], &dh = buffers[3], &dwp = buffers[4],
-                      &h = keep ? kept[0] : buffers[5], &act = keep ? kept[1] : buffers[6];
+  const torch::Tensor &rows_x = kept_x.defined() ? kept_x : buffers[0], &rows_g = buffers[1], &rows_w = buffers[2],
+                      &dh = buffers[3], &dwp = buffers[4], &h = keep ? kept[0] : buffers[5], &act = keep ? kept[1] : buffers[6];
   const int* pl = plan.data_ptr<int>();
   const int dwp_tiles = F_ / 32;
   const TokenMaps x_map = keep ? TokenMaps{} : make_token_maps(rows_x.data_ptr(), tk, D_);
   const TokenMaps g_map = make_token_maps(rows_g.data_ptr(), tk, D_), dh_map = make_token_maps(dh.data_ptr(), tk, 2 * F_);
-  const CUtensorMap x_mn = make_bf16_map_chunked(rows_x.data_ptr(), tk, D_, 64, 2), g_mn = make_bf16_map_chunked(rows_g.data_ptr(), tk, D_, 64, 2),
-                    act_mn = make_bf16_map_chunked(act.data_ptr(), tk, F_, 64, 2), dh_mn = make_bf16_map_chunked(dh.data_ptr(), tk, 2 * F_, 64, 2);
+  const CUtensorMap x_mn = make_bf16_map_chunked(rows_x.data_ptr(), tk, D_, 64, 2),
+                    g_mn = make_bf16_map_chunked(rows_g.data_ptr(), tk, D_, 64, 2),
+                    act_mn = make_bf16_map_chunked(act.data_ptr(), tk, F_, 64, 2),
+                    dh_mn = make_bf16_map_chunked(dh.data_ptr(), tk, 2 * F_, 64, 2);
   // d_act = w * (g Wd^T) needs g's rows; x's, where nothing has to be recomputed from them, follow beside that GEMM.
   const int64_t parts = whole_ranges(tk, L_, D_, F_, /*training=*/true, /*backward=*/true);
   const bool x_later = keep && parts > 1 && !kept_x.defined();
   inline_ = parts == 1;
   run_parts(parts, [&](int64_t first, int64_t last, cudaStream_t put_stream, cudaStream_t gemm_stream) {
     NvtxRange range("chunked_moe/bwd experts from", first);
-    put_whole(plan, inv_order, x, &g, w_flat, x_later || kept_x.defined() ? nullptr : bf16(rows_x), bf16(rows_g), rows_w.data_ptr<float>(), first, last,
-              put_stream, inline_, first > 0);
+    put_whole(plan, inv_order, x, &g, w_flat, x_later || kept_x.defined() ? nullptr : bf16(rows_x), bf16(rows_g),
+              rows_w.data_ptr<float>(), first, last, put_stream, inline_, first > 0);
     if (put_stream != gemm_stream) {
       cuda_check(cudaEventRecord(ev_put_[0], put_stream), "event record");
       cuda_check(cudaStreamWaitEvent(gemm_stream, ev_put_[0], 0), "wait put event");
@@ -1251,10 +1254,11 @@ void FusedRank::backward_whole(torch::Tensor x, torch::Tensor g, torch::Tensor w
   ++launches_;
 }
 
-// A forward of few tokens without autograd, on the caller's stream: plan, up-projection with its rows gathered, down-projection, sum of the
-// K rows a token. No put, no buffer of a slice and no arrival is involved, and up to 32 ids no plan kernel (`launch_few_swiglu`) where
-// nobody wants the plan: what that kernel leaves of one is enough for the two behind it, not for a backward. 64 tokens at D=7168 477 -> 462 us, one token 45 -> 41.5 us (the put
-// between was a launch and 5 us of latency). Up to 96 tokens the gather keeps up with the tensor cores, whatever the routing (gemm/row_gemm.cuh).
+// A forward of few tokens without autograd, on the caller's stream: plan, up-projection with its rows gathered, down-projection,
+// sum of the K rows a token. No put, no buffer of a slice and no arrival is involved, and up to 32 ids no plan kernel
+// (`launch_few_swiglu`) where nobody wants the plan: what that kernel leaves of one is enough for the two behind it, not for a
+// backward. With the put, a launch and 5 us of latency between plan and first GEMM, -> without: 64 tokens at D=7168 495 -> 481 us, one
+// token at D=1024 45.5 -> 42.9. Up to 96 tokens the gather keeps up with the tensor cores, whatever the routing (gemm/row_gemm.cuh).
 bool FusedRank::runs_brief(int64_t tokens, int64_t rows, bool training) const {
   return P_ == 1 && whole_passes_ && use_comm_stream_ && !training && !fp8_ && tokens > 0 && tokens <= kBriefTokens && rows <= S_ &&
          rows <= kPlanSmallIds && L_ <= kPlanSmallExperts;

@@ -1,8 +1,8 @@
 """Fused CUDA ops of the decoder around the MoE layers: residual add + RMSNorm, rotary embedding straight out of the
-qkv projection, the embedding table's gradient, the cross-entropy of bf16 logits, the sigmoid top-k router (everything after its logits GEMM) and the dense SwiGLU. Each is one kernel per direction (`csrc/model/`) instead of a
-chain of framework elementwise kernels, which took a third of a trainer step's device time. On CPU tensors (and for
-dtypes other than bf16) the same functions fall back to plain torch ops with identical semantics, so the model code
-has one path. The reference ships no model code; these serve `models/deepseek_tiny.py`.
+qkv projection, the embedding table's gradient, the cross-entropy of bf16 logits, the sigmoid top-k router (everything
+after its logits GEMM) and the dense SwiGLU. Each is one kernel per direction (`csrc/model/`) instead of a chain of
+framework elementwise kernels, which took a third of a trainer step's device time. On CPU tensors (and for dtypes other
+than bf16) the same functions fall back to plain torch ops with identical semantics, so the model code has one path. The reference ships no model code; these serve `models/deepseek_tiny.py`.
 """
 
 from __future__ import annotations

@@ -76,7 +76,8 @@ class FusedWorkspace:
             stripe=cfg.stripe_width, tk_cap=tk_cap, max_slices=self.max_slices,
             num_sms=int(os.environ.get("CEM_GEMM_GRID", cfg.num_sms)), fp8=self.fp8,
             arena=self.arena.local, peer_arenas=self.arena.peers, use_comm_stream=True,
-            spin_limit=int(os.environ.get("CEM_SPIN_LIMIT", _DEFAULT_SPIN_LIMIT)), put_blocks=int(os.environ.get("CEM_PUT_BLOCKS", _PUT_BLOCKS)))
+            spin_limit=int(os.environ.get("CEM_SPIN_LIMIT", _DEFAULT_SPIN_LIMIT)),
+            put_blocks=int(os.environ.get("CEM_PUT_BLOCKS", _PUT_BLOCKS)))
         self.rank.set_whole_passes(not cfg.always_slice)
         if "CEM_MBAR_LIMIT_US" in os.environ:
             self.rank.set_mbar_limit_us(int(os.environ["CEM_MBAR_LIMIT_US"]))
@@ -211,8 +212,8 @@ def expected_launches_alone(rows: int, experts: int, hidden: int, ffn: int, kept
 
     Forward: sort and plan (3, or 1 up to 2048 ids and 512 experts) + per range of experts (put, swiglu, down+combine) + combine
     reduce. Backward: per range (put, dswiglu, dW_down, dx+combine, dW_up, and swiglu+h or, beside the first GEMM of several kept
-    ranges, a put of x) + d_weight return + combine reduce. (A forward of one slice, up to 2048 ids and 512 experts, without autograd: 5, up to 96 tokens 4,
-    up to 32 ids 3.)
+    ranges, a put of x) + d_weight return + combine reduce. (A forward of one slice, up to 2048 ids and 512 experts, without
+    autograd: 5, also with `always_slice`; otherwise up to 96 tokens 4, up to 32 ids 3.)
     """
     ext = _build.load()
     forward, backward = [ext.whole_ranges(rows, experts, hidden, ffn, True, b) for b in (False, True)]
